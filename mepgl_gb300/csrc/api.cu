@@ -166,38 +166,10 @@ void fill_desc(mepgl_ctx *c, int si, int img_base, int tile_base)
     U.idx = 1.0 / s.dx;
     U.dx2 = s.dx * s.dx;
     U.dx = s.dx;
-    Uniform<float> &Uf = D.uf;
-    for (int k = 0; k < 2; ++k) {
-        Uf.a[k] = (float)U.a[k];
-        Uf.b[k] = (float)U.b[k];
-        Uf.hmx[k] = (float)U.hmx[k];
-        Uf.hmy[k] = (float)U.hmy[k];
-        Uf.aob[k] = (float)U.aob[k];
-        Uf.q[k] = (float)U.q[k];
-    }
-    Uf.eta = (float)U.eta;
-    Uf.gamma = (float)U.gamma;
-    Uf.delta = (float)U.delta;
-    Uf.h = (float)U.h;
-    Uf.idx = (float)U.idx;
-    Uf.dx2 = (float)s.dx * (float)s.dx;
-    Uf.dx = (float)s.dx;
-    Uniform<ff> &Up = D.uff;      // the double values split into float pairs
-    for (int k = 0; k < 2; ++k) {
-        Up.a[k] = ff(U.a[k]);
-        Up.b[k] = ff(U.b[k]);
-        Up.hmx[k] = ff(U.hmx[k]);
-        Up.hmy[k] = ff(U.hmy[k]);
-        Up.aob[k] = ff(U.aob[k]);
-        Up.q[k] = ff(U.q[k]);
-    }
-    Up.eta = ff(U.eta);
-    Up.gamma = ff(U.gamma);
-    Up.delta = ff(U.delta);
-    Up.h = ff(U.h);
-    Up.idx = ff(U.idx);
-    Up.dx2 = ff(U.dx2);
-    Up.dx = ff(U.dx);
+    fold_spacing(U);
+    round_uniform(D.uf, U);
+    D.uf.dx2 = (float)s.dx * (float)s.dx;
+    round_uniform(D.uff, U);      // the double values split into float pairs
     D.disc = c->opt.discretization;
     D.ph = s.dparams[8];
     D.mask = s.dmask;

@@ -84,7 +84,77 @@ template <class T>
 struct Uniform {
     T a[2], b[2], hmx[2], hmy[2], aob[2], q[2];
     T eta, gamma, delta, h, idx, dx2, dx;
+    // the same with the spacing folded in, as the stencils of site_pack.cuh
+    // use them: q dx, +- half of it, half of its square, (q + 1) dx, q / dx;
+    // -2 hm*, hm* / dx^2; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
+    // 1 / (4 dx), 1 / (8 dx^2)
+    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], a2[2], b2[2];
+    T etad, gammad, deltad, hd, idx4, idx8;
 };
+
+// The folded parameters from the plain ones (host, in double).
+inline void fold_spacing(Uniform<double> &U)
+{
+    for (int c = 0; c < 2; ++c) {
+        U.qd[c] = U.q[c] * U.dx;
+        U.hqd[c] = 0.5 * U.qd[c];
+        U.nhqd[c] = -U.hqd[c];
+        U.hqq[c] = U.hqd[c] * U.qd[c];
+        U.kq[c] = (U.q[c] + 1.0) * U.dx;
+        U.qi[c] = U.q[c] * U.idx;
+        U.n2hmx[c] = -2.0 * U.hmx[c];
+        U.n2hmy[c] = -2.0 * U.hmy[c];
+        U.hmxi[c] = U.hmx[c] * U.idx * U.idx;
+        U.hmyi[c] = U.hmy[c] * U.idx * U.idx;
+        U.a2[c] = 2.0 * U.a[c] * U.dx2;
+        U.b2[c] = 2.0 * U.b[c] * U.dx2;
+    }
+    U.idx4 = 0.25 * U.idx;
+    U.idx8 = 0.125 * U.idx * U.idx;
+    U.etad = U.eta * U.dx2;
+    U.gammad = U.gamma * U.dx2;
+    U.deltad = U.delta * U.dx2;
+    U.hd = U.h * U.dx;
+}
+
+// Rounded once from double: to float, or split into a float pair.
+template <class T>
+inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
+{
+    for (int c = 0; c < 2; ++c) {
+        r.a[c] = T(U.a[c]);
+        r.b[c] = T(U.b[c]);
+        r.hmx[c] = T(U.hmx[c]);
+        r.hmy[c] = T(U.hmy[c]);
+        r.aob[c] = T(U.aob[c]);
+        r.q[c] = T(U.q[c]);
+        r.qd[c] = T(U.qd[c]);
+        r.hqd[c] = T(U.hqd[c]);
+        r.nhqd[c] = T(U.nhqd[c]);
+        r.hqq[c] = T(U.hqq[c]);
+        r.kq[c] = T(U.kq[c]);
+        r.qi[c] = T(U.qi[c]);
+        r.n2hmx[c] = T(U.n2hmx[c]);
+        r.n2hmy[c] = T(U.n2hmy[c]);
+        r.hmxi[c] = T(U.hmxi[c]);
+        r.hmyi[c] = T(U.hmyi[c]);
+        r.a2[c] = T(U.a2[c]);
+        r.b2[c] = T(U.b2[c]);
+    }
+    r.eta = T(U.eta);
+    r.gamma = T(U.gamma);
+    r.delta = T(U.delta);
+    r.h = T(U.h);
+    r.idx = T(U.idx);
+    r.dx2 = T(U.dx2);
+    r.dx = T(U.dx);
+    r.etad = T(U.etad);
+    r.gammad = T(U.gammad);
+    r.deltad = T(U.deltad);
+    r.hd = T(U.hd);
+    r.idx4 = T(U.idx4);
+    r.idx8 = T(U.idx8);
+}
 
 // One string (one lattice, F images) as seen by the kernels.  Field buffers
 // hold three arrays each (A, psi_1, psi_2) of F*nx*ny pairs; psi_2 is null

@@ -24,8 +24,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
-#include "site_ops.cuh"
-#include "site_pair.cuh"
+#include "site_pack.cuh"
 
 namespace mepgl {
 
@@ -76,17 +75,6 @@ namespace mepgl {
 #ifndef MEPGL_MINB_STRIP_DIR
 #define MEPGL_MINB_STRIP_DIR MEPGL_MINB_STRIP
 #endif
-// strip row loop unrolled by the window period; interior sites with unit weights
-#ifndef MEPGL_STRIP_UNROLL
-#define MEPGL_STRIP_UNROLL 0
-#endif
-#ifndef MEPGL_STRIP_INTERIOR
-#define MEPGL_STRIP_INTERIOR 0
-#endif
-// two-component FP32 strips in packed FP32x2 arithmetic (site_pair.cuh)
-#ifndef MEPGL_STRIP_PAIR
-#define MEPGL_STRIP_PAIR 1
-#endif
 // FP32 NLCG steps as one persistent launch with per-image stage counters (strip.cuh)
 #ifndef MEPGL_STRIP_FUSED
 #define MEPGL_STRIP_FUSED 0
@@ -110,9 +98,11 @@ namespace mepgl {
 #if MEPGL_STRIP && MEPGL_SPLIT_DIR
 #error "MEPGL_SPLIT_DIR applies to the tile kernels; build it with MEPGL_STRIP=0"
 #endif
-// paired FP64 passes of two-component strings in packed float-float arithmetic
-#ifndef MEPGL_FF_PAIR
-#define MEPGL_FF_PAIR 1
+#ifndef MEPGL_MINB_GRAD_F64
+#define MEPGL_MINB_GRAD_F64 3
+#endif
+#ifndef MEPGL_MINB_DIR_F64
+#define MEPGL_MINB_DIR_F64 2
 #endif
 #ifndef MEPGL_MINB_GRAD_FF
 #define MEPGL_MINB_GRAD_FF 3
@@ -121,6 +111,7 @@ namespace mepgl {
 #define MEPGL_MINB_DIR_FF 2
 #endif
 template <class T> struct MinBlocks { static constexpr int grad = MEPGL_MINB_GRAD, dir = MEPGL_MINB_DIR; };
+template <> struct MinBlocks<double> { static constexpr int grad = MEPGL_MINB_GRAD_F64, dir = MEPGL_MINB_DIR_F64; };
 template <> struct MinBlocks<ff> { static constexpr int grad = MEPGL_MINB_GRAD_FF, dir = MEPGL_MINB_DIR_FF; };
 // Gradient tile kernels whose stencil spills at their register budget stage
 // one halo element at a time and read the previous gradient after the
@@ -142,10 +133,6 @@ template <class T> struct GradLean {
 template <class T> struct XPairs { static constexpr bool v = MEPGL_FF_XPAIRS != 0 && std::is_same<T, ff>::value; };
 
 template <class T> struct TileRows { static constexpr int v = sizeof(T) == 4 ? MEPGL_ROWS_F32 : MEPGL_ROWS_F64; };
-// Two-component float-float NLCG passes run the packed stencils (site_pair.cuh).
-template <class T, int NC> struct FFPacked {
-    static constexpr bool v = MEPGL_FF_PAIR && NC == 2 && std::is_same<T, ff>::value;
-};
 template <> struct TileRows<ff> { static constexpr int v = MEPGL_ROWS_F64; };
 
 int nlcg_step_launches() { return 2 + MEPGL_SPLIT_DIR; }
@@ -355,11 +342,22 @@ __device__ __forceinline__ TileRef flat_tile(const StringDesc &S, int tt)
     return t;
 }
 
-// Field h at a neighbour (per-site strings only).
-template <class T>
-__device__ __forceinline__ T h_site(const StringDesc &S, const SiteParams<T> &p, int s)
+// (h + h_neighbour) dx of the four neighbours of site s = (i, j).
+template <class T, int NC>
+__device__ __forceinline__ FieldSums<T> field_sums(const StringDesc &S, const PackParams<T, NC> &pp, int i, int j, int s)
 {
-    return S.per_site ? from_store<T>(static_cast<const store_t<T> *>(S.ph)[s]) : p.h;
+    const T hs = pp.hd + pp.hd;
+    FieldSums<T> f{hs, hs, hs, hs};
+    if (S.per_site) {
+        const store_t<T> *h = static_cast<const store_t<T> *>(S.ph);
+        const T dx = S.template u<T>().dx;
+        auto with = [&](int n) { return pp.hd + from_store<T>(h[n]) * dx; };
+        f.u = with(j + 1 < S.ny ? s + S.nx : s);
+        f.d = with(j > 0 ? s - S.nx : s);
+        f.r = with(i + 1 < S.nx ? s + 1 : s);
+        f.l = with(i > 0 ? s - 1 : s);
+    }
+    return f;
 }
 
 // --------------------------------------------------------------- line search
@@ -517,8 +515,8 @@ __global__ void __launch_bounds__(NT, MinBlocks<T>::grad) k_grad(const __grid_co
             gcur[c] = static_cast<W *>(S.g[f.gcur][c]) + off;
             gprev[c] = static_cast<const W *>(S.g[f.gprev][c]) + off;
         }
-        SiteParams<T> p;
-        p.load_uniform(S);
+        PackParams<T, NC> pp;
+        pp.load(S);
         __syncthreads();
         T v[2] = {(T)0, (T)0};
         const int lx = threadIdx.x & 31, gi = i0 + lx;
@@ -542,23 +540,10 @@ __global__ void __launch_bounds__(NT, MinBlocks<T>::grad) k_grad(const __grid_co
                 const int s = gi + S.nx * gj;
                 Wts<T> w;
                 w.load(t.m[ly + 1][lx + 1]);
-                T hr = p.h, hl = p.h, hu = p.h, hd = p.h;
-                if (S.per_site) {
-                    p.load_site(S, s, NC);
-                    hr = h_site(S, p, s + 1 < S.nx * S.ny ? s + 1 : s);
-                    hl = h_site(S, p, s > 0 ? s - 1 : s);
-                    hu = h_site(S, p, gj + 1 < S.ny ? s + S.nx : s);
-                    hd = h_site(S, p, gj > 0 ? s - S.nx : s);
-                }
+                if (S.per_site) pp.load_site(S, gi, gj, s);
                 T g[2 + 2 * NC];
-                if constexpr (FFPacked<T, NC>::v) {
-                    PairParams<T> pp;
-                    pp.set(p);
-                    site_gradient_pair<T>(pair_view_tile(t, lx + 1, ly + 1), p, pp, w, hr, hl, hu, hd, f.maxwell,
-                                          S.thin_film, g);
-                } else {
-                    site_gradient<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hr, hl, hu, hd, f.maxwell, S.thin_film, g);
-                }
+                site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s), f.maxwell,
+                                     S.thin_film, g);
                 if (GradLean<T>::v)
 #pragma unroll
                     for (int c = 0; c < 1 + NC; ++c) gold[r][c] = loadw<T>(gprev[c] + s);
@@ -673,8 +658,8 @@ __global__ void __launch_bounds__(NT, MinBlocks<T>::dir) k_dir_poly(const __grid
             cp_async_wait_all();
             }
         }
-        SiteParams<T> p;
-        p.load_uniform(S);
+        PackParams<T, NC> pp;
+        pp.load(S);
         __syncthreads();
         T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
         const int lx = threadIdx.x & 31, gi = i0 + lx;
@@ -684,16 +669,10 @@ __global__ void __launch_bounds__(NT, MinBlocks<T>::dir) k_dir_poly(const __grid
             if (gi < S.nx && gj < S.ny) {
                 Wts<T> w;
                 w.load(tx.m[ly + 1][lx + 1]);
-                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
+                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
                 T o[5];
-                if constexpr (FFPacked<T, NC>::v) {
-                    PairParams<T> pp;
-                    pp.set(p);
-                    site_poly_pair<T>(pair_view_tile(tx, lx + 1, ly + 1), pair_view_tile(td, lx + 1, ly + 1), p, pp,
-                                      w, f.poly_compat, S.thin_film, o);
-                } else {
-                    site_poly<T, NC, TYT>(tx, td, lx + 1, ly + 1, p, w, f.poly_compat, S.thin_film, o);
-                }
+                site_poly<T, NC>(pack_view_tile(tx, lx + 1, ly + 1), pack_view_tile(td, lx + 1, ly + 1), pp, w,
+                                 S.per_site, f.poly_compat, S.thin_film, o);
 #pragma unroll
                 for (int k = 0; k < 5; ++k) v[k] += o[k];
             }
@@ -703,10 +682,10 @@ __global__ void __launch_bounds__(NT, MinBlocks<T>::dir) k_dir_poly(const __grid
         if (finish_image<5>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot)) {
             if (threadIdx.x == 0) {
 #pragma unroll
-                for (int k = 0; k < 5; ++k) coef[k] = tot[k];
-                sc.fenergy[img] = tot[0];
+                for (int k = 0; k < 5; ++k) coef[k] = tot[k] * S.ud.dx2;
+                sc.fenergy[img] = coef[0];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = tot[1 + k];
+                for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = coef[1 + k];
             }
             __syncthreads();
             if (threadIdx.x < 32) {
@@ -786,8 +765,8 @@ __global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ Batch bt,
         ImagePtrs<T, NC> ip;
         image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, (size_t)tr.n * S.nx * S.ny);
         stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
-        SiteParams<T> p;
-        p.load_uniform(S);
+        PackParams<T, NC> pp;
+        pp.load(S);
         __syncthreads();
         T v[1] = {(T)0};
         const int lx = threadIdx.x & 31, gi = i0 + lx;
@@ -797,15 +776,21 @@ __global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ Batch bt,
             if (gi < S.nx && gj < S.ny) {
                 Wts<T> w;
                 w.load(t.m[ly + 1][lx + 1]);
-                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
-                v[0] += S.disc ? site_energy_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film)
-                               : site_energy<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film);
+                if (S.disc) {
+                    SiteParams<T> p;
+                    p.load_uniform(S);
+                    if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
+                    v[0] += site_energy_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film);
+                } else {
+                    if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
+                    v[0] += site_energy<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, S.per_site, S.thin_film);
+                }
             }
         }
         const int tpi = S.tiles_x * S.tiles_y;
         double tot[1];
         if (finish_image<1>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot) && threadIdx.x == 0)
-            out[img] = tot[0];
+            out[img] = S.disc ? tot[0] : tot[0] * S.ud.dx2;
         __syncthreads();
     }
 }
@@ -878,8 +863,8 @@ __global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ Ba
         ImagePtrs<T, NC> ip;
         image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, off);
         stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
-        SiteParams<T> p;
-        p.load_uniform(S);
+        PackParams<T, NC> pp;
+        pp.load(S);
         __syncthreads();
         const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
@@ -889,28 +874,31 @@ __global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ Ba
                 const int s = gi + S.nx * gj;
                 Wts<T> w;
                 w.load(t.m[ly + 1][lx + 1]);
-                T hr = p.h, hl = p.h, hu = p.h, hd = p.h;
-                if (S.per_site) {
-                    p.load_site(S, s, NC);
-                    hr = h_site(S, p, s + 1 < S.nx * S.ny ? s + 1 : s);
-                    hl = h_site(S, p, s > 0 ? s - 1 : s);
-                    hu = h_site(S, p, gj + 1 < S.ny ? s + S.nx : s);
-                    hd = h_site(S, p, gj > 0 ? s - S.nx : s);
-                }
                 T g[2 + 2 * NC];
-                if constexpr (std::is_same<T, ff>::value) {   // float-float: the reference form only
-                    site_gradient<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hr, hl, hu, hd, maxwell, S.thin_film, g);
-                } else if (S.disc) {
-                    T hmx_l[2] = {p.hmx[0], p.hmx[1]}, hmy_d[2] = {p.hmy[0], p.hmy[1]};
-                    if (S.per_site)
-                        for (int c = 0; c < NC; ++c) {
-                            if (gi > 0) hmx_l[c] = (T)0.5 / static_cast<const T *>(S.pmxx[c])[s - 1];
-                            if (gj > 0) hmy_d[c] = (T)0.5 / static_cast<const T *>(S.pmyy[c])[s - S.nx];
+                bool link = false;
+                if constexpr (!std::is_same<T, ff>::value) link = S.disc != 0;   // float-float: the reference form only
+                if (link) {
+                    if constexpr (!std::is_same<T, ff>::value) {
+                        SiteParams<T> p;
+                        p.load_uniform(S);
+                        T hl = p.h, hd = p.h;
+                        T hmx_l[2] = {p.hmx[0], p.hmx[1]}, hmy_d[2] = {p.hmy[0], p.hmy[1]};
+                        if (S.per_site) {
+                            p.load_site(S, s, NC);
+                            hl = static_cast<const T *>(S.ph)[s > 0 ? s - 1 : s];
+                            hd = static_cast<const T *>(S.ph)[gj > 0 ? s - S.nx : s];
+                            for (int c = 0; c < NC; ++c) {
+                                if (gi > 0) hmx_l[c] = (T)0.5 / static_cast<const T *>(S.pmxx[c])[s - 1];
+                                if (gj > 0) hmy_d[c] = (T)0.5 / static_cast<const T *>(S.pmyy[c])[s - S.nx];
+                            }
                         }
-                    site_gradient_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hl, hd, hmx_l, hmy_d, maxwell,
-                                                   S.thin_film, g);
+                        site_gradient_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hl, hd, hmx_l, hmy_d, maxwell,
+                                                       S.thin_film, g);
+                    }
                 } else {
-                    site_gradient<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hr, hl, hu, hd, maxwell, S.thin_film, g);
+                    if (S.per_site) pp.load_site(S, gi, gj, s);
+                    site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s),
+                                         maxwell, S.thin_film, g);
                 }
 #pragma unroll
                 for (int c = 0; c < 1 + NC; ++c) {
@@ -940,8 +928,8 @@ __global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ Batch bt, con
         ImagePtrs<T, NC> ip;
         image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, off);
         stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
-        SiteParams<T> p;
-        p.load_uniform(S);
+        PackParams<T, NC> pp;
+        pp.load(S);
         __syncthreads();
         const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
@@ -951,9 +939,9 @@ __global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ Batch bt, con
                 const size_t k = off + gi + (size_t)S.nx * gj;
                 Wts<T> w;
                 w.load(t.m[ly + 1][lx + 1]);
-                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
+                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
                 T o[1 + 2 * NC];
-                site_jb<T, NC, TYT>(t, lx + 1, ly + 1, p, w, o);
+                site_jb<T, NC>(pack_view_tile(t, lx + 1, ly + 1), S.template u<T>().idx, pp, w, o);
                 b[k] = o[0];
                 V v;
                 v.x = o[1];
@@ -2187,6 +2175,7 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
     S.ud.idx = 1.0 / dx;
     S.ud.dx2 = dx * dx;
     S.ud.dx = dx;
+    fold_spacing(S.ud);
     S.code_comp = comp_code;
     S.code_sc = sc_code;
     S.x[0][0] = const_cast<void *>(a);

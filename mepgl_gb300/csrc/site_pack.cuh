@@ -1,0 +1,579 @@
+// site_pack.cuh -- the per-site Ginzburg-Landau stencils: energy, gradient,
+// line quartic, B and J.
+//
+// Packs.  Every per-component quantity is a pack: the number itself for one
+// component, both components' values for two (FP32: a float2 on the packed
+// FP32x2 pipes; paired FP64: a packed float-float; FP64: two doubles).  What
+// carries no component (A, the magnetic views, the couplings) is scalar.
+//
+// Form of the terms.  A link i -> j with a = q A dx at its ends (lattice
+// units), Delta = psi_j - psi_i and the reference's linearised covariant
+// differences u0..u3 (nlcg.cu:149-203) has
+//
+//   sum u^2 / 2 = |Delta|^2 + s (y_i Dx - x_i Dy) + (a_i^2 |psi_i|^2 + a_j^2 |psi_j|^2) / 2,
+//   s = a_i + a_j,
+//
+// because y_i Dx - x_i Dy = y_j Dx - x_j Dy.  The last two terms belong to
+// the sites, with the weights of both links that meet there, so a link costs
+// the product of Delta with (Dx + s y, Dy - s x) and nothing per end; its
+// force on site i is -2 (Delta +- (s / 2) (y_j, -x_j)) + a_i^2 psi_i.  The
+// differences Delta are formed before anything is multiplied, as in u0..u3,
+// so the forms round alike.  Spacings are folded into the parameters: the
+// gradient's kinetic and magnetic terms carry no 1/dx (dx^2 / dx^2 = 1).
+//
+// Why: GB300 issues two FP64 operations per SM and clock, so the double
+// passes take 16 clocks per warp instruction and are bound by their count
+// alone (95 % of that rate measured); the float-float and FP32 passes are
+// bound by issue.  The forms the reference writes out cost 345 FP64
+// instructions per two-component site in the gradient and 486 in the
+// quartic.  With these forms, on the two-component 256 x 256 string of 64
+// images: an FP64 step 6.43 -> 4.60 ms, FP32 reparametrization and ten steps
+// 2.66 -> 2.42 ms; 1024 x 1024, FP32 passes: 3.46 -> 3.17 ms a step; the FP64
+// gradient and energy of 512 x 512 x 16, with its copies, 4.83 -> 4.00 ms.
+#pragma once
+
+#include "site_ops.cuh"
+
+namespace mepgl {
+
+// ------------------------------------------------------------------- packs
+struct dp2 {
+    double x, y;
+};
+
+template <class S, int NC> struct PackOf { using type = S; };
+template <> struct PackOf<float, 2> { using type = float2; };
+template <> struct PackOf<double, 2> { using type = dp2; };
+template <> struct PackOf<ff, 2> { using type = ffp; };
+template <class S, int NC> using pack_t = typename PackOf<S, NC>::type;
+
+__device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ ff fma1(ff a, ff b, ff c) { return a * b + c; }
+
+__device__ __forceinline__ float padd(float a, float b) { return a + b; }
+__device__ __forceinline__ float psub(float a, float b) { return a - b; }
+__device__ __forceinline__ float pmul(float a, float b) { return a * b; }
+__device__ __forceinline__ float pfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float pnfma(float a, float b, float c) { return __fmaf_rn(-a, b, c); }
+
+__device__ __forceinline__ double padd(double a, double b) { return a + b; }
+__device__ __forceinline__ double psub(double a, double b) { return a - b; }
+__device__ __forceinline__ double pmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double pfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double pnfma(double a, double b, double c) { return __fma_rn(-a, b, c); }
+
+__device__ __forceinline__ ff padd(ff a, ff b) { return a + b; }
+__device__ __forceinline__ ff psub(ff a, ff b) { return a - b; }
+__device__ __forceinline__ ff pmul(ff a, ff b) { return a * b; }
+__device__ __forceinline__ ff pfma(ff a, ff b, ff c) { return a * b + c; }
+__device__ __forceinline__ ff pnfma(ff a, ff b, ff c) { return c - a * b; }
+
+__device__ __forceinline__ dp2 padd(dp2 a, dp2 b) { return dp2{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ dp2 psub(dp2 a, dp2 b) { return dp2{a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ dp2 pmul(dp2 a, dp2 b) { return dp2{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ dp2 pfma(dp2 a, dp2 b, dp2 c) { return dp2{__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y)}; }
+__device__ __forceinline__ dp2 pnfma(dp2 a, dp2 b, dp2 c)
+{
+    return dp2{__fma_rn(-a.x, b.x, c.x), __fma_rn(-a.y, b.y, c.y)};
+}
+
+__device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+// a - b (b * -1 is exact, so this rounds once, as a - b does)
+__device__ __forceinline__ float2 psub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 pnfma(float2 a, float2 b, float2 c) { return __ffma2_rn(neg2f(a), b, c); }
+
+__device__ __forceinline__ ffp padd(ffp a, ffp b) { return a + b; }
+__device__ __forceinline__ ffp psub(ffp a, ffp b) { return a - b; }
+__device__ __forceinline__ ffp pmul(ffp a, ffp b) { return a * b; }
+__device__ __forceinline__ ffp pfma(ffp a, ffp b, ffp c) { return a * b + c; }
+__device__ __forceinline__ ffp pnfma(ffp a, ffp b, ffp c) { return c - a * b; }
+
+// same value in every component; one value per component; sum over them; one of them
+template <class S, int NC> struct Pk {
+    using P = pack_t<S, NC>;
+    static __device__ __forceinline__ P bc(S a)
+    {
+        if constexpr (NC == 1) return a;
+        else return mk(a, a);
+    }
+    static __device__ __forceinline__ P mk(S a, S b)
+    {
+        if constexpr (NC == 1) return a;
+        else if constexpr (std::is_same<S, ff>::value) return ffp{make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)};
+        else if constexpr (std::is_same<S, float>::value) return make_float2(a, b);
+        else return dp2{a, b};
+    }
+    template <int C> static __device__ __forceinline__ S lane(P p)
+    {
+        if constexpr (NC == 1) return p;
+        else if constexpr (std::is_same<S, ff>::value) return C == 0 ? ff(p.hi.x, p.lo.x) : ff(p.hi.y, p.lo.y);
+        else return C == 0 ? p.x : p.y;
+    }
+    static __device__ __forceinline__ S sum(P p)
+    {
+        if constexpr (NC == 1) return p;
+        else return lane<0>(p) + lane<1>(p);
+    }
+};
+
+// Neighbourhood of one site: A and Re / Im psi packs at (dx, dy) = [dy + 1][dx + 1].
+template <class S, int NC>
+struct PackView {
+    using P = pack_t<S, NC>;
+    vec2_t<S> a[3][3];
+    P px[3][3], py[3][3];
+};
+
+// Packed view of one site of a shared-memory tile.
+template <class S, int NC, int TYT>
+__device__ __forceinline__ PackView<S, NC> pack_view_tile(const TileF<S, NC, TYT> &t, int lx, int ly)
+{
+    PackView<S, NC> v;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            v.a[dy + 1][dx + 1] = t.A[ly + dy][lx + dx];
+            const vec2_t<S> p1 = t.P[0][ly + dy][lx + dx], p2 = t.P[NC - 1][ly + dy][lx + dx];
+            v.px[dy + 1][dx + 1] = Pk<S, NC>::mk(p1.x, p2.x);
+            v.py[dy + 1][dx + 1] = Pk<S, NC>::mk(p1.y, p2.y);
+        }
+    return v;
+}
+
+// Parameters as the stencils use them: read from the descriptor, and the
+// site's own where the string has per-site arrays.
+template <class S, int NC>
+struct PackParams {
+    using P = pack_t<S, NC>;
+    using K = Pk<S, NC>;
+    P qd, hqd, nhqd, hqq, kq, qi;   // q dx, +- half of it, half its square, (q + 1) dx, q / dx
+    P hmx, hmy, n2hmx, n2hmy;       // 1 / (2 m), -1 / m
+    P hmxi, hmyi, hmxil, hmyid;     // 1 / (2 m dx^2); at the left / lower neighbour (their forward links end here)
+    P aob, b, a2, b2;               // a / b, b; 2 a dx^2, 2 b dx^2
+    S eta, gamma, delta, h, idx, idx4, idx8;
+    S etad, gammad, deltad, hd;     // couplings times dx^2; h dx
+    __device__ __forceinline__ void load(const StringDesc &D)
+    {
+        const Uniform<S> &U = D.template u<S>();
+        qd = K::mk(U.qd[0], U.qd[1]);
+        hqd = K::mk(U.hqd[0], U.hqd[1]);
+        nhqd = K::mk(U.nhqd[0], U.nhqd[1]);
+        hqq = K::mk(U.hqq[0], U.hqq[1]);
+        kq = K::mk(U.kq[0], U.kq[1]);
+        qi = K::mk(U.qi[0], U.qi[1]);
+        hmx = K::mk(U.hmx[0], U.hmx[1]);
+        hmy = K::mk(U.hmy[0], U.hmy[1]);
+        hmxi = hmxil = K::mk(U.hmxi[0], U.hmxi[1]);
+        hmyi = hmyid = K::mk(U.hmyi[0], U.hmyi[1]);
+        n2hmx = K::mk(U.n2hmx[0], U.n2hmx[1]);
+        n2hmy = K::mk(U.n2hmy[0], U.n2hmy[1]);
+        aob = K::mk(U.aob[0], U.aob[1]);
+        b = K::mk(U.b[0], U.b[1]);
+        a2 = K::mk(U.a2[0], U.a2[1]);
+        b2 = K::mk(U.b2[0], U.b2[1]);
+        eta = U.eta;
+        gamma = U.gamma;
+        delta = U.delta;
+        h = U.h;
+        idx = U.idx;
+        idx4 = U.idx4;
+        idx8 = U.idx8;
+        etad = U.etad;
+        gammad = U.gammad;
+        deltad = U.deltad;
+        hd = U.hd;
+    }
+    // per-site strings: the parameters of site s = (i, j)
+    __device__ __forceinline__ void load_site(const StringDesc &D, int i, int j, int s)
+    {
+        SiteParams<S> p;
+        p.load_uniform(D);
+        p.load_site(D, s, NC);
+        using St = store_t<S>;
+        S x[2], y[2];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            x[c] = from_store<S>((St)0.5 / static_cast<const St *>(D.pmxx[c])[i > 0 ? s - 1 : s]);
+            y[c] = from_store<S>((St)0.5 / static_cast<const St *>(D.pmyy[c])[j > 0 ? s - D.nx : s]);
+        }
+        const S d2 = p.dx2, two = S(2.0f), n2 = S(-2.0f);
+        const P i2 = K::bc(idx * idx);
+        hmx = K::mk(p.hmx[0], p.hmx[NC - 1]);
+        hmy = K::mk(p.hmy[0], p.hmy[NC - 1]);
+        hmxi = pmul(hmx, i2);
+        hmyi = pmul(hmy, i2);
+        hmxil = pmul(K::mk(x[0], x[NC - 1]), i2);
+        hmyid = pmul(K::mk(y[0], y[NC - 1]), i2);
+        n2hmx = pmul(hmx, K::bc(n2));
+        n2hmy = pmul(hmy, K::bc(n2));
+        aob = K::mk(p.aob[0], p.aob[NC - 1]);
+        b = K::mk(p.b[0], p.b[NC - 1]);
+        a2 = K::mk(two * p.a[0] * d2, two * p.a[NC - 1] * d2);
+        b2 = K::mk(two * p.b[0] * d2, two * p.b[NC - 1] * d2);
+        h = p.h;
+        hd = p.h * p.dx;
+    }
+};
+
+// FP64: a biquadratic coupling of zero is skipped (a uniform branch; its 26
+// instructions cost 26 x 16 clocks per warp).  FP32 and float-float keep the
+// straight line (the branch measured slower there).
+template <class S> struct SkipZeroDelta { static constexpr bool v = std::is_same<S, double>::value; };
+
+// Four collocated views of (curl A - h) dx at one site, from the forward and
+// backward differences of A_y along x (yp, ym) and of A_x along y (xp, xm).
+template <class S>
+struct Curl {
+    S yp, ym, xp, xm;
+    template <class V> __device__ __forceinline__ Curl(const V (&a)[3][3])
+    {
+        yp = a[1][2].y - a[1][1].y;
+        ym = a[1][1].y - a[1][0].y;
+        xp = a[2][1].x - a[1][1].x;
+        xm = a[1][1].x - a[0][1].x;
+    }
+};
+
+// ------------------------------------------------------------------ energy
+// Free-energy density (freeEnergyDensity, nlcg.cu:105-214); the caller
+// multiplies the image's sum by dx^2.  per_site: pp.hmxil / hmyid differ from
+// pp.hmxi / hmyi.
+//
+// The energy and the quartic are sums of terms that cancel against one another
+// (the field's h^2 / 2 against the couplings' gain in the benchmark strings),
+// so their parameters stay as given and the spacing enters as one common
+// factor of the whole sum: folding dx^2 into each parameter, with a rounding
+// each, left an FP32 energy 6.4e-7 off where it is 3.6e-7 with the factor
+// outside.
+template <class S, int NC>
+__device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
+                                         int per_site, int thin_film)
+{
+    using K = Pk<S, NC>;
+    using P = pack_t<S, NC>;
+    const P X = v.px[1][1], Y = v.py[1][1];
+    const P r = pfma(Y, Y, pmul(X, X)), n = padd(r, pp.aob);
+    const P bh = pmul(pp.b, K::bc(S(0.5f) * w.area));
+    P e = pmul(pmul(bh, n), n);
+    P dg = K::bc(S(0.0f));
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const S Ai = dir == 0 ? v.a[1][1].x : v.a[1][1].y, Aj = dir == 0 ? v.a[1][2].x : v.a[2][1].y;
+        const P xj = dir == 0 ? v.px[1][2] : v.px[2][1], yj = dir == 0 ? v.py[1][2] : v.py[2][1];
+        const P hm = dir == 0 ? pp.hmxi : pp.hmyi, hb = dir == 0 ? pp.hmxil : pp.hmyid;
+        const S wf = dir == 0 ? w.wfx : w.wfy, wb = dir == 0 ? w.wbx : w.wby, ws = dir == 0 ? w.wsx : w.wsy;
+        const P f = pmul(hm, K::bc(wf));
+        const P Dx = psub(xj, X), Dy = psub(Y, yj);       // Dy: -(y_j - y_i)
+        const P s = pmul(pp.qd, K::bc(Ai + Aj));
+        e = pfma(pmul(f, Dx), pfma(s, Y, Dx), e);
+        e = pfma(pmul(f, Dy), pfma(s, X, Dy), e);
+        const P a = pmul(pp.qd, K::bc(Ai));
+        const P W = per_site ? pfma(hb, K::bc(wb), f) : pmul(hm, K::bc(ws));
+        dg = pfma(pmul(W, a), a, dg);
+    }
+    e = pfma(pmul(dg, K::bc(S(0.5f))), r, e);
+    S t = K::sum(e);
+    if constexpr (NC == 2) {
+        const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y);
+        const S x2 = K::template lane<1>(X), y2 = K::template lane<1>(Y);
+        const S r1 = K::template lane<0>(r), r2 = K::template lane<1>(r);
+        const S R = fma1(y1, y2, x1 * x2), I = fma1(x1, y2, -(y1 * x2));
+        S cp = pp.eta * R;
+        cp = fma1(S(0.5f) * pp.gamma * r1, r2, cp);
+        cp = fma1(S(0.5f) * pp.delta, fma1(R, R, -(I * I)), cp);
+        t = fma1(w.area, cp, t);
+    }
+    if (!thin_film) {
+        const Curl<S> c(v.a);
+        const S nh = -pp.h;
+        const S r0 = fma1(pp.idx, c.yp - c.xp, nh), r1 = fma1(pp.idx, c.ym - c.xp, nh);
+        const S r2 = fma1(pp.idx, c.ym - c.xm, nh), r3 = fma1(pp.idx, c.yp - c.xm, nh);
+        S em = (w.vUR * r0) * r0;
+        em = fma1(w.vUL * r1, r1, em);
+        em = fma1(w.vLL * r2, r2, em);
+        em = fma1(w.vLR * r3, r3, em);
+        t = fma1(S(0.125f), em, t);
+    }
+    return t;
+}
+
+// ---------------------------------------------------------------- gradient
+// (h + h_neighbour) dx towards the upper, lower, right and left neighbour.
+template <class S>
+struct FieldSums {
+    S u, d, r, l;
+};
+
+// Gradient dF/dA (out[0..1]) and dF/dpsi_c (out[2 + 2c..]) at one site,
+// restating gradientPsi (nlcg.cu:504-744) and gradientA (nlcg.cu:746-888).
+// Both link ends use the mass of this site, as the reference does.
+template <class S, int NC>
+__device__ __forceinline__ void site_gradient(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
+                                              const FieldSums<S> &h, int maxwell, int thin_film, S *out)
+{
+    using K = Pk<S, NC>;
+    using P = pack_t<S, NC>;
+    using V = vec2_t<S>;
+    const V A0 = v.a[1][1], Ar = v.a[1][2], Al = v.a[1][0], Au = v.a[2][1], Ad = v.a[0][1];
+    const P X = v.px[1][1], Y = v.py[1][1];
+    const P r2 = pfma(Y, Y, pmul(X, X));
+    const P m2r = pmul(r2, K::bc(S(-2.0f)));
+    P gx = K::bc(S(0.0f)), gy = gx, dg = gx, ga[2];
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const S A = dir == 0 ? A0.x : A0.y, Af = dir == 0 ? Ar.x : Au.y, Ab = dir == 0 ? Al.x : Ad.y;
+        const P xf = dir == 0 ? v.px[1][2] : v.px[2][1], yf = dir == 0 ? v.py[1][2] : v.py[2][1];
+        const P xb = dir == 0 ? v.px[1][0] : v.px[0][1], yb = dir == 0 ? v.py[1][0] : v.py[0][1];
+        // weights -2 w / (2 m) of the forward and backward link
+        const P f = pmul(dir == 0 ? pp.n2hmx : pp.n2hmy, K::bc(dir == 0 ? w.wfx : w.wfy));
+        const P b = pmul(dir == 0 ? pp.n2hmx : pp.n2hmy, K::bc(dir == 0 ? w.wbx : w.wby));
+        const P dxf = psub(xf, X), dyf = psub(yf, Y), dxb = psub(xb, X), dyb = psub(yb, Y);
+        const P sf = pmul(pp.hqd, K::bc(A + Af)), sb = pmul(pp.nhqd, K::bc(A + Ab));
+        gx = pfma(f, pfma(sf, yf, dxf), gx);
+        gx = pfma(b, pfma(sb, yb, dxb), gx);
+        gy = pfma(f, pnfma(sf, xf, dyf), gy);
+        gy = pfma(b, pnfma(sb, xb, dyb), gy);
+        // site term a^2 psi of both links, and the current through them
+        const P an = pmul(pp.nhqd, K::bc(A)), Wa = pmul(padd(f, b), an);   // -a / 2, W a
+        dg = pfma(Wa, an, dg);                                             // -W a^2 / 2
+        P c = pmul(Wa, m2r);
+        c = pfma(f, pnfma(X, dyf, pmul(Y, dxf)), c);
+        ga[dir] = pnfma(b, pnfma(X, dyb, pmul(Y, dxb)), c);
+    }
+    S g0 = K::sum(pmul(pp.nhqd, ga[0])), g1 = K::sum(pmul(pp.nhqd, ga[1]));
+    // condensation: 2 psi (a + b |psi|^2); density coupling with the other component
+    P k = pfma(pp.b2, r2, pp.a2);
+    if constexpr (NC == 2) {
+        const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y);
+        const S x2 = K::template lane<1>(X), y2 = K::template lane<1>(Y);
+        k = pfma(K::bc(pp.gammad), K::mk(K::template lane<1>(r2), K::template lane<0>(r2)), k);
+        k = pfma(k, K::bc(w.area), pmul(dg, K::bc(S(-2.0f))));
+        gx = pfma(k, X, gx);
+        gy = pfma(k, Y, gy);
+        // eta psi_2 + delta (psi_1* psi_2) psi_2-like terms: e = eta + delta R, i = delta I
+        const S R = fma1(y1, y2, x1 * x2), I = fma1(x1, y2, -(y1 * x2));
+        const S e = fma1(pp.deltad, R, pp.etad) * w.area, i = pp.deltad * I * w.area;
+        out[2] = fma1(-i, y2, fma1(e, x2, K::template lane<0>(gx)));
+        out[3] = fma1(i, x2, fma1(e, y2, K::template lane<0>(gy)));
+        out[4] = fma1(i, y1, fma1(e, x1, K::template lane<1>(gx)));
+        out[5] = fma1(-i, x1, fma1(e, y1, K::template lane<1>(gy)));
+    } else {
+        k = pfma(k, K::bc(w.area), pmul(dg, K::bc(S(-2.0f))));
+        out[2] = pfma(k, X, gx);
+        out[3] = pfma(k, Y, gy);
+    }
+    if (maxwell)
+#pragma unroll
+        for (int c = 2; c < 2 + 2 * NC; ++c) out[c] = S(0.0f);
+    if (!thin_film) {
+        // link differences ex(i,j) = A_y(i+1,j) - A_y(i,j), ey(i,j) = A_x(i,j+1) - A_x(i,j)
+        const S two = S(2.0f);
+        const S ex0 = Ar.y - A0.y, exm = A0.y - Al.y, ey0 = Au.x - A0.x, eym = A0.x - Ad.x;
+        const S exu = v.a[2][2].y - Au.y, exmu = Au.y - v.a[2][0].y;
+        const S exd = v.a[0][2].y - Ad.y, exmd = Ad.y - v.a[0][0].y;
+        const S eyr = v.a[2][2].x - Ar.x, eyrm = Ar.x - v.a[0][2].x;
+        const S eyl = v.a[2][0].x - Al.x, eylm = Al.x - v.a[0][0].x;
+        // the views of this site and the neighbours' views of the same plaquettes (nlcg.cu:852-883)
+        const S tu = fma1(two, ey0, h.u), td = fma1(two, eym, h.d);
+        const S tr = fma1(two, ex0, -h.r), tl = fma1(two, exm, -h.l);
+        S mx = w.vUR * ((ex0 + exu) - tu);
+        mx = fma1(w.vUL, (exm + exmu) - tu, mx);
+        mx = fma1(w.vLL, td - (exm + exmd), mx);
+        mx = fma1(w.vLR, td - (ex0 + exd), mx);
+        S my = w.vUR * ((ey0 + eyr) - tr);
+        my = fma1(w.vUL, tl - (ey0 + eyl), my);
+        my = fma1(w.vLL, tl - (eym + eylm), my);
+        my = fma1(w.vLR, (eym + eyrm) - tr, my);
+        out[0] = fma1(S(0.25f), mx, g0);
+        out[1] = fma1(S(0.25f), my, g1);
+    } else {
+        out[0] = S(0.0f);
+        out[1] = S(0.0f);
+    }
+}
+
+// ------------------------------------------------------------ line quartic
+// Coefficients {A, B, C, D, E} of F(x + t d) at one site, without the common
+// dx^2 (polynomialExpansion, nlcg.cu:997-1370).  compat keeps the reference's
+// x-link first-order slip (its t-linear field term uses charge -1) and the
+// halved cubic coefficient of the y-links, as corrections to the exact form.
+template <class S, int NC>
+__device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackView<S, NC> &dv,
+                                          const PackParams<S, NC> &pp, const Wts<S> &w, int per_site, int compat,
+                                          int thin_film, S *out)
+{
+    using K = Pk<S, NC>;
+    using P = pack_t<S, NC>;
+    const S half = S(0.5f);
+    const P X = v.px[1][1], Y = v.py[1][1], U = dv.px[1][1], Vd = dv.py[1][1];
+    // |psi + t d|^2 = r0 + n1 t + n2 t^2 (rh = n1 / 2); n0 = a / b + r0
+    const P r0 = pfma(Y, Y, pmul(X, X)), n0 = padd(r0, pp.aob);
+    const P rh = pfma(Y, Vd, pmul(X, U)), n1 = padd(rh, rh);
+    const P n2 = pfma(Vd, Vd, pmul(U, U));
+    P w0, w1, w2, kd_y;   // site term (a + t b)^2 |psi + t d|^2 / 2 of the links: coefficients of its first factor
+    P ka, kb, kc, kd;
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        // forward link i -> j: i the site, j its +x (dir 0) or +y (dir 1) neighbour
+        const S Ai = dir == 0 ? v.a[1][1].x : v.a[1][1].y, Aj = dir == 0 ? v.a[1][2].x : v.a[2][1].y;
+        const S ai = dir == 0 ? dv.a[1][1].x : dv.a[1][1].y, aj = dir == 0 ? dv.a[1][2].x : dv.a[2][1].y;
+        const P xj = dir == 0 ? v.px[1][2] : v.px[2][1], yj = dir == 0 ? v.py[1][2] : v.py[2][1];
+        const P uj = dir == 0 ? dv.px[1][2] : dv.px[2][1], vj = dir == 0 ? dv.py[1][2] : dv.py[2][1];
+        const P hm = dir == 0 ? pp.hmxi : pp.hmyi, hb = dir == 0 ? pp.hmxil : pp.hmyid;
+        const S wf = dir == 0 ? w.wfx : w.wfy, wb = dir == 0 ? w.wbx : w.wby, ws = dir == 0 ? w.wsx : w.wsy;
+        const P f = pmul(hm, K::bc(wf));
+        // W (q dx)^2 / 2 with W the weights of both links of this direction at the site
+        const P W = pmul(pp.hqq, per_site ? pfma(hb, K::bc(wb), f) : pmul(hm, K::bc(ws)));
+        const P W0 = K::bc(Ai * Ai), W1 = K::bc((Ai + Ai) * ai), W2 = K::bc(ai * ai);
+        // Delta (Dy, Ey with the opposite sign), and Delta + s (y, x)
+        const P Dx = psub(xj, X), Dy = psub(Y, yj), Ex = psub(uj, U), Ey = psub(Vd, vj);
+        const P s0 = pmul(pp.qd, K::bc(Ai + Aj)), s1 = pmul(pp.qd, K::bc(ai + aj));
+        const P P0 = pfma(s0, Y, Dx), P1 = pfma(s0, Vd, pfma(s1, Y, Ex)), P2 = pmul(s1, Vd);
+        const P Q0 = pfma(s0, X, Dy), Q1 = pfma(s0, U, pfma(s1, X, Ey)), Q2 = pmul(s1, U);
+        const P fDx = pmul(f, Dx), fDy = pmul(f, Dy), fEx = pmul(f, Ex), fEy = pmul(f, Ey);
+        if (dir == 0) {
+            w0 = pmul(W, W0);
+            w1 = pmul(W, W1);
+            w2 = pmul(W, W2);
+            ka = pmul(fDx, P0);
+            kb = pfma(fEx, P0, pmul(fDx, P1));
+            kc = pfma(fEx, P1, pmul(fDx, P2));
+            kd = pmul(fEx, P2);
+        } else {
+            w0 = pfma(W, W0, w0);
+            w1 = pfma(W, W1, w1);
+            w2 = pfma(W, W2, w2);
+            ka = pfma(fDx, P0, ka);
+            kb = pfma(fEx, P0, pfma(fDx, P1, kb));
+            kc = pfma(fEx, P1, pfma(fDx, P2, kc));
+            kd = pfma(fEx, P2, kd);
+        }
+        ka = pfma(fDy, Q0, ka);
+        kb = pfma(fEy, Q0, pfma(fDy, Q1, kb));
+        kc = pfma(fEy, Q1, pfma(fDy, Q2, kc));
+        kd = pfma(fEy, Q2, kd);
+        if (compat) {
+            if (dir == 0) {
+                // t1 carries charge -1 instead of q in its field term: t1 += e, e_k = (q + 1) dx a psi;
+                // B += t0.e, C += t1.e + e.e / 2, D += e.t2
+                const P ci = pmul(pp.kq, K::bc(ai)), cj = pmul(pp.kq, K::bc(aj));
+                const P Qi = pmul(pp.qd, K::bc(Ai)), Qj = pmul(pp.qd, K::bc(Aj));
+                const P qi = pmul(pp.qd, K::bc(ai)), qj = pmul(pp.qd, K::bc(aj));
+                const P rj = pfma(yj, yj, pmul(xj, xj)), rhj = pfma(yj, vj, pmul(xj, uj));
+                const P nK0 = pfma(X, Dy, pmul(Y, Dx));                 // -(x Dy - y Dx)
+                const P ti = padd(nK0, pmul(Qi, r0)), tj = padd(nK0, pmul(Qj, rj));
+                kb = pnfma(f, pfma(cj, tj, pmul(ci, ti)), kb);
+                const P si = pfma(qi, r0, pfma(Qi, rh, pfma(X, Ey, pmul(Y, Ex))));
+                const P sj = pfma(qj, rj, pfma(Qj, rhj, pfma(xj, Ey, pmul(yj, Ex))));
+                kc = pnfma(f, pfma(cj, sj, pmul(ci, si)), kc);
+                const P ee = pfma(pmul(cj, cj), rj, pmul(pmul(ci, ci), r0));
+                kc = pfma(pmul(f, K::bc(half)), ee, kc);
+                kd = pnfma(f, pfma(cj, pmul(qj, rhj), pmul(ci, pmul(qi, rh))), kd);
+            } else {
+                kd_y = pfma(n2, pmul(W, W1), pmul(n1, pmul(W, W2)));
+                kd_y = pfma(fEx, P2, pfma(fEy, Q2, kd_y));
+            }
+        }
+    }
+    // condensation b/2 (n0 + n1 t + n2 t^2)^2 and the site terms
+    const P bA = pmul(pp.b, K::bc(w.area)), bh = pmul(bA, K::bc(half));
+    const P U0 = pfma(bA, n0, w0), U1 = pfma(bA, n1, w1), V1 = pfma(bh, n1, w1), U2 = pfma(bh, n2, w2);
+    ka = pfma(w0, r0, pfma(pmul(bh, n0), n0, ka));
+    kb = pfma(w1, r0, pfma(n1, U0, kb));
+    kc = pfma(w2, r0, pfma(n1, V1, pfma(n2, U0, kc)));
+    kd = pfma(w2, n1, pfma(n2, U1, kd));
+    if (compat) kd = pnfma(kd_y, K::bc(half), kd);
+    const P ke = pmul(n2, U2);
+    S e = K::sum(ka), b1 = K::sum(kb), c2 = K::sum(kc), d3 = K::sum(kd), e4 = K::sum(ke);
+    if constexpr (NC == 2) {   // couplings between the components
+        const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y), x2 = K::template lane<1>(X), y2 = K::template lane<1>(Y);
+        const S u1 = K::template lane<0>(U), v1 = K::template lane<0>(Vd), u2 = K::template lane<1>(U), v2 = K::template lane<1>(Vd);
+        const S R0 = fma1(y1, y2, x1 * x2), R2 = fma1(v1, v2, u1 * u2);
+        const S R1 = fma1(y1, v2, fma1(x1, u2, fma1(v1, y2, u1 * x2)));
+        const S ea = pp.eta * w.area;
+        e = fma1(ea, R0, e);
+        b1 = fma1(ea, R1, b1);
+        c2 = fma1(ea, R2, c2);
+        const S ga = half * pp.gamma * w.area;
+        const S g0 = ga * K::template lane<0>(r0), g1 = ga * K::template lane<0>(n1), g2 = ga * K::template lane<0>(n2);
+        const S s0 = K::template lane<1>(r0), s1 = K::template lane<1>(n1), s2 = K::template lane<1>(n2);
+        e = fma1(g0, s0, e);
+        b1 = fma1(g1, s0, fma1(g0, s1, b1));
+        c2 = fma1(g2, s0, fma1(g1, s1, fma1(g0, s2, c2)));
+        d3 = fma1(g2, s1, fma1(g1, s2, d3));
+        e4 = fma1(g2, s2, e4);
+        if (!SkipZeroDelta<S>::v || pp.delta != S(0.0f)) {
+            const S I0 = fma1(x1, y2, -(y1 * x2)), I2 = fma1(u1, v2, -(v1 * u2));
+            const S I1 = fma1(-v1, x2, fma1(-y1, u2, fma1(u1, y2, x1 * v2)));
+            const S da = half * pp.delta * w.area, d2 = pp.delta * w.area;
+            e = fma1(da, fma1(R0, R0, -(I0 * I0)), e);
+            b1 = fma1(d2, fma1(R1, R0, -(I1 * I0)), b1);
+            c2 = fma1(da, fma1(R1, R1, -(I1 * I1)), c2);
+            c2 = fma1(d2, fma1(R0, R2, -(I0 * I2)), c2);
+            d3 = fma1(d2, fma1(R1, R2, -(I1 * I2)), d3);
+            e4 = fma1(da, fma1(R2, R2, -(I2 * I2)), e4);
+        }
+    }
+    if (!thin_film) {
+        const Curl<S> c(v.a), q(dv.a);
+        const S nh = -pp.h;
+        S em0 = S(0.0f), em1 = em0, em2 = em0;
+#define EMV(wv, yy, xx, dyy, dxx)                                                                        \
+    {                                                                                                    \
+        const S m0 = fma1(pp.idx, yy - xx, nh), m1 = dyy - dxx, z0 = wv * m0, z1 = wv * m1;              \
+        em0 = fma1(z0, m0, em0);                                                                         \
+        em1 = fma1(z0, m1, em1);                                                                         \
+        em2 = fma1(z1, m1, em2);                                                                         \
+    }
+        EMV(w.vUR, c.yp, c.xp, q.yp, q.xp)
+        EMV(w.vUL, c.ym, c.xp, q.ym, q.xp)
+        EMV(w.vLL, c.ym, c.xm, q.ym, q.xm)
+        EMV(w.vLR, c.yp, c.xm, q.yp, q.xm)
+#undef EMV
+        e = fma1(S(0.125f), em0, e);
+        b1 = fma1(pp.idx4, em1, b1);
+        c2 = fma1(pp.idx8, em2, c2);
+    }
+    out[0] = e;
+    out[1] = b1;
+    out[2] = c2;
+    out[3] = d3;
+    out[4] = e4;
+}
+
+// B and J at one site (computeJBKernel, nlcg.cu:243-364).
+template <class S, int NC>
+__device__ __forceinline__ void site_jb(const PackView<S, NC> &v, S idx, const PackParams<S, NC> &pp, const Wts<S> &w,
+                                        S *out /* 1+2NC */)
+{
+    using K = Pk<S, NC>;
+    using P = pack_t<S, NC>;
+    const Curl<S> c(v.a);
+    S bb = w.vUR * (c.yp - c.xp);
+    bb = fma1(w.vUL, c.ym - c.xp, bb);
+    bb = fma1(w.vLL, c.ym - c.xm, bb);
+    bb = fma1(w.vLR, c.yp - c.xm, bb);
+    out[0] = bb * idx * w.ivs;
+    const P X = v.px[1][1], Y = v.py[1][1];
+    const P r = pfma(Y, Y, pmul(X, X));
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const S A = dir == 0 ? v.a[1][1].x : v.a[1][1].y;
+        const P xf = dir == 0 ? v.px[1][2] : v.px[2][1], yf = dir == 0 ? v.py[1][2] : v.py[2][1];
+        const P xb = dir == 0 ? v.px[1][0] : v.px[0][1], yb = dir == 0 ? v.py[1][0] : v.py[0][1];
+        const P lf = K::bc(dir == 0 ? w.lfx : w.lfy), lb = K::bc(dir == 0 ? w.lbx : w.lby);
+        // lattice current of each link: x Dy - y Dx - a |psi|^2
+        const P ar = pmul(pmul(pp.qd, K::bc(A)), r);
+        const P jf = pnfma(Y, psub(xf, X), pfma(X, psub(yf, Y), pmul(ar, K::bc(S(-1.0f)))));
+        const P jb = pnfma(Y, psub(X, xb), pfma(X, psub(Y, yb), pmul(ar, K::bc(S(-1.0f)))));
+        const P j = pmul(pmul(dir == 0 ? pp.hmx : pp.hmy, pp.qi), pfma(lb, jb, pmul(lf, jf)));
+        out[1 + dir] = K::template lane<0>(j);
+        if (NC == 2) out[3 + dir] = K::template lane<1>(j);
+    }
+}
+
+}  // namespace mepgl

@@ -20,12 +20,12 @@
 
 constexpr int NTS = 32;   // threads per block of the strip kernels
 
-// Two-component FP32 strings run the packed stencils (site_pair.cuh): the
-// window then holds psi as (Re psi_1, Re psi_2), (Im psi_1, Im psi_2) in the
-// two pair slots of the components.
-template <class T, int NC>
+// The window of a two-component string holds psi as the stencils' packs,
+// (Re psi_1, Re psi_2) and (Im psi_1, Im psi_2), in the two pair slots of the
+// components.
+template <int NC>
 struct StripPacked {
-    static constexpr bool v = MEPGL_STRIP_PAIR && NC == 2 && std::is_same<T, float>::value;
+    static constexpr bool v = NC == 2;
 };
 
 // (re, im) of two components <-> (Re 1, Re 2), (Im 1, Im 2): a 2 x 2 transpose.
@@ -41,14 +41,12 @@ __device__ __forceinline__ void transpose_pair(V &a, V &b)
 
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
-// Register window of one site: A(dx, dy), P(c, dx, dy); the strip kernels
-// fill the entries their stencil reads and leave the others zero.
+// Register window of one site; the strip kernels fill the entries their
+// stencil reads and leave the others zero.
 template <class T, int NC>
 struct RegView {
     vec2_t<T> a[3][3];
     vec2_t<T> p[NC][3][3];
-    __device__ __forceinline__ vec2_t<T> A(int dx, int dy) const { return a[dy + 1][dx + 1]; }
-    __device__ __forceinline__ vec2_t<T> P(int c, int dx, int dy) const { return p[c][dy + 1][dx + 1]; }
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
@@ -62,19 +60,24 @@ struct RegView {
     }
 };
 
-// Packed view of a register window (PairView) from a RegView of the same
-// site whose psi slots already hold the packed pairs.
+// The stencils' view of a register window (for two components its psi slots
+// already hold the packs).
 template <class T, int NC>
-__device__ __forceinline__ PairView<T> pair_view(const RegView<T, NC> &r)
+__device__ __forceinline__ PackView<T, NC> pack_view(const RegView<T, NC> &r)
 {
-    PairView<T> v;
+    PackView<T, NC> v;
 #pragma unroll
     for (int y = 0; y < 3; ++y)
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
             v.a[y][x] = r.a[y][x];
-            v.px[y][x] = r.p[0][y][x];
-            v.py[y][x] = r.p[NC - 1][y][x];
+            if constexpr (NC == 1) {
+                v.px[y][x] = r.p[0][y][x].x;
+                v.py[y][x] = r.p[0][y][x].y;
+            } else {
+                v.px[y][x] = r.p[0][y][x];
+                v.py[y][x] = r.p[1][y][x];
+            }
         }
     return v;
 }
@@ -286,8 +289,8 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
     }
     const T alpha = (T)__ldcg(sc.alpha_pend + img);
     const unsigned fields = alpha != (T)0 ? 3u : 1u;   // d is not read when nothing is pending
-    SiteParams<T> p;
-    p.load_uniform(S);
+    PackParams<T, NC> pp;
+    pp.load(S);
     V rc[3][1 + NC];
     uint16_t rm;
     // raw row j -> window row (x + alpha d; left / right A by shuffles)
@@ -304,7 +307,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
             hx[c].y = hv.y + alpha * hd.y;
             R.gold[c] = raw[2][c];
         }
-        if constexpr (StripPacked<T, NC>::v) {
+        if constexpr (StripPacked<NC>::v) {
             transpose_pair(R.x[1], R.x[NC]);
             transpose_pair(hx[1], hx[NC]);
         }
@@ -332,11 +335,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
     }
     const int rows = S.ny - j0 < TYT ? S.ny - j0 : TYT;
     T v[2] = {(T)0, (T)0};
-#if MEPGL_STRIP_UNROLL
-#pragma unroll 3   // the window rotates with period 3: unrolled, its copies become renames
-#else
 #pragma unroll 1
-#endif
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
         take(Rp, j + 1, hp1, rc, rm);
@@ -346,7 +345,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
             V o[1 + NC];
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) o[c] = R0.x[c];
-            if constexpr (StripPacked<T, NC>::v) transpose_pair(o[1], o[NC]);
+            if constexpr (StripPacked<NC>::v) transpose_pair(o[1], o[NC]);
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) xout[c][s] = o[c];
         }
@@ -364,28 +363,11 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
             w3.p[c][1][2] = from_right<T>(R0.x[1 + c], hp0[c], L.lane);
         }
         if (L.cok) {
-            T hr = p.h, hl = p.h, hu = p.h, hd = p.h;
-            if (S.per_site) {
-                p.load_site(S, s, NC);
-                hr = h_site(S, p, s + 1 < S.nx * S.ny ? s + 1 : s);
-                hl = h_site(S, p, s > 0 ? s - 1 : s);
-                hu = h_site(S, p, j + 1 < S.ny ? s + S.nx : s);
-                hd = h_site(S, p, j > 0 ? s - S.nx : s);
-            }
+            if (S.per_site) pp.load_site(S, L.gi, j, s);
             T g[2 + 2 * NC];
             Wts<T> w;
-            if constexpr (StripPacked<T, NC>::v) {
-                w.load(R0.m);
-                PairParams<T> pp;
-                pp.set(p);
-                site_gradient_pair<T>(pair_view(w3), p, pp, w, hr, hl, hu, hd, f.maxwell, S.thin_film, g);
-            } else if (MEPGL_STRIP_INTERIOR && R0.m == 0xffffu) {   // interior site: unit weights, folded in
-                w.interior();
-                site_gradient_v<T, NC>(w3, p, w, hr, hl, hu, hd, f.maxwell, S.thin_film, g);
-            } else {
-                w.load(R0.m);
-                site_gradient_v<T, NC>(w3, p, w, hr, hl, hu, hd, f.maxwell, S.thin_film, g);
-            }
+            w.load(R0.m);
+            site_gradient<T, NC>(pack_view(w3), pp, w, field_sums(S, pp, L.gi, j, s), f.maxwell, S.thin_film, g);
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) {
                 V gv;
@@ -466,8 +448,8 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
         dout[c] = static_cast<V *>(S.d[f.dout][c]) + off;
     }
     const T beta = (T)__ldcg(sc.beta + img);
-    SiteParams<T> p;
-    p.load_uniform(S);
+    PackParams<T, NC> pp;
+    pp.load(S);
     V rc[3][1 + NC];
     uint16_t rm;
     auto take = [&](DirRow<T, NC> &R, const V (&raw)[3][1 + NC], uint16_t m) {
@@ -477,7 +459,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
             R.d[c].x = -raw[1][c].x + beta * raw[2][c].x;
             R.d[c].y = -raw[1][c].y + beta * raw[2][c].y;
         }
-        if constexpr (StripPacked<T, NC>::v) {
+        if constexpr (StripPacked<NC>::v) {
             transpose_pair(R.x[1], R.x[NC]);
             transpose_pair(R.d[1], R.d[NC]);
         }
@@ -503,11 +485,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
     }
     const int rows = S.ny - j0 < TYT ? S.ny - j0 : TYT;
     T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
-#if MEPGL_STRIP_UNROLL
-#pragma unroll 2   // the window rotates with period 2: unrolled, its copies become renames
-#else
 #pragma unroll 1
-#endif
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
         take(Rp, rc, rm);
@@ -519,7 +497,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
             V o[1 + NC];
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) o[c] = R0.d[c];
-            if constexpr (StripPacked<T, NC>::v) transpose_pair(o[1], o[NC]);
+            if constexpr (StripPacked<NC>::v) transpose_pair(o[1], o[NC]);
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) dout[c][s] = o[c];
         }
@@ -533,7 +511,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
             hd[c].x = -hg.x + beta * hdd.x;
             hd[c].y = -hg.y + beta * hdd.y;
         }
-        if constexpr (StripPacked<T, NC>::v) {
+        if constexpr (StripPacked<NC>::v) {
             transpose_pair(hx[1], hx[NC]);
             transpose_pair(hd[1], hd[NC]);
         }
@@ -560,21 +538,11 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
             vd.p[c][2][1] = Rp.d[1 + c];
         }
         if (L.cok) {
-            if (S.per_site) p.load_site(S, s, NC);
+            if (S.per_site) pp.load_site(S, L.gi, j, s);
             T o[5];
             Wts<T> w;
-            if constexpr (StripPacked<T, NC>::v) {
-                w.load(R0.m);
-                PairParams<T> pp;
-                pp.set(p);
-                site_poly_pair<T>(pair_view(vx), pair_view(vd), p, pp, w, f.poly_compat, S.thin_film, o);
-            } else if (MEPGL_STRIP_INTERIOR && R0.m == 0xffffu) {   // interior site: unit weights, folded in
-                w.interior();
-                site_poly_v<T, NC>(vx, vd, p, w, f.poly_compat, S.thin_film, o);
-            } else {
-                w.load(R0.m);
-                site_poly_v<T, NC>(vx, vd, p, w, f.poly_compat, S.thin_film, o);
-            }
+            w.load(R0.m);
+            site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, w, S.per_site, f.poly_compat, S.thin_film, o);
 #pragma unroll
             for (int k = 0; k < 5; ++k) v[k] += o[k];
         }
@@ -593,10 +561,10 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
     if (fin) {
         if (L.lane == 0) {
 #pragma unroll
-            for (int k = 0; k < 5; ++k) coef[k] = tot[k];
-            sc.fenergy[img] = tot[0];
+            for (int k = 0; k < 5; ++k) coef[k] = tot[k] * S.ud.dx2;
+            sc.fenergy[img] = coef[0];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = tot[1 + k];
+            for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = coef[1 + k];
         }
         __syncwarp();
         // the scan's grid and rounding follow the stored precision
