@@ -33,23 +33,14 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 TUNING = os.path.join(PKG, "tuning.json")
 
-# Strip candidates: rows per tile, single-warp blocks per SM for the
-# gradient and the direction pass (register budget 65536 / (32 x blocks)),
-# all steps of a call in one fused persistent launch, and its blocks per SM
-# or explicit register cap.
-STRIP = [(40, 16, 16, 1, 12, 0), (32, 16, 16, 1, 12, 0), (32, 16, 16, 1, 16, 152), (32, 16, 16, 1, 16, 144),
-         (32, 16, 16, 1, 16, 128), (32, 16, 16, 0, 16, 0)]
-# Tile candidates: rows per FP32 tile, min blocks per SM for the gradient
-# pass, for the direction pass, gradient-pass halo copy (0 through
-# registers, 1 cp.async), direction pass (0 fused, 1 split into a pointwise
-# update + polynomial pass), fused direction pass halo copy (0 x by cp.async
-# and g, d through registers, 1 all three by cp.async).
-TILE = [(16, 4, 4, 0, 0, 0)]
-CANDIDATES = [dict(MEPGL_STRIP=1, MEPGL_ROWS_F32=r, MEPGL_MINB_STRIP_GRAD=mg, MEPGL_MINB_STRIP_DIR=md,
-                   MEPGL_STRIP_FUSED=fu, MEPGL_MINB_STRIP_FUSED=mf, MEPGL_MAXREG_FUSED=mr)
-              for r, mg, md, fu, mf, mr in STRIP] + [
-    dict(MEPGL_STRIP=0, MEPGL_ROWS_F32=r, MEPGL_MINB_GRAD=g, MEPGL_MINB_DIR=d, MEPGL_GRAD_ASYNC=a,
-         MEPGL_SPLIT_DIR=sp, MEPGL_DIR_ASYNC=da) for r, g, d, a, sp, da in TILE]
+# Candidates for the FP32 NLCG passes: rows per strip, single-warp blocks per
+# SM for the gradient and the direction pass and for the fused launch
+# (register budget 65536 / (32 x blocks)), and whether batches of a few waves
+# run fused (0 waves: never).
+CANDIDATES = [dict(MEPGL_STRIP_ROWS_F32=r, MEPGL_MINB_STRIP_GRAD=mg, MEPGL_MINB_STRIP_DIR=md, MEPGL_MINB_STRIP_FUSED=mf,
+                   MEPGL_FUSE_WAVES=fw)
+              for r, mg, md, mf, fw in [(40, 16, 16, 12, 4), (32, 16, 16, 12, 4), (32, 16, 16, 16, 4),
+                                        (48, 16, 16, 12, 4), (32, 16, 16, 12, 0)]]
 
 
 def defines(c):

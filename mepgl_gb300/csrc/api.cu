@@ -201,6 +201,32 @@ void drop_graphs(mepgl_ctx *c)
     c->graphs.clear();
 }
 
+// Strips of the NLCG passes: rows per strip by launch batch, global strip order.
+int layout_strips(mepgl_ctx *c)
+{
+    const int slots = strip_pass_slots(c->precision, c->opt.fp64_arith == MEPGL_FP64_PAIRED, c->ncomp);
+    int base = 0;
+    c->batch_stile0.clear();
+    c->batch_nstiles.clear();
+    size_t si = 0;
+    for (Batch &B : c->batches) {
+        long most = 0;
+        for (int k = 0; k < B.n; ++k)
+            most += (long)B.s[k].F * B.s[k].tiles_x * ((B.s[k].ny + strip_rows_cap(c->precision) - 1) / strip_rows_cap(c->precision));
+        c->batch_stile0.push_back(base);
+        for (int k = 0; k < B.n; ++k, ++si) {
+            StringDesc &D = B.s[k];
+            D.rows = strip_rows(c->precision, D.ny, most, slots);
+            D.stiles_y = (D.ny + D.rows - 1) / D.rows;
+            D.stile_base = base;
+            base += D.F * D.tiles_x * D.stiles_y;
+            c->hdesc[si] = D;
+        }
+        c->batch_nstiles.push_back(base - c->batch_stile0.back());
+    }
+    return base;
+}
+
 // (Re)build tile table, descriptors and per-image arrays for the current strings.
 mepgl_status build_layout(mepgl_ctx *c)
 {
@@ -241,6 +267,7 @@ mepgl_status build_layout(mepgl_ctx *c)
                                   c->batch_tile0[b]);
     c->n_tiles = (int)tiles.size();
     c->total_images = img;
+    const int n_stiles = layout_strips(c);
     CK(c, cudaMalloc(&c->dtiles, sizeof(TileRef) * tiles.size()));
     CK(c, cudaMemcpy(c->dtiles, tiles.data(), sizeof(TileRef) * tiles.size(), cudaMemcpyHostToDevice));
     Scalars &S = c->sc;
@@ -248,7 +275,8 @@ mepgl_status build_layout(mepgl_ctx *c)
     for (double **p : {&S.gn0, &S.gn1, &S.gdg, &S.beta, &S.alpha, &S.alpha_pend, &S.fenergy})
         CK(c, cudaMalloc(p, I * sizeof(double)));
     CK(c, cudaMalloc(&S.poly, 4 * I * sizeof(double)));
-    CK(c, cudaMalloc(&S.part, (size_t)c->n_tiles * 8 * sizeof(double) + 4096 * sizeof(double)));
+    CK(c, cudaMalloc(&S.part, (size_t)(c->n_tiles > n_stiles ? c->n_tiles : n_stiles) * 8 * sizeof(double) +
+                                  4096 * sizeof(double)));
     CK(c, cudaMalloc(&S.ticket, I * sizeof(unsigned)));
     CK(c, cudaMemset(S.ticket, 0, I * sizeof(unsigned)));
     CK(c, cudaMalloc(&S.status, 16 * sizeof(int)));
@@ -315,6 +343,8 @@ Launch make_launch(mepgl_ctx *c, int batch, int si = -1)
     L.tile0 = t0;
     L.n_tiles = si >= 0 ? c->string_ntiles[si] : c->batch_ntiles[batch];
     L.grid = L.n_tiles;
+    L.stile0 = c->batch_stile0[batch];      // the NLCG passes cover whole batches
+    L.n_stiles = c->batch_nstiles[batch];
     L.precision = c->precision;
     L.paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED ? 1 : 0;
     L.ncomp = c->ncomp;
@@ -358,7 +388,7 @@ mepgl_status one_step(mepgl_ctx *c, int it, int use_cg, int maxwell)
     for (int b = 0; b < nb; ++b) CK(c, launch_dir_poly(make_launch(c, b), c->sc, f));
     c->xi ^= 1;
     c->di ^= 1;
-    c->launches += (int64_t)nlcg_step_launches() * nb;
+    c->launches += (int64_t)2 * nb;
     c->pending = true;
     return MEPGL_OK;
 }
@@ -391,25 +421,30 @@ mepgl_status two_step_graph(mepgl_ctx *c, int use_cg, int maxwell, cudaGraphExec
     return MEPGL_OK;
 }
 
-// Fused FP32 steps pay where a batch is a few waves of the pass kernels
-// (the kernel boundaries then idle much of the GPU); on larger batches the
-// pass kernels, which hold more warps per SM, are faster.
+// Fused steps pay where a batch is a few waves of the pass kernels (the kernel
+// boundaries then idle much of the GPU).  FP32: on larger batches the pass
+// kernels, which hold more warps per SM, are faster.  FP64: both forms hold 8
+// warps per SM and are bound by arithmetic, so the fused launch keeps a small
+// lead (256 x 256 x 64, 7 waves, two steps: 8.96 ms against 9.24); it is
+// bounded so that one call of a large string does not hold the GPU in a
+// single launch of seconds.
 bool use_fused(const mepgl_ctx *c)
 {
-    if (!nlcg_fused(c->precision) || c->opt.fp32_steps == MEPGL_FP32_STEPS_PASSES) return false;
-    if (c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED) return true;
-    const long long cap = (long long)fuse_waves() * strip_pass_slots(c->ncomp);
-    for (int n : c->batch_ntiles)
+    if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_PASSES) return false;
+    if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED) return true;
+    const int paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED;
+    const long long cap = (long long)fuse_waves(c->precision) * strip_pass_slots(c->precision, paired, c->ncomp);
+    for (int n : c->batch_nstiles)
         if (n > cap) return false;
     return true;
 }
 
-// Paired FP64 passes keep the fields x as float-float pairs (x_pairs()):
+// Paired FP64 passes keep the fields x as float-float pairs:
 // the current x of every string changes format before the passes and back
 // after them, so that every other kernel and copy sees double.
 bool paired_x(const mepgl_ctx *c)
 {
-    return c->precision == 1 && c->opt.fp64_arith == MEPGL_FP64_PAIRED && x_pairs();
+    return c->precision == 1 && c->opt.fp64_arith == MEPGL_FP64_PAIRED;
 }
 
 mepgl_status x_format(mepgl_ctx *c, int to_pairs)
@@ -469,7 +504,7 @@ mepgl_status nlcg_steps_body(mepgl_ctx *c, int iters, int use_cg, int maxwell)
         if (st != MEPGL_OK) return st;
         for (; it + 1 <= iters; it += 2) {
             CK(c, cudaGraphLaunch(ex, c->stream));
-            c->launches += 2 * (int64_t)nlcg_step_launches() * c->batches.size();
+            c->launches += 4 * (int64_t)c->batches.size();
         }
         c->pending = true;
     }
@@ -1292,7 +1327,8 @@ mepgl_status mepgl_info(const mepgl_ctx *c, int *n_images, int *precision, int64
 mepgl_status mepgl_pass_kernels(const mepgl_ctx *c, const char **grad, const char **dir_poly, const char **fused)
 {
     if (!c || !grad || !dir_poly || !fused) return MEPGL_ERR_INVALID_ARG;
-    nlcg_pass_kernels(c->precision, c->opt.fp64_arith == MEPGL_FP64_PAIRED, grad, dir_poly);
+    *grad = "k_grad_s";
+    *dir_poly = "k_dir_poly_s";
     *fused = use_fused(c) ? "k_nlcg_s" : "";
     return MEPGL_OK;
 }
@@ -1300,13 +1336,13 @@ mepgl_status mepgl_pass_kernels(const mepgl_ctx *c, const char **grad, const cha
 mepgl_status mepgl_fused_wait_selftest(mepgl_ctx *c, int *timed_out)
 {
     if (!c || !timed_out) return MEPGL_ERR_INVALID_ARG;
-    if (!nlcg_fused(c->precision))
+    if (c->precision != MEPGL_FP32)
         return fail(c, MEPGL_ERR_UNSUPPORTED, "mepgl_fused_wait_selftest: needs an FP32 context and fused steps");
     mepgl_status st = flush(c);
     if (st != MEPGL_OK) return st;
     const Launch L = make_launch(c, 0);
     CK(c, launch_nlcg_fused(L, c->sc, step_flags(c, 1, 1, 0), 1, 1, c->fqueue, c->fstage, c->total_images,
-                            (unsigned long long)L.n_tiles, 4096u));
+                            (unsigned long long)L.n_stiles, 4096u));
     c->launches += 1;
     int flag = 0;
     CK(c, cudaMemcpyAsync(&flag, c->sc.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1338,7 +1374,7 @@ mepgl_status mepgl_profile_passes(mepgl_ctx *c, int steps, int use_cg, double *m
         CK(c, cudaEventRecord(ev[2 * it], c->stream));
         c->xi ^= 1;
         c->di ^= 1;
-        c->launches += (int64_t)nlcg_step_launches() * nb;
+        c->launches += (int64_t)2 * nb;
         c->pending = true;
     }
     if (px) {

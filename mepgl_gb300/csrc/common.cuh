@@ -165,6 +165,8 @@ struct StringDesc {
     int tiles_x, tiles_y;     // tiles per image
     int img_base;             // first global image index of this string
     int tile_base;            // first global tile index of this string
+    int rows;                 // rows per warp strip of the NLCG passes
+    int stiles_y, stile_base; // strips per column of an image; first global strip index
     int thin_film;
     int disc;                 // 0: the reference's linearised differences, 1: gauge links
     int per_site;             // 1: parameters read from the arrays below

@@ -42,6 +42,7 @@ struct mepgl_ctx {
     // pass, its descriptors passed by value to the kernels
     std::vector<mepgl::Batch> batches;
     std::vector<int> batch_tile0, batch_ntiles, string_batch;
+    std::vector<int> batch_stile0, batch_nstiles;   // warp strips of the NLCG passes
     mepgl::TileRef *dtiles = nullptr;
     int n_tiles = 0, total_images = 0;
     unsigned long long *fqueue = nullptr;   // work counter of the fused NLCG launch

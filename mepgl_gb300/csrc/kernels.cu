@@ -2,25 +2,25 @@
 //
 // The NLCG iteration of the reference (nlcgSteps, mepgl/src/nlcg.cu:1462-1586:
 // ~12 kernels, 4 two-level reductions, ~10 device-wide syncs per step) is two
-// passes over the string here:
+// passes over the string here (strip.cuh):
 //
-//   k_grad      x <- x + alpha_pend d   (the previous step's update, fused)
+//   gradient    x <- x + alpha_pend d   (the previous step's update, fused)
 //               g  = dF/dx              (gradientPsi + gradientA)
 //               |g|^2, g.(g - g_prev)   (gradientDensity + 2 sums)
-//               last tile of an image:  beta (computeStepDirection's scalar)
-//   k_dir_poly  d <- -g + beta d        (computeStepDirection)
+//               last strip of an image: beta (computeStepDirection's scalar)
+//   direction   d <- -g + beta d        (computeStepDirection)
 //               quartic F(x + a d)      (polynomialExpansion + 2 sums)
-//               last tile of an image:  line search -> alpha (lineSearch)
+//               last strip of an image: line search -> alpha (lineSearch)
 //
 // so one step reads x, d, g_prev, g (twice with halo, served mostly by L2)
 // and writes x, g, d: 9 state-sized streams instead of the reference's ~20.
-// x and d are ping-ponged because neighbouring tiles read them as halo while
+// x and d are ping-ponged because neighbouring strips read them as halo while
 // they are being rewritten.
 //
-// Tiles are 32 x TileRows<T> sites (16 rows in FP32, 8 in FP64) staged with
-// a one-site halo in shared memory; each thread computes TileRows/8 sites of
-// one column.  Addresses inside an image are 32-bit offsets from per-tile
-// base pointers.
+// The energy, gradient, adjoint and B, J kernels work on tiles of 32 x
+// TileRows<T> sites staged with a one-site halo in shared memory; each thread
+// computes TileRows/8 sites of one column.  Addresses inside an image are
+// 32-bit offsets from per-tile base pointers.
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -28,125 +28,84 @@
 
 namespace mepgl {
 
-// Tuning knobs (compile time): tile rows per precision and the minimum
-// resident blocks per SM requested from ptxas for the two NLCG passes.
+// Tuning knobs (compile time): tile rows per precision.
 #ifndef MEPGL_ROWS_F32
-#define MEPGL_ROWS_F32 16
+#define MEPGL_ROWS_F32 40
 #endif
 #ifndef MEPGL_ROWS_F64
 #define MEPGL_ROWS_F64 8
 #endif
-#ifndef MEPGL_MINB_GRAD
-#define MEPGL_MINB_GRAD 4
-#endif
-#ifndef MEPGL_MINB_DIR
-#define MEPGL_MINB_DIR 4
-#endif
-
-// 1: the direction d = -g + beta d is formed by a pointwise pass and the
-// polynomial pass copies the x and d halo tiles with cp.async; 0: one fused
-// pass forms d over the halo tile in registers
-#ifndef MEPGL_SPLIT_DIR
-#define MEPGL_SPLIT_DIR 0
-#endif
-// 1: the direction pass of FP32 strings copies the raw x, g and d halo tiles
-// with cp.async and forms -g + beta d in shared memory; 0: x by cp.async,
-// g and d through registers
-#ifndef MEPGL_DIR_ASYNC
-#define MEPGL_DIR_ASYNC 0
-#endif
-// 1: the gradient pass copies the raw x and d halo tiles with cp.async and
-// forms x + alpha d in shared memory; 0: through registers (stage mode 1)
-#ifndef MEPGL_GRAD_ASYNC
-#define MEPGL_GRAD_ASYNC 0
-#endif
-
-// the float-float passes hold twice the registers of FP32 ones
-// FP32 NLCG passes as warp strips (strip.cuh) instead of shared-memory tiles
-#ifndef MEPGL_STRIP
-#define MEPGL_STRIP 1
-#endif
-#ifndef MEPGL_MINB_STRIP
-#define MEPGL_MINB_STRIP 16   // single-warp blocks per SM: 128 registers
-#endif
+// Resident single-warp blocks per SM asked of ptxas for the strip kernels
+// (registers per thread: 65536 / (32 x blocks)).  FP64 and float-float strips
+// hold twice the registers of FP32 ones; at 12 blocks they spill: a
+// float-float step of the 256 x 256 string took 2.1 ms instead of 1.5, FP64
+// gained nothing.
 #ifndef MEPGL_MINB_STRIP_GRAD
-#define MEPGL_MINB_STRIP_GRAD MEPGL_MINB_STRIP
+#define MEPGL_MINB_STRIP_GRAD 16
 #endif
 #ifndef MEPGL_MINB_STRIP_DIR
-#define MEPGL_MINB_STRIP_DIR MEPGL_MINB_STRIP
-#endif
-// FP32 NLCG steps as one persistent launch with per-image stage counters (strip.cuh)
-#ifndef MEPGL_STRIP_FUSED
-#define MEPGL_STRIP_FUSED 0
-#endif
-// FP32 strip launches of a single string use kernels specialised for it
-#ifndef MEPGL_STRIP_ONE
-#define MEPGL_STRIP_ONE 1
+#define MEPGL_MINB_STRIP_DIR 16
 #endif
 #ifndef MEPGL_MINB_STRIP_FUSED
-#define MEPGL_MINB_STRIP_FUSED MEPGL_MINB_STRIP
+#define MEPGL_MINB_STRIP_FUSED 12
 #endif
-// explicit register cap of the fused kernel (0: from MEPGL_MINB_STRIP_FUSED)
-#ifndef MEPGL_MAXREG_FUSED
-#define MEPGL_MAXREG_FUSED 0
+#ifndef MEPGL_MINB_STRIP_F64
+#define MEPGL_MINB_STRIP_F64 8
 #endif
-// fused steps only for batches of at most this many waves of the pass kernels
-// (beyond that the boundaries cost little and the pass kernels hold more warps)
+template <class T> struct StripBlocks {
+    static constexpr int grad = MEPGL_MINB_STRIP_F64, dir = MEPGL_MINB_STRIP_F64, fused = MEPGL_MINB_STRIP_F64;
+};
+template <> struct StripBlocks<float> {
+    static constexpr int grad = MEPGL_MINB_STRIP_GRAD, dir = MEPGL_MINB_STRIP_DIR, fused = MEPGL_MINB_STRIP_FUSED;
+};
+// Fused steps only for batches of at most this many waves of the pass kernels
+// (beyond that the boundaries cost little; FP32 pass kernels hold more warps)
 #ifndef MEPGL_FUSE_WAVES
 #define MEPGL_FUSE_WAVES 4
 #endif
-#if MEPGL_STRIP && MEPGL_SPLIT_DIR
-#error "MEPGL_SPLIT_DIR applies to the tile kernels; build it with MEPGL_STRIP=0"
+#ifndef MEPGL_FUSE_WAVES_F64
+#define MEPGL_FUSE_WAVES_F64 16
 #endif
-#ifndef MEPGL_MINB_GRAD_F64
-#define MEPGL_MINB_GRAD_F64 3
-#endif
-#ifndef MEPGL_MINB_DIR_F64
-#define MEPGL_MINB_DIR_F64 2
-#endif
-#ifndef MEPGL_MINB_GRAD_FF
-#define MEPGL_MINB_GRAD_FF 3
-#endif
-#ifndef MEPGL_MINB_DIR_FF
-#define MEPGL_MINB_DIR_FF 2
-#endif
-template <class T> struct MinBlocks { static constexpr int grad = MEPGL_MINB_GRAD, dir = MEPGL_MINB_DIR; };
-template <> struct MinBlocks<double> { static constexpr int grad = MEPGL_MINB_GRAD_F64, dir = MEPGL_MINB_DIR_F64; };
-template <> struct MinBlocks<ff> { static constexpr int grad = MEPGL_MINB_GRAD_FF, dir = MEPGL_MINB_DIR_FF; };
-// Gradient tile kernels whose stencil spills at their register budget stage
-// one halo element at a time and read the previous gradient after the
-// stencil.  MEPGL_GRAD_LEAN: 0 none, 1 the float-float kernels (default),
-// 2 every precision.
-#ifndef MEPGL_GRAD_LEAN
-#define MEPGL_GRAD_LEAN 1
-#endif
-template <class T> struct GradLean {
-    static constexpr bool v = MEPGL_GRAD_LEAN == 2 || (MEPGL_GRAD_LEAN == 1 && std::is_same<T, ff>::value);
-};
-
-// Paired FP64: while the NLCG passes run, the fields x hold float-float
-// pairs too (launch_x_format converts them in place before and after), so
-// the passes read and write them without double conversions.
-#ifndef MEPGL_FF_XPAIRS
-#define MEPGL_FF_XPAIRS 1
-#endif
-template <class T> struct XPairs { static constexpr bool v = MEPGL_FF_XPAIRS != 0 && std::is_same<T, ff>::value; };
 
 template <class T> struct TileRows { static constexpr int v = sizeof(T) == 4 ? MEPGL_ROWS_F32 : MEPGL_ROWS_F64; };
 template <> struct TileRows<ff> { static constexpr int v = MEPGL_ROWS_F64; };
 
-int nlcg_step_launches() { return 2 + MEPGL_SPLIT_DIR; }
+int fuse_waves(int precision) { return precision == 1 ? MEPGL_FUSE_WAVES_F64 : MEPGL_FUSE_WAVES; }
 
-bool nlcg_fused(int precision) { return MEPGL_STRIP && MEPGL_STRIP_FUSED && precision == 0; }
+// Rows per strip.  A strip walks its rows one after the other, so a string
+// with fewer strips than the GPU holds warps waits on a few long walks: ten
+// FP32 steps of 67 x 61 x 9 sites took 865 us with 40-row strips (54 of
+// them), 300 us with 2-row ones.  A long strip reads its two halo rows less
+// often; past 40 rows (FP32) the fused launch's per-image waits cost more
+// than that saves, and past 16 (FP64) nothing is gained, the passes being
+// bound by arithmetic.  So the rows shrink from the cap in proportion once a
+// batch has fewer strips than FILL per cent of the resident warps (ten steps
+// of 128 x 128 x 24 sites, one / two components, at 50, 100, 150, 200, 300 %:
+// FP32 389 / 508, 341 / 392, 316 / 347, 360 / 354, 359 / 403 us; FP64 3431 /
+// 6027, 2407 / 4279, 2329 / 4143, 2341 / 4154, 2397 / 4216 us; FP32 256 x
+// 256 x 40 loses 3 % from 150 on), down to the fewest rows that still gain.
+#ifndef MEPGL_STRIP_ROWS_F32
+#define MEPGL_STRIP_ROWS_F32 40
+#endif
+#ifndef MEPGL_STRIP_ROWS_F64
+#define MEPGL_STRIP_ROWS_F64 16
+#endif
+#ifndef MEPGL_STRIP_FILL_F32
+#define MEPGL_STRIP_FILL_F32 125
+#endif
+#ifndef MEPGL_STRIP_FILL_F64
+#define MEPGL_STRIP_FILL_F64 150
+#endif
+int strip_rows_cap(int precision) { return precision == 1 ? MEPGL_STRIP_ROWS_F64 : MEPGL_STRIP_ROWS_F32; }
 
-int fuse_waves() { return MEPGL_FUSE_WAVES; }
-
-void nlcg_pass_kernels(int precision, int paired, const char **grad, const char **dir_poly)
+int strip_rows(int precision, int ny, long tiles, int slots)
 {
-    (void)paired;
-    const bool strip = MEPGL_STRIP && precision == 0;
-    *grad = strip ? "k_grad_s" : "k_grad";
-    *dir_poly = strip ? "k_dir_poly_s" : "k_dir_poly";
+    const int cap = strip_rows_cap(precision), least = precision == 1 ? 1 : 2;
+    const long want = (long)slots * (precision == 1 ? MEPGL_STRIP_FILL_F64 : MEPGL_STRIP_FILL_F32) / 100;
+    long rows = tiles < want ? cap * tiles / want : cap;
+    if (rows < least) rows = least;
+    const long k = (ny + rows - 1) / rows;          // strips per column, of equal height
+    return (int)((ny + k - 1) / k);
 }
 
 int tile_rows(int precision) { return precision == 1 ? TileRows<double>::v : TileRows<float>::v; }
@@ -168,97 +127,50 @@ namespace {
 template <class T, int NC>
 struct ImagePtrs {                  // storage type (double for float-float)
     const vec2_t<store_t<T>> *in[1 + NC];
-    const vec2_t<store_t<T>> *aux[1 + NC];
-    vec2_t<store_t<T>> *out[1 + NC];
 };
 
 // ------------------------------------------------------------------ staging
 // The (TYT+2) x (TX+2) halo tile is split into flat element indices spread
 // over the block; each thread first issues every global load of all its
-// elements (independent, so they are in flight together), then combines and
-// stores them.  Out-of-lattice elements are zero.
-// mode 0: x = in;  mode 1: x = in + alpha * aux (and interior x -> out);
-// mode 2: x = -aux + beta * in, i.e. the new direction (interior -> out).
-// IN_WORK / AUX_WORK: in (and out) / aux are NLCG work arrays (g, d) rather
-// than fields.
-// CHUNK: one element's loads in flight at a time instead of all of them
-// (fewer registers live, for the kernels whose stencil is near its budget).
-template <class T, int NC, int TYT, int MODE, bool IN_WORK = false, bool AUX_WORK = false, bool CHUNK = false>
-__device__ __forceinline__ void stage(Tile<T, NC, TYT> &t, const StringDesc &S, const ImagePtrs<T, NC> &ip, int i0,
-                                      int j0, T coef, bool write_out, bool masks)
+// elements (independent, so they are in flight together), then stores them.
+// Out-of-lattice elements are zero.
+template <class T, int NC, int TYT>
+__device__ __forceinline__ void stage(Tile<T, NC, TYT> &t, const StringDesc &S, const ImagePtrs<T, NC> &ip, int i0, int j0)
 {
     using V = vec2_t<T>;
-    constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT, KB = CHUNK ? 1 : NI;
-    const bool aux = MODE == 2 || (MODE == 1 && coef != (T)0);
-    V f[NI][1 + NC], a[NI][1 + NC];
+    constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
+    V f[NI][1 + NC];
     uint16_t m[NI];
-    int sidx[NI];
-    bool ok[NI];
 #pragma unroll
-    for (int k0 = 0; k0 < NI; k0 += KB) {
-#pragma unroll
-    for (int k = k0; k < k0 + KB; ++k) {
+    for (int k = 0; k < NI; ++k) {
         const int e = threadIdx.x + k * NT;
         const int hy = e / HW, hx = e - hy * HW;
         const int gi = i0 + hx - 1, gj = j0 + hy - 1;
-        ok[k] = e < HE && gi >= 0 && gi < S.nx && gj >= 0 && gj < S.ny;
-        sidx[k] = ok[k] ? gi + S.nx * gj : 0;
+        const bool ok = e < HE && gi >= 0 && gi < S.nx && gj >= 0 && gj < S.ny;
         m[k] = 0;
 #pragma unroll
-        for (int c = 0; c < 1 + NC; ++c) {
-            f[k][c].x = f[k][c].y = (T)0;
-            a[k][c].x = a[k][c].y = (T)0;
-        }
-        if (ok[k]) {
-            const int s = sidx[k];
+        for (int c = 0; c < 1 + NC; ++c) f[k][c].x = f[k][c].y = (T)0;
+        if (ok) {
+            const int s = gi + S.nx * gj;
 #pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) f[k][c] = IN_WORK ? loadw<T>(ip.in[c] + s) : load2<T>(ip.in[c] + s);
-            if (aux)
-#pragma unroll
-                for (int c = 0; c < 1 + NC; ++c)
-                    a[k][c] = AUX_WORK ? loadw<T>(ip.aux[c] + s) : load2<T>(ip.aux[c] + s);
-            if (masks)
-                m[k] = S.mask ? S.mask[s]
-                              : (uint16_t)((S.code_comp[s] & 0xff) | ((S.code_sc[s] & 0xff) << 8));
+            for (int c = 0; c < 1 + NC; ++c) f[k][c] = load2<T>(ip.in[c] + s);
+            m[k] = S.mask ? S.mask[s] : (uint16_t)((S.code_comp[s] & 0xff) | ((S.code_sc[s] & 0xff) << 8));
         }
     }
 #pragma unroll
-    for (int k = k0; k < k0 + KB; ++k) {
+    for (int k = 0; k < NI; ++k) {
         const int e = threadIdx.x + k * NT;
         if (e >= HE) continue;
         const int hy = e / HW, hx = e - hy * HW;
-        V v[1 + NC];
+        t.A[hy][hx] = f[k][0];
 #pragma unroll
-        for (int c = 0; c < 1 + NC; ++c) {
-            if (MODE == 2) {
-                v[c].x = -a[k][c].x + coef * f[k][c].x;
-                v[c].y = -a[k][c].y + coef * f[k][c].y;
-            } else if (MODE == 1 && aux) {
-                v[c].x = f[k][c].x + coef * a[k][c].x;
-                v[c].y = f[k][c].y + coef * a[k][c].y;
-            } else {
-                v[c] = f[k][c];
-            }
-        }
-        if (write_out && ok[k] && hx >= 1 && hx <= TX && hy >= 1 && hy <= TYT)
-#pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) {
-                if (IN_WORK) storew<T>(ip.out[c] + sidx[k], v[c]);
-                else store2<T>(ip.out[c] + sidx[k], v[c]);
-            }
-        t.A[hy][hx] = v[0];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) t.P[c][hy][hx] = v[1 + c];
-        if (masks) t.m[hy][hx] = m[k];
-    }
+        for (int c = 0; c < NC; ++c) t.P[c][hy][hx] = f[k][1 + c];
+        t.m[hy][hx] = m[k];
     }
 }
 
-// Asynchronous copy of a plain halo tile (no arithmetic on the values):
-// cp.async per element, zero-filled outside the lattice, so its latency
-// overlaps the register-staged arrays that follow.  The neighbour codes
-// (2 bytes, below the 4-byte copy size) are loaded into m[] for the caller
-// to store; cp_async_wait_all() + a barrier complete the tile.
+// Asynchronous copy of one element to shared memory, zero-filled where it is
+// not valid.
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 template <int BYTES>
@@ -274,53 +186,11 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid)
                      : "memory");
 }
 
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-template <class T, int NC, int TYT>
-__device__ __forceinline__ void stage_async(TileF<T, NC, TYT> &t, const StringDesc &S,
-                                            const vec2_t<T> *const *src, int i0, int j0, uint16_t *m)
-{
-    using V = vec2_t<T>;
-    constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
-#pragma unroll
-    for (int k = 0; k < NI; ++k) {
-        const int e = threadIdx.x + k * NT;
-        if (m) m[k] = 0;
-        if (e >= HE) continue;
-        const int hy = e / HW, hx = e - hy * HW;
-        const int gi = i0 + hx - 1, gj = j0 + hy - 1;
-        const bool ok = gi >= 0 && gi < S.nx && gj >= 0 && gj < S.ny;
-        const int s = ok ? gi + S.nx * gj : 0;
-        cp_async<sizeof(V)>(&t.A[hy][hx], src[0] + s, ok);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) cp_async<sizeof(V)>(&t.P[c][hy][hx], src[1 + c] + s, ok);
-        if (m && ok) m[k] = S.mask[s];
-    }
-}
-
-template <class T, int NC, int TYT>
-__device__ __forceinline__ void store_codes(Tile<T, NC, TYT> &t,
-                                            const uint16_t (&m)[(((TYT + 2) * (TX + 2)) + NT - 1) / NT])
-{
-    constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
-#pragma unroll
-    for (int k = 0; k < NI; ++k) {
-        const int e = threadIdx.x + k * NT;
-        if (e < HE) t.m[e / HW][e % HW] = m[k];
-    }
-}
-
 template <class T, int NC>
-__device__ __forceinline__ void image_ptrs(ImagePtrs<T, NC> &ip, void *const *in, void *const *aux, void *const *out,
-                                           size_t off)
+__device__ __forceinline__ void image_ptrs(ImagePtrs<T, NC> &ip, void *const *in, size_t off)
 {
 #pragma unroll
-    for (int c = 0; c < 1 + NC; ++c) {
-        using W = vec2_t<store_t<T>>;
-        ip.in[c] = in ? static_cast<const W *>(in[c]) + off : nullptr;
-        ip.aux[c] = aux ? static_cast<const W *>(aux[c]) + off : nullptr;
-        ip.out[c] = out ? static_cast<W *>(out[c]) + off : nullptr;
-    }
+    for (int c = 0; c < 1 + NC; ++c) ip.in[c] = static_cast<const vec2_t<store_t<T>> *>(in[c]) + off;
 }
 
 // Slot of a tile's partial sums: the global tile index of (string, image, row,
@@ -375,13 +245,30 @@ __device__ __forceinline__ double quartic_rn(const double *c, double x)
 
 // lineSearch (nlcg.cu:1398-1445) by one warp: first p in 1..2000 with
 // f(x_p) > f(x_{p-1}) (else 2000); alpha = x_p / m in the working precision.
+//
+// Every FP64 instruction of a lone warp takes 64 clocks here whatever its
+// lanes do, and the grid starts at 1e-10, some 800 points below a usual
+// step: a scan from its start is 26 rounds of 32 points, 10 us.  So the
+// scan starts at the last multiple of 64 up to which the slope stays below
+// B / 2 (|B| at least twice the other terms of the derivative): there the
+// polynomial part falls by more than 1 % of |B| x from point to point, its
+// rounding is 1e-15 of that, and adding the energy rounds monotonically, so
+// no f(x_p) > f(x_{p-1}) is passed over.
 template <class T>
 __device__ double line_search_scan(const double *c, const double *xt)
 {
     const int lane = threadIdx.x & 31;
-    double f_prev = quartic_rn(c, xt[0]);
+    int p0 = 0;
+    {
+        const double x = xt[64 * lane];
+        const bool falls = c[1] <= -1e-200 && x * (4 * fabs(c[2]) + x * (6 * fabs(c[3]) + x * 8 * fabs(c[4]))) <= -c[1];
+        const unsigned bal = ~__ballot_sync(0xffffffffu, falls);
+        const int n = bal ? __ffs(bal) - 1 : 32;   // leading points that fall
+        if (n > 0) p0 = 64 * (n - 1);
+    }
+    double f_prev = quartic_rn(c, xt[p0]);
     int found = 0;
-    for (int base = 1; base <= 2000; base += 32) {
+    for (int base = p0 + 1; base <= 2000; base += 32) {
         const int p = base + lane;
         const double fp = p <= 2000 ? quartic_rn(c, xt[p]) : 0.0;
         double fl = __shfl_up_sync(0xffffffffu, fp, 1);
@@ -393,6 +280,58 @@ __device__ double line_search_scan(const double *c, const double *xt)
     const int j = found ? found : 2000;
     const T m = (T)1.025f;
     return (double)((T)xt[j] / m);
+}
+
+// Smallest positive root of the quartic's derivative f = a0 + a1 x + a2 x^2 +
+// a3 x^3 with a0 < 0 < a3 (its first local minimum: f crosses zero upwards
+// there) by Newton's method from a point from which it converges
+// monotonically.  f has its turning points at c1 <= c2 where D = a2^2 - 3 a1
+// a3 > 0 and its inflection at cm.  Left of cm it is concave: if f rises from
+// 0 to its root there, Newton from 0 stays left of it.  Right of cm it is
+// convex: Newton from a bound above the root stays right of it.  The steps
+// divide by a float reciprocal (each still gains seven digits).  False where
+// a case is out of the ordinary (no such bound in float range, slow
+// convergence); the caller then takes the closed form, whose acos, cos and
+// cbrt cost a lone warp about 10 us.
+__device__ bool first_minimum(double a0, double a1, double a2, double a3, double &root)
+{
+    if (!(a0 < 0.0)) return false;
+    if (a3 == 0.0 && a2 == 0.0) {
+        root = -a0 / a1;
+        return a1 > 0.0;
+    }
+    if (!(a3 > 0.0)) return false;
+    const double b2 = 2.0 * a2, b3 = 3.0 * a3, D = a2 * a2 - a1 * b3;
+    const double cm = -a2 / b3, fm = a0 + cm * (a1 + cm * (a2 + cm * a3));
+    double x = 0.0;
+    bool right = fm < 0.0;   // monotone f: right of the inflection if it is still negative there
+    if (D > 0.0) {
+        const double sd = sqrt(D), c1 = cm - sd / b3;
+        const double f1 = a0 + c1 * (a1 + c1 * (a2 + c1 * a3));
+        right = !(c1 > 0.0 && f1 > 0.0);
+    } else if (!right && !(a1 > 0.0)) {
+        return false;
+    }
+    if (right) {
+        // x - cm <= max(sqrt(2 |P|), cbrt(2 |Q|)) of the depressed cubic z^3 + P z + Q
+        const float P = (float)(2.0 * fabs(D) / (b3 * a3)), Q = (float)(2.0 * fabs(fm) / a3);
+        const float z = 1.0001f * fmaxf(sqrtf(P), cbrtf(Q));
+        if (!(z > 1e-30f && z < 1e30f)) return false;
+        x = cm + (double)z;
+        if (!(x > 0.0)) return false;
+    }
+    for (int it = 0; it < 24; ++it) {
+        const double f = a0 + x * (a1 + x * (a2 + x * a3)), df = a1 + x * (b2 + x * b3);
+        const float d = (float)df;
+        if (!(d > 1e-30f && d < 1e30f)) return false;
+        const double dx = f * (double)(1.0f / d);
+        x -= dx;
+        if (fabs(dx) <= 1e-9 * fabs(x)) {
+            root = x;
+            return x > 0.0;
+        }
+    }
+    return false;
 }
 
 // Exact version of the reference's scan: the first local minimum of the
@@ -443,311 +382,22 @@ __device__ double line_search_exact(const double *c, double fallback)
     return best < 0 ? fallback : best;
 }
 
+// The step of one image from its quartic, by one warp: the scan's answer, or
+// the exact first minimum (the scan's where there is none).  T: stored
+// precision, whose grid and rounding the scan follows.
+template <class T>
+__device__ double line_search(const double *coef, const Scalars &sc, int exact)
+{
+    if (exact) {
+        double x;
+        if (first_minimum(coef[1], 2 * coef[2], 3 * coef[3], 4 * coef[4], x)) return x;
+    }
+    const double alpha = line_search_scan<T>(coef, sizeof(T) == 8 ? sc.xtab_d : sc.xtab_f);
+    return exact ? line_search_exact(coef, alpha) : alpha;
+}
+
 // ------------------------------------------------------------------ kernels
-template <class T, int NC>
-__global__ void __launch_bounds__(NT, MinBlocks<T>::grad) k_grad(const __grid_constant__ Batch bt, const TileRef *__restrict__ tiles,
-                                             int n_tiles, Scalars sc, StepFlags f)
-{
-    constexpr int TYT = TileRows<T>::v;
-    using V = vec2_t<T>;
-    __shared__ Tile<T, NC, TYT> t;
-#if MEPGL_GRAD_ASYNC
-    __shared__ TileF<T, NC, TYT> dt;
-#endif
-    __shared__ double red[NT / 32 * 2];
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const int img = S.img_base + tr.n;
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        const size_t off = (size_t)tr.n * S.nx * S.ny;
-        ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[f.xin], S.d[f.din], S.x[f.xout], off);
-#if MEPGL_GRAD_ASYNC
-        if constexpr (std::is_same<T, ff>::value) {
-            stage<T, NC, TYT, 1, XPairs<T>::v, true, GradLean<T>::v>(t, S, ip, i0, j0, (T)sc.alpha_pend[img], true, true);
-        } else {
-            constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
-            const T alpha = (T)sc.alpha_pend[img];
-            uint16_t codes[NI];
-            stage_async<T, NC, TYT>(t, S, ip.in, i0, j0, codes);
-            if (alpha != (T)0) stage_async<T, NC, TYT>(dt, S, ip.aux, i0, j0, nullptr);
-            store_codes<T, NC, TYT>(t, codes);
-            cp_async_wait_all();
-            __syncthreads();
-            // x <- x + alpha d over the halo tile; interior x -> x[xout]
-#pragma unroll
-            for (int k = 0; k < NI; ++k) {
-                const int e = threadIdx.x + k * NT;
-                if (e >= HE) continue;
-                const int hy = e / HW, hx = e - hy * HW;
-                V v[1 + NC];
-                v[0] = t.A[hy][hx];
-#pragma unroll
-                for (int c = 0; c < NC; ++c) v[1 + c] = t.P[c][hy][hx];
-                if (alpha != (T)0) {
-                    V dv = dt.A[hy][hx];
-                    v[0].x = v[0].x + alpha * dv.x;
-                    v[0].y = v[0].y + alpha * dv.y;
-                    t.A[hy][hx] = v[0];
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        dv = dt.P[c][hy][hx];
-                        v[1 + c].x = v[1 + c].x + alpha * dv.x;
-                        v[1 + c].y = v[1 + c].y + alpha * dv.y;
-                        t.P[c][hy][hx] = v[1 + c];
-                    }
-                }
-                const int gi = i0 + hx - 1, gj = j0 + hy - 1;
-                if (hx >= 1 && hx <= TX && hy >= 1 && hy <= TYT && gi < S.nx && gj < S.ny)
-#pragma unroll
-                    for (int c = 0; c < 1 + NC; ++c) ip.out[c][gi + S.nx * gj] = v[c];
-            }
-        }
-#else
-        stage<T, NC, TYT, 1, XPairs<T>::v, true, GradLean<T>::v>(t, S, ip, i0, j0, (T)sc.alpha_pend[img], true, true);
-#endif
-        using W = vec2_t<store_t<T>>;
-        W *gcur[1 + NC];
-        const W *gprev[1 + NC];
-#pragma unroll
-        for (int c = 0; c < 1 + NC; ++c) {
-            gcur[c] = static_cast<W *>(S.g[f.gcur][c]) + off;
-            gprev[c] = static_cast<const W *>(S.g[f.gprev][c]) + off;
-        }
-        PackParams<T, NC> pp;
-        pp.load(S);
-        __syncthreads();
-        T v[2] = {(T)0, (T)0};
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
-        // previous gradient of this thread's sites, loaded before the stencil
-        // (lean kernels: after it, so that it holds no registers meanwhile)
-        V gold[TYT / 8][1 + NC];
-        if (!GradLean<T>::v)
-#pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int gj = j0 + (threadIdx.x >> 5) + 8 * r;
-#pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) {
-                gold[r][c].x = gold[r][c].y = (T)0;
-                if (gi < S.nx && gj < S.ny) gold[r][c] = loadw<T>(gprev[c] + gi + S.nx * gj);
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                const int s = gi + S.nx * gj;
-                Wts<T> w;
-                w.load(t.m[ly + 1][lx + 1]);
-                if (S.per_site) pp.load_site(S, gi, gj, s);
-                T g[2 + 2 * NC];
-                site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s), f.maxwell,
-                                     S.thin_film, g);
-                if (GradLean<T>::v)
-#pragma unroll
-                    for (int c = 0; c < 1 + NC; ++c) gold[r][c] = loadw<T>(gprev[c] + s);
-#pragma unroll
-                for (int c = 0; c < 1 + NC; ++c) {
-                    V gv;
-                    gv.x = g[2 * c];
-                    gv.y = g[2 * c + 1];
-                    storew<T>(gcur[c] + s, gv);
-                    const V go = gold[r][c];
-                    v[0] += gv.x * gv.x + gv.y * gv.y;
-                    v[1] += gv.x * (gv.x - go.x) + gv.y * (gv.y - go.y);
-                }
-            }
-        }
-        const int tpi = S.tiles_x * S.tiles_y;
-        double tot[2];
-        if (finish_image<2>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot) && threadIdx.x == 0) {
-            (f.gcur ? sc.gn1 : sc.gn0)[img] = tot[0];
-            sc.gdg[img] = tot[1];
-            double beta = 0.0;
-            if (f.use_cg) {
-                beta = tot[1] / (f.gprev ? sc.gn1 : sc.gn0)[img];
-                beta = beta > 0.0 ? beta : 0.0;   // Polak-Ribiere clipped at 0; NaN -> 0
-            }
-            sc.beta[img] = beta;
-        }
-        __syncthreads();
-    }
-}
-
-template <class T, int NC>
-__global__ void __launch_bounds__(NT, MinBlocks<T>::dir) k_dir_poly(const __grid_constant__ Batch bt,
-                                                 const TileRef *__restrict__ tiles, int n_tiles, Scalars sc,
-                                                 StepFlags f)
-{
-    constexpr int TYT = TileRows<T>::v;
-    __shared__ Tile<T, NC, TYT> tx;
-    __shared__ Tile<T, NC, TYT> td;
-    // raw gradient tile of the all-asynchronous FP32 variant (16 bytes otherwise)
-    constexpr bool DIR_ASYNC = MEPGL_DIR_ASYNC && !MEPGL_SPLIT_DIR && std::is_same<T, float>::value;
-    __shared__ __align__(16) unsigned char g_raw[DIR_ASYNC ? sizeof(TileF<T, NC, TYT>) : 16];
-    __shared__ double red[NT / 32 * 5];
-    __shared__ double coef[5];
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const int img = S.img_base + tr.n;
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        const size_t off = (size_t)tr.n * S.nx * S.ny;
-        ImagePtrs<T, NC> ipx, ipd;
-        image_ptrs<T, NC>(ipx, S.x[f.xout], nullptr, nullptr, off);
-        image_ptrs<T, NC>(ipd, S.d[f.din], S.g[f.gcur], S.d[f.dout], off);
-        if constexpr (std::is_same<T, ff>::value) {
-            // float-float tiles are staged through registers
-            stage<T, NC, TYT, 0, XPairs<T>::v>(tx, S, ipx, i0, j0, (T)0, false, true);
-#if MEPGL_SPLIT_DIR
-            ImagePtrs<T, NC> ipn;
-            image_ptrs<T, NC>(ipn, S.d[f.dout], nullptr, nullptr, off);
-            stage<T, NC, TYT, 0, true>(td, S, ipn, i0, j0, (T)0, false, false);
-#else
-            stage<T, NC, TYT, 2, true, true>(td, S, ipd, i0, j0, (T)sc.beta[img], true, false);
-#endif
-        } else {
-            uint16_t codes[((TYT + 2) * (TX + 2) + NT - 1) / NT];
-            stage_async<T, NC, TYT>(tx, S, ipx.in, i0, j0, codes);
-            if constexpr (DIR_ASYNC) {
-                TileF<T, NC, TYT> &tg = *reinterpret_cast<TileF<T, NC, TYT> *>(g_raw);
-                stage_async<T, NC, TYT>(tg, S, ipd.aux, i0, j0, nullptr);
-                stage_async<T, NC, TYT>(td, S, ipd.in, i0, j0, nullptr);
-                store_codes<T, NC, TYT>(tx, codes);
-                cp_async_wait_all();
-                __syncthreads();
-                // d <- -g + beta d over the halo tile; interior d -> d[dout]
-                using V = vec2_t<T>;
-                constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
-                const T beta = (T)sc.beta[img];
-#pragma unroll
-                for (int k = 0; k < NI; ++k) {
-                    const int e = threadIdx.x + k * NT;
-                    if (e >= HE) continue;
-                    const int hy = e / HW, hx = e - hy * HW;
-                    V v[1 + NC];
-                    {
-                        const V gv = tg.A[hy][hx], dv = td.A[hy][hx];
-                        v[0].x = -gv.x + beta * dv.x;
-                        v[0].y = -gv.y + beta * dv.y;
-                        td.A[hy][hx] = v[0];
-                    }
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const V gv = tg.P[c][hy][hx], dv = td.P[c][hy][hx];
-                        v[1 + c].x = -gv.x + beta * dv.x;
-                        v[1 + c].y = -gv.y + beta * dv.y;
-                        td.P[c][hy][hx] = v[1 + c];
-                    }
-                    const int gi = i0 + hx - 1, gj = j0 + hy - 1;
-                    if (hx >= 1 && hx <= TX && hy >= 1 && hy <= TYT && gi < S.nx && gj < S.ny)
-#pragma unroll
-                        for (int c = 0; c < 1 + NC; ++c) ipd.out[c][gi + S.nx * gj] = v[c];
-                }
-            } else {
-#if MEPGL_SPLIT_DIR
-            const vec2_t<T> *dsrc[1 + NC];
-#pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) dsrc[c] = ipd.out[c];
-            stage_async<T, NC, TYT>(td, S, dsrc, i0, j0, nullptr);
-#else
-            stage<T, NC, TYT, 2, true, true>(td, S, ipd, i0, j0, (T)sc.beta[img], true, false);
-#endif
-            store_codes<T, NC, TYT>(tx, codes);
-            cp_async_wait_all();
-            }
-        }
-        PackParams<T, NC> pp;
-        pp.load(S);
-        __syncthreads();
-        T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
-#pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                Wts<T> w;
-                w.load(tx.m[ly + 1][lx + 1]);
-                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
-                T o[5];
-                site_poly<T, NC>(pack_view_tile(tx, lx + 1, ly + 1), pack_view_tile(td, lx + 1, ly + 1), pp, w,
-                                 S.per_site, f.poly_compat, S.thin_film, o);
-#pragma unroll
-                for (int k = 0; k < 5; ++k) v[k] += o[k];
-            }
-        }
-        const int tpi = S.tiles_x * S.tiles_y;
-        double tot[5];
-        if (finish_image<5>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot)) {
-            if (threadIdx.x == 0) {
-#pragma unroll
-                for (int k = 0; k < 5; ++k) coef[k] = tot[k] * S.ud.dx2;
-                sc.fenergy[img] = coef[0];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = coef[1 + k];
-            }
-            __syncthreads();
-            if (threadIdx.x < 32) {
-                // the scan's grid and rounding follow the stored precision
-                const double *xt = sizeof(store_t<T>) == 8 ? sc.xtab_d : sc.xtab_f;
-                double alpha = line_search_scan<store_t<T>>(coef, xt);
-                if (f.ls_exact) alpha = line_search_exact(coef, alpha);
-                if (threadIdx.x == 0) {
-                    sc.alpha[img] = alpha;
-                    sc.alpha_pend[img] = alpha;
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
 #include "strip.cuh"
-
-// d[dout] = -g + beta d[din] at every site of the launch's tiles (the
-// pointwise half of computeStepDirection, nlcg.cu:955-994, when the
-// direction and polynomial passes are split).
-template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_dir_update(const __grid_constant__ Batch bt,
-                                                   const TileRef *__restrict__ tiles, int n_tiles, Scalars sc,
-                                                   StepFlags f)
-{
-    constexpr int TYT = TileRows<T>::v;
-    using V = vec2_t<T>;
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const T beta = (T)sc.beta[S.img_base + tr.n];
-        const size_t off = (size_t)tr.n * S.nx * S.ny;
-        const int gi = tr.tx * TX + (threadIdx.x & 31);
-        V gv[TYT / 8][1 + NC], dv[TYT / 8][1 + NC];
-#pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int gj = tr.ty * TYT + (threadIdx.x >> 5) + 8 * r;
-            if (gi < S.nx && gj < S.ny)
-#pragma unroll
-                for (int c = 0; c < 1 + NC; ++c) {
-                    const int s = gi + S.nx * gj;
-                    using W = vec2_t<store_t<T>>;
-                    gv[r][c] = loadw<T>(static_cast<const W *>(S.g[f.gcur][c]) + off + s);
-                    dv[r][c] = loadw<T>(static_cast<const W *>(S.d[f.din][c]) + off + s);
-                }
-        }
-#pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int gj = tr.ty * TYT + (threadIdx.x >> 5) + 8 * r;
-            if (gi < S.nx && gj < S.ny)
-#pragma unroll
-                for (int c = 0; c < 1 + NC; ++c) {
-                    V v;
-                    v.x = -gv[r][c].x + beta * dv[r][c].x;
-                    v.y = -gv[r][c].y + beta * dv[r][c].y;
-                    storew<T>(static_cast<vec2_t<store_t<T>> *>(S.d[f.dout][c]) + off + gi + S.nx * gj, v);
-                }
-        }
-    }
-}
 
 template <class T, int NC>
 __global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ Batch bt, const TileRef *__restrict__ tiles,
@@ -763,8 +413,8 @@ __global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ Batch bt,
         const int img = S.img_base + tr.n;
         const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
         ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, (size_t)tr.n * S.nx * S.ny);
-        stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
+        image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
+        stage<T, NC, TYT>(t, S, ip, i0, j0);
         PackParams<T, NC> pp;
         pp.load(S);
         __syncthreads();
@@ -810,8 +460,8 @@ __global__ void __launch_bounds__(NT) k_param_adjoint(const __grid_constant__ Ba
         const int img = S.img_base + tr.n;
         const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
         ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, (size_t)tr.n * S.nx * S.ny);
-        stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
+        image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
+        stage<T, NC, TYT>(t, S, ip, i0, j0);
         SiteParams<T> p;
         p.load_uniform(S);
         __syncthreads();
@@ -861,8 +511,8 @@ __global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ Ba
         const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
         const size_t off = (size_t)tr.n * S.nx * S.ny;
         ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, off);
-        stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
+        image_ptrs<T, NC>(ip, S.x[xbuf], off);
+        stage<T, NC, TYT>(t, S, ip, i0, j0);
         PackParams<T, NC> pp;
         pp.load(S);
         __syncthreads();
@@ -926,8 +576,8 @@ __global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ Batch bt, con
         const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
         const size_t off = (size_t)tr.n * S.nx * S.ny;
         ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], nullptr, nullptr, off);
-        stage<T, NC, TYT, 0>(t, S, ip, i0, j0, (T)0, false, true);
+        image_ptrs<T, NC>(ip, S.x[xbuf], off);
+        stage<T, NC, TYT>(t, S, ip, i0, j0);
         PackParams<T, NC> pp;
         pp.load(S);
         __syncthreads();
@@ -1649,122 +1299,98 @@ inline int grid_for(long n, int cap = 152 * 16)
         }                                                                                           \
     } while (0)
 
-// The NLCG passes also exist in float-float arithmetic (paired FP64 mode).
-#define DISPATCH_NLCG(L, KERNEL, ...)                                                               \
-    do {                                                                                            \
-        if ((L).paired && (L).precision == 1) {                                                     \
-            if ((L).ncomp == 2) KERNEL<ff, 2><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);        \
-            else KERNEL<ff, 1><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);                       \
-        } else {                                                                                    \
-            DISPATCH(L, KERNEL, __VA_ARGS__);                                                       \
-        }                                                                                           \
-    } while (0)
-
-// FP64 and float-float NLCG passes (tile kernels).
-#define DISPATCH_WIDE(L, KERNEL, ...)                                                               \
-    do {                                                                                            \
-        if ((L).paired) {                                                                           \
-            if ((L).ncomp == 2) KERNEL<ff, 2><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);        \
-            else KERNEL<ff, 1><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);                       \
-        } else {                                                                                    \
-            if ((L).ncomp == 2) KERNEL<double, 2><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);    \
-            else KERNEL<double, 1><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);                   \
-        }                                                                                           \
-    } while (0)
-
-// FP32 NLCG passes: one single-warp block per tile; launches of one string
-// take the kernels that read its descriptor at fixed offsets.
-#define DISPATCH_STRIP(L, KERNEL, ...)                                                              \
+// NLCG passes: one single-warp block per strip; launches of one string take
+// the kernels that read its descriptor at fixed offsets.
+#define DISPATCH_STRIP_T(L, KERNEL, T, ...)                                                         \
     do {                                                                                            \
         if (strip_one(L)) {                                                                         \
-            if ((L).ncomp == 2) KERNEL<float, 2, true><<<(L).n_tiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
-            else KERNEL<float, 1, true><<<(L).n_tiles, NTS, 0, (L).stream>>>(__VA_ARGS__);          \
+            if ((L).ncomp == 2) KERNEL<T, 2, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
+            else KERNEL<T, 1, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__);             \
         } else {                                                                                    \
-            if ((L).ncomp == 2) KERNEL<float, 2, false><<<(L).n_tiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
-            else KERNEL<float, 1, false><<<(L).n_tiles, NTS, 0, (L).stream>>>(__VA_ARGS__);         \
+            if ((L).ncomp == 2) KERNEL<T, 2, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
+            else KERNEL<T, 1, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__);            \
         }                                                                                           \
     } while (0)
+#define DISPATCH_STRIP(L, KERNEL, ...)                                                              \
+    do {                                                                                            \
+        if ((L).precision == 0) DISPATCH_STRIP_T(L, KERNEL, float, __VA_ARGS__);                    \
+        else if ((L).paired) DISPATCH_STRIP_T(L, KERNEL, ff, __VA_ARGS__);                          \
+        else DISPATCH_STRIP_T(L, KERNEL, double, __VA_ARGS__);                                      \
+    } while (0)
 
-// Single-string FP32 launch (MEPGL_STRIP_ONE = 0 sends every launch through
-// the indexed-descriptor kernels).
-static inline bool strip_one(const Launch &L) { return MEPGL_STRIP_ONE && L.batch->n == 1; }
+static inline bool strip_one(const Launch &L) { return L.batch->n == 1; }
 
 cudaError_t launch_grad(const Launch &L, const Scalars &sc, const StepFlags &f)
 {
-#if MEPGL_STRIP
-    if (L.precision == 0) DISPATCH_STRIP(L, k_grad_s, *L.batch, L.tile0, sc, f);
-    else DISPATCH_WIDE(L, k_grad, *L.batch, L.tiles, L.n_tiles, sc, f);
-#else
-    DISPATCH_NLCG(L, k_grad, *L.batch, L.tiles, L.n_tiles, sc, f);
-#endif
+    DISPATCH_STRIP(L, k_grad_s, *L.batch, L.stile0, sc, f);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dir_poly(const Launch &L, const Scalars &sc, const StepFlags &f)
 {
-#if MEPGL_SPLIT_DIR
-    {
-        Launch U = L;
-        U.grid = L.n_tiles < 152 * 16 ? L.n_tiles : 152 * 16;
-        DISPATCH_NLCG(U, k_dir_update, *U.batch, U.tiles, U.n_tiles, sc, f);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-#endif
-#if MEPGL_STRIP
-    if (L.precision == 0) DISPATCH_STRIP(L, k_dir_poly_s, *L.batch, L.tile0, sc, f);
-    else DISPATCH_WIDE(L, k_dir_poly, *L.batch, L.tiles, L.n_tiles, sc, f);
-#else
-    DISPATCH_NLCG(L, k_dir_poly, *L.batch, L.tiles, L.n_tiles, sc, f);
-#endif
+    DISPATCH_STRIP(L, k_dir_poly_s, *L.batch, L.stile0, sc, f);
     return cudaGetLastError();
 }
 
-int strip_pass_slots(int ncomp)
+// Resident blocks of one strip kernel on the current device.
+template <class K>
+static int resident(K kernel)
 {
-#if MEPGL_STRIP
+    int dev = 0, sms = 0, nb = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, NTS, 0) != cudaSuccess)
+        return 0;
+    return nb * sms;
+}
+
+template <class T>
+static int pass_slots(int ncomp)
+{
     static int slots[2] = {0, 0};
-    const int ci = ncomp == 2 ? 1 : 0;
+    int &n = slots[ncomp == 2];
+    if (n == 0) n = ncomp == 2 ? resident(k_dir_poly_s<T, 2, false>) : resident(k_dir_poly_s<T, 1, false>);
+    return n;
+}
+
+int strip_pass_slots(int precision, int paired, int ncomp)
+{
+    return precision == 0 ? pass_slots<float>(ncomp) : paired ? pass_slots<ff>(ncomp) : pass_slots<double>(ncomp);
+}
+
+template <class T>
+static cudaError_t nlcg_fused_launch(const Launch &L, const Scalars &sc, const StepPlan &plan, int steps,
+                                     unsigned long long *queue, unsigned *stage, unsigned max_polls)
+{
+    static int slots[4] = {0, 0, 0, 0};
+    const int ci = (L.ncomp == 2 ? 1 : 0) + (strip_one(L) ? 2 : 0);
     if (slots[ci] == 0) {
-        int dev = 0, sms = 0, nb = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return 0;
-        const cudaError_t e = ci ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_dir_poly_s<float, 2, false>, NTS, 0)
-                                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_dir_poly_s<float, 1, false>, NTS, 0);
-        if (e != cudaSuccess) return 0;
-        slots[ci] = nb * sms;
+        slots[ci] = ci == 0   ? resident(k_nlcg_s<T, 1, false>)
+                    : ci == 1 ? resident(k_nlcg_s<T, 2, false>)
+                    : ci == 2 ? resident(k_nlcg_s<T, 1, true>)
+                              : resident(k_nlcg_s<T, 2, true>);
+        if (slots[ci] == 0) {
+            const cudaError_t e = cudaGetLastError();
+            return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
+        }
     }
-    return slots[ci];
-#else
-    (void)ncomp;
-    return 0;
-#endif
+    const long long items = 2LL * L.n_stiles * steps;
+    const int grid = items < slots[ci] ? (int)items : slots[ci];
+#define FUSED_ARGS *L.batch, L.stile0, L.n_stiles, steps, plan, sc, queue, stage, max_polls
+    switch (ci) {
+    case 0: k_nlcg_s<T, 1, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
+    case 1: k_nlcg_s<T, 2, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
+    case 2: k_nlcg_s<T, 1, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
+    default: k_nlcg_s<T, 2, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
+    }
+#undef FUSED_ARGS
+    return cudaGetLastError();
 }
 
 cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlags &f0, int it0, int steps,
                               unsigned long long *queue, unsigned *stage, int n_stage, unsigned long long first_item,
                               unsigned max_polls)
 {
-#if MEPGL_STRIP
-    static int slots[4] = {0, 0, 0, 0};
-    const bool one = strip_one(L);
-    const int ci = (L.ncomp == 2 ? 1 : 0) + (one ? 2 : 0);
-    if (slots[ci] == 0) {
-        int dev = 0, sms = 0, nb = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) {
-            switch (ci) {
-            case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_nlcg_s<float, 1, false>, NTS, 0); break;
-            case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_nlcg_s<float, 2, false>, NTS, 0); break;
-            case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_nlcg_s<float, 1, true>, NTS, 0); break;
-            default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_nlcg_s<float, 2, true>, NTS, 0); break;
-            }
-        }
-        if (e != cudaSuccess) return e;
-        slots[ci] = nb * sms > 0 ? nb * sms : 1;
-    }
     StepPlan plan;
     plan.xi0 = f0.xin;
     plan.di0 = f0.din;
@@ -1775,22 +1401,9 @@ cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlag
     if (e == cudaSuccess && first_item) e = cudaStreamSynchronize(L.stream);   // first_item is a host local
     if (e == cudaSuccess) e = cudaMemsetAsync(stage, 0, sizeof(unsigned) * (size_t)n_stage, L.stream);
     if (e != cudaSuccess) return e;
-    const long long items = 2LL * L.n_tiles * steps;
-    const int grid = items < slots[ci] ? (int)items : slots[ci];
-#define FUSED_ARGS *L.batch, L.tile0, L.n_tiles, steps, plan, sc, queue, stage, max_polls
-    switch (ci) {
-    case 0: k_nlcg_s<float, 1, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    case 1: k_nlcg_s<float, 2, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    case 2: k_nlcg_s<float, 1, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    default: k_nlcg_s<float, 2, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    }
-#undef FUSED_ARGS
-    return cudaGetLastError();
-#else
-    (void)L; (void)sc; (void)f0; (void)it0; (void)steps; (void)queue; (void)stage; (void)n_stage;
-    (void)first_item; (void)max_polls;
-    return cudaErrorNotSupported;
-#endif
+    return L.precision == 0 ? nlcg_fused_launch<float>(L, sc, plan, steps, queue, stage, max_polls)
+           : L.paired       ? nlcg_fused_launch<ff>(L, sc, plan, steps, queue, stage, max_polls)
+                            : nlcg_fused_launch<double>(L, sc, plan, steps, queue, stage, max_polls);
 }
 
 cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *out)
@@ -2015,8 +1628,6 @@ cudaError_t launch_redist_cubic(int precision, const void *f, void *fnew, void *
                                                                F, F_new, p);
     return cudaGetLastError();
 }
-
-bool x_pairs() { return MEPGL_FF_XPAIRS != 0; }
 
 cudaError_t launch_x_format(void *x, long pairs, int to_pairs, cudaStream_t st)
 {

@@ -9,10 +9,6 @@ constexpr int LS_GRID = 2001;         // line-search grid points x_0 .. x_2000
 
 // Rows per lattice tile for a precision (0 float, 1 double); tiles are TX wide.
 int tile_rows(int precision);
-// Kernel launches per NLCG step and launch group (2, or 3 with the split direction pass).
-int nlcg_step_launches();
-// Kernel names of the two NLCG passes for a precision (0 float, 1 double) and arithmetic.
-void nlcg_pass_kernels(int precision, int paired, const char **grad, const char **dir_poly);
 // Copy the neighbour-code weight tables to constant memory (idempotent).
 cudaError_t upload_mask_tables();
 
@@ -22,6 +18,7 @@ struct Launch {
     int tile0;                   // global index of tiles[0] (tiles are in (string, image, row, column) order)
     int n_tiles;
     int grid;                    // blocks launched (grid-stride over tiles)
+    int stile0, n_stiles;        // the same for the warp strips of the NLCG passes
     int precision;               // 0 float, 1 double
     int paired;                  // 1: NLCG passes in float-float arithmetic on double fields
     int ncomp;                   // 1 or 2 (uniform over the strings of a context)
@@ -36,12 +33,14 @@ struct StepFlags {
     int poly_compat, ls_exact;
 };
 
-// True when this build has fused FP32 NLCG steps (one persistent launch per call).
-bool nlcg_fused(int precision);
-// Fused steps are used for batches of at most fuse_waves() x strip_pass_slots()
-// tiles: resident blocks of the FP32 pass kernels on the current device.
-int fuse_waves();
-int strip_pass_slots(int ncomp);
+// Rows per warp strip of an image column of ny rows, in a batch of `tiles`
+// strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
+int strip_rows_cap(int precision);
+int strip_rows(int precision, int ny, long tiles, int slots);
+// Steps are fused for batches of at most fuse_waves() x strip_pass_slots()
+// strips; strip_pass_slots(): resident warps of the pass kernels on the GPU.
+int fuse_waves(int precision);
+int strip_pass_slots(int precision, int paired, int ncomp);
 // `steps` NLCG steps (iterations it0, it0 + 1, ...; step 0 with the buffers
 // of f0) of the launch's tiles in one persistent launch; queue (one counter)
 // and stage (one per global image, n_stage) are reset on the stream first.
@@ -58,9 +57,8 @@ cudaError_t launch_grad(const Launch &L, const Scalars &sc, const StepFlags &f);
 // tile of each image runs the line search and sets alpha, alpha_pend.
 cudaError_t launch_dir_poly(const Launch &L, const Scalars &sc, const StepFlags &f);
 // x[xbuf] += alpha_pend d[dbuf]; alpha_pend = 0.
-// Paired FP64: whether the NLCG passes keep x as float-float pairs, and the
-// in-place conversion of `pairs` complex values of x to (1) or from (0) them.
-bool x_pairs();
+// Paired FP64: the NLCG passes keep x as float-float pairs; the in-place
+// conversion of `pairs` complex values of x to (1) or from (0) them.
 cudaError_t launch_x_format(void *x, long pairs, int to_pairs, cudaStream_t st);
 cudaError_t launch_apply_update(const Launch &L, const Scalars &sc, const StringDesc *host_strings, int n_strings,
                                 int xbuf, int dbuf);

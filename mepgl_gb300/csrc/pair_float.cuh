@@ -31,7 +31,7 @@ struct ff {
     __host__ __device__ explicit operator double() const { return (double)hi + (double)lo; }
 };
 
-struct ff2 {
+struct __align__(16) ff2 {   // one 16-byte access
     ff x, y;
 };
 
@@ -98,6 +98,18 @@ __device__ __forceinline__ double shfl_down(double v, int o) { return __shfl_dow
 __device__ __forceinline__ ff shfl_down(ff v, int o)
 {
     return ff(__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o));
+}
+
+// lane to the right (+1) / left (-1) of any lattice number type
+template <class T> __device__ __forceinline__ T shfl_right(T v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+template <class T> __device__ __forceinline__ T shfl_left(T v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+template <> __device__ __forceinline__ ff shfl_right<ff>(ff v)
+{
+    return ff(__shfl_down_sync(0xffffffffu, v.hi, 1), __shfl_down_sync(0xffffffffu, v.lo, 1));
+}
+template <> __device__ __forceinline__ ff shfl_left<ff>(ff v)
+{
+    return ff(__shfl_up_sync(0xffffffffu, v.hi, 1), __shfl_up_sync(0xffffffffu, v.lo, 1));
 }
 
 // ------------------------------------------------ packed pairs of float-floats

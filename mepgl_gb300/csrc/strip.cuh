@@ -1,21 +1,27 @@
-// strip.cuh -- the two NLCG passes as warp strips (FP32 fields), launched
-// as two pass kernels per step or as one fused persistent launch per call
-// (end of file).  Included by kernels.cu inside its anonymous namespace,
-// after the tile kernels, whose helpers (part_slot, h_site, line search) it
-// uses.
+// strip.cuh -- the two NLCG passes as warp strips, for float, double and
+// float-float fields, launched as two pass kernels per step or as one fused
+// persistent launch per call (end of file).  Included by kernels.cu inside
+// its anonymous namespace.
 //
-// A block is one warp.  In the pass kernels it owns one tile of the usual
-// tiling (TX = 32 columns x TYT rows of one image); in the fused kernel it
-// takes tiles from a work queue.  Everything that depends on the tile
-// (pointers, parameters, row numbers) is uniform over the block.  Lane l holds column i0 + l and walks down the
-// tile's rows with a three-row window of its column in registers; the
-// x-neighbours come from the adjacent lanes by shuffles.  Lanes 0 and 31
-// copy the halo column next to them (i0 - 1, i0 + 32) into a three-row ring
-// in shared memory with cp.async and read it back themselves, so no lane
-// waits for another.  Rows j0 - 1 and j0 + TYT are read as halo rows.
-// While a row is computed, the loads of the next row are in flight.  Every
-// tile leaves one partial per quantity in the slot the tile kernels use,
-// and the last tile of an image (atomic ticket) finishes it.
+// A block is one warp.  In the pass kernels it owns one strip (TX = 32
+// columns x S.rows rows of one image); in the fused kernel it takes strips
+// from a work queue.  Everything that depends on the strip (pointers,
+// parameters, row numbers) is uniform over the block.  Lane l holds column
+// i0 + l and walks down the strip's rows with a three-row window of its
+// column in registers; the x-neighbours come from the adjacent lanes by
+// shuffles.  Lanes 0 and 31 copy the halo column next to them (i0 - 1, i0 +
+// 32) into a three-row ring in shared memory with cp.async and read it back
+// themselves, so no lane waits for another.  Rows j0 - 1 and j0 + S.rows are
+// read as halo rows.  While a row is computed, the loads of the next row are
+// in flight.  Every strip leaves one partial per quantity, and the last strip
+// of an image (atomic ticket) finishes it.
+//
+// FP64: bound by the FP64 pipe, 64 clocks per warp instruction and SM
+// quarter, so 8 warps per SM (255 registers, no spills) keep it busy and the
+// strips' equal sharing of the quarters counts.  256 x 256 x 64, two
+// components, per step: 4.48 ms, 4.66 as shared-memory tiles of 256 threads
+// and two launches; 64 x 64 x 16, ten steps with reparametrization: 744 us
+// against 1070.  Float-float: 1.53 ms per step against 1.68.
 #pragma once
 
 constexpr int NTS = 32;   // threads per block of the strip kernels
@@ -75,8 +81,8 @@ __device__ __forceinline__ PackView<T, NC> pack_view(const RegView<T, NC> &r)
                 v.px[y][x] = r.p[0][y][x].x;
                 v.py[y][x] = r.p[0][y][x].y;
             } else {
-                v.px[y][x] = r.p[0][y][x];
-                v.py[y][x] = r.p[1][y][x];
+                v.px[y][x] = Pk<T, NC>::mk(r.p[0][y][x].x, r.p[0][y][x].y);
+                v.py[y][x] = Pk<T, NC>::mk(r.p[1][y][x].x, r.p[1][y][x].y);
             }
         }
     return v;
@@ -95,8 +101,8 @@ template <class T>
 __device__ __forceinline__ vec2_t<T> from_right(vec2_t<T> v, vec2_t<T> halo, int lane)
 {
     vec2_t<T> r;
-    r.x = __shfl_down_sync(FULL_MASK, v.x, 1);
-    r.y = __shfl_down_sync(FULL_MASK, v.y, 1);
+    r.x = shfl_right(v.x);
+    r.y = shfl_right(v.y);
     return lane == TX - 1 ? halo : r;
 }
 
@@ -104,7 +110,7 @@ __device__ __forceinline__ vec2_t<T> from_right(vec2_t<T> v, vec2_t<T> halo, int
 template <class T>
 __device__ __forceinline__ T from_left(T v, T halo, int lane)
 {
-    const T l = __shfl_up_sync(FULL_MASK, v, 1);
+    const T l = shfl_left(v);
     return lane == 0 ? halo : l;
 }
 
@@ -178,8 +184,8 @@ __device__ __forceinline__ void strip_halo(vec2_t<T> (&slot)[2][NR][1 + NC], con
 template <int N>
 __device__ __forceinline__ void cp_async_wait_groups() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Tile g of the global tile order (strings in order, each from its
-// tile_base: image, tile row, tile column), derived from the block index and
+// Strip g of the global strip order (strings in order, each from its
+// stile_base: image, strip row, column), derived from the block index and
 // the descriptors alone so that it is uniform over the block.
 // ONE: the launch covers a single string (bt.n == 1); its descriptor is
 // then read at fixed offsets, i.e. as constant operands, not through
@@ -190,18 +196,29 @@ __device__ __forceinline__ TileRef strip_tile(const Batch &bt, int g)
     int s = 0;
     if (!ONE)
         for (int k = 1; k < bt.n; ++k)
-            if (g >= bt.s[k].tile_base) s = k;
-    TileRef t = flat_tile(bt.s[s], g - bt.s[s].tile_base);
+            if (g >= bt.s[k].stile_base) s = k;
+    const StringDesc &S = bt.s[s];
+    const int r = g - S.stile_base, tpi = S.tiles_x * S.stiles_y, n = r / tpi, u = r - n * tpi, ty = u / S.tiles_x;
+    TileRef t;
     t.s = (int16_t)s;
+    t.ty = (int16_t)ty;
+    t.tx = (int16_t)(u - ty * S.tiles_x);
+    t.pad = 0;
+    t.n = n;
     return t;
+}
+
+// Slot of a strip's partial sums.
+__device__ __forceinline__ int strip_slot(const StringDesc &S, const TileRef &tr)
+{
+    return S.stile_base + (tr.n * S.stiles_y + tr.ty) * S.tiles_x + tr.tx;
 }
 
 // Packed neighbour codes of the lane's site in row j (0 outside the lattice).
 __device__ __forceinline__ uint16_t strip_code(const StringDesc &S, const StripLane &L, int j)
 {
     if (!(j >= 0 && j < S.ny && L.cok)) return 0;
-    const int s = L.gi + S.nx * j;
-    return S.mask ? S.mask[s] : (uint16_t)((S.code_comp[s] & 0xff) | ((S.code_sc[s] & 0xff) << 8));
+    return S.mask[L.gi + S.nx * j];
 }
 
 // Warp form of finish_image: the tile's NV partials leave from lane 0; if
@@ -260,21 +277,20 @@ struct GradRow {
 template <class T, int NC>
 using GradRing = vec2_t<T>[3][2][2][1 + NC];
 
-// Pass A on one tile as a warp strip: x <- x + alpha_pend d over the tile
-// (+ halo), the gradient of every site, |g|^2 and g . (g - g_prev); the last
-// tile of an image computes beta.  Same semantics as k_grad.  Returns true
-// (in every lane) when this tile finished its image.  Before the tile's
-// partials are counted every lane fences its field stores, so that a
-// consumer that has seen the image finished (same launch) reads them.
+// Gradient pass on one strip: x <- x + alpha_pend d over the strip (+ halo),
+// the gradient of every site, |g|^2 and g . (g - g_prev); the last strip of an
+// image computes beta.  Returns true (in every lane) when this strip finished
+// its image.  Before the strip's partials are counted every lane fences its
+// field stores, so that a consumer that has seen the image finished (same
+// launch) reads them.
 template <class T, int NC, bool ONE>
 __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
 {
-    constexpr int TYT = TileRows<T>::v;
     using V = vec2_t<T>;
     const StringDesc &S = bt.s[ONE ? 0 : tr.s];
     const int img = S.img_base + tr.n;
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    const int i0 = tr.tx * TX, j0 = tr.ty * S.rows;
     const size_t off = (size_t)tr.n * S.nx * S.ny;
     const StripLane L = strip_lane(S, i0);
     const V *src[3][1 + NC];
@@ -333,7 +349,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
         take(Rm, j0 - 1, hp0, ra, ma);
         take(R0, j0, hp0, rb, mb);
     }
-    const int rows = S.ny - j0 < TYT ? S.ny - j0 : TYT;
+    const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
     T v[2] = {(T)0, (T)0};
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
@@ -384,11 +400,11 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
 #pragma unroll
         for (int c = 0; c < NC; ++c) hp0[c] = hp1[c];
     }
-    const int tpi = S.tiles_x * S.tiles_y;
+    const int tpi = S.tiles_x * S.stiles_y;
     double tot[2];
     __threadfence();
     __syncwarp();
-    const bool fin = finish_image_warp<2>(v, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot);
+    const bool fin = finish_image_warp<2>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
     if (fin && L.lane == 0) {
         (f.gcur ? sc.gn1 : sc.gn0)[img] = tot[0];
         sc.gdg[img] = tot[1];
@@ -403,7 +419,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, MEPGL_MINB_STRIP_GRAD) k_grad_s(const __grid_constant__ Batch bt,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::grad) k_grad_s(const __grid_constant__ Batch bt,
                                                                   int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) GradRing<T, NC> ring;
@@ -422,20 +438,18 @@ struct DirRow {
 template <class T, int NC>
 using DirRing = vec2_t<T>[3][2][3][1 + NC];
 
-// Pass B on one tile as a warp strip: d <- -g + beta d over the tile
-// (+ halo), the quartic coefficients of F(x + a d); the last tile of an
-// image runs the line search.  Same semantics as k_dir_poly.  Returns true
-// (in every lane) when this tile finished its image; field stores are
-// fenced as in grad_tile.
+// Direction pass on one strip: d <- -g + beta d over the strip (+ halo), the
+// quartic coefficients of F(x + a d); the last strip of an image runs the line
+// search.  Returns true (in every lane) when this strip finished its image;
+// field stores are fenced as in grad_tile.
 template <class T, int NC, bool ONE>
 __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
                                          DirRing<T, NC> &ring, double (&coef)[5])
 {
-    constexpr int TYT = TileRows<T>::v;
     using V = vec2_t<T>;
     const StringDesc &S = bt.s[ONE ? 0 : tr.s];
     const int img = S.img_base + tr.n;
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    const int i0 = tr.tx * TX, j0 = tr.ty * S.rows;
     const size_t off = (size_t)tr.n * S.nx * S.ny;
     const StripLane L = strip_lane(S, i0);
     const V *src[3][1 + NC];
@@ -483,7 +497,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
         dm_ax = R0.d[0].x;
         take(R0, rb, mb);
     }
-    const int rows = S.ny - j0 < TYT ? S.ny - j0 : TYT;
+    const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
     T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
@@ -553,11 +567,11 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
     // the halo copy of the row below the tile may still be in flight: complete it before the
     // ring can be reused (the fused kernel runs more tiles in the same block)
     cp_async_wait_groups<0>();
-    const int tpi = S.tiles_x * S.tiles_y;
+    const int tpi = S.tiles_x * S.stiles_y;
     double tot[5];
     __threadfence();
     __syncwarp();
-    const bool fin = finish_image_warp<5>(v, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot);
+    const bool fin = finish_image_warp<5>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
     if (fin) {
         if (L.lane == 0) {
 #pragma unroll
@@ -567,10 +581,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
             for (int k = 0; k < 4; ++k) sc.poly[4 * img + k] = coef[1 + k];
         }
         __syncwarp();
-        // the scan's grid and rounding follow the stored precision
-        const double *xt = sizeof(store_t<T>) == 8 ? sc.xtab_d : sc.xtab_f;
-        double alpha = line_search_scan<store_t<T>>(coef, xt);
-        if (f.ls_exact) alpha = line_search_exact(coef, alpha);
+        const double alpha = line_search<store_t<T>>(coef, sc, f.ls_exact);
         if (L.lane == 0) {
             sc.alpha[img] = alpha;
             sc.alpha_pend[img] = alpha;
@@ -581,7 +592,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, MEPGL_MINB_STRIP_DIR) k_dir_poly_s(const __grid_constant__ Batch bt,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::dir) k_dir_poly_s(const __grid_constant__ Batch bt,
                                                                       int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) DirRing<T, NC> ring;
@@ -654,16 +665,8 @@ __device__ __forceinline__ void publish_stage(unsigned *stage, unsigned value)
     __syncwarp();
 }
 
-// Register budget of the fused kernel: an explicit cap, or the one
-// resident-block target implies.
-#if MEPGL_MAXREG_FUSED
-#define MEPGL_FUSED_BOUNDS __maxnreg__(MEPGL_MAXREG_FUSED)
-#else
-#define MEPGL_FUSED_BOUNDS __launch_bounds__(NTS, MEPGL_MINB_STRIP_FUSED)
-#endif
-
 template <class T, int NC, bool ONE>
-__global__ void MEPGL_FUSED_BOUNDS k_nlcg_s(const __grid_constant__ Batch bt, int tile0, int n_tiles, int steps,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __grid_constant__ Batch bt, int tile0, int n_tiles, int steps,
                                             StepPlan plan, Scalars sc, unsigned long long *queue, unsigned *stage,
                                             unsigned max_polls)
 {
