@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <tuple>
@@ -27,8 +28,6 @@ thread_local std::string g_create_error;
 }  // namespace
 
 namespace {
-
-const double INF = INFINITY;
 
 mepgl_status fail(mepgl_ctx *c, mepgl_status st, const std::string &msg)
 {
@@ -129,7 +128,7 @@ mepgl_status upload_string_params(mepgl_ctx *c, StringHost &s)
     return MEPGL_OK;
 }
 
-void fill_desc(mepgl_ctx *c, int si, int img_base, int tile_base)
+void fill_desc(mepgl_ctx *c, int si, int img_base)
 {
     StringHost &s = c->strings[si];
     StringDesc &D = c->hdesc[si];
@@ -141,7 +140,6 @@ void fill_desc(mepgl_ctx *c, int si, int img_base, int tile_base)
     D.tiles_x = (s.nx + TX - 1) / TX;
     D.tiles_y = (s.ny + tile_rows(c->precision) - 1) / tile_rows(c->precision);
     D.img_base = img_base;
-    D.tile_base = tile_base;
     D.thin_film = c->thin_film;
     D.per_site = s.uniform ? 0 : 1;
     // uniform parameters, formed in double and rounded once per precision
@@ -184,15 +182,14 @@ void fill_desc(mepgl_ctx *c, int si, int img_base, int tile_base)
 void free_scalars(mepgl_ctx *c)
 {
     Scalars &S = c->sc;
-    cudaFree(S.gn0); cudaFree(S.gn1); cudaFree(S.gdg); cudaFree(S.beta); cudaFree(S.alpha);
-    cudaFree(S.alpha_pend); cudaFree(S.fenergy); cudaFree(S.poly); cudaFree(S.part); cudaFree(S.ticket);
-    cudaFree(S.xtab_f); cudaFree(S.xtab_d); cudaFree(S.status);
     memset(&S, 0, sizeof(S));
-    cudaFree(c->fqueue); c->fqueue = nullptr;
-    cudaFree(c->fstage); c->fstage = nullptr;
-    cudaFree(c->dscratch); c->dscratch = nullptr;
-    cudaFree(c->ds); cudaFree(c->ds_jb); c->ds = c->ds_jb = nullptr;
-    cudaFree(c->dtiles); c->dtiles = nullptr;
+    cudaFree(c->slab);
+    c->slab = c->dscratch = c->ds = c->ds_jb = nullptr;
+    c->fqueue = nullptr;
+    c->fstage = nullptr;
+    cudaFreeHost(c->mail);
+    c->mail = nullptr;
+    c->mail_cap = 0;
 }
 
 void drop_graphs(mepgl_ctx *c)
@@ -204,19 +201,19 @@ void drop_graphs(mepgl_ctx *c)
 // Strips of the NLCG passes: rows per strip by launch batch, global strip order.
 int layout_strips(mepgl_ctx *c)
 {
-    const int slots = strip_pass_slots(c->precision, c->opt.fp64_arith == MEPGL_FP64_PAIRED, c->ncomp);
+    const int paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED;
+    const int slots = strip_pass_slots(c->precision, paired, c->ncomp), cap = strip_rows_cap(c->precision, paired);
     int base = 0;
     c->batch_stile0.clear();
     c->batch_nstiles.clear();
     size_t si = 0;
     for (Batch &B : c->batches) {
-        long most = 0;
-        for (int k = 0; k < B.n; ++k)
-            most += (long)B.s[k].F * B.s[k].tiles_x * ((B.s[k].ny + strip_rows_cap(c->precision) - 1) / strip_rows_cap(c->precision));
+        long most = 0;   // strips of the most rows
+        for (int k = 0; k < B.n; ++k) most += (long)B.s[k].F * B.s[k].tiles_x * ((B.s[k].ny + cap - 1) / cap);
         c->batch_stile0.push_back(base);
         for (int k = 0; k < B.n; ++k, ++si) {
             StringDesc &D = B.s[k];
-            D.rows = strip_rows(c->precision, D.ny, most, slots);
+            D.rows = strip_rows(c->precision, paired, D.ny, most, slots);
             D.stiles_y = (D.ny + D.rows - 1) / D.rows;
             D.stile_base = base;
             base += D.F * D.tiles_x * D.stiles_y;
@@ -233,118 +230,99 @@ mepgl_status build_layout(mepgl_ctx *c)
     drop_graphs(c);
     free_scalars(c);
     c->hdesc.assign(c->strings.size(), StringDesc{});
-    std::vector<TileRef> tiles;
-    int img = 0;
-    c->string_tile0.clear();
-    c->string_ntiles.clear();
+    int img = 0, most_tiles = 0;
     c->batches.clear();
-    c->batch_tile0.clear();
-    c->batch_ntiles.clear();
     c->string_batch.clear();
     for (size_t si = 0; si < c->strings.size(); ++si) {
         const int in_batch = (int)(si % MAX_STRINGS);
         if (in_batch == 0) {
             c->batches.emplace_back();
             memset(&c->batches.back(), 0, sizeof(Batch));
-            c->batch_tile0.push_back((int)tiles.size());
         }
-        fill_desc(c, (int)si, img, (int)tiles.size());
+        fill_desc(c, (int)si, img);
         const StringDesc &D = c->hdesc[si];
         Batch &B = c->batches.back();
         B.s[in_batch] = D;
         B.n = in_batch + 1;
         c->string_batch.push_back((int)c->batches.size() - 1);
-        c->string_tile0.push_back((int)tiles.size());
-        for (int n = 0; n < D.F; ++n)
-            for (int ty = 0; ty < D.tiles_y; ++ty)
-                for (int tx = 0; tx < D.tiles_x; ++tx)
-                    tiles.push_back(TileRef{(int16_t)in_batch, (int16_t)ty, (int16_t)tx, 0, n});
-        c->string_ntiles.push_back((int)tiles.size() - c->string_tile0.back());
+        const int tiles = D.F * D.tiles_x * D.tiles_y;
+        most_tiles = most_tiles > tiles ? most_tiles : tiles;
         img += D.F;
     }
-    for (size_t b = 0; b < c->batches.size(); ++b)
-        c->batch_ntiles.push_back((b + 1 < c->batches.size() ? c->batch_tile0[b + 1] : (int)tiles.size()) -
-                                  c->batch_tile0[b]);
-    c->n_tiles = (int)tiles.size();
     c->total_images = img;
     const int n_stiles = layout_strips(c);
-    CK(c, cudaMalloc(&c->dtiles, sizeof(TileRef) * tiles.size()));
-    CK(c, cudaMemcpy(c->dtiles, tiles.data(), sizeof(TileRef) * tiles.size(), cudaMemcpyHostToDevice));
     Scalars &S = c->sc;
     const size_t I = (size_t)img;
-    for (double **p : {&S.gn0, &S.gn1, &S.gdg, &S.beta, &S.alpha, &S.alpha_pend, &S.fenergy})
-        CK(c, cudaMalloc(p, I * sizeof(double)));
-    CK(c, cudaMalloc(&S.poly, 4 * I * sizeof(double)));
-    CK(c, cudaMalloc(&S.part, (size_t)(c->n_tiles > n_stiles ? c->n_tiles : n_stiles) * 8 * sizeof(double) +
-                                  4096 * sizeof(double)));
-    CK(c, cudaMalloc(&S.ticket, I * sizeof(unsigned)));
-    CK(c, cudaMemset(S.ticket, 0, I * sizeof(unsigned)));
-    CK(c, cudaMalloc(&S.status, 16 * sizeof(int)));
-    CK(c, cudaMemset(S.status, 0, 16 * sizeof(int)));
-    CK(c, cudaMalloc(&c->fqueue, sizeof(unsigned long long)));
-    CK(c, cudaMalloc(&c->fstage, I * sizeof(unsigned)));
+    int fmax = 0;
+    for (auto &s : c->strings) fmax = fmax > s.F ? fmax : s.F;
+    // one allocation: the line-search grids, then what starts at zero, then the partial sums
+    const size_t n_part = (size_t)(most_tiles > n_stiles ? most_tiles : n_stiles) * 8 + 4096;
+    size_t at = 0;
+    auto take = [&](size_t doubles) {
+        const size_t o = at;
+        at += (doubles + 31) & ~(size_t)31;
+        return o;
+    };
+    const size_t o_xf = take(LS_GRID), o_xd = take(LS_GRID), tables = at;
+    size_t o_img[7];
+    for (size_t &o : o_img) o = take(I);
+    const size_t o_poly = take(4 * I), o_scr = take(3 * I + 64), o_ds = take(fmax + 1), o_jb = take(fmax + 1),
+                 o_tick = take((I + 1) / 2), o_stage = take((I + 1) / 2), o_queue = take(1), o_status = take(8), zeroed = at,
+                 o_part = take(n_part);
+    CK(c, cudaMalloc(&c->slab, at * sizeof(double)));
+    double **dst[7] = {&S.gn0, &S.gn1, &S.gdg, &S.beta, &S.alpha, &S.alpha_pend, &S.fenergy};
+    for (int k = 0; k < 7; ++k) *dst[k] = c->slab + o_img[k];
+    S.poly = c->slab + o_poly;
+    S.part = c->slab + o_part;
+    S.ticket = (unsigned *)(c->slab + o_tick);
+    S.status = (int *)(c->slab + o_status);
+    S.xtab_f = c->slab + o_xf;
+    S.xtab_d = c->slab + o_xd;
+    c->dscratch = c->slab + o_scr;
+    c->ds = c->slab + o_ds;
+    c->ds_jb = c->slab + o_jb;
+    c->fqueue = (unsigned long long *)(c->slab + o_queue);
+    c->fstage = (unsigned *)(c->slab + o_stage);
     // line-search grid x_p = x_0 * m^p rounded to float / double at every step
-    std::vector<double> xf(LS_GRID), xd(LS_GRID);
+    std::vector<double> grid(tables, 0.0);
     float fx = 1e-10f;
     const float fm = 1.025f;
     double dxx = 1e-10;
     const double dm = (double)1.025f;
     for (int p = 0; p < LS_GRID; ++p) {
-        xf[p] = fx;
-        xd[p] = dxx;
+        grid[o_xf + p] = fx;
+        grid[o_xd + p] = dxx;
         fx = fx * fm;
         dxx = dxx * dm;
     }
-    CK(c, cudaMalloc(&S.xtab_f, LS_GRID * sizeof(double)));
-    CK(c, cudaMalloc(&S.xtab_d, LS_GRID * sizeof(double)));
-    CK(c, cudaMemcpy(S.xtab_f, xf.data(), LS_GRID * sizeof(double), cudaMemcpyHostToDevice));
-    CK(c, cudaMemcpy(S.xtab_d, xd.data(), LS_GRID * sizeof(double), cudaMemcpyHostToDevice));
-    CK(c, cudaMalloc(&c->dscratch, (3 * I + 64) * sizeof(double)));
-    int fmax = 0;
-    for (auto &s : c->strings) fmax = fmax > s.F ? fmax : s.F;
-    CK(c, cudaMalloc(&c->ds, (fmax + 1) * sizeof(double)));
-    CK(c, cudaMalloc(&c->ds_jb, (fmax + 1) * sizeof(double)));
-    CK(c, cudaMemset(c->ds, 0, (fmax + 1) * sizeof(double)));
-    CK(c, cudaMemset(c->ds_jb, 0, (fmax + 1) * sizeof(double)));
+    CK(c, cudaMemset(c->slab + tables, 0, (zeroed - tables) * sizeof(double)));
+    CK(c, cudaMemcpy(c->slab, grid.data(), tables * sizeof(double), cudaMemcpyHostToDevice));   // waits for the zeros too
+    c->mail_cap = 3 * I;
+    CK(c, cudaMallocHost(&c->mail, (c->mail_cap + 8) * sizeof(double)));
     c->host_s.assign(fmax, 0.0);
     c->host_sjb.assign(fmax, 0.0);
     return MEPGL_OK;
 }
 
-// Restart NLCG history: zero g and d, |g|^2 = inf, nothing pending.
+// Restart the NLCG history: |g|^2 = inf, nothing pending.  The gradients and
+// directions are left as they are: no pass reads them before it has written
+// them (beta is 0 after a restart).
 mepgl_status reset_history(mepgl_ctx *c)
 {
-    for (auto &s : c->strings) {
-        const size_t bytes = (size_t)s.F * s.M() * 2 * real_size(c->precision);
-        for (int b = 0; b < 2; ++b)
-            for (int f = 0; f < 1 + c->ncomp; ++f) {
-                CK(c, cudaMemsetAsync(s.g[b][f], 0, bytes, c->stream));
-                CK(c, cudaMemsetAsync(s.d[b][f], 0, bytes, c->stream));
-            }
-    }
-    std::vector<double> inf(c->total_images, INF);
-    CK(c, cudaMemcpyAsync(c->sc.gn0, inf.data(), inf.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaMemcpyAsync(c->sc.gn1, inf.data(), inf.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    for (double *p : {c->sc.alpha, c->sc.alpha_pend, c->sc.fenergy, c->sc.beta, c->sc.gdg})
-        CK(c, cudaMemsetAsync(p, 0, c->total_images * 8, c->stream));
-    CK(c, cudaMemsetAsync(c->sc.poly, 0, c->total_images * 32, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
+    CK(c, launch_reset_history(c->sc, c->total_images, c->stream));
     c->pending = false;
     return MEPGL_OK;
 }
 
-// Launch covering a whole batch of strings, or (si >= 0) the tiles of one string.
-Launch make_launch(mepgl_ctx *c, int batch, int si = -1)
+// Launch of the NLCG passes over a whole batch of strings.
+Launch make_launch(mepgl_ctx *c, int batch)
 {
     Launch L;
     L.batch = &c->batches[batch];
-    const int t0 = si >= 0 ? c->string_tile0[si] : c->batch_tile0[batch];
-    L.tiles = c->dtiles + t0;
-    L.tile0 = t0;
-    L.n_tiles = si >= 0 ? c->string_ntiles[si] : c->batch_ntiles[batch];
-    L.grid = L.n_tiles;
-    L.stile0 = c->batch_stile0[batch];      // the NLCG passes cover whole batches
+    L.stile0 = c->batch_stile0[batch];
     L.n_stiles = c->batch_nstiles[batch];
+    L.str = &L.batch->s[0];
+    L.n_tiles = 0;
     L.precision = c->precision;
     L.paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED ? 1 : 0;
     L.ncomp = c->ncomp;
@@ -352,13 +330,22 @@ Launch make_launch(mepgl_ctx *c, int batch, int si = -1)
     return L;
 }
 
-Launch string_launch(mepgl_ctx *c, int si) { return make_launch(c, c->string_batch[si], si); }
+// Launch of the tile kernels over one string.
+Launch string_launch(mepgl_ctx *c, int si)
+{
+    Launch L = make_launch(c, c->string_batch[si]);
+    L.str = &c->hdesc[si];
+    L.n_tiles = L.str->F * L.str->tiles_x * L.str->tiles_y;
+    return L;
+}
 
 mepgl_status flush(mepgl_ctx *c)
 {
     if (!c->pending) return MEPGL_OK;
-    CK(c, launch_apply_update(make_launch(c, 0), c->sc, c->hdesc.data(), (int)c->hdesc.size(), c->xi, c->di));
-    c->launches += (int64_t)c->strings.size() * (1 + c->ncomp);
+    for (size_t b = 0; b < c->batches.size(); ++b)
+        CK(c, launch_apply_update(make_launch(c, (int)b), c->sc, c->xi, c->di));
+    CK(c, cudaMemsetAsync(c->sc.alpha_pend, 0, sizeof(double) * c->total_images, c->stream));
+    c->launches += (int64_t)c->batches.size();
     c->pending = false;
     return MEPGL_OK;
 }
@@ -520,11 +507,49 @@ mepgl_status nlcg_steps_body(mepgl_ctx *c, int iters, int use_cg, int maxwell)
 // per-image scalars after NLCG steps, a string of zero or non-finite arc
 // length.  Read on the stream after the work before it, then cleared; the
 // first raised flag is reported.
+int *mail_status(mepgl_ctx *c) { return reinterpret_cast<int *>(c->mail + c->mail_cap); }
+
+mepgl_status report_device_status(mepgl_ctx *c);
+
 mepgl_status check_device_status(mepgl_ctx *c)
 {
-    int st[4] = {0, 0, 0, 0};
-    CK(c, cudaMemcpyAsync(st, c->sc.status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemcpyAsync(mail_status(c), c->sc.status, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
+    return report_device_status(c);
+}
+
+// Device doubles to the caller's arrays (NULL: skipped) through the pinned
+// buffer, with one wait for all of them and (check) the status flags.
+struct Fetch {
+    double *dst;
+    const double *src;
+    size_t n;
+};
+
+mepgl_status fetch(mepgl_ctx *c, std::initializer_list<Fetch> items, bool check)
+{
+    size_t at = 0;
+    for (const Fetch &f : items) {
+        if (!f.dst) continue;
+        CK(c, cudaMemcpyAsync(c->mail + at, f.src, f.n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        at += f.n;
+    }
+    if (check) CK(c, cudaMemcpyAsync(mail_status(c), c->sc.status, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    at = 0;
+    for (const Fetch &f : items) {
+        if (!f.dst) continue;
+        memcpy(f.dst, c->mail + at, f.n * sizeof(double));
+        at += f.n;
+    }
+    return check ? report_device_status(c) : MEPGL_OK;
+}
+
+// The flags that the last copy brought; raised ones are cleared on the device.
+mepgl_status report_device_status(mepgl_ctx *c)
+{
+    int st[4];
+    memcpy(st, mail_status(c), sizeof(st));
     if (!(st[STATUS_WAIT] | st[STATUS_NONFINITE] | st[STATUS_ARC])) return MEPGL_OK;
     CK(c, cudaMemsetAsync(c->sc.status, 0, sizeof(st), c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
@@ -543,7 +568,9 @@ mepgl_status check_device_status(mepgl_ctx *c)
                 "it was taken as uniform, so a linear resample kept the images");
 }
 
-mepgl_status copy_fields(mepgl_ctx *c, StringHost &s, void *const *dst, const void *const *src, int memory, bool in)
+// wait: until the copies are done
+mepgl_status copy_fields(mepgl_ctx *c, StringHost &s, void *const *dst, const void *const *src, int memory, bool in,
+                         bool wait = true)
 {
     const size_t bytes = (size_t)s.F * s.M() * 2 * real_size(c->precision);
     const cudaMemcpyKind k = memory == MEPGL_DEVICE ? cudaMemcpyDeviceToDevice
@@ -553,7 +580,7 @@ mepgl_status copy_fields(mepgl_ctx *c, StringHost &s, void *const *dst, const vo
         if (!(in ? src[f] : dst[f])) continue;
         CK(c, cudaMemcpyAsync(dst[f], src[f], bytes, k, c->stream));
     }
-    CK(c, cudaStreamSynchronize(c->stream));
+    if (wait) CK(c, cudaStreamSynchronize(c->stream));
     return MEPGL_OK;
 }
 
@@ -722,10 +749,7 @@ mepgl_status reset_cg(mepgl_ctx *c, int first, int last)
     if (first < 0 || last > c->total_images || first > last)
         return fail(c, MEPGL_ERR_INVALID_ARG, "reset_cg: image range out of bounds");
     if (first == last) return MEPGL_OK;
-    std::vector<double> inf(last - first, INF);
-    CK(c, cudaMemcpyAsync(c->sc.gn0 + first, inf.data(), inf.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaMemcpyAsync(c->sc.gn1 + first, inf.data(), inf.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
+    CK(c, launch_restart_cg(c->sc, first, last, c->stream));
     return MEPGL_OK;
 }
 
@@ -845,6 +869,8 @@ mepgl_status mepgl_create_batch(const mepgl_problem *probs, int n_strings, const
     }
     if (st == MEPGL_OK) st = build_layout(c);
     if (st == MEPGL_OK) st = reset_history(c);
+    if (st == MEPGL_OK && cudaStreamSynchronize(c->stream) != cudaSuccess)
+        st = fail(c, MEPGL_ERR_CUDA, "mepgl_create: setting up the buffers failed");
     if (st != MEPGL_OK) {
         g_create_error = c->err;
         mepgl_destroy(c);
@@ -896,6 +922,8 @@ mepgl_status mepgl_set_state(mepgl_ctx *c, const void *a, const void *psi_1, con
         for (int f = 0; f < 1 + c->ncomp; ++f)
             CK(c, cudaMemcpyAsync(s.x[c->xi][f], c->stage[f], c->stage_bytes, cudaMemcpyDeviceToDevice, c->stream));
         c->staged = false;
+        // the host arrays and the staging buffer are free again when this call returns
+        CK(c, cudaStreamSynchronize(c->stream));
         return reset_history(c);
     }
     if (!a || !psi_1 || (c->ncomp == 2 && !psi_2))
@@ -1026,8 +1054,8 @@ mepgl_status mepgl_batch_get_state(mepgl_ctx *c, int string, void *a, void *psi_
     StringHost &s = c->strings[string];
     void *dst[3] = {a, psi_1, psi_2};
     const void *src[3] = {s.x[c->xi][0], s.x[c->xi][1], s.x[c->xi][2]};
-    st = copy_fields(c, s, dst, src, memory, false);
-    if (st == MEPGL_OK) st = check_device_status(c);
+    st = copy_fields(c, s, dst, src, memory, false, false);
+    if (st == MEPGL_OK) st = check_device_status(c);   // waits for the copies too
     return st;
 }
 
@@ -1041,10 +1069,7 @@ mepgl_status mepgl_batch_free_energy(mepgl_ctx *c, int string, double *fenergy)
     if (st != MEPGL_OK) return st;
     CK(c, launch_energy(string_launch(c, string), c->sc, c->xi, c->dscratch));
     c->launches += 1;
-    CK(c, cudaMemcpyAsync(fenergy, c->dscratch + c->hdesc[string].img_base, c->strings[string].F * sizeof(double),
-                          cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    st = check_device_status(c);
+    st = fetch(c, {{fenergy, c->dscratch + c->hdesc[string].img_base, (size_t)c->strings[string].F}}, true);
     if (st != MEPGL_OK) return st;
     for (int n = 0; n < c->strings[string].F; ++n)
         if (!std::isfinite(fenergy[n]))
@@ -1068,9 +1093,8 @@ mepgl_status mepgl_batch_param_adjoint(mepgl_ctx *c, int string, double *dF_dH, 
     c->launches += 1;
     const int F = c->strings[string].F;
     std::vector<double> h(3 * (size_t)F);
-    CK(c, cudaMemcpyAsync(h.data(), c->dscratch + 3 * (size_t)c->hdesc[string].img_base, h.size() * sizeof(double),
-                          cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
+    st = fetch(c, {{h.data(), c->dscratch + 3 * (size_t)c->hdesc[string].img_base, h.size()}}, false);
+    if (st != MEPGL_OK) return st;
     for (int n = 0; n < F; ++n) {
         if (dF_dH) dF_dH[n] = h[3 * n];
         if (dF_deta) dF_deta[n] = h[3 * n + 1];
@@ -1147,12 +1171,9 @@ mepgl_status mepgl_batch_image_scalars(mepgl_ctx *c, int string, double *fenergy
 {
     if (!c || string < 0 || string >= (int)c->strings.size()) return fail(c, MEPGL_ERR_INVALID_ARG, "bad string");
     const int F = c->strings[string].F, o = c->hdesc[string].img_base;
-    if (fenergy) CK(c, cudaMemcpyAsync(fenergy, c->sc.fenergy + o, F * 8, cudaMemcpyDeviceToHost, c->stream));
     // loop()'s g_norm2 is the slot nlcgSteps writes on even substeps
-    if (g_norm2) CK(c, cudaMemcpyAsync(g_norm2, c->sc.gn0 + o, F * 8, cudaMemcpyDeviceToHost, c->stream));
-    if (alpha) CK(c, cudaMemcpyAsync(alpha, c->sc.alpha + o, F * 8, cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    return check_device_status(c);
+    const size_t n = (size_t)F;
+    return fetch(c, {{fenergy, c->sc.fenergy + o, n}, {g_norm2, c->sc.gn0 + o, n}, {alpha, c->sc.alpha + o, n}}, true);
 }
 
 mepgl_status mepgl_compute_jb(mepgl_ctx *c, void *b, void *j_1, void *j_2, int memory)
@@ -1204,12 +1225,9 @@ mepgl_status mepgl_batch_observables(mepgl_ctx *c, int string, int inset, double
                              c->stream));
         c->launches += 1;
     }
-    if (flux) CK(c, cudaMemcpyAsync(flux, out, F * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (winding_1) CK(c, cudaMemcpyAsync(winding_1, out + F, F * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (winding_2 && c->ncomp == 2)
-        CK(c, cudaMemcpyAsync(winding_2, out + 2 * (size_t)F, F * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    return MEPGL_OK;
+    const size_t n = (size_t)F;
+    return fetch(c, {{flux, out, n}, {winding_1, out + F, n}, {c->ncomp == 2 ? winding_2 : nullptr, out + 2 * (size_t)F, n}},
+                 false);
 }
 
 mepgl_status mepgl_arc_length(mepgl_ctx *c, int metric, double *s)
@@ -1224,9 +1242,7 @@ mepgl_status mepgl_batch_arc_length(mepgl_ctx *c, int string, int metric, double
     double *where = nullptr;
     mepgl_status st = arc_length(c, string, metric, &where);
     if (st != MEPGL_OK) return st;
-    CK(c, cudaMemcpyAsync(s, where, c->strings[string].F * 8, cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    return check_device_status(c);
+    return fetch(c, {{s, where, (size_t)c->strings[string].F}}, true);
 }
 
 mepgl_status mepgl_redistribute(mepgl_ctx *c, int kind, int F_new)
@@ -1237,12 +1253,13 @@ mepgl_status mepgl_redistribute(mepgl_ctx *c, int kind, int F_new)
         return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_redistribute: unknown kind");
     mepgl_status st = redistribute(c, kind, F_new);
     if (st != MEPGL_OK) return st;
-    CK(c, cudaStreamSynchronize(c->stream));
+    int *bad = mail_status(c) + 4;   // a singular spline matrix (cubic only), read with the status flags
+    *bad = 0;
+    if (kind == MEPGL_REDIST_CUBIC)
+        CK(c, cudaMemcpyAsync(bad, c->plan.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     st = check_device_status(c);
     if (st != MEPGL_OK) return st;
-    int bad = 0;
-    CK(c, cudaMemcpy(&bad, c->plan.status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (bad) {
+    if (*bad) {
         CK(c, cudaMemset(c->plan.status, 0, sizeof(int)));
         return fail(c, MEPGL_ERR_NAN, "spline matrix is singular (coincident images)");
     }
@@ -1399,7 +1416,6 @@ mepgl_status mepgl_profile_passes(mepgl_ctx *c, int steps, int use_cg, double *m
 mepgl_status mepgl_synchronize(mepgl_ctx *c)
 {
     if (!c) return MEPGL_ERR_INVALID_ARG;
-    CK(c, cudaStreamSynchronize(c->stream));
     return check_device_status(c);
 }
 

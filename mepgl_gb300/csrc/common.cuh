@@ -164,7 +164,6 @@ struct StringDesc {
     int nx, ny, F, ncomp;
     int tiles_x, tiles_y;     // tiles per image
     int img_base;             // first global image index of this string
-    int tile_base;            // first global tile index of this string
     int rows;                 // rows per warp strip of the NLCG passes
     int stiles_y, stile_base; // strips per column of an image; first global strip index
     int thin_film;
@@ -186,10 +185,15 @@ template <> __host__ __device__ inline const Uniform<ff> &StringDesc::u<ff>() co
 
 // Descriptors of the strings covered by one launch; passed by value as a
 // __grid_constant__ kernel parameter, i.e. read through the constant cache.
-struct Batch {
+// Launches of a single string pass only its own: every launch copies its
+// parameters, and sixteen descriptors are 20 KB of them.
+template <int N>
+struct BatchOf {
     int n;
-    StringDesc s[MAX_STRINGS];
+    StringDesc s[N];
 };
+using Batch = BatchOf<MAX_STRINGS>;
+template <bool ONE> using batch_t = BatchOf<ONE ? 1 : MAX_STRINGS>;
 
 struct TileRef {
     int16_t s;        // string within the batch

@@ -41,14 +41,13 @@ struct mepgl_ctx {
     // strings are grouped MAX_STRINGS at a time; each group is one launch per
     // pass, its descriptors passed by value to the kernels
     std::vector<mepgl::Batch> batches;
-    std::vector<int> batch_tile0, batch_ntiles, string_batch;
+    std::vector<int> string_batch;
     std::vector<int> batch_stile0, batch_nstiles;   // warp strips of the NLCG passes
-    mepgl::TileRef *dtiles = nullptr;
-    int n_tiles = 0, total_images = 0;
+    int total_images = 0;
     unsigned long long *fqueue = nullptr;   // work counter of the fused NLCG launch
     unsigned *fstage = nullptr;             // per-image stage counters of the fused NLCG launch
-    std::vector<int> string_tile0, string_ntiles;
     mepgl::Scalars sc{};
+    double *slab = nullptr;       // one allocation for the per-image scalars and everything below up to the arc lengths
     double *dscratch = nullptr;   // per-image temporaries (energies, 3 adjoints)
     double *ds = nullptr, *ds_jb = nullptr;   // arc lengths of string 0
     mepgl::RedistPlan plan{};
@@ -59,6 +58,8 @@ struct mepgl_ctx {
     bool pending = false;         // an NLCG update not yet applied to x
     int64_t launches = 0;
     std::string err;
+    double *mail = nullptr;       // pinned: results on their way to the caller, then the status flags
+    size_t mail_cap = 0;          // doubles of results it holds
     std::map<std::tuple<int, int, int, int>, cudaGraphExec_t> graphs;
     std::vector<double> host_s, host_sjb;
     int sm_count = 152;

@@ -84,6 +84,9 @@ int fuse_waves(int precision) { return precision == 1 ? MEPGL_FUSE_WAVES_F64 : M
 // FP32 389 / 508, 341 / 392, 316 / 347, 360 / 354, 359 / 403 us; FP64 3431 /
 // 6027, 2407 / 4279, 2329 / 4143, 2341 / 4154, 2397 / 4216 us; FP32 256 x
 // 256 x 40 loses 3 % from 150 on), down to the fewest rows that still gain.
+// Float-float strips are bound by issue, and a second wave of them costs more
+// than long ones: four steps of 128 x 128 x 24 take 447 / 845 us at 80 % (one
+// wave of 12 rows), 613 / 1029 at 110 %, 522 / 903 at 150 %.
 #ifndef MEPGL_STRIP_ROWS_F32
 #define MEPGL_STRIP_ROWS_F32 40
 #endif
@@ -96,12 +99,22 @@ int fuse_waves(int precision) { return precision == 1 ? MEPGL_FUSE_WAVES_F64 : M
 #ifndef MEPGL_STRIP_FILL_F64
 #define MEPGL_STRIP_FILL_F64 150
 #endif
-int strip_rows_cap(int precision) { return precision == 1 ? MEPGL_STRIP_ROWS_F64 : MEPGL_STRIP_ROWS_F32; }
-
-int strip_rows(int precision, int ny, long tiles, int slots)
+#ifndef MEPGL_STRIP_ROWS_FF
+#define MEPGL_STRIP_ROWS_FF 16
+#endif
+#ifndef MEPGL_STRIP_FILL_FF
+#define MEPGL_STRIP_FILL_FF 80
+#endif
+int strip_rows_cap(int precision, int paired)
 {
-    const int cap = strip_rows_cap(precision), least = precision == 1 ? 1 : 2;
-    const long want = (long)slots * (precision == 1 ? MEPGL_STRIP_FILL_F64 : MEPGL_STRIP_FILL_F32) / 100;
+    return precision == 0 ? MEPGL_STRIP_ROWS_F32 : paired ? MEPGL_STRIP_ROWS_FF : MEPGL_STRIP_ROWS_F64;
+}
+
+int strip_rows(int precision, int paired, int ny, long tiles, int slots)
+{
+    const int cap = strip_rows_cap(precision, paired), least = precision == 0 ? 2 : 1;
+    const int fill = precision == 0 ? MEPGL_STRIP_FILL_F32 : paired ? MEPGL_STRIP_FILL_FF : MEPGL_STRIP_FILL_F64;
+    const long want = (long)slots * fill / 100;
     long rows = tiles < want ? cap * tiles / want : cap;
     if (rows < least) rows = least;
     const long k = (ny + rows - 1) / rows;          // strips per column, of equal height
@@ -193,13 +206,7 @@ __device__ __forceinline__ void image_ptrs(ImagePtrs<T, NC> &ip, void *const *in
     for (int c = 0; c < 1 + NC; ++c) ip.in[c] = static_cast<const vec2_t<store_t<T>> *>(in[c]) + off;
 }
 
-// Slot of a tile's partial sums: the global tile index of (string, image, row,
-// column), independent of which launch (whole batch or one string) covers it.
-__device__ __forceinline__ int part_slot(const StringDesc &S, const TileRef &tr)
-{
-    return S.tile_base + (tr.n * S.tiles_y + tr.ty) * S.tiles_x + tr.tx;
-}
-
+// Tile tt of a string, in (image, row, column) order.
 __device__ __forceinline__ TileRef flat_tile(const StringDesc &S, int tt)
 {
     const int tpi = S.tiles_x * S.tiles_y, n = tt / tpi, r = tt - n * tpi, ty = r / S.tiles_x;
@@ -400,238 +407,249 @@ __device__ double line_search(const double *coef, const Scalars &sc, int exact)
 #include "strip.cuh"
 
 template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ Batch bt, const TileRef *__restrict__ tiles,
-                                               int n_tiles, Scalars sc, int xbuf, double *out)
+__global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ StringDesc S, Scalars sc, int xbuf, double *out)
 {
     constexpr int TYT = TileRows<T>::v;
     __shared__ Tile<T, NC, TYT> t;
     __shared__ double red[NT / 32];
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        // without a tile table: one string, tiles in (image, row, column) order
-        const TileRef tr = tiles ? tiles[tt] : flat_tile(bt.s[0], tt);
-        const StringDesc &S = bt.s[tr.s];
-        const int img = S.img_base + tr.n;
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
-        stage<T, NC, TYT>(t, S, ip, i0, j0);
-        PackParams<T, NC> pp;
-        pp.load(S);
-        __syncthreads();
-        T v[1] = {(T)0};
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
+    const int tt = blockIdx.x;
+    const TileRef tr = flat_tile(S, tt);
+    const int img = S.img_base + tr.n;
+    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    ImagePtrs<T, NC> ip;
+    image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
+    stage<T, NC, TYT>(t, S, ip, i0, j0);
+    PackParams<T, NC> pp;
+    pp.load(S);
+    __syncthreads();
+    T v[1] = {(T)0};
+    const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                Wts<T> w;
-                w.load(t.m[ly + 1][lx + 1]);
-                if (S.disc) {
-                    SiteParams<T> p;
-                    p.load_uniform(S);
-                    if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
-                    v[0] += site_energy_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film);
-                } else {
-                    if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
-                    v[0] += site_energy<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, S.per_site, S.thin_film);
-                }
+    for (int r = 0; r < TYT / 8; ++r) {
+        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
+        if (gi < S.nx && gj < S.ny) {
+            Wts<T> w;
+            w.load(t.m[ly + 1][lx + 1]);
+            if (S.disc) {
+                SiteParams<T> p;
+                p.load_uniform(S);
+                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
+                v[0] += site_energy_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film);
+            } else {
+                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
+                v[0] += site_energy<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, S.per_site, S.thin_film);
             }
         }
-        const int tpi = S.tiles_x * S.tiles_y;
-        double tot[1];
-        if (finish_image<1>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot) && threadIdx.x == 0)
-            out[img] = S.disc ? tot[0] : tot[0] * S.ud.dx2;
-        __syncthreads();
     }
+    const int tpi = S.tiles_x * S.tiles_y;
+    double tot[1];
+    if (finish_image<1>(v, red, sc, tt, tr.n * tpi, tpi, img, tot) && threadIdx.x == 0)
+        out[img] = S.disc ? tot[0] : tot[0] * S.ud.dx2;
 }
 
 // Per-image dF/dH, dF/deta, dF/dgamma at fixed fields (out[3 img + k]).
 template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_param_adjoint(const __grid_constant__ Batch bt,
-                                                      const TileRef *__restrict__ tiles, int n_tiles, Scalars sc,
+__global__ void __launch_bounds__(NT) k_param_adjoint(const __grid_constant__ StringDesc S, Scalars sc,
                                                       int xbuf, double *out)
 {
     constexpr int TYT = TileRows<T>::v;
     __shared__ Tile<T, NC, TYT> t;
     __shared__ double red[NT / 32 * 3];
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const int img = S.img_base + tr.n;
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
-        stage<T, NC, TYT>(t, S, ip, i0, j0);
-        SiteParams<T> p;
-        p.load_uniform(S);
-        __syncthreads();
-        T v[3] = {(T)0, (T)0, (T)0};
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
+    const int tt = blockIdx.x;
+    const TileRef tr = flat_tile(S, tt);
+    const int img = S.img_base + tr.n;
+    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    ImagePtrs<T, NC> ip;
+    image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
+    stage<T, NC, TYT>(t, S, ip, i0, j0);
+    SiteParams<T> p;
+    p.load_uniform(S);
+    __syncthreads();
+    T v[3] = {(T)0, (T)0, (T)0};
+    const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                Wts<T> w;
-                w.load(t.m[ly + 1][lx + 1]);
-                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
-                if (S.disc) {
-                    T u[3] = {(T)0, v[1], v[2]};
-                    site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, 1, u);
-                    v[1] = u[1];
-                    v[2] = u[2];
-                    if (!S.thin_film) v[0] += site_dh_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w);
-                } else {
-                    site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film, v);
-                }
+    for (int r = 0; r < TYT / 8; ++r) {
+        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
+        if (gi < S.nx && gj < S.ny) {
+            Wts<T> w;
+            w.load(t.m[ly + 1][lx + 1]);
+            if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
+            if (S.disc) {
+                T u[3] = {(T)0, v[1], v[2]};
+                site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, 1, u);
+                v[1] = u[1];
+                v[2] = u[2];
+                if (!S.thin_film) v[0] += site_dh_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w);
+            } else {
+                site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film, v);
             }
         }
-        const int tpi = S.tiles_x * S.tiles_y;
-        double tot[3];
-        if (finish_image<3>(v, red, sc, part_slot(S, tr), S.tile_base + tr.n * tpi, tpi, img, tot) &&
-            threadIdx.x == 0) {
-            out[3 * img] = tot[0];
-            out[3 * img + 1] = tot[1];
-            out[3 * img + 2] = tot[2];
-        }
-        __syncthreads();
+    }
+    const int tpi = S.tiles_x * S.tiles_y;
+    double tot[3];
+    if (finish_image<3>(v, red, sc, tt, tr.n * tpi, tpi, img, tot) &&
+        threadIdx.x == 0) {
+        out[3 * img] = tot[0];
+        out[3 * img + 1] = tot[1];
+        out[3 * img + 2] = tot[2];
     }
 }
 
 template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ Batch bt,
-                                                      const TileRef *__restrict__ tiles, int n_tiles, int xbuf,
+__global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ StringDesc S, int xbuf,
                                                       FieldPtrs out, int maxwell)
 {
     constexpr int TYT = TileRows<T>::v;
     using V = vec2_t<T>;
     __shared__ Tile<T, NC, TYT> t;
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        const size_t off = (size_t)tr.n * S.nx * S.ny;
-        ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], off);
-        stage<T, NC, TYT>(t, S, ip, i0, j0);
-        PackParams<T, NC> pp;
-        pp.load(S);
-        __syncthreads();
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
+    const int tt = blockIdx.x;
+    const TileRef tr = flat_tile(S, tt);
+    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    const size_t off = (size_t)tr.n * S.nx * S.ny;
+    ImagePtrs<T, NC> ip;
+    image_ptrs<T, NC>(ip, S.x[xbuf], off);
+    stage<T, NC, TYT>(t, S, ip, i0, j0);
+    PackParams<T, NC> pp;
+    pp.load(S);
+    __syncthreads();
+    const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                const int s = gi + S.nx * gj;
-                Wts<T> w;
-                w.load(t.m[ly + 1][lx + 1]);
-                T g[2 + 2 * NC];
-                bool link = false;
-                if constexpr (!std::is_same<T, ff>::value) link = S.disc != 0;   // float-float: the reference form only
-                if (link) {
-                    if constexpr (!std::is_same<T, ff>::value) {
-                        SiteParams<T> p;
-                        p.load_uniform(S);
-                        T hl = p.h, hd = p.h;
-                        T hmx_l[2] = {p.hmx[0], p.hmx[1]}, hmy_d[2] = {p.hmy[0], p.hmy[1]};
-                        if (S.per_site) {
-                            p.load_site(S, s, NC);
-                            hl = static_cast<const T *>(S.ph)[s > 0 ? s - 1 : s];
-                            hd = static_cast<const T *>(S.ph)[gj > 0 ? s - S.nx : s];
-                            for (int c = 0; c < NC; ++c) {
-                                if (gi > 0) hmx_l[c] = (T)0.5 / static_cast<const T *>(S.pmxx[c])[s - 1];
-                                if (gj > 0) hmy_d[c] = (T)0.5 / static_cast<const T *>(S.pmyy[c])[s - S.nx];
-                            }
+    for (int r = 0; r < TYT / 8; ++r) {
+        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
+        if (gi < S.nx && gj < S.ny) {
+            const int s = gi + S.nx * gj;
+            Wts<T> w;
+            w.load(t.m[ly + 1][lx + 1]);
+            T g[2 + 2 * NC];
+            bool link = false;
+            if constexpr (!std::is_same<T, ff>::value) link = S.disc != 0;   // float-float: the reference form only
+            if (link) {
+                if constexpr (!std::is_same<T, ff>::value) {
+                    SiteParams<T> p;
+                    p.load_uniform(S);
+                    T hl = p.h, hd = p.h;
+                    T hmx_l[2] = {p.hmx[0], p.hmx[1]}, hmy_d[2] = {p.hmy[0], p.hmy[1]};
+                    if (S.per_site) {
+                        p.load_site(S, s, NC);
+                        hl = static_cast<const T *>(S.ph)[s > 0 ? s - 1 : s];
+                        hd = static_cast<const T *>(S.ph)[gj > 0 ? s - S.nx : s];
+                        for (int c = 0; c < NC; ++c) {
+                            if (gi > 0) hmx_l[c] = (T)0.5 / static_cast<const T *>(S.pmxx[c])[s - 1];
+                            if (gj > 0) hmy_d[c] = (T)0.5 / static_cast<const T *>(S.pmyy[c])[s - S.nx];
                         }
-                        site_gradient_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hl, hd, hmx_l, hmy_d, maxwell,
-                                                       S.thin_film, g);
                     }
-                } else {
-                    if (S.per_site) pp.load_site(S, gi, gj, s);
-                    site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s),
-                                         maxwell, S.thin_film, g);
+                    site_gradient_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hl, hd, hmx_l, hmy_d, maxwell,
+                                                   S.thin_film, g);
                 }
+            } else {
+                if (S.per_site) pp.load_site(S, gi, gj, s);
+                site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s),
+                                     maxwell, S.thin_film, g);
+            }
 #pragma unroll
-                for (int c = 0; c < 1 + NC; ++c) {
-                    V gv;
-                    gv.x = g[2 * c];
-                    gv.y = g[2 * c + 1];
-                    store2<T>(static_cast<vec2_t<store_t<T>> *>(out.p[c]) + off + s, gv);
-                }
+            for (int c = 0; c < 1 + NC; ++c) {
+                V gv;
+                gv.x = g[2 * c];
+                gv.y = g[2 * c + 1];
+                store2<T>(static_cast<vec2_t<store_t<T>> *>(out.p[c]) + off + s, gv);
             }
         }
-        __syncthreads();
     }
 }
 
 template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ Batch bt, const TileRef *__restrict__ tiles,
-                                           int n_tiles, int xbuf, T *b, vec2_t<T> *j1, vec2_t<T> *j2)
+__global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ StringDesc S, int xbuf, T *b, vec2_t<T> *j1, vec2_t<T> *j2)
 {
     constexpr int TYT = TileRows<T>::v;
     using V = vec2_t<T>;
     __shared__ Tile<T, NC, TYT> t;
-    for (int tt = blockIdx.x; tt < n_tiles; tt += gridDim.x) {
-        const TileRef tr = tiles[tt];
-        const StringDesc &S = bt.s[tr.s];
-        const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-        const size_t off = (size_t)tr.n * S.nx * S.ny;
-        ImagePtrs<T, NC> ip;
-        image_ptrs<T, NC>(ip, S.x[xbuf], off);
-        stage<T, NC, TYT>(t, S, ip, i0, j0);
-        PackParams<T, NC> pp;
-        pp.load(S);
-        __syncthreads();
-        const int lx = threadIdx.x & 31, gi = i0 + lx;
+    const int tt = blockIdx.x;
+    const TileRef tr = flat_tile(S, tt);
+    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
+    const size_t off = (size_t)tr.n * S.nx * S.ny;
+    ImagePtrs<T, NC> ip;
+    image_ptrs<T, NC>(ip, S.x[xbuf], off);
+    stage<T, NC, TYT>(t, S, ip, i0, j0);
+    PackParams<T, NC> pp;
+    pp.load(S);
+    __syncthreads();
+    const int lx = threadIdx.x & 31, gi = i0 + lx;
 #pragma unroll
-        for (int r = 0; r < TYT / 8; ++r) {
-            const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-            if (gi < S.nx && gj < S.ny) {
-                const size_t k = off + gi + (size_t)S.nx * gj;
-                Wts<T> w;
-                w.load(t.m[ly + 1][lx + 1]);
-                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
-                T o[1 + 2 * NC];
-                site_jb<T, NC>(pack_view_tile(t, lx + 1, ly + 1), S.template u<T>().idx, pp, w, o);
-                b[k] = o[0];
-                V v;
-                v.x = o[1];
-                v.y = o[2];
-                j1[k] = v;
-                if (NC == 2) {
-                    v.x = o[3];
-                    v.y = o[4];
-                    j2[k] = v;
-                }
+    for (int r = 0; r < TYT / 8; ++r) {
+        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
+        if (gi < S.nx && gj < S.ny) {
+            const size_t k = off + gi + (size_t)S.nx * gj;
+            Wts<T> w;
+            w.load(t.m[ly + 1][lx + 1]);
+            if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
+            T o[1 + 2 * NC];
+            site_jb<T, NC>(pack_view_tile(t, lx + 1, ly + 1), S.template u<T>().idx, pp, w, o);
+            b[k] = o[0];
+            V v;
+            v.x = o[1];
+            v.y = o[2];
+            j1[k] = v;
+            if (NC == 2) {
+                v.x = o[3];
+                v.y = o[4];
+                j2[k] = v;
             }
         }
-        __syncthreads();
     }
 }
 
-// x += alpha_pend[image] d over one image per blockIdx.y.  W: the compute
-// type of the NLCG passes that wrote d (ff: d holds float-float pairs, the
-// update runs in double on their values).
-template <class T, class W = T>
-__global__ void __launch_bounds__(NT) k_apply_update(vec2_t<T> *x, const vec2_t<T> *d, const double *alpha_pend,
-                                                     long M)
+// x += alpha_pend[image] d over every string of a batch: block (chunk, image
+// of the batch, field).  W: the compute type of the NLCG passes that wrote d
+// (ff: d holds float-float pairs, the update runs in double on their values).
+template <class T, class W, bool ONE>
+__global__ void __launch_bounds__(NT) k_apply_update(const __grid_constant__ batch_t<ONE> bt, const double *alpha_pend,
+                                                     int img0, int xbuf, int dbuf)
 {
-    const T a = (T)alpha_pend[blockIdx.y];
+    const int img = img0 + blockIdx.y;
+    int si = 0;
+    if (!ONE)
+        for (int k = 1; k < bt.n; ++k)
+            if (img >= bt.s[k].img_base) si = k;
+    const StringDesc &S = bt.s[si];
+    const T a = (T)alpha_pend[img];
     if (a == (T)0) return;
-    const long off = (long)blockIdx.y * M;
+    const long M = (long)S.nx * S.ny, off = (long)(img - S.img_base) * M;
+    vec2_t<T> *x = static_cast<vec2_t<T> *>(S.x[xbuf][blockIdx.z]) + off;
+    const vec2_t<T> *d = static_cast<const vec2_t<T> *>(S.d[dbuf][blockIdx.z]) + off;
     for (long p = blockIdx.x * (long)NT + threadIdx.x; p < M; p += (long)gridDim.x * NT) {
-        vec2_t<T> v = x[off + p];
+        vec2_t<T> v = x[p];
         vec2_t<T> dd;
         if constexpr (std::is_same<W, ff>::value) {
-            const ff2 w = loadw<ff>(d + off + p);
+            const ff2 w = loadw<ff>(d + p);
             dd.x = to_double(w.x);
             dd.y = to_double(w.y);
         } else {
-            dd = d[off + p];
+            dd = d[p];
         }
         v.x = v.x + a * dd.x;
         v.y = v.y + a * dd.y;
-        x[off + p] = v;
+        x[p] = v;
     }
+}
+
+// NLCG history of every image: |g|^2 = infinity (the next beta is 0, and the
+// passes then read neither the old gradient nor the old direction, whose
+// contents no longer matter), no step pending, scalars zero.
+__global__ void k_reset_history(Scalars sc, int n_images)
+{
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= n_images) return;
+    sc.gn0[n] = sc.gn1[n] = INFINITY;
+    sc.gdg[n] = sc.beta[n] = sc.alpha[n] = sc.alpha_pend[n] = sc.fenergy[n] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sc.poly[4 * n + k] = 0.0;
+}
+
+// |g|^2 = infinity for images [first, last).
+__global__ void k_restart_cg(Scalars sc, int first, int last)
+{
+    const int n = first + blockIdx.x * blockDim.x + threadIdx.x;
+    if (n < last) sc.gn0[n] = sc.gn1[n] = INFINITY;
 }
 
 // Fields x between double pairs and float-float pairs, in place (an ff2
@@ -1291,11 +1309,11 @@ inline int grid_for(long n, int cap = 152 * 16)
 #define DISPATCH(L, KERNEL, ...)                                                                    \
     do {                                                                                            \
         if ((L).precision == 1) {                                                                   \
-            if ((L).ncomp == 2) KERNEL<double, 2><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);   \
-            else KERNEL<double, 1><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);                  \
+            if ((L).ncomp == 2) KERNEL<double, 2><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);   \
+            else KERNEL<double, 1><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);                  \
         } else {                                                                                    \
-            if ((L).ncomp == 2) KERNEL<float, 2><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);    \
-            else KERNEL<float, 1><<<(L).grid, NT, 0, (L).stream>>>(__VA_ARGS__);                   \
+            if ((L).ncomp == 2) KERNEL<float, 2><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);    \
+            else KERNEL<float, 1><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);                   \
         }                                                                                           \
     } while (0)
 
@@ -1304,11 +1322,12 @@ inline int grid_for(long n, int cap = 152 * 16)
 #define DISPATCH_STRIP_T(L, KERNEL, T, ...)                                                         \
     do {                                                                                            \
         if (strip_one(L)) {                                                                         \
-            if ((L).ncomp == 2) KERNEL<T, 2, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
-            else KERNEL<T, 1, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__);             \
+            const batch_t<true> one = only_string(L);                                               \
+            if ((L).ncomp == 2) KERNEL<T, 2, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(one, __VA_ARGS__); \
+            else KERNEL<T, 1, true><<<(L).n_stiles, NTS, 0, (L).stream>>>(one, __VA_ARGS__);        \
         } else {                                                                                    \
-            if ((L).ncomp == 2) KERNEL<T, 2, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__); \
-            else KERNEL<T, 1, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(__VA_ARGS__);            \
+            if ((L).ncomp == 2) KERNEL<T, 2, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(*(L).batch, __VA_ARGS__); \
+            else KERNEL<T, 1, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(*(L).batch, __VA_ARGS__); \
         }                                                                                           \
     } while (0)
 #define DISPATCH_STRIP(L, KERNEL, ...)                                                              \
@@ -1319,16 +1338,23 @@ inline int grid_for(long n, int cap = 152 * 16)
     } while (0)
 
 static inline bool strip_one(const Launch &L) { return L.batch->n == 1; }
+static inline batch_t<true> only_string(const Launch &L)
+{
+    batch_t<true> b;
+    b.n = 1;
+    b.s[0] = L.batch->s[0];
+    return b;
+}
 
 cudaError_t launch_grad(const Launch &L, const Scalars &sc, const StepFlags &f)
 {
-    DISPATCH_STRIP(L, k_grad_s, *L.batch, L.stile0, sc, f);
+    DISPATCH_STRIP(L, k_grad_s, L.stile0, sc, f);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dir_poly(const Launch &L, const Scalars &sc, const StepFlags &f)
 {
-    DISPATCH_STRIP(L, k_dir_poly_s, *L.batch, L.stile0, sc, f);
+    DISPATCH_STRIP(L, k_dir_poly_s, L.stile0, sc, f);
     return cudaGetLastError();
 }
 
@@ -1376,12 +1402,12 @@ static cudaError_t nlcg_fused_launch(const Launch &L, const Scalars &sc, const S
     }
     const long long items = 2LL * L.n_stiles * steps;
     const int grid = items < slots[ci] ? (int)items : slots[ci];
-#define FUSED_ARGS *L.batch, L.stile0, L.n_stiles, steps, plan, sc, queue, stage, max_polls
+#define FUSED_ARGS L.stile0, L.n_stiles, steps, plan, sc, queue, stage, max_polls
     switch (ci) {
-    case 0: k_nlcg_s<T, 1, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    case 1: k_nlcg_s<T, 2, false><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    case 2: k_nlcg_s<T, 1, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
-    default: k_nlcg_s<T, 2, true><<<grid, NTS, 0, L.stream>>>(FUSED_ARGS); break;
+    case 0: k_nlcg_s<T, 1, false><<<grid, NTS, 0, L.stream>>>(*L.batch, FUSED_ARGS); break;
+    case 1: k_nlcg_s<T, 2, false><<<grid, NTS, 0, L.stream>>>(*L.batch, FUSED_ARGS); break;
+    case 2: k_nlcg_s<T, 1, true><<<grid, NTS, 0, L.stream>>>(only_string(L), FUSED_ARGS); break;
+    default: k_nlcg_s<T, 2, true><<<grid, NTS, 0, L.stream>>>(only_string(L), FUSED_ARGS); break;
     }
 #undef FUSED_ARGS
     return cudaGetLastError();
@@ -1408,7 +1434,7 @@ cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlag
 
 cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *out)
 {
-    DISPATCH(L, k_energy, *L.batch, L.tiles, L.n_tiles, sc, xbuf, out);
+    DISPATCH(L, k_energy, *L.str, sc, xbuf, out);
     return cudaGetLastError();
 }
 
@@ -1417,18 +1443,18 @@ cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *
 // no float-float form and stays IEEE double.
 cudaError_t launch_gradient_only(const Launch &L, int xbuf, FieldPtrs out, int maxwell)
 {
-    if (L.paired && L.precision == 1 && !L.batch->s[0].disc) {
-        if (L.ncomp == 2) k_gradient_only<ff, 2><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, out, maxwell);
-        else k_gradient_only<ff, 1><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, out, maxwell);
+    if (L.paired && L.precision == 1 && !L.str->disc) {
+        if (L.ncomp == 2) k_gradient_only<ff, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, out, maxwell);
+        else k_gradient_only<ff, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, out, maxwell);
     } else {
-        DISPATCH(L, k_gradient_only, *L.batch, L.tiles, L.n_tiles, xbuf, out, maxwell);
+        DISPATCH(L, k_gradient_only, *L.str, xbuf, out, maxwell);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_param_adjoint(const Launch &L, const Scalars &sc, int xbuf, double *out)
 {
-    DISPATCH(L, k_param_adjoint, *L.batch, L.tiles, L.n_tiles, sc, xbuf, out);
+    DISPATCH(L, k_param_adjoint, *L.str, sc, xbuf, out);
     return cudaGetLastError();
 }
 
@@ -1437,46 +1463,57 @@ cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *const 
     (void)sc;
     if (L.precision == 1) {
         if (L.ncomp == 2)
-            k_jb<double, 2><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, (double *)b[0],
+            k_jb<double, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (double *)b[0],
                                                          (double2 *)j[0][0], (double2 *)j[0][1]);
         else
-            k_jb<double, 1><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, (double *)b[0],
+            k_jb<double, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (double *)b[0],
                                                          (double2 *)j[0][0], (double2 *)j[0][1]);
     } else {
         if (L.ncomp == 2)
-            k_jb<float, 2><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, (float *)b[0],
+            k_jb<float, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (float *)b[0],
                                                         (float2 *)j[0][0], (float2 *)j[0][1]);
         else
-            k_jb<float, 1><<<L.grid, NT, 0, L.stream>>>(*L.batch, L.tiles, L.n_tiles, xbuf, (float *)b[0],
+            k_jb<float, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (float *)b[0],
                                                         (float2 *)j[0][0], (float2 *)j[0][1]);
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_apply_update(const Launch &L, const Scalars &sc, const StringDesc *hs, int n_strings, int xbuf,
-                                int dbuf)
+template <class T, class W>
+static void apply_update(const Launch &L, const Scalars &sc, int xbuf, int dbuf)
 {
-    for (int si = 0; si < n_strings; ++si) {
-        const StringDesc &S = hs[si];
-        const long M = (long)S.nx * S.ny;
-        for (int c = 0; c < 1 + S.ncomp; ++c) {
-            const dim3 grid((unsigned)((M + NT - 1) / NT < 64 ? (M + NT - 1) / NT : 64), (unsigned)S.F);
-            if (L.precision == 1 && L.paired)   // d holds float-float pairs (paired passes)
-                k_apply_update<double, ff><<<grid, NT, 0, L.stream>>>(
-                    (double2 *)S.x[xbuf][c], (const double2 *)S.d[dbuf][c], sc.alpha_pend + S.img_base, M);
-            else if (L.precision == 1)
-                k_apply_update<double><<<grid, NT, 0, L.stream>>>(
-                    (double2 *)S.x[xbuf][c], (const double2 *)S.d[dbuf][c], sc.alpha_pend + S.img_base, M);
-            else
-                k_apply_update<float><<<grid, NT, 0, L.stream>>>(
-                    (float2 *)S.x[xbuf][c], (const float2 *)S.d[dbuf][c], sc.alpha_pend + S.img_base, M);
-        }
+    const Batch &B = *L.batch;
+    long M = 0;
+    for (int k = 0; k < B.n; ++k) M = M > (long)B.s[k].nx * B.s[k].ny ? M : (long)B.s[k].nx * B.s[k].ny;
+    const int img0 = B.s[0].img_base, images = B.s[B.n - 1].img_base + B.s[B.n - 1].F - img0;
+    const long chunks = (M + NT - 1) / NT;
+    constexpr int MOST = 65535;   // images per launch (grid y)
+    for (int i = 0; i < images; i += MOST) {
+        const int n = images - i < MOST ? images - i : MOST;
+        const dim3 grid((unsigned)(chunks < 64 ? chunks : 64), (unsigned)n, (unsigned)(1 + L.ncomp));
+        if (strip_one(L)) k_apply_update<T, W, true><<<grid, NT, 0, L.stream>>>(only_string(L), sc.alpha_pend, img0 + i, xbuf, dbuf);
+        else k_apply_update<T, W, false><<<grid, NT, 0, L.stream>>>(B, sc.alpha_pend, img0 + i, xbuf, dbuf);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    int total_images = 0;
-    for (int si = 0; si < n_strings; ++si) total_images += hs[si].F;
-    return cudaMemsetAsync(sc.alpha_pend, 0, sizeof(double) * total_images, L.stream);
+}
+
+cudaError_t launch_apply_update(const Launch &L, const Scalars &sc, int xbuf, int dbuf)
+{
+    if (L.precision == 0) apply_update<float, float>(L, sc, xbuf, dbuf);
+    else if (L.paired) apply_update<double, ff>(L, sc, xbuf, dbuf);   // d holds float-float pairs (paired passes)
+    else apply_update<double, double>(L, sc, xbuf, dbuf);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reset_history(const Scalars &sc, int n_images, cudaStream_t st)
+{
+    k_reset_history<<<(n_images + NT - 1) / NT, NT, 0, st>>>(sc, n_images);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_restart_cg(const Scalars &sc, int first, int last, cudaStream_t st)
+{
+    k_restart_cg<<<(last - first + NT - 1) / NT, NT, 0, st>>>(sc, first, last);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_check_scalars(const Scalars &sc, int n_images, int slot, cudaStream_t st)
@@ -1757,10 +1794,8 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
     cudaError_t e = noalloc_setup(dev, &scr);
     if (e != cudaSuccess) return noalloc_fail(MEPGL_ERR_CUDA, std::string("scratch setup: ") + cudaGetErrorString(e));
 
-    Batch bt;
-    memset(&bt, 0, sizeof(bt));
-    bt.n = 1;
-    StringDesc &S = bt.s[0];
+    StringDesc S;
+    memset(&S, 0, sizeof(S));
     S.nx = nx;
     S.ny = ny;
     S.F = n_images;
@@ -1801,9 +1836,9 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
     e = cudaMemsetAsync(scr.ticket, 0, sizeof(unsigned) * n_images, st);
     if (e != cudaSuccess) return noalloc_fail(MEPGL_ERR_CUDA, std::string("ticket reset: ") + cudaGetErrorString(e));
     if (multicomponent)
-        k_energy<double, 2><<<(unsigned)n_tiles, NT, 0, st>>>(bt, nullptr, (int)n_tiles, sc, 0, fenergy);
+        k_energy<double, 2><<<(unsigned)n_tiles, NT, 0, st>>>(S, sc, 0, fenergy);
     else
-        k_energy<double, 1><<<(unsigned)n_tiles, NT, 0, st>>>(bt, nullptr, (int)n_tiles, sc, 0, fenergy);
+        k_energy<double, 1><<<(unsigned)n_tiles, NT, 0, st>>>(S, sc, 0, fenergy);
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(MEPGL_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return MEPGL_OK;

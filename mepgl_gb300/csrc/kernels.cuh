@@ -13,12 +13,10 @@ int tile_rows(int precision);
 cudaError_t upload_mask_tables();
 
 struct Launch {
-    const Batch *batch;          // host copy; passed by value to the kernels
-    const TileRef *tiles;        // device
-    int tile0;                   // global index of tiles[0] (tiles are in (string, image, row, column) order)
-    int n_tiles;
-    int grid;                    // blocks launched (grid-stride over tiles)
-    int stile0, n_stiles;        // the same for the warp strips of the NLCG passes
+    const Batch *batch;          // strings of the NLCG passes (host copy; passed by value to the kernels)
+    int stile0, n_stiles;        // their strips
+    const StringDesc *str;       // string of the tile kernels
+    int n_tiles;                 // its tiles
     int precision;               // 0 float, 1 double
     int paired;                  // 1: NLCG passes in float-float arithmetic on double fields
     int ncomp;                   // 1 or 2 (uniform over the strings of a context)
@@ -35,8 +33,8 @@ struct StepFlags {
 
 // Rows per warp strip of an image column of ny rows, in a batch of `tiles`
 // strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
-int strip_rows_cap(int precision);
-int strip_rows(int precision, int ny, long tiles, int slots);
+int strip_rows_cap(int precision, int paired);
+int strip_rows(int precision, int paired, int ny, long tiles, int slots);
 // Steps are fused for batches of at most fuse_waves() x strip_pass_slots()
 // strips; strip_pass_slots(): resident warps of the pass kernels on the GPU.
 int fuse_waves(int precision);
@@ -56,12 +54,14 @@ cudaError_t launch_grad(const Launch &L, const Scalars &sc, const StepFlags &f);
 // Pass 2: d <- -g + beta d (into d[dout]); quartic of F(x + a d); the last
 // tile of each image runs the line search and sets alpha, alpha_pend.
 cudaError_t launch_dir_poly(const Launch &L, const Scalars &sc, const StepFlags &f);
-// x[xbuf] += alpha_pend d[dbuf]; alpha_pend = 0.
 // Paired FP64: the NLCG passes keep x as float-float pairs; the in-place
 // conversion of `pairs` complex values of x to (1) or from (0) them.
 cudaError_t launch_x_format(void *x, long pairs, int to_pairs, cudaStream_t st);
-cudaError_t launch_apply_update(const Launch &L, const Scalars &sc, const StringDesc *host_strings, int n_strings,
-                                int xbuf, int dbuf);
+// x[xbuf] += alpha_pend d[dbuf] over a batch (alpha_pend stays).
+cudaError_t launch_apply_update(const Launch &L, const Scalars &sc, int xbuf, int dbuf);
+// Scalars of every image as after a restart; |g|^2 = infinity for images [first, last).
+cudaError_t launch_reset_history(const Scalars &sc, int n_images, cudaStream_t st);
+cudaError_t launch_restart_cg(const Scalars &sc, int first, int last, cudaStream_t st);
 // Energy of x[xbuf] into sc.fenergy_out (per image).
 cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *out);
 cudaError_t launch_param_adjoint(const Launch &L, const Scalars &sc, int xbuf, double *out);

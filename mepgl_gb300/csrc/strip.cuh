@@ -191,7 +191,7 @@ __device__ __forceinline__ void cp_async_wait_groups() { asm volatile("cp.async.
 // then read at fixed offsets, i.e. as constant operands, not through
 // indexed constant loads.
 template <bool ONE>
-__device__ __forceinline__ TileRef strip_tile(const Batch &bt, int g)
+__device__ __forceinline__ TileRef strip_tile(const batch_t<ONE> &bt, int g)
 {
     int s = 0;
     if (!ONE)
@@ -284,7 +284,7 @@ using GradRing = vec2_t<T>[3][2][2][1 + NC];
 // field stores, so that a consumer that has seen the image finished (same
 // launch) reads them.
 template <class T, int NC, bool ONE>
-__device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
+__device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
 {
     using V = vec2_t<T>;
@@ -305,6 +305,8 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
     }
     const T alpha = (T)__ldcg(sc.alpha_pend + img);
     const unsigned fields = alpha != (T)0 ? 3u : 1u;   // d is not read when nothing is pending
+    // nor g_prev when it does not enter beta (restarted image, steepest descent)
+    const bool hist = f.use_cg && __ldcg((f.gprev ? sc.gn1 : sc.gn0) + img) <= 1.7976931348623157e308;
     PackParams<T, NC> pp;
     pp.load(S);
     V rc[3][1 + NC];
@@ -334,7 +336,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
         R.m = m;
     };
     auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, bool gold) {
-        strip_load<T, NC, 3>(raw, src, S, L, j, gold ? fields | 4u : fields);
+        strip_load<T, NC, 3>(raw, src, S, L, j, gold && hist ? fields | 4u : fields);
         strip_halo<T, NC, 2, 3>(ring[(j + 3) % 3], src, S, L, j, fields, true);
         m = strip_code(S, L, j);
     };
@@ -419,7 +421,7 @@ __device__ __forceinline__ bool grad_tile(const Batch &bt, const TileRef tr, con
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::grad) k_grad_s(const __grid_constant__ Batch bt,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::grad) k_grad_s(const __grid_constant__ batch_t<ONE> bt,
                                                                   int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) GradRing<T, NC> ring;
@@ -443,7 +445,7 @@ using DirRing = vec2_t<T>[3][2][3][1 + NC];
 // search.  Returns true (in every lane) when this strip finished its image;
 // field stores are fenced as in grad_tile.
 template <class T, int NC, bool ONE>
-__device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
+__device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
                                          DirRing<T, NC> &ring, double (&coef)[5])
 {
     using V = vec2_t<T>;
@@ -462,6 +464,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
         dout[c] = static_cast<V *>(S.d[f.dout][c]) + off;
     }
     const T beta = (T)__ldcg(sc.beta + img);
+    const unsigned fields = beta != (T)0 ? 7u : 3u;    // d is not read when it does not enter
     PackParams<T, NC> pp;
     pp.load(S);
     V rc[3][1 + NC];
@@ -480,8 +483,8 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
         R.m = m;
     };
     auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, bool issue) {
-        strip_load<T, NC, 3>(raw, src, S, L, j, issue ? 7u : 0u);
-        strip_halo<T, NC, 3, 3>(ring[(j + 3) % 3], src, S, L, j, 7u, issue);
+        strip_load<T, NC, 3>(raw, src, S, L, j, issue ? fields : 0u);
+        strip_halo<T, NC, 3, 3>(ring[(j + 3) % 3], src, S, L, j, fields, issue);
         m = strip_code(S, L, j);
     };
     DirRow<T, NC> R0, Rp;
@@ -521,7 +524,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
 #pragma unroll
         for (int c = 0; c < 1 + NC; ++c) {
             hx[c] = h[0][c];
-            const V hg = h[1][c], hdd = h[2][c];
+            const V hg = h[1][c], hdd = fields & 4u ? h[2][c] : zero2<T>();
             hd[c].x = -hg.x + beta * hdd.x;
             hd[c].y = -hg.y + beta * hdd.y;
         }
@@ -592,7 +595,7 @@ __device__ __forceinline__ bool dir_tile(const Batch &bt, const TileRef tr, cons
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::dir) k_dir_poly_s(const __grid_constant__ Batch bt,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::dir) k_dir_poly_s(const __grid_constant__ batch_t<ONE> bt,
                                                                       int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) DirRing<T, NC> ring;
@@ -666,7 +669,7 @@ __device__ __forceinline__ void publish_stage(unsigned *stage, unsigned value)
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __grid_constant__ Batch bt, int tile0, int n_tiles, int steps,
+__global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __grid_constant__ batch_t<ONE> bt, int tile0, int n_tiles, int steps,
                                             StepPlan plan, Scalars sc, unsigned long long *queue, unsigned *stage,
                                             unsigned max_polls)
 {
