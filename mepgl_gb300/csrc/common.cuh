@@ -86,9 +86,9 @@ struct Uniform {
     T eta, gamma, delta, h, idx, dx2, dx;
     // the same with the spacing folded in, as the stencils of site_pack.cuh
     // use them: q dx, +- half of it, half of its square, (q + 1) dx, q / dx;
-    // -2 hm*, hm* / dx^2; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
+    // -2 hm*, hm* / dx^2, and that times half of (q dx)^2; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
     // 1 / (4 dx), 1 / (8 dx^2)
-    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], a2[2], b2[2];
+    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hqmx[2], hqmy[2], a2[2], b2[2];
     T etad, gammad, deltad, hd, idx4, idx8;
 };
 
@@ -106,6 +106,8 @@ inline void fold_spacing(Uniform<double> &U)
         U.n2hmy[c] = -2.0 * U.hmy[c];
         U.hmxi[c] = U.hmx[c] * U.idx * U.idx;
         U.hmyi[c] = U.hmy[c] * U.idx * U.idx;
+        U.hqmx[c] = U.hqq[c] * U.hmxi[c];
+        U.hqmy[c] = U.hqq[c] * U.hmyi[c];
         U.a2[c] = 2.0 * U.a[c] * U.dx2;
         U.b2[c] = 2.0 * U.b[c] * U.dx2;
     }
@@ -138,6 +140,8 @@ inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
         r.n2hmy[c] = T(U.n2hmy[c]);
         r.hmxi[c] = T(U.hmxi[c]);
         r.hmyi[c] = T(U.hmyi[c]);
+        r.hqmx[c] = T(U.hqmx[c]);
+        r.hqmy[c] = T(U.hqmy[c]);
         r.a2[c] = T(U.a2[c]);
         r.b2[c] = T(U.b2[c]);
     }

@@ -152,6 +152,7 @@ struct PackParams {
     using K = Pk<S, NC>;
     P qd, hqd, nhqd, hqq, kq, qi;   // q dx, +- half of it, half its square, (q + 1) dx, q / dx
     P hmx, hmy, n2hmx, n2hmy;       // 1 / (2 m), -1 / m
+    P hqmx, hqmy;                   // hqq / (2 m dx^2)
     P hmxi, hmyi, hmxil, hmyid;     // 1 / (2 m dx^2); at the left / lower neighbour (their forward links end here)
     P aob, b, a2, b2;               // a / b, b; 2 a dx^2, 2 b dx^2
     S eta, gamma, delta, h, idx, idx4, idx8;
@@ -169,6 +170,8 @@ struct PackParams {
         hmy = K::mk(U.hmy[0], U.hmy[1]);
         hmxi = hmxil = K::mk(U.hmxi[0], U.hmxi[1]);
         hmyi = hmyid = K::mk(U.hmyi[0], U.hmyi[1]);
+        hqmx = K::mk(U.hqmx[0], U.hqmx[1]);
+        hqmy = K::mk(U.hqmy[0], U.hqmy[1]);
         n2hmx = K::mk(U.n2hmx[0], U.n2hmx[1]);
         n2hmy = K::mk(U.n2hmy[0], U.n2hmy[1]);
         aob = K::mk(U.aob[0], U.aob[1]);
@@ -217,6 +220,15 @@ struct PackParams {
         h = p.h;
         hd = p.h * p.dx;
     }
+};
+
+// Weights of a site whose neighbours all lie inside both domains, as
+// constants (FP64 strips: a row of such sites drops every multiplication by a
+// weight, 26 of 212 instructions of the gradient and 24 of 290 of the quartic).
+struct Ones {
+    static constexpr bool interior = true;
+    static constexpr double area = 1, wfx = 1, wbx = 1, wfy = 1, wby = 1, wsx = 2, wsy = 2;
+    static constexpr double vUR = 1, vUL = 1, vLL = 1, vLR = 1;
 };
 
 // FP64: a biquadratic coupling of zero is skipped (a uniform branch; its 26
@@ -269,13 +281,11 @@ __device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackPar
         const P f = pmul(hm, K::bc(wf));
         const P Dx = psub(xj, X), Dy = psub(Y, yj);       // Dy: -(y_j - y_i)
         const P s = pmul(pp.qd, K::bc(Ai + Aj));
-        e = pfma(pmul(f, Dx), pfma(s, Y, Dx), e);
-        e = pfma(pmul(f, Dy), pfma(s, X, Dy), e);
-        const P a = pmul(pp.qd, K::bc(Ai));
-        const P W = per_site ? pfma(hb, K::bc(wb), f) : pmul(hm, K::bc(ws));
-        dg = pfma(pmul(W, a), a, dg);
+        e = pfma(f, pfma(Dy, pfma(s, X, Dy), pmul(Dx, pfma(s, Y, Dx))), e);
+        const P W = per_site ? pmul(pp.hqq, pfma(hb, K::bc(wb), f)) : pmul(dir == 0 ? pp.hqmx : pp.hqmy, K::bc(ws));
+        dg = pfma(W, K::bc(Ai * Ai), dg);
     }
-    e = pfma(pmul(dg, K::bc(S(0.5f))), r, e);
+    e = pfma(dg, r, e);
     S t = K::sum(e);
     if constexpr (NC == 2) {
         const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y);
@@ -308,86 +318,154 @@ struct FieldSums {
     S u, d, r, l;
 };
 
-// Gradient dF/dA (out[0..1]) and dF/dpsi_c (out[2 + 2c..]) at one site,
-// restating gradientPsi (nlcg.cu:504-744) and gradientA (nlcg.cu:746-888).
-// Both link ends use the mass of this site, as the reference does.
+// What a walk down a column hands from row to row: of the y-link below the
+// row (from row j - 1 to row j) its pull on the upper site and its current,
+// without the mass; of the magnetic views below it the sums and differences
+// that both rows read.
 template <class S, int NC>
-__device__ __forceinline__ void site_gradient(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
-                                              const FieldSums<S> &h, int maxwell, int thin_film, S *out)
+struct GradCarry {
+    pack_t<S, NC> tx, ty, cr;
+    S s1, s2, tu, ql, qr, ex, exm;
+};
+
+// A row of the window as the gradient reads it: A and psi of the column, A of
+// the columns left and right of it.
+template <class S, int NC>
+struct GradView {
+    vec2_t<S> a, al, ar;
+    pack_t<S, NC> x, y;
+};
+
+// The upper side of row c (the carry into the row above, u): its y-link and
+// magnetic views.  wy: weight of the link; hu: (h + h_above) dx.
+template <class S, int NC>
+__device__ __forceinline__ void grad_up(const GradView<S, NC> &c, const GradView<S, NC> &u, const PackParams<S, NC> &pp,
+                                        S wy, S hu, S ex0, S exm0, GradCarry<S, NC> &k)
 {
     using K = Pk<S, NC>;
     using P = pack_t<S, NC>;
-    using V = vec2_t<S>;
-    const V A0 = v.a[1][1], Ar = v.a[1][2], Al = v.a[1][0], Au = v.a[2][1], Ad = v.a[0][1];
-    const P X = v.px[1][1], Y = v.py[1][1];
+    const P w = K::bc(wy), dx = psub(u.x, c.x), dy = psub(u.y, c.y), sf = pmul(pp.hqd, K::bc(c.a.y + u.a.y));
+    k.tx = pmul(w, pfma(sf, c.y, dx));
+    k.ty = pmul(w, pnfma(sf, c.x, dy));
+    k.cr = pmul(w, pnfma(c.x, dy, pmul(c.y, dx)));
+    const S ey0 = u.a.x - c.a.x, eyr = u.ar.x - c.ar.x, eyl = u.al.x - c.al.x;
+    k.ex = u.ar.y - u.a.y;
+    k.exm = u.a.y - u.al.y;
+    k.s1 = ex0 + k.ex;
+    k.s2 = exm0 + k.exm;
+    k.tu = fma1(S(2.0f), ey0, hu);
+    k.qr = ey0 + eyr;
+    k.ql = ey0 + eyl;
+}
+
+// Gradient dF/dA (out[0..1]) and dF/dpsi_c (out[2 + 2c..]) at one site of row c
+// with the row u above it, restating gradientPsi (nlcg.cu:504-744) and
+// gradientA (nlcg.cu:746-888).  Both link ends use the mass of this site, as
+// the reference does.  xl, yl, xr, yr: psi of the columns left and right.  k:
+// the carry from the row below, replaced by the one into the row above.  W:
+// Wts or Ones.
+template <class S, int NC, class W>
+__device__ __forceinline__ void site_gradient(const GradView<S, NC> &c, const GradView<S, NC> &u,
+                                              const pack_t<S, NC> &xl, const pack_t<S, NC> &yl,
+                                              const pack_t<S, NC> &xr, const pack_t<S, NC> &yr,
+                                              const PackParams<S, NC> &pp, const W &w, const FieldSums<S> &h,
+                                              int maxwell, int thin_film, GradCarry<S, NC> &k, S *out)
+{
+    using K = Pk<S, NC>;
+    using P = pack_t<S, NC>;
+    constexpr bool ones = W::interior;
+    const P X = c.x, Y = c.y;
     const P r2 = pfma(Y, Y, pmul(X, X));
     const P m2r = pmul(r2, K::bc(S(-2.0f)));
-    P gx = K::bc(S(0.0f)), gy = gx, dg = gx, ga[2];
-#pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-        const S A = dir == 0 ? A0.x : A0.y, Af = dir == 0 ? Ar.x : Au.y, Ab = dir == 0 ? Al.x : Ad.y;
-        const P xf = dir == 0 ? v.px[1][2] : v.px[2][1], yf = dir == 0 ? v.py[1][2] : v.py[2][1];
-        const P xb = dir == 0 ? v.px[1][0] : v.px[0][1], yb = dir == 0 ? v.py[1][0] : v.py[0][1];
-        // weights -2 w / (2 m) of the forward and backward link
-        const P f = pmul(dir == 0 ? pp.n2hmx : pp.n2hmy, K::bc(dir == 0 ? w.wfx : w.wfy));
-        const P b = pmul(dir == 0 ? pp.n2hmx : pp.n2hmy, K::bc(dir == 0 ? w.wbx : w.wby));
-        const P dxf = psub(xf, X), dyf = psub(yf, Y), dxb = psub(xb, X), dyb = psub(yb, Y);
-        const P sf = pmul(pp.hqd, K::bc(A + Af)), sb = pmul(pp.nhqd, K::bc(A + Ab));
-        gx = pfma(f, pfma(sf, yf, dxf), gx);
-        gx = pfma(b, pfma(sb, yb, dxb), gx);
-        gy = pfma(f, pnfma(sf, xf, dyf), gy);
-        gy = pfma(b, pnfma(sb, xb, dyb), gy);
+    P gx, gy, dg, ga0, ga1;
+    {   // x-links; weights -2 w / (2 m) of the forward and backward one
+        const P f = ones ? pp.n2hmx : pmul(pp.n2hmx, K::bc(S(w.wfx)));
+        const P b = ones ? pp.n2hmx : pmul(pp.n2hmx, K::bc(S(w.wbx)));
+        const P dxf = psub(xr, X), dyf = psub(yr, Y), dxb = psub(xl, X), dyb = psub(yl, Y);
+        const P sf = pmul(pp.hqd, K::bc(c.a.x + c.ar.x)), sb = pmul(pp.nhqd, K::bc(c.a.x + c.al.x));
+        gx = pfma(b, pfma(sb, yl, dxb), pmul(f, pfma(sf, yr, dxf)));
+        gy = pfma(b, pnfma(sb, xl, dyb), pmul(f, pnfma(sf, xr, dyf)));
         // site term a^2 psi of both links, and the current through them
-        const P an = pmul(pp.nhqd, K::bc(A)), Wa = pmul(padd(f, b), an);   // -a / 2, W a
-        dg = pfma(Wa, an, dg);                                             // -W a^2 / 2
-        P c = pmul(Wa, m2r);
-        c = pfma(f, pnfma(X, dyf, pmul(Y, dxf)), c);
-        ga[dir] = pnfma(b, pnfma(X, dyb, pmul(Y, dxb)), c);
+        const P an = pmul(pp.nhqd, K::bc(c.a.x)), Wa = pmul(pmul(pp.n2hmx, K::bc(S(w.wsx))), an);   // -a / 2, W a
+        dg = pmul(Wa, an);                                                                          // -W a^2 / 2
+        const P cu = pfma(f, pnfma(X, dyf, pmul(Y, dxf)), pmul(Wa, m2r));
+        ga0 = pnfma(b, pnfma(X, dyb, pmul(Y, dxb)), cu);
     }
-    S g0 = K::sum(pmul(pp.nhqd, ga[0])), g1 = K::sum(pmul(pp.nhqd, ga[1]));
+    const P cr_below = k.cr;
+    {   // y-links: the one above, and the carried pull of the one below
+        const P dx = psub(u.x, X), dy = psub(u.y, Y), sf = pmul(pp.hqd, K::bc(c.a.y + u.a.y));
+        const P f = ones ? pp.n2hmy : pmul(pp.n2hmy, K::bc(S(w.wfy)));
+        gx = pfma(f, pfma(sf, u.y, dx), pnfma(pp.n2hmy, k.tx, gx));
+        gy = pfma(f, pnfma(sf, u.x, dy), pnfma(pp.n2hmy, k.ty, gy));
+        const P tx = pfma(sf, Y, dx), ty = pnfma(sf, X, dy), cr = pnfma(X, dy, pmul(Y, dx));
+        const P wf = K::bc(S(w.wfy));
+        k.tx = ones ? tx : pmul(wf, tx);
+        k.ty = ones ? ty : pmul(wf, ty);
+        k.cr = ones ? cr : pmul(wf, cr);
+        const P an = pmul(pp.nhqd, K::bc(c.a.y)), Wa = pmul(pmul(pp.n2hmy, K::bc(S(w.wsy))), an);
+        dg = pfma(Wa, an, dg);
+        ga1 = pfma(pp.n2hmy, padd(k.cr, cr_below), pmul(Wa, m2r));
+    }
+    const S g0 = K::sum(pmul(pp.nhqd, ga0)), g1 = K::sum(pmul(pp.nhqd, ga1));
     // condensation: 2 psi (a + b |psi|^2); density coupling with the other component
-    P k = pfma(pp.b2, r2, pp.a2);
+    P kk = pfma(pp.b2, r2, pp.a2);
+    const P m2 = K::bc(S(-2.0f));
     if constexpr (NC == 2) {
         const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y);
         const S x2 = K::template lane<1>(X), y2 = K::template lane<1>(Y);
-        k = pfma(K::bc(pp.gammad), K::mk(K::template lane<1>(r2), K::template lane<0>(r2)), k);
-        k = pfma(k, K::bc(w.area), pmul(dg, K::bc(S(-2.0f))));
-        gx = pfma(k, X, gx);
-        gy = pfma(k, Y, gy);
+        kk = pfma(K::bc(pp.gammad), K::mk(K::template lane<1>(r2), K::template lane<0>(r2)), kk);
+        kk = ones ? pfma(dg, m2, kk) : pfma(kk, K::bc(S(w.area)), pmul(dg, m2));
+        gx = pfma(kk, X, gx);
+        gy = pfma(kk, Y, gy);
         // eta psi_2 + delta (psi_1* psi_2) psi_2-like terms: e = eta + delta R, i = delta I
         const S R = fma1(y1, y2, x1 * x2), I = fma1(x1, y2, -(y1 * x2));
-        const S e = fma1(pp.deltad, R, pp.etad) * w.area, i = pp.deltad * I * w.area;
+        S e = fma1(pp.deltad, R, pp.etad), i = pp.deltad * I;
+        if (!ones) {
+            e = e * S(w.area);
+            i = i * S(w.area);
+        }
         out[2] = fma1(-i, y2, fma1(e, x2, K::template lane<0>(gx)));
         out[3] = fma1(i, x2, fma1(e, y2, K::template lane<0>(gy)));
         out[4] = fma1(i, y1, fma1(e, x1, K::template lane<1>(gx)));
         out[5] = fma1(-i, x1, fma1(e, y1, K::template lane<1>(gy)));
     } else {
-        k = pfma(k, K::bc(w.area), pmul(dg, K::bc(S(-2.0f))));
-        out[2] = pfma(k, X, gx);
-        out[3] = pfma(k, Y, gy);
+        kk = ones ? pfma(dg, m2, kk) : pfma(kk, K::bc(S(w.area)), pmul(dg, m2));
+        out[2] = pfma(kk, X, gx);
+        out[3] = pfma(kk, Y, gy);
     }
     if (maxwell)
 #pragma unroll
-        for (int c = 2; c < 2 + 2 * NC; ++c) out[c] = S(0.0f);
+        for (int q = 2; q < 2 + 2 * NC; ++q) out[q] = S(0.0f);
+    // magnetic views of this site and the neighbours' views of the same plaquettes
+    // (nlcg.cu:852-883), from the link differences ex(i,j) = A_y(i+1,j) - A_y(i,j)
+    // and ey(i,j) = A_x(i,j+1) - A_x(i,j); the lower side comes with the carry
+    const S s3 = k.s2, s4 = k.s1, td = k.tu, ql = k.ql, qr = k.qr, ex0 = k.ex, exm = k.exm, two = S(2.0f);
+    {
+        const S ey0 = u.a.x - c.a.x, eyr = u.ar.x - c.ar.x, eyl = u.al.x - c.al.x;
+        k.ex = u.ar.y - u.a.y;
+        k.exm = u.a.y - u.al.y;
+        k.s1 = ex0 + k.ex;
+        k.s2 = exm + k.exm;
+        k.tu = fma1(two, ey0, h.u);
+        k.qr = ey0 + eyr;
+        k.ql = ey0 + eyl;
+    }
     if (!thin_film) {
-        // link differences ex(i,j) = A_y(i+1,j) - A_y(i,j), ey(i,j) = A_x(i,j+1) - A_x(i,j)
-        const S two = S(2.0f);
-        const S ex0 = Ar.y - A0.y, exm = A0.y - Al.y, ey0 = Au.x - A0.x, eym = A0.x - Ad.x;
-        const S exu = v.a[2][2].y - Au.y, exmu = Au.y - v.a[2][0].y;
-        const S exd = v.a[0][2].y - Ad.y, exmd = Ad.y - v.a[0][0].y;
-        const S eyr = v.a[2][2].x - Ar.x, eyrm = Ar.x - v.a[0][2].x;
-        const S eyl = v.a[2][0].x - Al.x, eylm = Al.x - v.a[0][0].x;
-        // the views of this site and the neighbours' views of the same plaquettes (nlcg.cu:852-883)
-        const S tu = fma1(two, ey0, h.u), td = fma1(two, eym, h.d);
         const S tr = fma1(two, ex0, -h.r), tl = fma1(two, exm, -h.l);
-        S mx = w.vUR * ((ex0 + exu) - tu);
-        mx = fma1(w.vUL, (exm + exmu) - tu, mx);
-        mx = fma1(w.vLL, td - (exm + exmd), mx);
-        mx = fma1(w.vLR, td - (ex0 + exd), mx);
-        S my = w.vUR * ((ey0 + eyr) - tr);
-        my = fma1(w.vUL, tl - (ey0 + eyl), my);
-        my = fma1(w.vLL, tl - (eym + eylm), my);
-        my = fma1(w.vLR, (eym + eyrm) - tr, my);
+        S mx, my;
+        if constexpr (ones) {
+            mx = fma1(two, td - k.tu, (k.s1 + k.s2) - (s3 + s4));
+            my = fma1(two, tl - tr, (k.qr + qr) - (k.ql + ql));
+        } else {
+            mx = S(w.vUR) * (k.s1 - k.tu);
+            mx = fma1(S(w.vUL), k.s2 - k.tu, mx);
+            mx = fma1(S(w.vLL), td - s3, mx);
+            mx = fma1(S(w.vLR), td - s4, mx);
+            my = S(w.vUR) * (k.qr - tr);
+            my = fma1(S(w.vUL), tl - k.ql, my);
+            my = fma1(S(w.vLL), tl - ql, my);
+            my = fma1(S(w.vLR), qr - tr, my);
+        }
         out[0] = fma1(S(0.25f), mx, g0);
         out[1] = fma1(S(0.25f), my, g1);
     } else {
@@ -396,16 +474,52 @@ __device__ __forceinline__ void site_gradient(const PackView<S, NC> &v, const Pa
     }
 }
 
+// The same from a nine-point view (tile kernels): the carry is formed from the row below.
+template <class S, int NC>
+__device__ __forceinline__ void site_gradient(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
+                                              const FieldSums<S> &h, int maxwell, int thin_film, S *out)
+{
+    const GradView<S, NC> d{v.a[0][1], v.a[0][0], v.a[0][2], v.px[0][1], v.py[0][1]};
+    const GradView<S, NC> c{v.a[1][1], v.a[1][0], v.a[1][2], v.px[1][1], v.py[1][1]};
+    const GradView<S, NC> u{v.a[2][1], v.a[2][0], v.a[2][2], v.px[2][1], v.py[2][1]};
+    GradCarry<S, NC> k;
+    grad_up<S, NC>(d, c, pp, w.wby, h.d, d.ar.y - d.a.y, d.a.y - d.al.y, k);
+    site_gradient<S, NC>(c, u, v.px[1][0], v.py[1][0], v.px[1][2], v.py[1][2], pp, w, h, maxwell, thin_film, k, out);
+}
+
 // ------------------------------------------------------------ line quartic
-// Coefficients {A, B, C, D, E} of F(x + t d) at one site, without the common
-// dx^2 (polynomialExpansion, nlcg.cu:997-1370).  compat keeps the reference's
+// Sums of the coefficients {A, B, C, D, E} of F(x + t d): per-component packs,
+// scalars, and the magnetic sums with their factors outside.
+template <class S, int NC>
+struct PolySum {
+    pack_t<S, NC> ka, kb, kc, kd, ke;
+    S e, b, c, d, e4, em0, em1, em2;
+    __device__ __forceinline__ void zero()
+    {
+        ka = kb = kc = kd = ke = Pk<S, NC>::bc(S(0.0f));
+        e = b = c = d = e4 = em0 = em1 = em2 = S(0.0f);
+    }
+    __device__ __forceinline__ void total(const PackParams<S, NC> &pp, S (&o)[5]) const
+    {
+        using K = Pk<S, NC>;
+        o[0] = fma1(S(0.125f), em0, e + K::sum(ka));
+        o[1] = fma1(pp.idx4, em1, b + K::sum(kb));
+        o[2] = fma1(pp.idx8, em2, c + K::sum(kc));
+        o[3] = d + K::sum(kd);
+        o[4] = e4 + K::sum(ke);
+    }
+};
+
+// Adds the coefficients {A, B, C, D, E} of F(x + t d) at one site, without the
+// common dx^2 (polynomialExpansion, nlcg.cu:997-1370).  compat keeps the reference's
 // x-link first-order slip (its t-linear field term uses charge -1) and the
 // halved cubic coefficient of the y-links, as corrections to the exact form.
-template <class S, int NC>
+template <class S, int NC, class Wt>
 __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackView<S, NC> &dv,
-                                          const PackParams<S, NC> &pp, const Wts<S> &w, int per_site, int compat,
-                                          int thin_film, S *out)
+                                          const PackParams<S, NC> &pp, const Wt &w, int per_site, int compat,
+                                          int thin_film, PolySum<S, NC> &sum)
 {
+    constexpr bool ones = Wt::interior;
     using K = Pk<S, NC>;
     using P = pack_t<S, NC>;
     const S half = S(0.5f);
@@ -415,7 +529,7 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
     const P rh = pfma(Y, Vd, pmul(X, U)), n1 = padd(rh, rh);
     const P n2 = pfma(Vd, Vd, pmul(U, U));
     P w0, w1, w2, kd_y;   // site term (a + t b)^2 |psi + t d|^2 / 2 of the links: coefficients of its first factor
-    P ka, kb, kc, kd;
+    P ka = sum.ka, kb = sum.kb, kc = sum.kc, kd = sum.kd;
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
         // forward link i -> j: i the site, j its +x (dir 0) or +y (dir 1) neighbour
@@ -424,10 +538,10 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
         const P xj = dir == 0 ? v.px[1][2] : v.px[2][1], yj = dir == 0 ? v.py[1][2] : v.py[2][1];
         const P uj = dir == 0 ? dv.px[1][2] : dv.px[2][1], vj = dir == 0 ? dv.py[1][2] : dv.py[2][1];
         const P hm = dir == 0 ? pp.hmxi : pp.hmyi, hb = dir == 0 ? pp.hmxil : pp.hmyid;
-        const S wf = dir == 0 ? w.wfx : w.wfy, wb = dir == 0 ? w.wbx : w.wby, ws = dir == 0 ? w.wsx : w.wsy;
-        const P f = pmul(hm, K::bc(wf));
+        const S wf = S(dir == 0 ? w.wfx : w.wfy), wb = S(dir == 0 ? w.wbx : w.wby), ws = S(dir == 0 ? w.wsx : w.wsy);
+        const P f = ones ? hm : pmul(hm, K::bc(wf));
         // W (q dx)^2 / 2 with W the weights of both links of this direction at the site
-        const P W = pmul(pp.hqq, per_site ? pfma(hb, K::bc(wb), f) : pmul(hm, K::bc(ws)));
+        const P W = per_site ? pmul(pp.hqq, pfma(hb, K::bc(wb), f)) : pmul(dir == 0 ? pp.hqmx : pp.hqmy, K::bc(ws));
         const P W0 = K::bc(Ai * Ai), W1 = K::bc((Ai + Ai) * ai), W2 = K::bc(ai * ai);
         // Delta (Dy, Ey with the opposite sign), and Delta + s (y, x)
         const P Dx = psub(xj, X), Dy = psub(Y, yj), Ex = psub(uj, U), Ey = psub(Vd, vj);
@@ -439,19 +553,15 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
             w0 = pmul(W, W0);
             w1 = pmul(W, W1);
             w2 = pmul(W, W2);
-            ka = pmul(fDx, P0);
-            kb = pfma(fEx, P0, pmul(fDx, P1));
-            kc = pfma(fEx, P1, pmul(fDx, P2));
-            kd = pmul(fEx, P2);
         } else {
             w0 = pfma(W, W0, w0);
             w1 = pfma(W, W1, w1);
             w2 = pfma(W, W2, w2);
-            ka = pfma(fDx, P0, ka);
-            kb = pfma(fEx, P0, pfma(fDx, P1, kb));
-            kc = pfma(fEx, P1, pfma(fDx, P2, kc));
-            kd = pfma(fEx, P2, kd);
         }
+        ka = pfma(fDx, P0, ka);
+        kb = pfma(fEx, P0, pfma(fDx, P1, kb));
+        kc = pfma(fEx, P1, pfma(fDx, P2, kc));
+        kd = pfma(fEx, P2, kd);
         ka = pfma(fDy, Q0, ka);
         kb = pfma(fEy, Q0, pfma(fDy, Q1, kb));
         kc = pfma(fEy, Q1, pfma(fDy, Q2, kc));
@@ -480,25 +590,26 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
         }
     }
     // condensation b/2 (n0 + n1 t + n2 t^2)^2 and the site terms
-    const P bA = pmul(pp.b, K::bc(w.area)), bh = pmul(bA, K::bc(half));
+    const P bA = ones ? pp.b : pmul(pp.b, K::bc(S(w.area))), bh = pmul(bA, K::bc(half));
     const P U0 = pfma(bA, n0, w0), U1 = pfma(bA, n1, w1), V1 = pfma(bh, n1, w1), U2 = pfma(bh, n2, w2);
-    ka = pfma(w0, r0, pfma(pmul(bh, n0), n0, ka));
-    kb = pfma(w1, r0, pfma(n1, U0, kb));
-    kc = pfma(w2, r0, pfma(n1, V1, pfma(n2, U0, kc)));
+    sum.ka = pfma(w0, r0, pfma(pmul(bh, n0), n0, ka));
+    sum.kb = pfma(w1, r0, pfma(n1, U0, kb));
+    sum.kc = pfma(w2, r0, pfma(n1, V1, pfma(n2, U0, kc)));
     kd = pfma(w2, n1, pfma(n2, U1, kd));
     if (compat) kd = pnfma(kd_y, K::bc(half), kd);
-    const P ke = pmul(n2, U2);
-    S e = K::sum(ka), b1 = K::sum(kb), c2 = K::sum(kc), d3 = K::sum(kd), e4 = K::sum(ke);
+    sum.kd = kd;
+    sum.ke = pfma(n2, U2, sum.ke);
     if constexpr (NC == 2) {   // couplings between the components
         const S x1 = K::template lane<0>(X), y1 = K::template lane<0>(Y), x2 = K::template lane<1>(X), y2 = K::template lane<1>(Y);
         const S u1 = K::template lane<0>(U), v1 = K::template lane<0>(Vd), u2 = K::template lane<1>(U), v2 = K::template lane<1>(Vd);
         const S R0 = fma1(y1, y2, x1 * x2), R2 = fma1(v1, v2, u1 * u2);
         const S R1 = fma1(y1, v2, fma1(x1, u2, fma1(v1, y2, u1 * x2)));
-        const S ea = pp.eta * w.area;
+        S e = sum.e, b1 = sum.b, c2 = sum.c, d3 = sum.d, e4 = sum.e4;
+        const S ea = ones ? pp.eta : pp.eta * S(w.area);
         e = fma1(ea, R0, e);
         b1 = fma1(ea, R1, b1);
         c2 = fma1(ea, R2, c2);
-        const S ga = half * pp.gamma * w.area;
+        const S ga = ones ? half * pp.gamma : half * pp.gamma * S(w.area);
         const S g0 = ga * K::template lane<0>(r0), g1 = ga * K::template lane<0>(n1), g2 = ga * K::template lane<0>(n2);
         const S s0 = K::template lane<1>(r0), s1 = K::template lane<1>(n1), s2 = K::template lane<1>(n2);
         e = fma1(g0, s0, e);
@@ -509,7 +620,7 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
         if (!SkipZeroDelta<S>::v || pp.delta != S(0.0f)) {
             const S I0 = fma1(x1, y2, -(y1 * x2)), I2 = fma1(u1, v2, -(v1 * u2));
             const S I1 = fma1(-v1, x2, fma1(-y1, u2, fma1(u1, y2, x1 * v2)));
-            const S da = half * pp.delta * w.area, d2 = pp.delta * w.area;
+            const S d2 = ones ? pp.delta : pp.delta * S(w.area), da = half * d2;
             e = fma1(da, fma1(R0, R0, -(I0 * I0)), e);
             b1 = fma1(d2, fma1(R1, R0, -(I1 * I0)), b1);
             c2 = fma1(da, fma1(R1, R1, -(I1 * I1)), c2);
@@ -517,14 +628,20 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
             d3 = fma1(d2, fma1(R1, R2, -(I1 * I2)), d3);
             e4 = fma1(da, fma1(R2, R2, -(I2 * I2)), e4);
         }
+        sum.e = e;
+        sum.b = b1;
+        sum.c = c2;
+        sum.d = d3;
+        sum.e4 = e4;
     }
     if (!thin_film) {
         const Curl<S> c(v.a), q(dv.a);
         const S nh = -pp.h;
-        S em0 = S(0.0f), em1 = em0, em2 = em0;
+        S em0 = sum.em0, em1 = sum.em1, em2 = sum.em2;
 #define EMV(wv, yy, xx, dyy, dxx)                                                                        \
     {                                                                                                    \
-        const S m0 = fma1(pp.idx, yy - xx, nh), m1 = dyy - dxx, z0 = wv * m0, z1 = wv * m1;              \
+        const S m0 = fma1(pp.idx, yy - xx, nh), m1 = dyy - dxx;                                          \
+        const S z0 = ones ? m0 : S(wv) * m0, z1 = ones ? m1 : S(wv) * m1;                                \
         em0 = fma1(z0, m0, em0);                                                                         \
         em1 = fma1(z0, m1, em1);                                                                         \
         em2 = fma1(z1, m1, em2);                                                                         \
@@ -534,15 +651,10 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
         EMV(w.vLL, c.ym, c.xm, q.ym, q.xm)
         EMV(w.vLR, c.yp, c.xm, q.yp, q.xm)
 #undef EMV
-        e = fma1(S(0.125f), em0, e);
-        b1 = fma1(pp.idx4, em1, b1);
-        c2 = fma1(pp.idx8, em2, c2);
+        sum.em0 = em0;
+        sum.em1 = em1;
+        sum.em2 = em2;
     }
-    out[0] = e;
-    out[1] = b1;
-    out[2] = c2;
-    out[3] = d3;
-    out[4] = e4;
 }
 
 // B and J at one site (computeJBKernel, nlcg.cu:243-364).

@@ -21,7 +21,10 @@
 // strips' equal sharing of the quarters counts.  256 x 256 x 64, two
 // components, per step: 4.48 ms, 4.66 as shared-memory tiles of 256 threads
 // and two launches; 64 x 64 x 16, ten steps with reparametrization: 744 us
-// against 1070.  Float-float: 1.53 ms per step against 1.68.
+// against 1070.  Float-float: 1.53 ms per step against 1.68.  With what the
+// wider types save on top (the carry from row to row, rows of interior sites
+// without weights, one running sum per coefficient): FP64 3.92 ms, float-float
+// 1.43 ms per step.
 #pragma once
 
 constexpr int NTS = 32;   // threads per block of the strip kernels
@@ -273,6 +276,37 @@ struct GradRow {
     uint16_t m;
 };
 
+// Re and Im psi packs from a window row's psi slots.
+template <class T, int NC>
+__device__ __forceinline__ pack_t<T, NC> psi_x(const vec2_t<T> *p)
+{
+    if constexpr (NC == 1) return p[0].x;
+    else return Pk<T, NC>::mk(p[0].x, p[0].y);
+}
+template <class T, int NC>
+__device__ __forceinline__ pack_t<T, NC> psi_y(const vec2_t<T> *p)
+{
+    if constexpr (NC == 1) return p[0].y;
+    else return Pk<T, NC>::mk(p[NC - 1].x, p[NC - 1].y);
+}
+
+template <class T, int NC>
+__device__ __forceinline__ GradView<T, NC> grad_view(const GradRow<T, NC> &R)
+{
+    return GradView<T, NC>{R.x[0], R.al, R.ar, psi_x<T, NC>(R.x + 1), psi_y<T, NC>(R.x + 1)};
+}
+
+// The carry into row c from the row d below it.
+template <class T, int NC>
+__device__ __forceinline__ GradCarry<T, NC> grad_below(const GradRow<T, NC> &d, const GradRow<T, NC> &c,
+                                                       const PackParams<T, NC> &pp, const Wts<T> &w, T hd)
+{
+    GradCarry<T, NC> k;
+    const GradView<T, NC> vd = grad_view(d);
+    grad_up<T, NC>(vd, grad_view(c), pp, w.wby, hd, vd.ar.y - vd.a.y, vd.a.y - vd.al.y, k);
+    return k;
+}
+
 // Halo ring of the gradient pass: [row % 3][side][x, d][field].
 template <class T, int NC>
 using GradRing = vec2_t<T>[3][2][2][1 + NC];
@@ -340,8 +374,14 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef 
         strip_halo<T, NC, 2, 3>(ring[(j + 3) % 3], src, S, L, j, fields, true);
         m = strip_code(S, L, j);
     };
+    // FP64 and float-float rows hand their upper y-link and views on to the next
+    // (21 of 233 FP64 instructions); FP32 forms them again from the row below,
+    // because the carry costs 20 registers, i.e. warps (sweep of 16 strings:
+    // 15.8 ms against 16.5 with the carry)
+    constexpr bool CARRY = !std::is_same<T, float>::value;
     GradRow<T, NC> Rm, R0, Rp;
     V hp0[NC], hp1[NC];
+    GradCarry<T, NC> up;   // from the row below
     {   // the first three rows are loaded together: one memory latency, not three
         V ra[3][1 + NC], rb[3][1 + NC];
         uint16_t ma, mb;
@@ -350,6 +390,18 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef 
         load(rc, rm, j0 + 1, true);
         take(Rm, j0 - 1, hp0, ra, ma);
         take(R0, j0, hp0, rb, mb);
+        if constexpr (CARRY) {
+            // the link from row j0 - 1 with the weight and field sum that row j0 knows it by
+            Wts<T> w;
+            w.load(R0.m);
+            T hd = pp.hd + pp.hd;
+            if (S.per_site && L.cok) {
+                PackParams<T, NC> q = pp;
+                q.load_site(S, L.gi, j0, L.gi + S.nx * j0);
+                hd = field_sums(S, q, L.gi, j0, L.gi + S.nx * j0).d;
+            }
+            up = grad_below(Rm, R0, pp, w, hd);
+        }
     }
     const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
     T v[2] = {(T)0, (T)0};
@@ -367,25 +419,30 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef 
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) xout[c][s] = o[c];
         }
-        RegView<T, NC> w3;
-        w3.clear();
-        w3.a[0][0] = Rm.al; w3.a[0][1] = Rm.x[0]; w3.a[0][2] = Rm.ar;
-        w3.a[1][0] = R0.al; w3.a[1][1] = R0.x[0]; w3.a[1][2] = R0.ar;
-        w3.a[2][0] = Rp.al; w3.a[2][1] = Rp.x[0]; w3.a[2][2] = Rp.ar;
+        V pl[NC], pr[NC];   // psi of the columns left and right
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            w3.p[c][0][1] = Rm.x[1 + c];
-            w3.p[c][1][1] = R0.x[1 + c];
-            w3.p[c][2][1] = Rp.x[1 + c];
-            w3.p[c][1][0] = from_left2<T>(R0.x[1 + c], hp0[c], L.lane);
-            w3.p[c][1][2] = from_right<T>(R0.x[1 + c], hp0[c], L.lane);
+            pl[c] = from_left2<T>(R0.x[1 + c], hp0[c], L.lane);
+            pr[c] = from_right<T>(R0.x[1 + c], hp0[c], L.lane);
         }
+        bool inner = false;
+        if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
             if (S.per_site) pp.load_site(S, L.gi, j, s);
+            const GradView<T, NC> vc = grad_view(R0), vu = grad_view(Rp);
+            const FieldSums<T> h = field_sums(S, pp, L.gi, j, s);
             T g[2 + 2 * NC];
-            Wts<T> w;
-            w.load(R0.m);
-            site_gradient<T, NC>(pack_view(w3), pp, w, field_sums(S, pp, L.gi, j, s), f.maxwell, S.thin_film, g);
+            if (inner) {
+                if constexpr (std::is_same<T, double>::value)
+                    site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr),
+                                         pp, Ones(), h, f.maxwell, S.thin_film, up, g);
+            } else {
+                Wts<T> w;
+                w.load(R0.m);
+                if constexpr (!CARRY) up = grad_below(Rm, R0, pp, w, h.d);
+                site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr), pp,
+                                     w, h, f.maxwell, S.thin_film, up, g);
+            }
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) {
                 V gv;
@@ -393,11 +450,11 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef 
                 gv.y = g[2 * c + 1];
                 gcur[c][s] = gv;
                 const V go = R0.gold[c];
-                v[0] += gv.x * gv.x + gv.y * gv.y;
-                v[1] += gv.x * (gv.x - go.x) + gv.y * (gv.y - go.y);
+                v[0] = fma1(gv.x, gv.x, fma1(gv.y, gv.y, v[0]));
+                v[1] = fma1(gv.x, gv.x - go.x, fma1(gv.y, gv.y - go.y, v[1]));
             }
         }
-        Rm = R0;
+        if constexpr (!CARRY) Rm = R0;
         R0 = Rp;
 #pragma unroll
         for (int c = 0; c < NC; ++c) hp0[c] = hp1[c];
@@ -502,6 +559,10 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const TileRef t
     }
     const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
     T v[5] = {(T)0, (T)0, (T)0, (T)0, (T)0};
+    // FP32 adds up a site's terms first (they cancel); the wider types the strip's
+    constexpr bool WIDE = !std::is_same<T, float>::value;
+    PolySum<T, NC> sum;
+    sum.zero();
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
@@ -554,14 +615,25 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const TileRef t
             vx.p[c][2][1] = Rp.x[1 + c];
             vd.p[c][2][1] = Rp.d[1 + c];
         }
+        bool inner = false;
+        if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
             if (S.per_site) pp.load_site(S, L.gi, j, s);
-            T o[5];
-            Wts<T> w;
-            w.load(R0.m);
-            site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, w, S.per_site, f.poly_compat, S.thin_film, o);
+            if constexpr (!WIDE) sum.zero();
+            if (inner) {
+                if constexpr (std::is_same<T, double>::value)
+                    site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, Ones(), S.per_site, f.poly_compat, S.thin_film, sum);
+            } else {
+                Wts<T> w;
+                w.load(R0.m);
+                site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, w, S.per_site, f.poly_compat, S.thin_film, sum);
+            }
+            if constexpr (!WIDE) {
+                T o[5];
+                sum.total(pp, o);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) v[k] += o[k];
+                for (int k = 0; k < 5; ++k) v[k] += o[k];
+            }
         }
         xm_ax = R0.x[0].x;
         dm_ax = R0.d[0].x;
@@ -570,6 +642,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const TileRef t
     // the halo copy of the row below the tile may still be in flight: complete it before the
     // ring can be reused (the fused kernel runs more tiles in the same block)
     cp_async_wait_groups<0>();
+    if constexpr (WIDE) sum.total(pp, v);
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[5];
     __threadfence();
