@@ -8,6 +8,7 @@
 // scalars and per-tile partials.  The reference instead allocated and freed
 // scratch inside every call (mepgl/src/nlcg.cu:225-239,
 // mepgl/src/parallel_sum.cu:49-67, mepgl/src/interpolation.cu:410-480).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -138,7 +139,6 @@ void fill_desc(mepgl_ctx *c, int si, int img_base)
     D.F = s.F;
     D.ncomp = c->ncomp;
     D.tiles_x = (s.nx + TX - 1) / TX;
-    D.tiles_y = (s.ny + tile_rows(c->precision) - 1) / tile_rows(c->precision);
     D.img_base = img_base;
     D.thin_film = c->thin_film;
     D.per_site = s.uniform ? 0 : 1;
@@ -187,9 +187,7 @@ void free_scalars(mepgl_ctx *c)
     c->slab = c->dscratch = c->ds = c->ds_jb = nullptr;
     c->fqueue = nullptr;
     c->fstage = nullptr;
-    cudaFreeHost(c->mail);
-    c->mail = nullptr;
-    c->mail_cap = 0;
+    c->mail.clear();
 }
 
 void drop_graphs(mepgl_ctx *c)
@@ -216,6 +214,8 @@ int layout_strips(mepgl_ctx *c)
             D.rows = strip_rows(c->precision, paired, D.ny, most, slots);
             D.stiles_y = (D.ny + D.rows - 1) / D.rows;
             D.stile_base = base;
+            D.wrows = walk_rows(c->precision, D.ny, (long)D.F * D.tiles_x, c->sm_count);
+            D.wtiles_y = (D.ny + D.wrows - 1) / D.wrows;
             base += D.F * D.tiles_x * D.stiles_y;
             c->hdesc[si] = D;
         }
@@ -230,7 +230,7 @@ mepgl_status build_layout(mepgl_ctx *c)
     drop_graphs(c);
     free_scalars(c);
     c->hdesc.assign(c->strings.size(), StringDesc{});
-    int img = 0, most_tiles = 0;
+    int img = 0;
     c->batches.clear();
     c->string_batch.clear();
     for (size_t si = 0; si < c->strings.size(); ++si) {
@@ -245,8 +245,6 @@ mepgl_status build_layout(mepgl_ctx *c)
         B.s[in_batch] = D;
         B.n = in_batch + 1;
         c->string_batch.push_back((int)c->batches.size() - 1);
-        const int tiles = D.F * D.tiles_x * D.tiles_y;
-        most_tiles = most_tiles > tiles ? most_tiles : tiles;
         img += D.F;
     }
     c->total_images = img;
@@ -256,7 +254,12 @@ mepgl_status build_layout(mepgl_ctx *c)
     int fmax = 0;
     for (auto &s : c->strings) fmax = fmax > s.F ? fmax : s.F;
     // one allocation: the line-search grids, then what starts at zero, then the partial sums
-    const size_t n_part = (size_t)(most_tiles > n_stiles ? most_tiles : n_stiles) * 8 + 4096;
+    size_t n_part = (size_t)n_stiles * 8;
+    for (size_t k = 0; k < c->strings.size(); ++k) {   // also of the walks, and of the arc lengths per image and site block
+        const StringDesc &D = c->hdesc[k];
+        const size_t w = (size_t)D.F * D.tiles_x * D.wtiles_y * 8, arc = 2 * (size_t)D.F * arc_blocks(D);
+        n_part = std::max(n_part, std::max(w, arc));
+    }
     size_t at = 0;
     auto take = [&](size_t doubles) {
         const size_t o = at;
@@ -265,12 +268,14 @@ mepgl_status build_layout(mepgl_ctx *c)
     };
     const size_t o_xf = take(LS_GRID), o_xd = take(LS_GRID), tables = at;
     size_t o_img[7];
-    for (size_t &o : o_img) o = take(I);
-    const size_t o_poly = take(4 * I), o_scr = take(3 * I + 64), o_ds = take(fmax + 1), o_jb = take(fmax + 1),
-                 o_tick = take((I + 1) / 2), o_stage = take((I + 1) / 2), o_queue = take(1), o_status = take(8), zeroed = at,
+    for (int k = 0; k < 4; ++k) o_img[k] = take(I);
+    const size_t o_poly = take(4 * I), o_tick = take((I + 1) / 2), o_stage = take((I + 1) / 2), o_queue = take(1),
+                 o_mail = at;   // from here on what fetch() brings to the host
+    for (int k = 4; k < 7; ++k) o_img[k] = take(I);
+    const size_t o_status = take(8), o_scr = take(3 * I + 64), o_ds = take(fmax + 1), o_jb = take(fmax + 1), zeroed = at,
                  o_part = take(n_part);
     CK(c, cudaMalloc(&c->slab, at * sizeof(double)));
-    double **dst[7] = {&S.gn0, &S.gn1, &S.gdg, &S.beta, &S.alpha, &S.alpha_pend, &S.fenergy};
+    double **dst[7] = {&S.gn1, &S.gdg, &S.beta, &S.alpha_pend, &S.alpha, &S.gn0, &S.fenergy};
     for (int k = 0; k < 7; ++k) *dst[k] = c->slab + o_img[k];
     S.poly = c->slab + o_poly;
     S.part = c->slab + o_part;
@@ -297,8 +302,7 @@ mepgl_status build_layout(mepgl_ctx *c)
     }
     CK(c, cudaMemset(c->slab + tables, 0, (zeroed - tables) * sizeof(double)));
     CK(c, cudaMemcpy(c->slab, grid.data(), tables * sizeof(double), cudaMemcpyHostToDevice));   // waits for the zeros too
-    c->mail_cap = 3 * I;
-    CK(c, cudaMallocHost(&c->mail, (c->mail_cap + 8) * sizeof(double)));
+    c->mail.resize(zeroed - o_mail);
     c->host_s.assign(fmax, 0.0);
     c->host_sjb.assign(fmax, 0.0);
     return MEPGL_OK;
@@ -335,7 +339,7 @@ Launch string_launch(mepgl_ctx *c, int si)
 {
     Launch L = make_launch(c, c->string_batch[si]);
     L.str = &c->hdesc[si];
-    L.n_tiles = L.str->F * L.str->tiles_x * L.str->tiles_y;
+    L.n_tiles = L.str->F * L.str->tiles_x * L.str->wtiles_y;
     return L;
 }
 
@@ -507,19 +511,22 @@ mepgl_status nlcg_steps_body(mepgl_ctx *c, int iters, int use_cg, int maxwell)
 // per-image scalars after NLCG steps, a string of zero or non-finite arc
 // length.  Read on the stream after the work before it, then cleared; the
 // first raised flag is reported.
-int *mail_status(mepgl_ctx *c) { return reinterpret_cast<int *>(c->mail + c->mail_cap); }
-
-mepgl_status report_device_status(mepgl_ctx *c);
+mepgl_status report_device_status(mepgl_ctx *c, const int *st);
 
 mepgl_status check_device_status(mepgl_ctx *c)
 {
-    CK(c, cudaMemcpyAsync(mail_status(c), c->sc.status, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    int st[4];
+    CK(c, cudaMemcpyAsync(st, c->sc.status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    return report_device_status(c);
+    return report_device_status(c, st);
 }
 
-// Device doubles to the caller's arrays (NULL: skipped) through the pinned
-// buffer, with one wait for all of them and (check) the status flags.
+// Device doubles to the caller's arrays (NULL: skipped) and, with check, the
+// status flags.  All of them lie in the slab's mail part, so that one copy of
+// the range around them, and one wait, brings them; the unasked-for doubles
+// in between are a few KB.  The copy goes to pageable memory, which holds the
+// host until it is done: as quick as pinned memory at these sizes, and pinned
+// memory cost 150 us when the context went.
 struct Fetch {
     double *dst;
     const double *src;
@@ -528,30 +535,30 @@ struct Fetch {
 
 mepgl_status fetch(mepgl_ctx *c, std::initializer_list<Fetch> items, bool check)
 {
-    size_t at = 0;
+    const double *status = reinterpret_cast<const double *>(c->sc.status), *lo = check ? status : nullptr,
+                 *hi = check ? status + 2 : nullptr;
     for (const Fetch &f : items) {
         if (!f.dst) continue;
-        CK(c, cudaMemcpyAsync(c->mail + at, f.src, f.n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        at += f.n;
+        if (!lo || f.src < lo) lo = f.src;
+        if (!hi || f.src + f.n > hi) hi = f.src + f.n;
     }
-    if (check) CK(c, cudaMemcpyAsync(mail_status(c), c->sc.status, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (!lo) return MEPGL_OK;
+    double *mail = c->mail.data();
+    CK(c, cudaMemcpyAsync(mail, lo, (hi - lo) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    at = 0;
-    for (const Fetch &f : items) {
-        if (!f.dst) continue;
-        memcpy(f.dst, c->mail + at, f.n * sizeof(double));
-        at += f.n;
-    }
-    return check ? report_device_status(c) : MEPGL_OK;
+    for (const Fetch &f : items)
+        if (f.dst) memcpy(f.dst, mail + (f.src - lo), f.n * sizeof(double));
+    if (!check) return MEPGL_OK;
+    int st[4];
+    memcpy(st, mail + (status - lo), sizeof(st));
+    return report_device_status(c, st);
 }
 
-// The flags that the last copy brought; raised ones are cleared on the device.
-mepgl_status report_device_status(mepgl_ctx *c)
+// The flags that a copy brought; raised ones are cleared on the device.
+mepgl_status report_device_status(mepgl_ctx *c, const int *st)
 {
-    int st[4];
-    memcpy(st, mail_status(c), sizeof(st));
     if (!(st[STATUS_WAIT] | st[STATUS_NONFINITE] | st[STATUS_ARC])) return MEPGL_OK;
-    CK(c, cudaMemsetAsync(c->sc.status, 0, sizeof(st), c->stream));
+    CK(c, cudaMemsetAsync(c->sc.status, 0, 4 * sizeof(int), c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     if (st[STATUS_WAIT])
         return fail(c, MEPGL_ERR_CUDA, "fused NLCG launch: a per-image stage wait ran out; the steps are incomplete");
@@ -584,32 +591,27 @@ mepgl_status copy_fields(mepgl_ctx *c, StringHost &s, void *const *dst, const vo
     return MEPGL_OK;
 }
 
+// Squared distances between the images of string si, in the field metric
+// (metrics & 1, c->ds) and the (B, J) metric (metrics & 2, c->ds_jb).
+mepgl_status arc_distances(mepgl_ctx *c, int si, int metrics)
+{
+    mepgl_status st = flush(c);
+    if (st != MEPGL_OK) return st;
+    // B and J, where they are stored, go to the spare direction buffer (its contents are not needed)
+    CK(c, launch_arc_distances(string_launch(c, si), c->sc, c->xi, metrics, c->sm_count, c->strings[si].d[c->di ^ 1], c->ds,
+                               c->ds_jb));
+    c->launches += 2;
+    return MEPGL_OK;
+}
+
 // Arc length of string si into c->ds (fields) or c->ds_jb (B, J).
 mepgl_status arc_length(mepgl_ctx *c, int si, int metric, double **where)
 {
-    StringHost &s = c->strings[si];
-    mepgl_status st = flush(c);
+    *where = metric == MEPGL_METRIC_FIELDS ? c->ds : c->ds_jb;
+    mepgl_status st = arc_distances(c, si, metric == MEPGL_METRIC_FIELDS ? 1 : 2);
     if (st != MEPGL_OK) return st;
-    const void *fl[3];
-    int w[3];
-    int nf = 1 + c->ncomp;
-    if (metric == MEPGL_METRIC_FIELDS) {
-        for (int f = 0; f < nf; ++f) { fl[f] = s.x[c->xi][f]; w[f] = 2; }
-        *where = c->ds;
-    } else {
-        // B, J into the spare direction buffer (its contents are not needed)
-        void *b[1] = {s.d[c->di ^ 1][0]};
-        void *j[1][2] = {{s.d[c->di ^ 1][1], c->ncomp == 2 ? s.d[c->di ^ 1][2] : s.d[c->di ^ 1][1]}};
-        CK(c, launch_jb(string_launch(c, si), c->sc, c->xi, b, j));
-        c->launches += 1;
-        fl[0] = b[0]; w[0] = 1;
-        fl[1] = j[0][0]; w[1] = 2;
-        fl[2] = j[0][1]; w[2] = 2;
-        *where = c->ds_jb;
-    }
-    CK(c, launch_arc_length(c->precision, fl, w, nf, s.M(), s.F, c->sc.part, *where, c->sc.status + STATUS_ARC,
-                            c->stream));
-    c->launches += 2;
+    CK(c, launch_arc_cumulate(c->strings[si].F, *where, c->sc.status + STATUS_ARC, c->stream));
+    c->launches += 1;
     return MEPGL_OK;
 }
 
@@ -619,12 +621,10 @@ mepgl_status ensure_plan(mepgl_ctx *c, int F, int F_new)
     if (need <= c->plan_cap) return MEPGL_OK;
     RedistPlan &p = c->plan;
     cudaFree(p.k); cudaFree(p.w); cudaFree(p.h); cudaFree(p.dl); cudaFree(p.d); cudaFree(p.du); cudaFree(p.du2);
-    cudaFree(p.ipiv); cudaFree(p.status); cudaFree(p.aux);
+    cudaFree(p.ipiv); cudaFree(p.aux);
     CK(c, cudaMalloc(&p.aux, redist_aux_size(need) * sizeof(double)));
     CK(c, cudaMalloc(&p.k, need * sizeof(int)));
     CK(c, cudaMalloc(&p.ipiv, need * sizeof(int)));
-    CK(c, cudaMalloc(&p.status, 4 * sizeof(int)));
-    CK(c, cudaMemset(p.status, 0, 4 * sizeof(int)));
     for (double **q : {&p.w, &p.h, &p.dl, &p.d, &p.du, &p.du2}) CK(c, cudaMalloc(q, need * sizeof(double)));
     c->plan_cap = need;
     return MEPGL_OK;
@@ -657,16 +657,14 @@ mepgl_status redistribute(mepgl_ctx *c, int kind, int F_new)
     if (F < 2 || F_new < 2) return fail(c, MEPGL_ERR_INVALID_ARG, "redistribute: need at least 2 images");
     if (kind == MEPGL_REDIST_CUBIC && F < 4)
         return fail(c, MEPGL_ERR_INVALID_ARG, "cubic reparametrization needs at least 4 images");
-    double *sp = nullptr;
-    mepgl_status st = arc_length(c, 0, MEPGL_METRIC_FIELDS, &sp);
-    if (st != MEPGL_OK) return st;
-    st = arc_length(c, 0, MEPGL_METRIC_JB, &sp);
+    mepgl_status st = arc_distances(c, 0, 3);
     if (st != MEPGL_OK) return st;
     double *s_use = c->opt.metric == MEPGL_METRIC_FIELDS ? c->ds : c->ds_jb;
     st = ensure_plan(c, F, F_new);
     if (st != MEPGL_OK) return st;
     const int cubic = kind == MEPGL_REDIST_CUBIC;
-    CK(c, launch_redist_plan(s_use, F, F_new, cubic, c->opt.spline, c->plan, c->stream));
+    CK(c, launch_redist_plan(c->ds, c->ds_jb, s_use, c->sc.status, F, F_new, cubic, c->opt.spline, c->plan,
+                              c->stream));
     c->launches += 1;
     void *target[3] = {};
     const size_t rs = real_size(c->precision);
@@ -723,14 +721,13 @@ mepgl_status redistribute_into_spare(mepgl_ctx *c, int si, int kind)
     if (F < 2) return fail(c, MEPGL_ERR_INVALID_ARG, "redistribute: need at least 2 images");
     const int cubic = kind == MEPGL_REDIST_CUBIC;
     if (cubic && F < 4) return fail(c, MEPGL_ERR_INVALID_ARG, "cubic reparametrization needs at least 4 images");
-    double *sp = nullptr;
-    mepgl_status st = arc_length(c, si, MEPGL_METRIC_FIELDS, &sp);
-    if (st == MEPGL_OK) st = arc_length(c, si, MEPGL_METRIC_JB, &sp);
+    mepgl_status st = arc_distances(c, si, 3);
     if (st == MEPGL_OK) st = ensure_plan(c, F, F);
     if (st == MEPGL_OK && cubic) st = ensure_cubic_scratch(c, redist_cubic_scratch_bytes(c->precision, s.M(), F, F));
     if (st != MEPGL_OK) return st;
     double *s_use = c->opt.metric == MEPGL_METRIC_FIELDS ? c->ds : c->ds_jb;
-    CK(c, launch_redist_plan(s_use, F, F, cubic, c->opt.spline, c->plan, c->stream));
+    CK(c, launch_redist_plan(c->ds, c->ds_jb, s_use, c->sc.status, F, F, cubic, c->opt.spline, c->plan,
+                              c->stream));
     c->launches += 1;
     for (int f = 0; f < 1 + c->ncomp; ++f) {
         if (cubic)
@@ -894,7 +891,7 @@ mepgl_status mepgl_destroy(mepgl_ctx *c)
     c->refine = nullptr;
     RedistPlan &p = c->plan;
     cudaFree(p.k); cudaFree(p.w); cudaFree(p.h); cudaFree(p.dl); cudaFree(p.d); cudaFree(p.du); cudaFree(p.du2);
-    cudaFree(p.ipiv); cudaFree(p.status); cudaFree(p.aux);
+    cudaFree(p.ipiv); cudaFree(p.aux);
     cudaFree(c->cubic_scratch);
     if (c->copy_stream) {
         cudaStreamSynchronize(c->copy_stream);
@@ -1135,7 +1132,7 @@ mepgl_status mepgl_energy_grad(mepgl_ctx *c, double *fenergy, void *g_a, void *g
     }
     Launch L = string_launch(c, 0);
     L.paired = 0;   // the gradient a caller asks for is IEEE double in every FP64 mode
-    CK(c, launch_gradient_only(L, c->xi, out, 0));
+    CK(c, launch_gradient_only(L, c->sc, c->xi, out, 0));
     c->launches += 1;
     if (direct) {
         CK(c, cudaStreamSynchronize(c->stream));
@@ -1182,15 +1179,14 @@ mepgl_status mepgl_compute_jb(mepgl_ctx *c, void *b, void *j_1, void *j_2, int m
     mepgl_status st = flush(c);
     if (st != MEPGL_OK) return st;
     StringHost &s = c->strings[0];
-    void *bb[1] = {s.d[c->di ^ 1][0]};
-    void *jj[1][2] = {{s.d[c->di ^ 1][1], c->ncomp == 2 ? s.d[c->di ^ 1][2] : s.d[c->di ^ 1][1]}};
-    CK(c, launch_jb(string_launch(c, 0), c->sc, c->xi, bb, jj));
+    void *const *o = s.d[c->di ^ 1];
+    CK(c, launch_jb(string_launch(c, 0), c->sc, c->xi, o[0], o[1], o[2]));
     c->launches += 1;
     const size_t rs = real_size(c->precision), n = (size_t)s.F * s.M();
     const cudaMemcpyKind k = memory == MEPGL_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (b) CK(c, cudaMemcpyAsync(b, bb[0], n * rs, k, c->stream));
-    if (j_1) CK(c, cudaMemcpyAsync(j_1, jj[0][0], 2 * n * rs, k, c->stream));
-    if (j_2 && c->ncomp == 2) CK(c, cudaMemcpyAsync(j_2, jj[0][1], 2 * n * rs, k, c->stream));
+    if (b) CK(c, cudaMemcpyAsync(b, o[0], n * rs, k, c->stream));
+    if (j_1) CK(c, cudaMemcpyAsync(j_1, o[1], 2 * n * rs, k, c->stream));
+    if (j_2 && c->ncomp == 2) CK(c, cudaMemcpyAsync(j_2, o[2], 2 * n * rs, k, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     return MEPGL_OK;
 }
@@ -1213,11 +1209,8 @@ mepgl_status mepgl_batch_observables(mepgl_ctx *c, int string, int inset, double
     const int F = s.F;
     double *out = c->dscratch;      // flux, winding 1, winding 2: 3F doubles
     if (flux) {
-        void *bb[1] = {s.d[c->di ^ 1][0]};
-        void *jj[1][2] = {{s.d[c->di ^ 1][1], c->ncomp == 2 ? s.d[c->di ^ 1][2] : s.d[c->di ^ 1][1]}};
-        CK(c, launch_jb(string_launch(c, string), c->sc, c->xi, bb, jj));
-        CK(c, launch_flux(c->precision, bb[0], s.M(), F, s.dx * s.dx, out, c->stream));
-        c->launches += 2;
+        CK(c, launch_flux(string_launch(c, string), c->sc, c->xi, out));
+        c->launches += 1;
     }
     for (int k = 0; k < c->ncomp; ++k) {
         if (!(k == 0 ? winding_1 : winding_2)) continue;
@@ -1253,14 +1246,13 @@ mepgl_status mepgl_redistribute(mepgl_ctx *c, int kind, int F_new)
         return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_redistribute: unknown kind");
     mepgl_status st = redistribute(c, kind, F_new);
     if (st != MEPGL_OK) return st;
-    int *bad = mail_status(c) + 4;   // a singular spline matrix (cubic only), read with the status flags
-    *bad = 0;
-    if (kind == MEPGL_REDIST_CUBIC)
-        CK(c, cudaMemcpyAsync(bad, c->plan.status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    st = check_device_status(c);
+    int flags[5];
+    CK(c, cudaMemcpyAsync(flags, c->sc.status, sizeof(flags), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    st = report_device_status(c, flags);
     if (st != MEPGL_OK) return st;
-    if (*bad) {
-        CK(c, cudaMemset(c->plan.status, 0, sizeof(int)));
+    if (kind == MEPGL_REDIST_CUBIC && flags[STATUS_SPLINE]) {
+        CK(c, cudaMemset(c->sc.status + STATUS_SPLINE, 0, sizeof(int)));
         return fail(c, MEPGL_ERR_NAN, "spline matrix is singular (coincident images)");
     }
     return MEPGL_OK;

@@ -1,12 +1,12 @@
 // common.cuh -- shared device-side definitions of libmepgl_gb300.
 //
-// Work decomposition.  Every pass over the string is a list of tiles; a
-// tile is TX x TY sites of one image of one string.  Kernels walk the tile
-// list with a grid-stride loop, so one launch covers every image of up to
-// MAX_STRINGS strings (strings may differ in size and image count).
-// Per-image reductions are deterministic: each tile writes one partial per
-// quantity, and the last tile of an image to finish (atomic ticket per
-// image) sums that image's partials in a fixed order.
+// Work decomposition.  Every kernel over the lattice shares a string out as
+// strips of TX columns x some rows of one image, one warp each; a launch of
+// the NLCG passes covers every image of up to MAX_STRINGS strings (strings
+// may differ in size and image count).  Per-image reductions are
+// deterministic: each strip writes one partial per quantity, and the last
+// strip of an image to finish (atomic ticket per image) sums that image's
+// partials in a fixed order.
 //
 // Precision.  Fields are float or double (T).  Sums are formed in T inside
 // a block (fixed pairwise shuffle trees), then in double across tiles and
@@ -86,9 +86,10 @@ struct Uniform {
     T eta, gamma, delta, h, idx, dx2, dx;
     // the same with the spacing folded in, as the stencils of site_pack.cuh
     // use them: q dx, +- half of it, half of its square, (q + 1) dx, q / dx;
-    // -2 hm*, hm* / dx^2, and that times half of (q dx)^2; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
+    // -2 hm*, hm* / dx^2, and that times half of (q dx)^2; hm* q / dx; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
     // 1 / (4 dx), 1 / (8 dx^2)
-    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hqmx[2], hqmy[2], a2[2], b2[2];
+    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hqmx[2], hqmy[2], jmx[2], jmy[2],
+        a2[2], b2[2];
     T etad, gammad, deltad, hd, idx4, idx8;
 };
 
@@ -108,6 +109,8 @@ inline void fold_spacing(Uniform<double> &U)
         U.hmyi[c] = U.hmy[c] * U.idx * U.idx;
         U.hqmx[c] = U.hqq[c] * U.hmxi[c];
         U.hqmy[c] = U.hqq[c] * U.hmyi[c];
+        U.jmx[c] = U.hmx[c] * U.qi[c];
+        U.jmy[c] = U.hmy[c] * U.qi[c];
         U.a2[c] = 2.0 * U.a[c] * U.dx2;
         U.b2[c] = 2.0 * U.b[c] * U.dx2;
     }
@@ -142,6 +145,8 @@ inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
         r.hmyi[c] = T(U.hmyi[c]);
         r.hqmx[c] = T(U.hqmx[c]);
         r.hqmy[c] = T(U.hqmy[c]);
+        r.jmx[c] = T(U.jmx[c]);
+        r.jmy[c] = T(U.jmy[c]);
         r.a2[c] = T(U.a2[c]);
         r.b2[c] = T(U.b2[c]);
     }
@@ -166,10 +171,11 @@ inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
 // slots), d (direction, ping-pong).
 struct StringDesc {
     int nx, ny, F, ncomp;
-    int tiles_x, tiles_y;     // tiles per image
+    int tiles_x;              // strips across an image
     int img_base;             // first global image index of this string
     int rows;                 // rows per warp strip of the NLCG passes
-    int stiles_y, stile_base; // strips per column of an image; first global strip index
+    int stiles_y, stile_base; // strips down an image; first global strip index
+    int wrows, wtiles_y;      // the same of the walks over one string (walk.cuh)
     int thin_film;
     int disc;                 // 0: the reference's linearised differences, 1: gauge links
     int per_site;             // 1: parameters read from the arrays below
@@ -199,12 +205,10 @@ struct BatchOf {
 using Batch = BatchOf<MAX_STRINGS>;
 template <bool ONE> using batch_t = BatchOf<ONE ? 1 : MAX_STRINGS>;
 
-struct TileRef {
-    int16_t s;        // string within the batch
-    int16_t ty;       // tile row
-    int16_t tx;       // tile column
-    int16_t pad;
-    int32_t n;        // image
+struct StripRef {
+    int s;        // string within the batch
+    int ty, tx;   // strip row and column
+    int n;        // image
 };
 
 // Per-image scalars of the whole context (index = img_base + n).
@@ -271,39 +275,6 @@ __device__ __forceinline__ void block_sum(const T (&v)[NV], double (&out)[NV], d
         }
     }
     __syncthreads();
-}
-
-// Write this tile's NV partials; return true (in every thread) if this
-// block is the last of its image, in which case `tot` holds the image sums
-// (in thread 0) computed over the image's partials in index order.
-template <int NV, class T>
-__device__ __forceinline__ bool finish_image(const T (&v)[NV], double *smem, const Scalars &sc, int tile,
-                                             int first_tile, int tiles_per_image, int img, double (&tot)[NV])
-{
-    __shared__ bool last;
-    double mine[NV];
-    block_sum<NV>(v, mine, smem);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sc.part[(size_t)tile * 8 + k] = mine[k];
-        __threadfence();
-        const unsigned prev = atomicAdd(&sc.ticket[img], 1u);
-        last = (prev == (unsigned)tiles_per_image - 1);
-    }
-    __syncthreads();
-    if (!last) return false;
-    __threadfence();
-    double acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0;
-    for (int t = threadIdx.x; t < tiles_per_image; t += NT) {
-        const double *p = sc.part + (size_t)(first_tile + t) * 8;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) acc[k] += __ldcg(p + k);
-    }
-    block_sum<NV>(acc, tot, smem);
-    if (threadIdx.x == 0) sc.ticket[img] = 0;
-    return true;
 }
 
 }  // namespace mepgl

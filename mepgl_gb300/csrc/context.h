@@ -58,8 +58,7 @@ struct mepgl_ctx {
     bool pending = false;         // an NLCG update not yet applied to x
     int64_t launches = 0;
     std::string err;
-    double *mail = nullptr;       // pinned: results on their way to the caller, then the status flags
-    size_t mail_cap = 0;          // doubles of results it holds
+    std::vector<double> mail;     // results on their way to the caller, with the status flags
     std::map<std::tuple<int, int, int, int>, cudaGraphExec_t> graphs;
     std::vector<double> host_s, host_sjb;
     int sm_count = 152;

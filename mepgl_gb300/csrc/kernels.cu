@@ -17,10 +17,8 @@
 // x and d are ping-ponged because neighbouring strips read them as halo while
 // they are being rewritten.
 //
-// The energy, gradient, adjoint and B, J kernels work on tiles of 32 x
-// TileRows<T> sites staged with a one-site halo in shared memory; each thread
-// computes TileRows/8 sites of one column.  Addresses inside an image are
-// 32-bit offsets from per-tile base pointers.
+// Energies, gradients, adjoints and B, J of a string are formed by the same
+// kind of walk (walk.cuh).
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -28,13 +26,6 @@
 
 namespace mepgl {
 
-// Tuning knobs (compile time): tile rows per precision.
-#ifndef MEPGL_ROWS_F32
-#define MEPGL_ROWS_F32 40
-#endif
-#ifndef MEPGL_ROWS_F64
-#define MEPGL_ROWS_F64 8
-#endif
 // Resident single-warp blocks per SM asked of ptxas for the strip kernels
 // (registers per thread: 65536 / (32 x blocks)).  FP64 and float-float strips
 // hold twice the registers of FP32 ones; at 12 blocks they spill: a
@@ -66,9 +57,6 @@ template <> struct StripBlocks<float> {
 #ifndef MEPGL_FUSE_WAVES_F64
 #define MEPGL_FUSE_WAVES_F64 16
 #endif
-
-template <class T> struct TileRows { static constexpr int v = sizeof(T) == 4 ? MEPGL_ROWS_F32 : MEPGL_ROWS_F64; };
-template <> struct TileRows<ff> { static constexpr int v = MEPGL_ROWS_F64; };
 
 int fuse_waves(int precision) { return precision == 1 ? MEPGL_FUSE_WAVES_F64 : MEPGL_FUSE_WAVES; }
 
@@ -110,18 +98,33 @@ int strip_rows_cap(int precision, int paired)
     return precision == 0 ? MEPGL_STRIP_ROWS_F32 : paired ? MEPGL_STRIP_ROWS_FF : MEPGL_STRIP_ROWS_F64;
 }
 
-int strip_rows(int precision, int paired, int ny, long tiles, int slots)
+// ny rows in strips of equal height: `cap` rows, fewer (`least` at least) where
+// `tiles` strips of cap rows are fewer than `want`
+static int equal_rows(int ny, int cap, int least, long tiles, long want)
 {
-    const int cap = strip_rows_cap(precision, paired), least = precision == 0 ? 2 : 1;
-    const int fill = precision == 0 ? MEPGL_STRIP_FILL_F32 : paired ? MEPGL_STRIP_FILL_FF : MEPGL_STRIP_FILL_F64;
-    const long want = (long)slots * fill / 100;
     long rows = tiles < want ? cap * tiles / want : cap;
     if (rows < least) rows = least;
-    const long k = (ny + rows - 1) / rows;          // strips per column, of equal height
+    const long k = (ny + rows - 1) / rows;
     return (int)((ny + k - 1) / k);
 }
 
-int tile_rows(int precision) { return precision == 1 ? TileRows<double>::v : TileRows<float>::v; }
+int strip_rows(int precision, int paired, int ny, long tiles, int slots)
+{
+    const int fill = precision == 0 ? MEPGL_STRIP_FILL_F32 : paired ? MEPGL_STRIP_FILL_FF : MEPGL_STRIP_FILL_F64;
+    return equal_rows(ny, strip_rows_cap(precision, paired), precision == 0 ? 2 : 1, tiles, (long)slots * fill / 100);
+}
+
+#ifndef MEPGL_WALK_ROWS_F32
+#define MEPGL_WALK_ROWS_F32 8
+#endif
+#ifndef MEPGL_WALK_ROWS_F64
+#define MEPGL_WALK_ROWS_F64 8
+#endif
+int walk_rows(int precision, int ny, long columns, int sms)
+{
+    const int cap = precision == 0 ? MEPGL_WALK_ROWS_F32 : MEPGL_WALK_ROWS_F64;
+    return equal_rows(ny, cap, precision == 0 ? 2 : 1, columns * ((ny + cap - 1) / cap), (long)sms * 16);
+}
 
 cudaError_t upload_mask_tables()
 {
@@ -135,52 +138,6 @@ cudaError_t upload_mask_tables()
 }
 
 namespace {
-
-// Base pointers of one image's fields for one tile.
-template <class T, int NC>
-struct ImagePtrs {                  // storage type (double for float-float)
-    const vec2_t<store_t<T>> *in[1 + NC];
-};
-
-// ------------------------------------------------------------------ staging
-// The (TYT+2) x (TX+2) halo tile is split into flat element indices spread
-// over the block; each thread first issues every global load of all its
-// elements (independent, so they are in flight together), then stores them.
-// Out-of-lattice elements are zero.
-template <class T, int NC, int TYT>
-__device__ __forceinline__ void stage(Tile<T, NC, TYT> &t, const StringDesc &S, const ImagePtrs<T, NC> &ip, int i0, int j0)
-{
-    using V = vec2_t<T>;
-    constexpr int HW = TX + 2, HE = (TYT + 2) * HW, NI = (HE + NT - 1) / NT;
-    V f[NI][1 + NC];
-    uint16_t m[NI];
-#pragma unroll
-    for (int k = 0; k < NI; ++k) {
-        const int e = threadIdx.x + k * NT;
-        const int hy = e / HW, hx = e - hy * HW;
-        const int gi = i0 + hx - 1, gj = j0 + hy - 1;
-        const bool ok = e < HE && gi >= 0 && gi < S.nx && gj >= 0 && gj < S.ny;
-        m[k] = 0;
-#pragma unroll
-        for (int c = 0; c < 1 + NC; ++c) f[k][c].x = f[k][c].y = (T)0;
-        if (ok) {
-            const int s = gi + S.nx * gj;
-#pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) f[k][c] = load2<T>(ip.in[c] + s);
-            m[k] = S.mask ? S.mask[s] : (uint16_t)((S.code_comp[s] & 0xff) | ((S.code_sc[s] & 0xff) << 8));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NI; ++k) {
-        const int e = threadIdx.x + k * NT;
-        if (e >= HE) continue;
-        const int hy = e / HW, hx = e - hy * HW;
-        t.A[hy][hx] = f[k][0];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) t.P[c][hy][hx] = f[k][1 + c];
-        t.m[hy][hx] = m[k];
-    }
-}
 
 // Asynchronous copy of one element to shared memory, zero-filled where it is
 // not valid.
@@ -197,26 +154,6 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid)
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES),
                      "r"(n)
                      : "memory");
-}
-
-template <class T, int NC>
-__device__ __forceinline__ void image_ptrs(ImagePtrs<T, NC> &ip, void *const *in, size_t off)
-{
-#pragma unroll
-    for (int c = 0; c < 1 + NC; ++c) ip.in[c] = static_cast<const vec2_t<store_t<T>> *>(in[c]) + off;
-}
-
-// Tile tt of a string, in (image, row, column) order.
-__device__ __forceinline__ TileRef flat_tile(const StringDesc &S, int tt)
-{
-    const int tpi = S.tiles_x * S.tiles_y, n = tt / tpi, r = tt - n * tpi, ty = r / S.tiles_x;
-    TileRef t;
-    t.s = 0;
-    t.ty = (int16_t)ty;
-    t.tx = (int16_t)(r - ty * S.tiles_x);
-    t.pad = 0;
-    t.n = n;
-    return t;
 }
 
 // (h + h_neighbour) dx of the four neighbours of site s = (i, j).
@@ -406,197 +343,7 @@ __device__ double line_search(const double *coef, const Scalars &sc, int exact)
 // ------------------------------------------------------------------ kernels
 #include "strip.cuh"
 
-template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_energy(const __grid_constant__ StringDesc S, Scalars sc, int xbuf, double *out)
-{
-    constexpr int TYT = TileRows<T>::v;
-    __shared__ Tile<T, NC, TYT> t;
-    __shared__ double red[NT / 32];
-    const int tt = blockIdx.x;
-    const TileRef tr = flat_tile(S, tt);
-    const int img = S.img_base + tr.n;
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-    ImagePtrs<T, NC> ip;
-    image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
-    stage<T, NC, TYT>(t, S, ip, i0, j0);
-    PackParams<T, NC> pp;
-    pp.load(S);
-    __syncthreads();
-    T v[1] = {(T)0};
-    const int lx = threadIdx.x & 31, gi = i0 + lx;
-#pragma unroll
-    for (int r = 0; r < TYT / 8; ++r) {
-        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-        if (gi < S.nx && gj < S.ny) {
-            Wts<T> w;
-            w.load(t.m[ly + 1][lx + 1]);
-            if (S.disc) {
-                SiteParams<T> p;
-                p.load_uniform(S);
-                if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
-                v[0] += site_energy_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film);
-            } else {
-                if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
-                v[0] += site_energy<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, S.per_site, S.thin_film);
-            }
-        }
-    }
-    const int tpi = S.tiles_x * S.tiles_y;
-    double tot[1];
-    if (finish_image<1>(v, red, sc, tt, tr.n * tpi, tpi, img, tot) && threadIdx.x == 0)
-        out[img] = S.disc ? tot[0] : tot[0] * S.ud.dx2;
-}
-
-// Per-image dF/dH, dF/deta, dF/dgamma at fixed fields (out[3 img + k]).
-template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_param_adjoint(const __grid_constant__ StringDesc S, Scalars sc,
-                                                      int xbuf, double *out)
-{
-    constexpr int TYT = TileRows<T>::v;
-    __shared__ Tile<T, NC, TYT> t;
-    __shared__ double red[NT / 32 * 3];
-    const int tt = blockIdx.x;
-    const TileRef tr = flat_tile(S, tt);
-    const int img = S.img_base + tr.n;
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-    ImagePtrs<T, NC> ip;
-    image_ptrs<T, NC>(ip, S.x[xbuf], (size_t)tr.n * S.nx * S.ny);
-    stage<T, NC, TYT>(t, S, ip, i0, j0);
-    SiteParams<T> p;
-    p.load_uniform(S);
-    __syncthreads();
-    T v[3] = {(T)0, (T)0, (T)0};
-    const int lx = threadIdx.x & 31, gi = i0 + lx;
-#pragma unroll
-    for (int r = 0; r < TYT / 8; ++r) {
-        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-        if (gi < S.nx && gj < S.ny) {
-            Wts<T> w;
-            w.load(t.m[ly + 1][lx + 1]);
-            if (S.per_site) p.load_site(S, gi + S.nx * gj, NC);
-            if (S.disc) {
-                T u[3] = {(T)0, v[1], v[2]};
-                site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, 1, u);
-                v[1] = u[1];
-                v[2] = u[2];
-                if (!S.thin_film) v[0] += site_dh_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w);
-            } else {
-                site_param_adjoint<T, NC, TYT>(t, lx + 1, ly + 1, p, w, S.thin_film, v);
-            }
-        }
-    }
-    const int tpi = S.tiles_x * S.tiles_y;
-    double tot[3];
-    if (finish_image<3>(v, red, sc, tt, tr.n * tpi, tpi, img, tot) &&
-        threadIdx.x == 0) {
-        out[3 * img] = tot[0];
-        out[3 * img + 1] = tot[1];
-        out[3 * img + 2] = tot[2];
-    }
-}
-
-template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_gradient_only(const __grid_constant__ StringDesc S, int xbuf,
-                                                      FieldPtrs out, int maxwell)
-{
-    constexpr int TYT = TileRows<T>::v;
-    using V = vec2_t<T>;
-    __shared__ Tile<T, NC, TYT> t;
-    const int tt = blockIdx.x;
-    const TileRef tr = flat_tile(S, tt);
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-    const size_t off = (size_t)tr.n * S.nx * S.ny;
-    ImagePtrs<T, NC> ip;
-    image_ptrs<T, NC>(ip, S.x[xbuf], off);
-    stage<T, NC, TYT>(t, S, ip, i0, j0);
-    PackParams<T, NC> pp;
-    pp.load(S);
-    __syncthreads();
-    const int lx = threadIdx.x & 31, gi = i0 + lx;
-#pragma unroll
-    for (int r = 0; r < TYT / 8; ++r) {
-        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-        if (gi < S.nx && gj < S.ny) {
-            const int s = gi + S.nx * gj;
-            Wts<T> w;
-            w.load(t.m[ly + 1][lx + 1]);
-            T g[2 + 2 * NC];
-            bool link = false;
-            if constexpr (!std::is_same<T, ff>::value) link = S.disc != 0;   // float-float: the reference form only
-            if (link) {
-                if constexpr (!std::is_same<T, ff>::value) {
-                    SiteParams<T> p;
-                    p.load_uniform(S);
-                    T hl = p.h, hd = p.h;
-                    T hmx_l[2] = {p.hmx[0], p.hmx[1]}, hmy_d[2] = {p.hmy[0], p.hmy[1]};
-                    if (S.per_site) {
-                        p.load_site(S, s, NC);
-                        hl = static_cast<const T *>(S.ph)[s > 0 ? s - 1 : s];
-                        hd = static_cast<const T *>(S.ph)[gj > 0 ? s - S.nx : s];
-                        for (int c = 0; c < NC; ++c) {
-                            if (gi > 0) hmx_l[c] = (T)0.5 / static_cast<const T *>(S.pmxx[c])[s - 1];
-                            if (gj > 0) hmy_d[c] = (T)0.5 / static_cast<const T *>(S.pmyy[c])[s - S.nx];
-                        }
-                    }
-                    site_gradient_link<T, NC, TYT>(t, lx + 1, ly + 1, p, w, hl, hd, hmx_l, hmy_d, maxwell,
-                                                   S.thin_film, g);
-                }
-            } else {
-                if (S.per_site) pp.load_site(S, gi, gj, s);
-                site_gradient<T, NC>(pack_view_tile(t, lx + 1, ly + 1), pp, w, field_sums(S, pp, gi, gj, s),
-                                     maxwell, S.thin_film, g);
-            }
-#pragma unroll
-            for (int c = 0; c < 1 + NC; ++c) {
-                V gv;
-                gv.x = g[2 * c];
-                gv.y = g[2 * c + 1];
-                store2<T>(static_cast<vec2_t<store_t<T>> *>(out.p[c]) + off + s, gv);
-            }
-        }
-    }
-}
-
-template <class T, int NC>
-__global__ void __launch_bounds__(NT) k_jb(const __grid_constant__ StringDesc S, int xbuf, T *b, vec2_t<T> *j1, vec2_t<T> *j2)
-{
-    constexpr int TYT = TileRows<T>::v;
-    using V = vec2_t<T>;
-    __shared__ Tile<T, NC, TYT> t;
-    const int tt = blockIdx.x;
-    const TileRef tr = flat_tile(S, tt);
-    const int i0 = tr.tx * TX, j0 = tr.ty * TYT;
-    const size_t off = (size_t)tr.n * S.nx * S.ny;
-    ImagePtrs<T, NC> ip;
-    image_ptrs<T, NC>(ip, S.x[xbuf], off);
-    stage<T, NC, TYT>(t, S, ip, i0, j0);
-    PackParams<T, NC> pp;
-    pp.load(S);
-    __syncthreads();
-    const int lx = threadIdx.x & 31, gi = i0 + lx;
-#pragma unroll
-    for (int r = 0; r < TYT / 8; ++r) {
-        const int ly = (threadIdx.x >> 5) + 8 * r, gj = j0 + ly;
-        if (gi < S.nx && gj < S.ny) {
-            const size_t k = off + gi + (size_t)S.nx * gj;
-            Wts<T> w;
-            w.load(t.m[ly + 1][lx + 1]);
-            if (S.per_site) pp.load_site(S, gi, gj, gi + S.nx * gj);
-            T o[1 + 2 * NC];
-            site_jb<T, NC>(pack_view_tile(t, lx + 1, ly + 1), S.template u<T>().idx, pp, w, o);
-            b[k] = o[0];
-            V v;
-            v.x = o[1];
-            v.y = o[2];
-            j1[k] = v;
-            if (NC == 2) {
-                v.x = o[3];
-                v.y = o[4];
-                j2[k] = v;
-            }
-        }
-    }
-}
+#include "walk.cuh"
 
 // x += alpha_pend[image] d over every string of a batch: block (chunk, image
 // of the batch, field).  W: the compute type of the NLCG passes that wrote d
@@ -672,8 +419,8 @@ __global__ void __launch_bounds__(NT) k_x_format(double2 *x, long n)
     }
 }
 
-// Arc length: squared image-to-image distance over every site (no mask, no
-// dx^2; interpolation.cu:39-92).  Block (bx, n) covers sites
+// Arc length from stored arrays: squared image-to-image distance over every
+// site (no mask, no dx^2; interpolation.cu:39-92).  Block (bx, n) covers sites
 // [bx * NT * ARC_SPT, ...) of image n against image n - 1: each thread issues
 // all its loads of both images, then adds them in the fixed order (site,
 // field, component), so each (image, site block) partial is the same sum
@@ -820,22 +567,6 @@ __global__ void k_generate(vec2_t<T> *a, vec2_t<T> *p1, vec2_t<T> *p2, int nx, i
     }
 }
 
-// Magnetic flux of every image: Phi_n = dx^2 sum_sites B (post.py:131-133);
-// one block per image, double sums in a fixed order.
-template <class T>
-__global__ void k_flux(const T *__restrict__ b, long M, int F, double dx2, double *out)
-{
-    __shared__ double red[NT / 32];
-    for (int n = blockIdx.x; n < F; n += gridDim.x) {
-        const T *bn = b + (size_t)n * M;
-        double v[1] = {0.0};
-        for (long s = threadIdx.x; s < M; s += NT) v[0] += (double)bn[s];
-        double tot[1];
-        block_sum<1>(v, tot, red);
-        if (threadIdx.x == 0) out[n] = tot[0] * dx2;
-    }
-}
-
 // Winding sum of one field per image (compute_winding, gl_utils.py:10-41):
 // around the rectangle `inset` sites inside the lattice edge, counter-
 // clockwise from the lower-left corner, sum of the linearised phase steps
@@ -876,17 +607,23 @@ __global__ void k_winding(const vec2_t<T> *__restrict__ psi, int nx, int ny, int
     }
 }
 
-// computeArcLength (interpolation.cu:126-140), first half: block n adds
-// image n's partials.
-__global__ void k_arc_sum(const double *part, int nblocks, double *s)
+// computeArcLength (interpolation.cu:126-140), first half: block (n, metric)
+// adds image n's partials.
+__global__ void k_arc_sum(const double *part_f, const double *part_jb, int nblocks, double *s_f, double *s_jb)
 {
     __shared__ double red[NT / 32];
     const int n = blockIdx.x;
-    double v[1] = {0.0};
-    for (int b = threadIdx.x; b < nblocks; b += NT) v[0] += part[(size_t)n * nblocks + b];
-    double tot[1];
-    block_sum<1>(v, tot, red);
-    if (threadIdx.x == 0) s[n] = tot[0];
+    const double *part = blockIdx.y ? part_jb : part_f;
+    double v = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += NT) v += part[(size_t)n * nblocks + b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < NT / 32; ++k) v += red[k];
+        (blockIdx.y ? s_jb : s_f)[n] = v;
+    }
 }
 
 // Second half: cumulative sqrt, normalised so that s[F-1] = 1.  The square
@@ -904,42 +641,53 @@ constexpr int ARC_CUM_MAX = 4096;
 
 __device__ __forceinline__ bool arc_total_ok(double t) { return t > 0.0 && t <= 1.7976931348623157e308; }
 
-__global__ void k_arc_cumulate(int F, double *s, int *bad)
+// By a whole block, for one or two metrics (s[1] null: one), whose additions
+// run at the same time in the first threads of two warps; r: 2 F doubles of
+// shared memory, or null (then everything in those threads).
+__device__ void arc_cumulate(int F, double *const (&s)[2], int *bad, double *r)
 {
-    __shared__ double r[ARC_CUM_MAX];
-    __shared__ double total;
+    __shared__ double total[2];
+    const int metrics = s[1] ? 2 : 1;
     if (F == 1) {     // a single image has no length to normalise
-        if (threadIdx.x == 0) s[0] = 0.0;
+        if (threadIdx.x == 0)
+            for (int m = 0; m < metrics; ++m) s[m][0] = 0.0;
         return;
     }
-    if (F > ARC_CUM_MAX) {
-        if (threadIdx.x == 0) {
-            double acc = 0.0;
-            s[0] = 0.0;
-            for (int n = 1; n < F; ++n) {
-                acc += sqrt(s[n]);
-                s[n] = acc;
-            }
-            const bool ok = arc_total_ok(acc);
-            if (!ok) atomicExch(bad, 1);
-            for (int n = 0; n < F; ++n) s[n] = ok ? s[n] / acc : (double)n / (double)(F - 1);
-        }
-        return;
-    }
-    for (int n = threadIdx.x; n < F; n += blockDim.x) r[n] = n == 0 ? 0.0 : sqrt(s[n]);
+    if (r)
+        for (int m = 0; m < metrics; ++m)
+            for (int n = threadIdx.x; n < F; n += blockDim.x) r[m * F + n] = n == 0 ? 0.0 : sqrt(s[m][n]);
     __syncthreads();
-    if (threadIdx.x == 0) {
+    const int m = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0 && m < metrics) {
         double acc = 0.0;
-        for (int n = 1; n < F; ++n) {
-            acc += r[n];
-            r[n] = acc;
+        if (r) {
+            for (int n = 1; n < F; ++n) {
+                acc += r[m * F + n];
+                r[m * F + n] = acc;
+            }
+        } else {
+            s[m][0] = 0.0;
+            for (int n = 1; n < F; ++n) {
+                acc += sqrt(s[m][n]);
+                s[m][n] = acc;
+            }
         }
-        total = acc;
+        total[m] = acc;
         if (!arc_total_ok(acc)) atomicExch(bad, 1);
     }
     __syncthreads();
-    const bool ok = arc_total_ok(total);
-    for (int n = threadIdx.x; n < F; n += blockDim.x) s[n] = ok ? r[n] / total : (double)n / (double)(F - 1);
+    for (int k = 0; k < metrics; ++k) {
+        const bool ok = arc_total_ok(total[k]);
+        const double *from = r ? r + k * F : s[k];
+        for (int n = threadIdx.x; n < F; n += blockDim.x) s[k][n] = ok ? from[n] / total[k] : (double)n / (double)(F - 1);
+    }
+}
+
+__global__ void k_arc_cumulate(int F, double *s_f, double *s_jb, int *bad, int use_smem)
+{
+    extern __shared__ double cum_sm[];
+    double *const s[2] = {s_f ? s_f : s_jb, s_f ? s_jb : nullptr};
+    arc_cumulate(F, s, bad, use_smem ? cum_sm : nullptr);
 }
 
 // Finiteness of the per-image scalars after a call's NLCG steps: the energy
@@ -962,20 +710,26 @@ __global__ void k_check_scalars(const double *fenergy, const double *gn, int n_i
 // Redistribution plan: segment and weight per output image, and for the
 // cubic spline the Forsythe-Malcolm-Moler matrix (buildHMatrix,
 // interpolation.cu:252-290) factorised once by Gaussian elimination with
-// partial pivoting (the LAPACK gtsv algorithm) for every site's system.
-// One block of 32 threads.  The segment walk and the elimination are
-// sequential (thread 0); everything that is not (differences h, output
-// positions, weights, and the reciprocals and per-image coefficients that
-// spare the cubic resample its divisions) is spread over the block, because
-// every FP64 division and square root is slow on this GPU.  The arrays live
-// in shared memory when they fit, else in the plan's global arrays.
+// partial pivoting (the LAPACK gtsv algorithm) for every site's system.  One
+// block.
+//
+// What bounds it is the chain of dependent FP64 operations: an addition takes
+// tens of clocks here, a division hundreds.  So the segments are found by
+// bisection, one thread per output image, and the elimination's pivots come
+// from the continuants p_q = d_q p_{q-1} - dl_q du_{q-1} p_{q-2} (a multiply-add
+// per image; d'_q = p_q / p_{q-1} are then independent divisions), polished by
+// two sweeps of d'_q = d_q - dl_q du_{q-1} / d'_{q-1}, each of which shrinks an
+// error by dl_q du_{q-1} / d'_{q-1}^2 <= 1/4.  If a pivot would have been exchanged, or one is not
+// a normal number, the elimination runs as written.  With both
+// cumulations before it, 32 images, cubic: 45 us -> 26; 64 images, linear: 34 us
+// -> 14.  The arrays live in shared memory when they fit, else in the plan's
+// global arrays (elimination by one thread).
 
-// Shared-memory bytes of the plan kernel: s, h, dl, d, du, du2 [F or F+1],
-// output positions and segment starts [F_new] as doubles; ipiv [F] and the
-// segments [F_new] as ints.
+// Shared-memory bytes of the plan kernel: s, h, dl, d, du, du2 and two more
+// [F or F+1] as doubles; ipiv [F] and the segments [F_new] as ints.
 __host__ __device__ inline size_t redist_plan_smem(int F, int F_new)
 {
-    return (size_t)(6 * F + 1 + 2 * F_new) * sizeof(double) + (size_t)(F + F_new) * sizeof(int);
+    return (size_t)(8 * F + 1) * sizeof(double) + (size_t)(F + F_new) * sizeof(int);
 }
 
 // Weight of the segment's end image.  A segment of zero length (two equal
@@ -983,13 +737,59 @@ __host__ __device__ inline size_t redist_plan_smem(int F, int F_new)
 // both ends are the same state.
 __device__ __forceinline__ double redist_weight(double num, double len) { return len != 0.0 ? num / len : 1.0; }
 
-__global__ void k_redist_plan(const double *s_in, int F, int F_new, int cubic, int spline, RedistPlan p, int use_smem)
+// Smallest k in [1, last] with e[k] >= x, else last (e does not decrease).
+__device__ __forceinline__ int first_not_below(const double *e, double x, int last)
 {
-    if (blockIdx.x != 0) return;
+    int lo = 1, hi = last;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (e[mid] < x) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// gtsv's elimination, in place, by one thread.
+__device__ void eliminate(int F, double *dl, double *d, double *du, double *du2, int *ipiv)
+{
+    for (int q = 0; q < F - 1; ++q) {
+        const double sub = dl[q + 1];
+        if (fabs(d[q]) >= fabs(sub)) {
+            if (d[q] != 0) {
+                const double l = sub / d[q];
+                dl[q + 1] = l;
+                d[q + 1] = d[q + 1] - l * du[q];
+            } else {
+                dl[q + 1] = 0;
+            }
+        } else {
+            const double l = d[q] / sub;
+            d[q] = sub;
+            dl[q + 1] = l;
+            const double tmp = du[q];
+            du[q] = d[q + 1];
+            d[q + 1] = tmp - l * d[q + 1];
+            if (q < F - 2) {
+                du2[q] = du[q + 1];
+                du[q + 1] = -l * du[q + 1];
+            }
+            ipiv[q] = 1;
+        }
+    }
+}
+
+// s_f and s_jb hold squared distances, which become arc lengths first (the
+// plan is made on s_use, one of the two).
+__global__ void k_redist_plan(double *s_f, double *s_jb, const double *s_use, int *status, int F, int F_new, int cubic,
+                              int spline, RedistPlan p, int use_smem)
+{
     extern __shared__ double plan_sm[];
     const int t = threadIdx.x, nt = blockDim.x;
-    const double *s = s_in;
-    double *h = p.h, *dl = p.dl, *d = p.d, *du = p.du, *du2 = p.du2, *snew = nullptr, *sst = nullptr;
+    double *const both[2] = {s_f, s_jb};
+    arc_cumulate(F, both, status + STATUS_ARC, use_smem ? plan_sm : nullptr);
+    __syncthreads();
+    const double *s = s_use;
+    double *h = p.h, *dl = p.dl, *d = p.d, *du = p.du, *du2 = p.du2, *w1 = nullptr, *w2 = nullptr;
     int *ipiv = p.ipiv, *kk = p.k;
     if (use_smem) {
         double *ss = plan_sm;
@@ -998,84 +798,94 @@ __global__ void k_redist_plan(const double *s_in, int F, int F_new, int cubic, i
         d = dl + F;
         du = d + F;
         du2 = du + F;
-        snew = du2 + F;
-        sst = snew + F_new;
-        ipiv = reinterpret_cast<int *>(sst + F_new);
+        w1 = du2 + F;
+        w2 = w1 + F;
+        ipiv = reinterpret_cast<int *>(w2 + F);
         kk = ipiv + F;
-        for (int n = t; n < F; n += nt) ss[n] = s_in[n];
+        for (int n = t; n < F; n += nt) ss[n] = s_use[n];
         s = ss;
         __syncthreads();
     }
     // h[n] = s[n] - s[n-1]; output positions n / (F_new - 1)
     for (int n = t; n <= F; n += nt) h[n] = n == 0 ? 0.0 : (n == F ? INFINITY : s[n] - s[n - 1]);
-    if (use_smem)
-        for (int n = t; n < F_new; n += nt) snew[n] = (double)n / (double)(F_new - 1);
     __syncthreads();
-    const bool walk_sum = cubic && spline == 0;
-    if (t == 0) {
-        // segment walk (comparisons and additions only when the positions are staged)
-        int k = 1;
-        double seg_start = 0.0, seg_end = walk_sum ? h[1] : s[1];
-        for (int n = 0; n < F_new; ++n) {
-            const double s_new = use_smem ? snew[n] : (double)n / (double)(F_new - 1);
-            if (walk_sum) {
-                while (seg_end < s_new) { k++; seg_start += h[k - 1]; seg_end += h[k]; }
-            } else {
-                while (seg_end < s_new && k < F - 1) { k++; seg_start = s[k - 1]; seg_end = s[k]; }
-            }
-            if (k >= F) k = F - 1;
-            kk[n] = k;
-            if (use_smem) sst[n] = seg_start;
-            else p.w[n] = redist_weight(s_new - seg_start, cubic ? h[k] : (s[k] - s[k - 1]));
-        }
+    // Segment k ends at s[k].  The reference's cubic walks by running sums of h
+    // (interpolation.cu:380-386), which are s again up to rounding; where theirs
+    // ends below 1 it reads past its array, and the last image comes from the
+    // wrong segment.  s itself ends at 1.
+    for (int n = t; n < F_new; n += nt) {
+        const double s_new = (double)n / (double)(F_new - 1);
+        const int k = first_not_below(s, s_new, F - 1);
+        const double start = k > 1 ? s[k - 1] : 0.0;
+        kk[n] = k;
+        p.k[n] = k;
+        p.w[n] = redist_weight(s_new - start, cubic ? h[k] : (s[k] - s[k - 1]));
     }
     __syncthreads();
-    if (use_smem)
-        for (int n = t; n < F_new; n += nt) {
-            const int k = kk[n];
-            p.k[n] = k;
-            p.w[n] = redist_weight(snew[n] - sst[n], cubic ? h[k] : (s[k] - s[k - 1]));
-        }
     if (!cubic) {
         if (use_smem)
             for (int n = t; n <= F; n += nt) p.h[n] = h[n];
         return;
     }
-    if (t == 0) {
-        for (int n = 0; n < F; ++n) { dl[n] = d[n] = du[n] = du2[n] = 0.0; ipiv[n] = 0; }
-        d[0] = -h[1];
-        du[0] = h[1];
-        for (int n = 1; n < F - 1; ++n) { dl[n] = h[n]; d[n] = 2 * (h[n] + h[n + 1]); du[n] = h[n + 1]; }
-        dl[F - 1] = h[F - 1];
-        d[F - 1] = -h[F - 1];
-        for (int q = 0; q < F - 1; ++q) {
-            const double sub = dl[q + 1];
-            if (fabs(d[q]) >= fabs(sub)) {
-                if (d[q] != 0) {
-                    const double l = sub / d[q];
-                    dl[q + 1] = l;
-                    d[q + 1] = d[q + 1] - l * du[q];
-                } else {
-                    dl[q + 1] = 0;
-                }
-            } else {
-                const double l = d[q] / sub;
-                d[q] = sub;
-                dl[q + 1] = l;
-                const double tmp = du[q];
-                du[q] = d[q + 1];
-                d[q + 1] = tmp - l * d[q + 1];
-                if (q < F - 2) {
-                    du2[q] = du[q + 1];
-                    du[q + 1] = -l * du[q + 1];
-                }
-                ipiv[q] = 1;
-            }
-        }
-        for (int q = 0; q < F; ++q)
-            if (d[q] == 0 && p.status) *p.status = 1;
+    for (int n = t; n < F; n += nt) {
+        const bool ends = n == 0 || n == F - 1;
+        dl[n] = n == 0 ? 0.0 : h[n];
+        d[n] = n == 0 ? -h[1] : (n == F - 1 ? -h[F - 1] : 2 * (h[n] + h[n + 1]));
+        du[n] = n == 0 ? h[1] : (ends ? 0.0 : h[n + 1]);
+        du2[n] = 0.0;
+        ipiv[n] = 0;
     }
     __syncthreads();
+    bool done = false;
+    if (use_smem) {
+        // continuants p_q of the matrix times F: w1 = p_q, w2 = p_{q-1} (rescaled together)
+        const double sc = (double)F;
+        for (int q = t; q < F; q += nt) {
+            w1[q] = d[q] * sc;
+            w2[q] = q > 0 ? -(dl[q] * sc) * (du[q - 1] * sc) : 0.0;
+        }
+        __syncthreads();
+        if (t == 0) {
+            double pm = 1.0, pq = w1[0];
+            w2[0] = 1.0;
+            for (int q = 1; q < F; ++q) {
+                const double pn = fma(w1[q], pq, w2[q] * pm);
+                pm = pq;
+                pq = pn;
+                w1[q] = pq;
+                w2[q] = pm;
+                const int ex = (__double2hiint(pq) >> 20) & 0x7ff;
+                if (ex > 1023 + 400 || ex < 1023 - 400) {   // out of 10^+-120: bring both back
+                    const double r = ex > 1023 ? 1e-120 : 1e120;
+                    pq *= r;
+                    pm *= r;
+                }
+            }
+        }
+        __syncthreads();
+        int good = 1;
+        for (int q = t; q < F; q += nt) w1[q] = w1[q] / (w2[q] * (double)F);
+        __syncthreads();
+        for (int it = 0; it < 2; ++it) {
+            for (int q = t; q < F; q += nt) w2[q] = q == 0 ? d[0] : d[q] - (dl[q] * du[q - 1]) / w1[q - 1];
+            __syncthreads();
+            for (int q = t; q < F; q += nt) w1[q] = w2[q];
+            __syncthreads();
+        }
+        // no exchange and every pivot a normal number, except that the last may be anything
+        for (int q = t; q < F - 1; q += nt)
+            if (!(fabs(w1[q]) >= fabs(dl[q + 1])) || !(fabs(w1[q]) > 1e-280) || !(fabs(w1[q]) < 1e280)) good = 0;
+        done = __syncthreads_and(good);
+        if (done) {
+            for (int q = t; q < F; q += nt) d[q] = w1[q];
+            for (int q = t; q < F; q += nt)
+                if (q > 0) dl[q] = dl[q] / w1[q - 1];
+        }
+    }
+    if (!done && t == 0) eliminate(F, dl, d, du, du2, ipiv);
+    __syncthreads();
+    for (int q = t; q < F; q += nt)
+        if (d[q] == 0) status[STATUS_SPLINE] = 1;
     // factors out (from shared memory), and the cubic resample's uniform coefficients
     double *rh = p.aux, *rd = rh + F, *ev = rd + F, *ends = ev + 4 * F_new;
     for (int n = t; n <= F; n += nt) {
@@ -1104,6 +914,7 @@ __global__ void k_redist_plan(const double *s_in, int F, int F_new, int cubic, i
         ends[1] = 1.0 / (h[2] + h[1]);
         ends[2] = 1.0 / (h[3] + h[2] + h[1]);
         ends[3] = h[1] * h[1];
+    } else if (t == 32) {
         ends[4] = 1.0 / (h[F - 1] + h[F - 2]);
         ends[5] = 1.0 / (h[F - 2] + h[F - 3]);
         ends[6] = 1.0 / (h[F - 1] + h[F - 2] + h[F - 3]);
@@ -1306,16 +1117,20 @@ inline int grid_for(long n, int cap = 152 * 16)
 }  // namespace
 
 // ----------------------------------------------------------------- launchers
-#define DISPATCH(L, KERNEL, ...)                                                                    \
-    do {                                                                                            \
-        if ((L).precision == 1) {                                                                   \
-            if ((L).ncomp == 2) KERNEL<double, 2><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);   \
-            else KERNEL<double, 1><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);                  \
-        } else {                                                                                    \
-            if ((L).ncomp == 2) KERNEL<float, 2><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);    \
-            else KERNEL<float, 1><<<(L).n_tiles, NT, 0, (L).stream>>>(__VA_ARGS__);                   \
-        }                                                                                           \
-    } while (0)
+// One operation over every strip of the launch's string.
+template <class T, class Op>
+static cudaError_t walk(const Launch &L, const Scalars &sc, int xbuf, const Op &op)
+{
+    if (L.ncomp == 2) k_walk<T, 2, Op><<<L.n_tiles, NTS, 0, L.stream>>>(*L.str, sc, xbuf, op);
+    else k_walk<T, 1, Op><<<L.n_tiles, NTS, 0, L.stream>>>(*L.str, sc, xbuf, op);
+    return cudaGetLastError();
+}
+
+template <class Op>
+static cudaError_t walk(const Launch &L, const Scalars &sc, int xbuf, const Op &op)
+{
+    return L.precision == 1 ? walk<double>(L, sc, xbuf, op) : walk<float>(L, sc, xbuf, op);
+}
 
 // NLCG passes: one single-warp block per strip; launches of one string take
 // the kernels that read its descriptor at fixed offsets.
@@ -1434,49 +1249,32 @@ cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlag
 
 cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *out)
 {
-    DISPATCH(L, k_energy, *L.str, sc, xbuf, out);
-    return cudaGetLastError();
+    return walk(L, sc, xbuf, EnergyOp{out});
 }
 
 // FP64 launches with L.paired compute in float-float on the double fields
 // (about 48 bits) and store double gradients; the link discretisation has
 // no float-float form and stays IEEE double.
-cudaError_t launch_gradient_only(const Launch &L, int xbuf, FieldPtrs out, int maxwell)
+cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell)
 {
-    if (L.paired && L.precision == 1 && !L.str->disc) {
-        if (L.ncomp == 2) k_gradient_only<ff, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, out, maxwell);
-        else k_gradient_only<ff, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, out, maxwell);
-    } else {
-        DISPATCH(L, k_gradient_only, *L.str, xbuf, out, maxwell);
-    }
-    return cudaGetLastError();
+    const GradientOp op{{out.p[0], out.p[1], out.p[2]}, maxwell};
+    if (L.paired && L.precision == 1 && !L.str->disc) return walk<ff>(L, sc, xbuf, op);
+    return walk(L, sc, xbuf, op);
 }
 
 cudaError_t launch_param_adjoint(const Launch &L, const Scalars &sc, int xbuf, double *out)
 {
-    DISPATCH(L, k_param_adjoint, *L.str, sc, xbuf, out);
-    return cudaGetLastError();
+    return walk(L, sc, xbuf, AdjointOp{out});
 }
 
-cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *const *b, void *const (*j)[2])
+cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *b, void *j1, void *j2)
 {
-    (void)sc;
-    if (L.precision == 1) {
-        if (L.ncomp == 2)
-            k_jb<double, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (double *)b[0],
-                                                         (double2 *)j[0][0], (double2 *)j[0][1]);
-        else
-            k_jb<double, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (double *)b[0],
-                                                         (double2 *)j[0][0], (double2 *)j[0][1]);
-    } else {
-        if (L.ncomp == 2)
-            k_jb<float, 2><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (float *)b[0],
-                                                        (float2 *)j[0][0], (float2 *)j[0][1]);
-        else
-            k_jb<float, 1><<<L.n_tiles, NT, 0, L.stream>>>(*L.str, xbuf, (float *)b[0],
-                                                        (float2 *)j[0][0], (float2 *)j[0][1]);
-    }
-    return cudaGetLastError();
+    return walk(L, sc, xbuf, JbOp{b, j1, j2});
+}
+
+cudaError_t launch_flux(const Launch &L, const Scalars &sc, int xbuf, double *out)
+{
+    return walk(L, sc, xbuf, FluxOp{out});
 }
 
 template <class T, class W>
@@ -1522,21 +1320,77 @@ cudaError_t launch_check_scalars(const Scalars &sc, int n_images, int slot, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_arc_length(int precision, const void *const *fields, const int *width, int nf, long sites, int F,
-                              double *part, double *s, int *bad, cudaStream_t st)
+// Distances by one walk (k_arc_walk) or from stored B and J.  The walk reads
+// each image once but forms B and J of every chunk's first image again and has
+// few, long blocks: it pays in FP32, which is bound by memory, once there are
+// blocks for every SM (256 x 256 x 64: 77 us against 104; 64 x 64 x 16 in FP64:
+// 97 us against 24).
+static bool arc_by_walk(const Launch &L, int metrics, int sms)
 {
-    const int nb = (int)((sites + (long)NT * ARC_SPT - 1) / ((long)NT * ARC_SPT));
-    const dim3 grid(nb, F);
-    const void *f[3] = {nf > 0 ? fields[0] : nullptr, nf > 1 ? fields[1] : nullptr, nf > 2 ? fields[2] : nullptr};
-    const int w[3] = {nf > 0 ? width[0] : 0, nf > 1 ? width[1] : 0, nf > 2 ? width[2] : 0};
-    if (precision == 1)
-        k_arc_partial<double><<<grid, NT, 0, st>>>((const double *)f[0], (const double *)f[1], (const double *)f[2],
-                                                   w[0], w[1], w[2], sites, part);
-    else
-        k_arc_partial<float><<<grid, NT, 0, st>>>((const float *)f[0], (const float *)f[1], (const float *)f[2],
-                                                  w[0], w[1], w[2], sites, part);
-    k_arc_sum<<<F, NT, 0, st>>>(part, nb, s);
-    k_arc_cumulate<<<1, NT, 0, st>>>(F, s, bad);
+    const StringDesc &S = *L.str;
+    return L.precision == 0 && metrics == 3 && (long)S.tiles_x * ((S.ny + ARC_ROWS - 1) / ARC_ROWS) * S.F >= 64L * sms;
+}
+
+size_t arc_blocks(const StringDesc &S)
+{
+    const size_t walk = (size_t)S.tiles_x * ((S.ny + ARC_ROWS - 1) / ARC_ROWS);
+    const size_t flat = ((size_t)S.nx * S.ny + NT * ARC_SPT - 1) / (NT * ARC_SPT);
+    return walk > flat ? walk : flat;
+}
+
+template <int NC>
+static void arc_walk(const Launch &L, int xbuf, int nb, int sms, double *part_f, double *part_jb)
+{
+    const StringDesc &S = *L.str;
+    // images per block: long enough to spare the image read twice at a chunk's
+    // start, short enough that there is a wave of blocks
+    int chunk = (int)((long)nb * S.F / ((long)sms * 16));
+    chunk = chunk < 4 ? 4 : (chunk > 32 ? 32 : chunk);
+    const dim3 grid((unsigned)nb, (unsigned)((S.F + chunk - 1) / chunk));
+    k_arc_walk<NC><<<grid, NTS, 0, L.stream>>>(S, xbuf, chunk, part_f, part_jb);
+}
+
+template <class T>
+static void arc_flat(const Launch &L, const void *const *f, int w0, int nb, double *part)
+{
+    const StringDesc &S = *L.str;
+    k_arc_partial<T><<<dim3(nb, S.F), NT, 0, L.stream>>>((const T *)f[0], (const T *)f[1], L.ncomp == 2 ? (const T *)f[2] : nullptr,
+                                                         w0, 2, 2, (long)S.nx * S.ny, part);
+}
+
+cudaError_t launch_arc_distances(const Launch &L, const Scalars &sc, int xbuf, int metrics, int sms, void *const *spare,
+                                 double *s_f, double *s_jb)
+{
+    const StringDesc &S = *L.str;
+    double *part = sc.part, *part_jb = part + (metrics == 3 ? arc_blocks(S) * S.F : 0);
+    int nb;
+    if (arc_by_walk(L, metrics, sms)) {
+        nb = S.tiles_x * ((S.ny + ARC_ROWS - 1) / ARC_ROWS);
+        if (L.ncomp == 2) arc_walk<2>(L, xbuf, nb, sms, part, part_jb);
+        else arc_walk<1>(L, xbuf, nb, sms, part, part_jb);
+    } else {
+        nb = (int)(((long)S.nx * S.ny + NT * ARC_SPT - 1) / (NT * ARC_SPT));
+        if (metrics & 2) {
+            const cudaError_t e = launch_jb(L, sc, xbuf, spare[0], spare[1], spare[2]);
+            if (e != cudaSuccess) return e;
+            if (L.precision == 1) arc_flat<double>(L, spare, 1, nb, part_jb);
+            else arc_flat<float>(L, spare, 1, nb, part_jb);
+        }
+        if (metrics & 1) {
+            if (L.precision == 1) arc_flat<double>(L, S.x[xbuf], 2, nb, part);
+            else arc_flat<float>(L, S.x[xbuf], 2, nb, part);
+        }
+    }
+    const double *pf = metrics & 1 ? part : part_jb;
+    double *sf = metrics & 1 ? s_f : s_jb;
+    k_arc_sum<<<dim3(S.F, metrics == 3 ? 2 : 1), NT, 0, L.stream>>>(pf, part_jb, nb, sf, s_jb);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_arc_cumulate(int F, double *s, int *bad, cudaStream_t st)
+{
+    const int smem = F <= ARC_CUM_MAX;
+    k_arc_cumulate<<<1, NT, smem ? F * sizeof(double) : 0, st>>>(F, s, nullptr, bad, smem);
     return cudaGetLastError();
 }
 
@@ -1556,14 +1410,6 @@ cudaError_t launch_generate(int precision, void *a, void *p1, void *p2, int nx, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_flux(int precision, const void *b, long M, int F, double dx2, double *out, cudaStream_t st)
-{
-    const int grid = F < 152 * 4 ? F : 152 * 4;
-    if (precision == 1) k_flux<double><<<grid, NT, 0, st>>>((const double *)b, M, F, dx2, out);
-    else k_flux<float><<<grid, NT, 0, st>>>((const float *)b, M, F, dx2, out);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_winding(int precision, const void *psi, int nx, int ny, int F, int inset, double *out,
                            cudaStream_t st)
 {
@@ -1573,12 +1419,16 @@ cudaError_t launch_winding(int precision, const void *psi, int nx, int ny, int F
     return cudaGetLastError();
 }
 
-cudaError_t launch_redist_plan(const double *s, int F, int F_new, int cubic, int spline, const RedistPlan &p,
-                               cudaStream_t st)
+cudaError_t launch_redist_plan(double *s_f, double *s_jb, const double *s_use, int *status, int F, int F_new, int cubic,
+                               int spline, const RedistPlan &p, cudaStream_t st)
 {
     const size_t sm = redist_plan_smem(F, F_new);
-    const int use_smem = sm <= 48 * 1024;
-    k_redist_plan<<<1, 32, use_smem ? sm : 0, st>>>(s, F, F_new, cubic, spline, p, use_smem);
+    const int use_smem = sm <= 200 * 1024;   // about 2,300 images
+    if (use_smem && sm > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_redist_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
+    }
+    k_redist_plan<<<1, 128, use_smem ? sm : 0, st>>>(s_f, s_jb, s_use, status, F, F_new, cubic, spline, p, use_smem);
     return cudaGetLastError();
 }
 
@@ -1765,7 +1615,7 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
                                                   double *fenergy, void *stream)
 {
     using namespace mepgl;
-    constexpr int rows = MEPGL_ROWS_F64;
+    constexpr int rows = 8;   // per strip
     if (nx < 2 || ny < 2 || n_images < 1 || !(dx > 0))
         return noalloc_fail(MEPGL_ERR_INVALID_ARG, "need nx, ny >= 2, n_images >= 1, dx > 0");
     if (!comp_code || !sc_code || !a_1 || !b_1 || !m_xx_1 || !m_yy_1 || !h || !a || !psi_1 || !fenergy ||
@@ -1773,7 +1623,7 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
         return noalloc_fail(MEPGL_ERR_INVALID_ARG, "null device pointer");
     const long tiles_x = (nx + TX - 1) / TX, tiles_y = (ny + rows - 1) / rows;
     const long n_tiles = tiles_x * tiles_y * n_images;
-    // tile coordinates are 16-bit (TileRef), as in mepgl_create
+    // the lattice limits of mepgl_create
     if (nx > 32767 * TX || ny > 32767 * rows || (long)nx * ny >= (1L << 31))
         return noalloc_fail(MEPGL_ERR_INVALID_ARG, "lattice too large: need nx <= 32767*32, ny <= 32767*8 "
                                                    "and nx * ny < 2^31");
@@ -1801,7 +1651,8 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
     S.F = n_images;
     S.ncomp = multicomponent ? 2 : 1;
     S.tiles_x = (int)tiles_x;
-    S.tiles_y = (int)tiles_y;
+    S.wtiles_y = (int)tiles_y;
+    S.wrows = rows;
     S.thin_film = thin_film ? 1 : 0;
     S.per_site = 1;
     const double *pa[2] = {a_1, multicomponent ? a_2 : a_1}, *pb[2] = {b_1, multicomponent ? b_2 : b_1};
@@ -1836,9 +1687,9 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
     e = cudaMemsetAsync(scr.ticket, 0, sizeof(unsigned) * n_images, st);
     if (e != cudaSuccess) return noalloc_fail(MEPGL_ERR_CUDA, std::string("ticket reset: ") + cudaGetErrorString(e));
     if (multicomponent)
-        k_energy<double, 2><<<(unsigned)n_tiles, NT, 0, st>>>(S, sc, 0, fenergy);
+        k_walk<double, 2, EnergyOp><<<(unsigned)n_tiles, NTS, 0, st>>>(S, sc, 0, EnergyOp{fenergy});
     else
-        k_energy<double, 1><<<(unsigned)n_tiles, NT, 0, st>>>(S, sc, 0, fenergy);
+        k_walk<double, 1, EnergyOp><<<(unsigned)n_tiles, NTS, 0, st>>>(S, sc, 0, EnergyOp{fenergy});
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(MEPGL_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return MEPGL_OK;

@@ -7,16 +7,14 @@ namespace mepgl {
 
 constexpr int LS_GRID = 2001;         // line-search grid points x_0 .. x_2000
 
-// Rows per lattice tile for a precision (0 float, 1 double); tiles are TX wide.
-int tile_rows(int precision);
 // Copy the neighbour-code weight tables to constant memory (idempotent).
 cudaError_t upload_mask_tables();
 
 struct Launch {
     const Batch *batch;          // strings of the NLCG passes (host copy; passed by value to the kernels)
     int stile0, n_stiles;        // their strips
-    const StringDesc *str;       // string of the tile kernels
-    int n_tiles;                 // its tiles
+    const StringDesc *str;       // string of the walks over one string
+    int n_tiles;                 // its strips
     int precision;               // 0 float, 1 double
     int paired;                  // 1: NLCG passes in float-float arithmetic on double fields
     int ncomp;                   // 1 or 2 (uniform over the strings of a context)
@@ -35,6 +33,8 @@ struct StepFlags {
 // strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
 int strip_rows_cap(int precision, int paired);
 int strip_rows(int precision, int paired, int ny, long tiles, int slots);
+// The same for the walks over one string, of `columns` image columns of strips.
+int walk_rows(int precision, int ny, long columns, int sms);
 // Steps are fused for batches of at most fuse_waves() x strip_pass_slots()
 // strips; strip_pass_slots(): resident warps of the pass kernels on the GPU.
 int fuse_waves(int precision);
@@ -68,20 +68,27 @@ cudaError_t launch_param_adjoint(const Launch &L, const Scalars &sc, int xbuf, d
 // Gradient of x[xbuf] into the three arrays of `out` (single string).
 struct FieldPtrs { void *p[3]; };
 // Gradient of every image into `out` (FP64 launches with L.paired: float-float arithmetic).
-cudaError_t launch_gradient_only(const Launch &L, int xbuf, FieldPtrs out, int maxwell);
-// B, J of x[xbuf] written to per-string arrays (b: F*M reals, j: F*M pairs).
-cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *const *b, void *const (*j)[2]);
+cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell);
+// B, J of x[xbuf] (b: F*M reals, j1, j2: F*M pairs); flux dx^2 sum B per image of the string.
+cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *b, void *j1, void *j2);
+cudaError_t launch_flux(const Launch &L, const Scalars &sc, int xbuf, double *out);
 
-// Arc length of one string over nf per-image arrays of `width` reals per site
-// (reals of the context precision).  Result: s[0..F) (device doubles), using
-// part (>= tiles_per_image * F doubles) as scratch.  A string of zero or
+// Partial sums per image of an arc length (upper bound).
+size_t arc_blocks(const StringDesc &S);
+// Squared distances of each image of the launch's string to the one before, in
+// the field metric (metrics & 1) into s_f[0..F) and the (B, J) metric
+// (metrics & 2) into s_jb[0..F) (device doubles).  spare: three arrays of the
+// fields' size for B, J_1, J_2; sc.part holds 2 arc_blocks F doubles.
+cudaError_t launch_arc_distances(const Launch &L, const Scalars &sc, int xbuf, int metrics, int sms, void *const *spare,
+                                 double *s_f, double *s_jb);
+// Squared distances to normalised arc length, in place.  A string of zero or
 // non-finite length sets *bad (device int) and gets the uniform s = n/(F-1).
-cudaError_t launch_arc_length(int precision, const void *const *fields, const int *width, int nf, long sites, int F,
-                              double *part, double *s, int *bad, cudaStream_t st);
+cudaError_t launch_arc_cumulate(int F, double *s, int *bad, cudaStream_t st);
 // Device status flags (Scalars::status): [0] a stage wait of the fused NLCG
 // launch ran out; [1] count of non-finite per-image scalars after NLCG steps,
-// [2] the first such image + 1; [3] a string of zero or non-finite arc length.
-constexpr int STATUS_WAIT = 0, STATUS_NONFINITE = 1, STATUS_NONFINITE_IMAGE = 2, STATUS_ARC = 3;
+// [2] the first such image + 1; [3] a string of zero or non-finite arc length;
+// [4] a singular spline matrix.
+constexpr int STATUS_WAIT = 0, STATUS_NONFINITE = 1, STATUS_NONFINITE_IMAGE = 2, STATUS_ARC = 3, STATUS_SPLINE = 4;
 // Checks energy and |g|^2 (slot 0 or 1) of n_images images (see STATUS_NONFINITE).
 cudaError_t launch_check_scalars(const Scalars &sc, int n_images, int slot, cudaStream_t st);
 // Initial-guess parameters of launch_generate (see mepgl_guess).
@@ -96,30 +103,28 @@ struct GuessParams {
 cudaError_t launch_generate(int precision, void *a, void *p1, void *p2, int nx, int ny, int F, int ncomp,
                             const int32_t *comp, const int32_t *sc, const double *tracks, int n_tracks,
                             const GuessParams &g, cudaStream_t st);
-// out[n] = dx2 * sum of b over image n (M reals per image, context precision).
-cudaError_t launch_flux(int precision, const void *b, long M, int F, double dx2, double *out, cudaStream_t st);
 // out[n] = winding sum of psi (pairs) of image n around the rectangle `inset`
 // sites inside the lattice edge (requires nx, ny > 2 inset + 1).
 cudaError_t launch_winding(int precision, const void *psi, int nx, int ny, int F, int inset, double *out,
                            cudaStream_t st);
-// Plan of a redistribution from F to F_new images on the arc length s:
-// segment k and weight w per output image; for cubic also h and the
-// factorised spline matrix (dl, d, du, du2, ipiv) -- all in `plan`.
+// Plan of a redistribution from F to F_new images: the squared distances s_f
+// and s_jb become arc lengths, and on s_use (one of them) the segment k and
+// weight w per output image; for cubic also h and the factorised spline matrix
+// (dl, d, du, du2, ipiv) -- all in `plan`.  `status` is Scalars::status.
 struct RedistPlan {
     int *k;          // [F_new]
     double *w;       // [F_new]
     double *h;       // [F + 1]
     double *dl, *d, *du, *du2;   // [F]
     int *ipiv;       // [F]
-    int *status;
     // cubic: 1 / h [F], 1 / d [F], per output image {w, 1 - w, h_k^2 (w^3 - w),
     // h_k^2 (wm^3 - wm)} [4 F_new], the end conditions' factors [8]
     double *aux;
 };
 // doubles of RedistPlan::aux for a plan of capacity `cap` images
 inline size_t redist_aux_size(int cap) { return (size_t)6 * cap + 8; }
-cudaError_t launch_redist_plan(const double *s, int F, int F_new, int cubic, int spline, const RedistPlan &p,
-                               cudaStream_t st);
+cudaError_t launch_redist_plan(double *s_f, double *s_jb, const double *s_use, int *status, int F, int F_new, int cubic,
+                               int spline, const RedistPlan &p, cudaStream_t st);
 // Linear resample of `pairs` interleaved pairs per image (precision real).
 cudaError_t launch_redist_linear(int precision, const void *f, void *fnew, long pairs, int F_new, const RedistPlan &p,
                                  cudaStream_t st);

@@ -905,7 +905,7 @@ struct Ctx {
         for (int f = 0; f < 3; ++f) fp.p[f] = f < w->nf ? out.p[f] : nullptr;
         ++grads;
         c->launches += 1;
-        return launch_gradient_only(L, xbuf, fp, 0);
+        return launch_gradient_only(L, c->sc, xbuf, fp, 0);
     }
     cudaError_t lin(const LinArgs &a)
     {
@@ -1052,7 +1052,7 @@ mepgl_status hess_vec(Ctx &R, const Vec &u, const Vec &y, bool with_mu)
     Lh.stream = R.st;
     R.grads += 2;
     R.c->launches += 1;
-    RK(launch_gradient_only(Lh, 0, fp, 0));
+    RK(launch_gradient_only(Lh, w->hvc->sc, 0, fp, 0));
     a = lin_args(y);
     add_term(a, gp, 1.0, S_INV2H);
     add_term(a, gm, -1.0, S_INV2H);
@@ -1355,7 +1355,7 @@ mepgl_status wide_gauge_gradients(Ctx &R, const GaugeBasis &B, double h, std::ve
         RK(cudaGetLastError());
         FieldPtrs fp;
         for (int f = 0; f < 3; ++f) fp.p[f] = f < w->nf ? gw.p[f] : nullptr;
-        RK(launch_gradient_only(Lw, 0, fp, 0));
+        RK(launch_gradient_only(Lw, wc->sc, 0, fp, 0));
         mepgl_status st = orbit_gradients(R, B, xw, gw, nW, w->wide_gd + (size_t)w0 * m, m, 0);
         if (st != MEPGL_OK) return st;
         c->launches += 2;

@@ -1,6 +1,5 @@
-// site_ops.cuh -- what the per-site stencils share: mask weights, tiles,
-// site parameters; and the terms without a packed form: parameter adjoints
-// and the gauge-link functional.
+// site_ops.cuh -- what the per-site stencils share: mask weights and site
+// parameters; and the gauge-link functional, which has no packed form.
 //
 // The discretisation is the reference's (mepgl/src/nlcg.cu): psi and A live
 // on sites; on a link i -> j along e the kinetic term uses the linearised
@@ -89,19 +88,6 @@ inline void build_mask_table(MaskTable<T> &M)
     }
 }
 
-// Fields of a tile of TYT rows (+ halo): A, psi_1[, psi_2].
-template <class T, int NC, int TYT>
-struct TileF {
-    vec2_t<T> A[TYT + 2][TX + 2];
-    vec2_t<T> P[NC][TYT + 2][TX + 2];
-};
-
-// The same with the packed neighbour codes of each site.
-template <class T, int NC, int TYT>
-struct Tile : TileF<T, NC, TYT> {
-    uint16_t m[TYT + 2][TX + 2];
-};
-
 // Parameters of one site (uniform strings read the descriptor).
 template <class T>
 struct SiteParams {
@@ -132,30 +118,8 @@ struct SiteParams {
     }
 };
 
-#define TA(dx_, dy_) (t.A[ly + (dy_)][lx + (dx_)])
-#define TP(c_, dx_, dy_) (t.P[c_][ly + (dy_)][lx + (dx_)])
-
-// Partial derivatives of site_energy at fixed fields with respect to a
-// uniform shift of the applied field h, to eta and to gamma (no reference
-// counterpart): out[0] = -1/4 sum_views w_v (curl - h), out[1] = area Re(psi1
-// psi2*), out[2] = area |psi1|^2 |psi2|^2 / 2, each times dx^2.
-template <class T, int NC, int TYT>
-__device__ __forceinline__ void site_param_adjoint(const Tile<T, NC, TYT> &t, int lx, int ly,
-                                                   const SiteParams<T> &p, const Wts<T> &w, int thin_film, T *out)
-{
-    if (NC == 2) {
-        const vec2_t<T> P1 = TP(0, 0, 0), P2 = TP(NC - 1, 0, 0);
-        out[1] += (P1.x * P2.x + P1.y * P2.y) * w.area * p.dx2;
-        out[2] += (T)0.5 * (P1.x * P1.x + P1.y * P1.y) * (P2.x * P2.x + P2.y * P2.y) * w.area * p.dx2;
-    }
-    if (!thin_film) {
-        const vec2_t<T> A0 = TA(0, 0);
-        const T ayp = (TA(1, 0).y - A0.y) * p.idx, aym = (A0.y - TA(-1, 0).y) * p.idx;
-        const T axp = (TA(0, 1).x - A0.x) * p.idx, axm = (A0.x - TA(0, -1).x) * p.idx;
-        const T r0 = ayp - axp - p.h, r1 = aym - axp - p.h, r2 = aym - axm - p.h, r3 = ayp - axm - p.h;
-        out[0] -= (T)0.25 * (w.vUR * r0 + w.vUL * r1 + w.vLL * r2 + w.vLR * r3) * p.dx2;
-    }
-}
+#define TA(dx_, dy_) (t.A((dx_), (dy_)))
+#define TP(c_, dx_, dy_) (t.P((c_), (dx_), (dy_)))
 
 // ------------------------------------------------------- gauge links
 // The link (Peierls) discretisation of the same functional (no reference
@@ -185,8 +149,8 @@ __device__ __forceinline__ T cond_density(const vec2_t<T> *P, int nc, const Site
     return nl;
 }
 
-template <class T, int NC, int TYT>
-__device__ __forceinline__ T site_energy_link(const Tile<T, NC, TYT> &t, int lx, int ly, const SiteParams<T> &p,
+template <class T, int NC, class View>
+__device__ __forceinline__ T site_energy_link(const View &t, const SiteParams<T> &p,
                                               const Wts<T> &w, int thin_film)
 {
     vec2_t<T> P0[NC];
@@ -219,8 +183,8 @@ __device__ __forceinline__ T site_energy_link(const Tile<T, NC, TYT> &t, int lx,
 // forward links, the backward links owned by its -x / -y neighbours (whose
 // masses are hmx_l / hmy_d = 1 / (2 m) there), and the plaquettes with
 // lower-left corners s, s-x, s-y (applied fields h, hl, hd).
-template <class T, int NC, int TYT>
-__device__ __forceinline__ void site_gradient_link(const Tile<T, NC, TYT> &t, int lx, int ly, const SiteParams<T> &p,
+template <class T, int NC, class View>
+__device__ __forceinline__ void site_gradient_link(const View &t, const SiteParams<T> &p,
                                                    const Wts<T> &w, T hl, T hd, const T *hmx_l, const T *hmy_d,
                                                    int maxwell, int thin_film, T *out)
 {
@@ -286,8 +250,8 @@ __device__ __forceinline__ void site_gradient_link(const Tile<T, NC, TYT> &t, in
 }
 
 // dF/dH of the link functional at one site: -v_UR (B - h) dx^2.
-template <class T, int NC, int TYT>
-__device__ __forceinline__ T site_dh_link(const Tile<T, NC, TYT> &t, int lx, int ly, const SiteParams<T> &p,
+template <class T, int NC, class View>
+__device__ __forceinline__ T site_dh_link(const View &t, const SiteParams<T> &p,
                                           const Wts<T> &w)
 {
     return -w.vUR * ((TA(0, 0).x + TA(1, 0).y - TA(0, 1).x - TA(0, 0).y) * p.idx - p.h) * p.dx2;

@@ -127,23 +127,6 @@ struct PackView {
     P px[3][3], py[3][3];
 };
 
-// Packed view of one site of a shared-memory tile.
-template <class S, int NC, int TYT>
-__device__ __forceinline__ PackView<S, NC> pack_view_tile(const TileF<S, NC, TYT> &t, int lx, int ly)
-{
-    PackView<S, NC> v;
-#pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-            v.a[dy + 1][dx + 1] = t.A[ly + dy][lx + dx];
-            const vec2_t<S> p1 = t.P[0][ly + dy][lx + dx], p2 = t.P[NC - 1][ly + dy][lx + dx];
-            v.px[dy + 1][dx + 1] = Pk<S, NC>::mk(p1.x, p2.x);
-            v.py[dy + 1][dx + 1] = Pk<S, NC>::mk(p1.y, p2.y);
-        }
-    return v;
-}
-
 // Parameters as the stencils use them: read from the descriptor, and the
 // site's own where the string has per-site arrays.
 template <class S, int NC>
@@ -153,6 +136,7 @@ struct PackParams {
     P qd, hqd, nhqd, hqq, kq, qi;   // q dx, +- half of it, half its square, (q + 1) dx, q / dx
     P hmx, hmy, n2hmx, n2hmy;       // 1 / (2 m), -1 / m
     P hqmx, hqmy;                   // hqq / (2 m dx^2)
+    P jmx, jmy;                     // qi / (2 m)
     P hmxi, hmyi, hmxil, hmyid;     // 1 / (2 m dx^2); at the left / lower neighbour (their forward links end here)
     P aob, b, a2, b2;               // a / b, b; 2 a dx^2, 2 b dx^2
     S eta, gamma, delta, h, idx, idx4, idx8;
@@ -170,6 +154,8 @@ struct PackParams {
         hmy = K::mk(U.hmy[0], U.hmy[1]);
         hmxi = hmxil = K::mk(U.hmxi[0], U.hmxi[1]);
         hmyi = hmyid = K::mk(U.hmyi[0], U.hmyi[1]);
+        jmx = K::mk(U.jmx[0], U.jmx[1]);
+        jmy = K::mk(U.jmy[0], U.jmy[1]);
         hqmx = K::mk(U.hqmx[0], U.hqmx[1]);
         hqmy = K::mk(U.hqmy[0], U.hqmy[1]);
         n2hmx = K::mk(U.n2hmx[0], U.n2hmx[1]);
@@ -211,6 +197,8 @@ struct PackParams {
         hmyi = pmul(hmy, i2);
         hmxil = pmul(K::mk(x[0], x[NC - 1]), i2);
         hmyid = pmul(K::mk(y[0], y[NC - 1]), i2);
+        jmx = pmul(hmx, qi);
+        jmy = pmul(hmy, qi);
         n2hmx = pmul(hmx, K::bc(n2));
         n2hmy = pmul(hmy, K::bc(n2));
         aob = K::mk(p.aob[0], p.aob[NC - 1]);
@@ -228,7 +216,8 @@ struct PackParams {
 struct Ones {
     static constexpr bool interior = true;
     static constexpr double area = 1, wfx = 1, wbx = 1, wfy = 1, wby = 1, wsx = 2, wsy = 2;
-    static constexpr double vUR = 1, vUL = 1, vLL = 1, vLR = 1;
+    static constexpr double lfx = 1, lbx = 1, lfy = 1, lby = 1;
+    static constexpr double vUR = 1, vUL = 1, vLL = 1, vLR = 1, ivs = 0.25;
 };
 
 // FP64: a biquadratic coupling of zero is skipped (a uniform branch; its 26
@@ -261,15 +250,16 @@ struct Curl {
 // factor of the whole sum: folding dx^2 into each parameter, with a rounding
 // each, left an FP32 energy 6.4e-7 off where it is 3.6e-7 with the factor
 // outside.
-template <class S, int NC>
-__device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
+template <class S, int NC, class Wt>
+__device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wt &w,
                                          int per_site, int thin_film)
 {
     using K = Pk<S, NC>;
     using P = pack_t<S, NC>;
+    constexpr bool ones = Wt::interior;
     const P X = v.px[1][1], Y = v.py[1][1];
     const P r = pfma(Y, Y, pmul(X, X)), n = padd(r, pp.aob);
-    const P bh = pmul(pp.b, K::bc(S(0.5f) * w.area));
+    const P bh = pmul(pp.b, K::bc(ones ? S(0.5f) : S(0.5f) * S(w.area)));
     P e = pmul(pmul(bh, n), n);
     P dg = K::bc(S(0.0f));
 #pragma unroll
@@ -277,8 +267,8 @@ __device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackPar
         const S Ai = dir == 0 ? v.a[1][1].x : v.a[1][1].y, Aj = dir == 0 ? v.a[1][2].x : v.a[2][1].y;
         const P xj = dir == 0 ? v.px[1][2] : v.px[2][1], yj = dir == 0 ? v.py[1][2] : v.py[2][1];
         const P hm = dir == 0 ? pp.hmxi : pp.hmyi, hb = dir == 0 ? pp.hmxil : pp.hmyid;
-        const S wf = dir == 0 ? w.wfx : w.wfy, wb = dir == 0 ? w.wbx : w.wby, ws = dir == 0 ? w.wsx : w.wsy;
-        const P f = pmul(hm, K::bc(wf));
+        const S wf = S(dir == 0 ? w.wfx : w.wfy), wb = S(dir == 0 ? w.wbx : w.wby), ws = S(dir == 0 ? w.wsx : w.wsy);
+        const P f = ones ? hm : pmul(hm, K::bc(wf));
         const P Dx = psub(xj, X), Dy = psub(Y, yj);       // Dy: -(y_j - y_i)
         const P s = pmul(pp.qd, K::bc(Ai + Aj));
         e = pfma(f, pfma(Dy, pfma(s, X, Dy), pmul(Dx, pfma(s, Y, Dx))), e);
@@ -295,20 +285,53 @@ __device__ __forceinline__ S site_energy(const PackView<S, NC> &v, const PackPar
         S cp = pp.eta * R;
         cp = fma1(S(0.5f) * pp.gamma * r1, r2, cp);
         cp = fma1(S(0.5f) * pp.delta, fma1(R, R, -(I * I)), cp);
-        t = fma1(w.area, cp, t);
+        t = ones ? t + cp : fma1(S(w.area), cp, t);
     }
     if (!thin_film) {
         const Curl<S> c(v.a);
         const S nh = -pp.h;
         const S r0 = fma1(pp.idx, c.yp - c.xp, nh), r1 = fma1(pp.idx, c.ym - c.xp, nh);
         const S r2 = fma1(pp.idx, c.ym - c.xm, nh), r3 = fma1(pp.idx, c.yp - c.xm, nh);
-        S em = (w.vUR * r0) * r0;
-        em = fma1(w.vUL * r1, r1, em);
-        em = fma1(w.vLL * r2, r2, em);
-        em = fma1(w.vLR * r3, r3, em);
+        S em = ones ? r0 * r0 : (S(w.vUR) * r0) * r0;
+        em = fma1(ones ? r1 : S(w.vUL) * r1, r1, em);
+        em = fma1(ones ? r2 : S(w.vLL) * r2, r2, em);
+        em = fma1(ones ? r3 : S(w.vLR) * r3, r3, em);
         t = fma1(S(0.125f), em, t);
     }
     return t;
+}
+
+// Partial derivatives of the energy at fixed fields with respect to a uniform
+// shift of the applied field h, to eta and to gamma (no reference
+// counterpart), summed without their constants: h += sum over the views of
+// w_v (curl - h) (times -dx^2 / 4), eta += area Re(psi1 psi2*) (dx^2), gamma
+// += area |psi1|^2 |psi2|^2 (dx^2 / 2).
+template <class S, int NC, class Wt>
+__device__ __forceinline__ void site_param_adjoint(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wt &w,
+                                                   int thin_film, S &h, S &eta, S &gamma)
+{
+    using K = Pk<S, NC>;
+    constexpr bool ones = Wt::interior;
+    if constexpr (NC == 2) {
+        const S x1 = K::template lane<0>(v.px[1][1]), y1 = K::template lane<0>(v.py[1][1]);
+        const S x2 = K::template lane<1>(v.px[1][1]), y2 = K::template lane<1>(v.py[1][1]);
+        const S R = fma1(y1, y2, x1 * x2), r1 = fma1(y1, y1, x1 * x1), r2 = fma1(y2, y2, x2 * x2);
+        eta = ones ? eta + R : fma1(S(w.area), R, eta);
+        gamma = fma1(ones ? r1 : S(w.area) * r1, r2, gamma);
+    }
+    if (!thin_film) {
+        const Curl<S> c(v.a);
+        const S nh = -pp.h;
+        if constexpr (ones) {   // the four views add up to twice the central differences
+            const S d = (c.yp + c.ym) - (c.xp + c.xm);
+            h = h + fma1(S(2.0f) * pp.idx, d, S(4.0f) * nh);
+        } else {
+            h = fma1(S(w.vUR), fma1(pp.idx, c.yp - c.xp, nh), h);
+            h = fma1(S(w.vUL), fma1(pp.idx, c.ym - c.xp, nh), h);
+            h = fma1(S(w.vLL), fma1(pp.idx, c.ym - c.xm, nh), h);
+            h = fma1(S(w.vLR), fma1(pp.idx, c.yp - c.xm, nh), h);
+        }
+    }
 }
 
 // ---------------------------------------------------------------- gradient
@@ -472,19 +495,6 @@ __device__ __forceinline__ void site_gradient(const GradView<S, NC> &c, const Gr
         out[0] = S(0.0f);
         out[1] = S(0.0f);
     }
-}
-
-// The same from a nine-point view (tile kernels): the carry is formed from the row below.
-template <class S, int NC>
-__device__ __forceinline__ void site_gradient(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wts<S> &w,
-                                              const FieldSums<S> &h, int maxwell, int thin_film, S *out)
-{
-    const GradView<S, NC> d{v.a[0][1], v.a[0][0], v.a[0][2], v.px[0][1], v.py[0][1]};
-    const GradView<S, NC> c{v.a[1][1], v.a[1][0], v.a[1][2], v.px[1][1], v.py[1][1]};
-    const GradView<S, NC> u{v.a[2][1], v.a[2][0], v.a[2][2], v.px[2][1], v.py[2][1]};
-    GradCarry<S, NC> k;
-    grad_up<S, NC>(d, c, pp, w.wby, h.d, d.ar.y - d.a.y, d.a.y - d.al.y, k);
-    site_gradient<S, NC>(c, u, v.px[1][0], v.py[1][0], v.px[1][2], v.py[1][2], pp, w, h, maxwell, thin_film, k, out);
 }
 
 // ------------------------------------------------------------ line quartic
@@ -657,32 +667,49 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
     }
 }
 
+// B at one site: mean of the views inside the domain.
+template <class S, class Wt>
+__device__ __forceinline__ S site_b(const vec2_t<S> (&a)[3][3], S idx, const Wt &w)
+{
+    const Curl<S> c(a);
+    if constexpr (Wt::interior) {
+        return ((c.yp + c.ym) - (c.xp + c.xm)) * (S(0.5f) * idx);
+    } else {
+        S b = S(w.vUR) * (c.yp - c.xp);
+        b = fma1(S(w.vUL), c.ym - c.xp, b);
+        b = fma1(S(w.vLL), c.ym - c.xm, b);
+        b = fma1(S(w.vLR), c.yp - c.xm, b);
+        return b * idx * S(w.ivs);
+    }
+}
+
 // B and J at one site (computeJBKernel, nlcg.cu:243-364).
-template <class S, int NC>
-__device__ __forceinline__ void site_jb(const PackView<S, NC> &v, S idx, const PackParams<S, NC> &pp, const Wts<S> &w,
+template <class S, int NC, class Wt>
+__device__ __forceinline__ void site_jb(const PackView<S, NC> &v, const PackParams<S, NC> &pp, const Wt &w,
                                         S *out /* 1+2NC */)
 {
     using K = Pk<S, NC>;
     using P = pack_t<S, NC>;
-    const Curl<S> c(v.a);
-    S bb = w.vUR * (c.yp - c.xp);
-    bb = fma1(w.vUL, c.ym - c.xp, bb);
-    bb = fma1(w.vLL, c.ym - c.xm, bb);
-    bb = fma1(w.vLR, c.yp - c.xm, bb);
-    out[0] = bb * idx * w.ivs;
+    constexpr bool ones = Wt::interior;
+    out[0] = site_b<S>(v.a, pp.idx, w);
     const P X = v.px[1][1], Y = v.py[1][1];
-    const P r = pfma(Y, Y, pmul(X, X));
+    const P nqr = pmul(pmul(pp.nhqd, K::bc(S(2.0f))), pfma(Y, Y, pmul(X, X)));   // -q dx |psi|^2
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
         const S A = dir == 0 ? v.a[1][1].x : v.a[1][1].y;
         const P xf = dir == 0 ? v.px[1][2] : v.px[2][1], yf = dir == 0 ? v.py[1][2] : v.py[2][1];
         const P xb = dir == 0 ? v.px[1][0] : v.px[0][1], yb = dir == 0 ? v.py[1][0] : v.py[0][1];
-        const P lf = K::bc(dir == 0 ? w.lfx : w.lfy), lb = K::bc(dir == 0 ? w.lbx : w.lby);
         // lattice current of each link: x Dy - y Dx - a |psi|^2
-        const P ar = pmul(pmul(pp.qd, K::bc(A)), r);
-        const P jf = pnfma(Y, psub(xf, X), pfma(X, psub(yf, Y), pmul(ar, K::bc(S(-1.0f)))));
-        const P jb = pnfma(Y, psub(X, xb), pfma(X, psub(Y, yb), pmul(ar, K::bc(S(-1.0f)))));
-        const P j = pmul(pmul(dir == 0 ? pp.hmx : pp.hmy, pp.qi), pfma(lb, jb, pmul(lf, jf)));
+        const P nar = pmul(nqr, K::bc(A));
+        P j;
+        if constexpr (ones) {
+            j = pnfma(Y, psub(xf, xb), pfma(X, psub(yf, yb), padd(nar, nar)));
+        } else {
+            const P jf = pnfma(Y, psub(xf, X), pfma(X, psub(yf, Y), nar));
+            const P jb = pnfma(Y, psub(X, xb), pfma(X, psub(Y, yb), nar));
+            j = pfma(K::bc(S(dir == 0 ? w.lbx : w.lby)), jb, pmul(K::bc(S(dir == 0 ? w.lfx : w.lfy)), jf));
+        }
+        j = pmul(dir == 0 ? pp.jmx : pp.jmy, j);
         out[1 + dir] = K::template lane<0>(j);
         if (NC == 2) out[3 + dir] = K::template lane<1>(j);
     }

@@ -194,7 +194,7 @@ __device__ __forceinline__ void cp_async_wait_groups() { asm volatile("cp.async.
 // then read at fixed offsets, i.e. as constant operands, not through
 // indexed constant loads.
 template <bool ONE>
-__device__ __forceinline__ TileRef strip_tile(const batch_t<ONE> &bt, int g)
+__device__ __forceinline__ StripRef strip_tile(const batch_t<ONE> &bt, int g)
 {
     int s = 0;
     if (!ONE)
@@ -202,17 +202,16 @@ __device__ __forceinline__ TileRef strip_tile(const batch_t<ONE> &bt, int g)
             if (g >= bt.s[k].stile_base) s = k;
     const StringDesc &S = bt.s[s];
     const int r = g - S.stile_base, tpi = S.tiles_x * S.stiles_y, n = r / tpi, u = r - n * tpi, ty = u / S.tiles_x;
-    TileRef t;
-    t.s = (int16_t)s;
-    t.ty = (int16_t)ty;
-    t.tx = (int16_t)(u - ty * S.tiles_x);
-    t.pad = 0;
+    StripRef t;
+    t.s = s;
+    t.ty = ty;
+    t.tx = u - ty * S.tiles_x;
     t.n = n;
     return t;
 }
 
 // Slot of a strip's partial sums.
-__device__ __forceinline__ int strip_slot(const StringDesc &S, const TileRef &tr)
+__device__ __forceinline__ int strip_slot(const StringDesc &S, const StripRef &tr)
 {
     return S.stile_base + (tr.n * S.stiles_y + tr.ty) * S.tiles_x + tr.tx;
 }
@@ -318,7 +317,7 @@ using GradRing = vec2_t<T>[3][2][2][1 + NC];
 // field stores, so that a consumer that has seen the image finished (same
 // launch) reads them.
 template <class T, int NC, bool ONE>
-__device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
+__device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
 {
     using V = vec2_t<T>;
@@ -502,7 +501,7 @@ using DirRing = vec2_t<T>[3][2][3][1 + NC];
 // search.  Returns true (in every lane) when this strip finished its image;
 // field stores are fenced as in grad_tile.
 template <class T, int NC, bool ONE>
-__device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const TileRef tr, const Scalars &sc, const StepFlags &f,
+__device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                          DirRing<T, NC> &ring, double (&coef)[5])
 {
     using V = vec2_t<T>;
@@ -759,7 +758,7 @@ __global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __g
         const int k = (int)(item / per_step);
         const int r = (int)(item - (unsigned long long)k * per_step);
         const int pass = r >= n_tiles ? 1 : 0, u = r - pass * n_tiles;
-        const TileRef tr = strip_tile<ONE>(bt, tile0 + u);
+        const StripRef tr = strip_tile<ONE>(bt, tile0 + u);
         const int img = bt.s[ONE ? 0 : tr.s].img_base + tr.n;
         const unsigned need = 2u * (unsigned)k + (unsigned)pass;
         if (need > 0 && !wait_stage(stage + img, need, max_polls, sc.status)) return;
