@@ -205,6 +205,15 @@ mepgl_status mepgl_free_energy(mepgl_ctx *ctx, double *fenergy);
 mepgl_status mepgl_energy_grad(mepgl_ctx *ctx, double *fenergy, void *g_a, void *g_psi_1, void *g_psi_2,
                                int memory);
 
+/* What a backward pass wants of the free energy F_n, in one walk over the
+ * fields: weights[n] dF_n/d(A, psi) into device arrays of the fields' layout,
+ * and (adjoint non-NULL: host array of 3 F doubles) dF_n/d(H, eta, gamma)
+ * without the weights at adjoint[3 n + k].  `weights` is a device array of F
+ * doubles, rounded to the precision of the fields first.  g_psi_2 is ignored
+ * with one component; the other arrays must not be NULL. */
+mepgl_status mepgl_weighted_grad(mepgl_ctx *ctx, const double *weights, double *adjoint, void *g_a, void *g_psi_1,
+                                 void *g_psi_2);
+
 /* `iterations` nonlinear-conjugate-gradient steps on every image.
  * use_cg = 0 gives steepest descent; maxwell_only = 1 freezes psi (mode M).
  * Replaces nlcgSteps (mepgl/src/nlcg.cu:1462-1586), with its gradient

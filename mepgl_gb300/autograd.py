@@ -5,8 +5,8 @@ free energies (float64, shape (F,)) of fields held in CUDA tensors of shape
 (F, ny, nx, 2) in the reference's device layout.  The forward pass is the
 library's energy kernel (computeFreeEnergy, mepgl/src/nlcg.cu:217-240); the
 backward pass is its hand-written gradient kernel (gradientPsi / gradientA,
-nlcg.cu:504-888) scaled by the incoming per-image weights, and the
-parameter-adjoint kernel for ``theta``:
+nlcg.cu:504-888) scaled by the incoming per-image weights, with the parameter
+adjoints for ``theta`` from the same walk over the fields:
 
 * ``theta`` = (H_shift, eta, gamma), float64, shape (3,): a uniform shift
   added to the problem's applied field h, and the couplings eta and gamma.
@@ -94,20 +94,24 @@ class _FreeEnergy(torch.autograd.Function):
     def backward(ctx, grad_out):
         a, p1, p2, theta = ctx.saved_tensors
         g: GLEnergy = ctx.g
-        c = _load(g, theta, a, p1, p2)
-        w = grad_out.detach().to(torch.float64)
-        ga = gp1 = gp2 = gth = None
-        need_fields = ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
-        if need_fields:
-            ta, t1 = torch.empty_like(a), torch.empty_like(p1)
-            t2 = torch.empty_like(p2) if p2 is not None else None
-            c.energy_grad_device(ta.data_ptr(), t1.data_ptr(), None if t2 is None else t2.data_ptr(),
-                                 with_energy=False)
-            scale = w.to(device=a.device, dtype=a.dtype).view(-1, 1, 1, 1)
-            ga = ta * scale if ctx.needs_input_grad[0] else None
-            gp1 = t1 * scale if ctx.needs_input_grad[1] else None
-            gp2 = t2 * scale if (t2 is not None and ctx.needs_input_grad[2]) else None
+        w = grad_out.detach().to(device=a.device, dtype=torch.float64).contiguous()
+        c = _load(g, theta, a, p1, p2)         # waits for w too
+        ga = gp1 = gp2 = gth = adj = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
+            ga, gp1 = torch.empty_like(a), torch.empty_like(p1)
+            gp2 = torch.empty_like(p2) if p2 is not None else None
+            at = (ga.data_ptr(), gp1.data_ptr(), None if gp2 is None else gp2.data_ptr())
+            try:
+                at_w = w.data_ptr()
+            except RuntimeError:     # weights without storage (vmap over backward passes): the scaling is PyTorch's
+                c.energy_grad_device(*at, with_energy=False)
+                scale = w.to(a.dtype).view(-1, 1, 1, 1)
+                ga, gp1, gp2 = (None if v is None else v * scale for v in (ga, gp1, gp2))
+            else:
+                adj = c.weighted_grad_device(at_w, *at, with_adjoint=ctx.needs_input_grad[3])
         if ctx.needs_input_grad[3]:
-            adj = torch.from_numpy(np.ascontiguousarray(c.param_adjoint()))   # (F, 3)
-            gth = (w.cpu().view(-1, 1) * adj).sum(0).to(theta.device, theta.dtype)
-        return ga, gp1, gp2, gth, None
+            if adj is None:
+                adj = np.ascontiguousarray(c.param_adjoint())
+            gth = (w.cpu().view(-1, 1) * torch.from_numpy(adj)).sum(0).to(theta.device, theta.dtype)
+        return (ga if ctx.needs_input_grad[0] else None, gp1 if ctx.needs_input_grad[1] else None,
+                gp2 if ctx.needs_input_grad[2] else None, gth, None)

@@ -1143,6 +1143,24 @@ mepgl_status mepgl_energy_grad(mepgl_ctx *c, double *fenergy, void *g_a, void *g
     return copy_fields(c, s, dst, src, memory, false);
 }
 
+mepgl_status mepgl_weighted_grad(mepgl_ctx *c, const double *weights, double *adjoint, void *g_a, void *g_psi_1,
+                                 void *g_psi_2)
+{
+    if (!c) return MEPGL_ERR_INVALID_ARG;
+    if (!weights || !g_a || !g_psi_1 || (c->ncomp == 2 && !g_psi_2))
+        return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_weighted_grad: null argument");
+    mepgl_status st = flush(c);
+    if (st != MEPGL_OK) return st;
+    Launch L = string_launch(c, 0);
+    L.paired = 0;   // as mepgl_energy_grad
+    CK(c, launch_gradient_only(L, c->sc, c->xi, FieldPtrs{{g_a, g_psi_1, c->ncomp == 2 ? g_psi_2 : nullptr}}, 0, weights,
+                               adjoint ? c->dscratch : nullptr));
+    c->launches += 1;
+    if (adjoint) return fetch(c, {{adjoint, c->dscratch, 3 * (size_t)c->strings[0].F}}, false);
+    CK(c, cudaStreamSynchronize(c->stream));
+    return MEPGL_OK;
+}
+
 mepgl_status mepgl_nlcg_steps(mepgl_ctx *c, int iterations, int use_cg, int maxwell_only)
 {
     if (c) ++c->state_version;

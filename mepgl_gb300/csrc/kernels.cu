@@ -1255,9 +1255,12 @@ cudaError_t launch_energy(const Launch &L, const Scalars &sc, int xbuf, double *
 // FP64 launches with L.paired compute in float-float on the double fields
 // (about 48 bits) and store double gradients; the link discretisation has
 // no float-float form and stays IEEE double.
-cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell)
+cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell,
+                                 const double *weights, double *adjoint)
 {
-    const GradientOp op{{out.p[0], out.p[1], out.p[2]}, maxwell};
+    if (adjoint)
+        return walk(L, sc, xbuf, GradientOp<true>{{out.p[0], out.p[1], out.p[2]}, maxwell, weights, adjoint});
+    const GradientOp<false> op{{out.p[0], out.p[1], out.p[2]}, maxwell, weights, nullptr};
     if (L.paired && L.precision == 1 && !L.str->disc) return walk<ff>(L, sc, xbuf, op);
     return walk(L, sc, xbuf, op);
 }

@@ -68,7 +68,11 @@ cudaError_t launch_param_adjoint(const Launch &L, const Scalars &sc, int xbuf, d
 // Gradient of x[xbuf] into the three arrays of `out` (single string).
 struct FieldPtrs { void *p[3]; };
 // Gradient of every image into `out` (FP64 launches with L.paired: float-float arithmetic).
-cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell);
+// weights (device, per image of the string; null: 1) multiply each image's
+// gradient; adjoint (null: none): dF/dH, dF/deta, dF/dgamma at [3 img + k],
+// formed by the same walk (not in float-float).
+cudaError_t launch_gradient_only(const Launch &L, const Scalars &sc, int xbuf, FieldPtrs out, int maxwell,
+                                 const double *weights = nullptr, double *adjoint = nullptr);
 // B, J of x[xbuf] (b: F*M reals, j1, j2: F*M pairs); flux dx^2 sum B per image of the string.
 cudaError_t launch_jb(const Launch &L, const Scalars &sc, int xbuf, void *b, void *j1, void *j2);
 cudaError_t launch_flux(const Launch &L, const Scalars &sc, int xbuf, double *out);

@@ -99,6 +99,7 @@ _SIGS = {
     "mepgl_get_state": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]),
     "mepgl_free_energy": (C.c_int, [C.c_void_p, C.c_void_p]),
     "mepgl_energy_grad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]),
+    "mepgl_weighted_grad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "mepgl_nlcg_steps": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int]),
     "mepgl_reset_cg": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "mepgl_image_scalars": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
@@ -290,6 +291,13 @@ class StringContext:
         e = np.zeros(self.F) if with_energy else None
         self._check(self.L.mepgl_energy_grad(self.h, _ptr(e), _ptr(g_a), _ptr(g_psi_1), _ptr(g_psi_2), DEVICE))
         return e
+
+    def weighted_grad_device(self, weights, g_a, g_psi_1, g_psi_2=None, with_adjoint=False):
+        """weights[n] dF_n/dfields into device arrays; with_adjoint: also the (F, 3) of param_adjoint, unweighted."""
+        adj = np.empty((self.F, 3)) if with_adjoint else None
+        self._check(self.L.mepgl_weighted_grad(self.h, _ptr(weights), _ptr(adj), _ptr(g_a), _ptr(g_psi_1),
+                                               _ptr(g_psi_2)))
+        return adj
 
     def nlcg_steps(self, iterations: int, nlcg: bool = True, maxwell: bool = False):
         self._check(self.L.mepgl_nlcg_steps(self.h, int(iterations), int(nlcg), int(maxwell)))

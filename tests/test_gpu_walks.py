@@ -36,6 +36,7 @@ def relmax(a, b):
     (True, False, False, True), (False, False, True, True)])
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 def test_walks(nx, ny, images, mc, film, uniform, link, precision):
+    torch = pytest.importorskip("torch")
     from mepgl_gb300 import native
     rng = np.random.default_rng(nx * 1000 + ny)
     prob = problem(rng, nx, ny, mc, film, uniform, 0.0 if link else 0.1)
@@ -64,6 +65,17 @@ def test_walks(nx, ny, images, mc, film, uniform, link, precision):
         for k in range(3):
             if np.any(wa[:, k]):
                 assert relmax(adj[:, k], wa[:, k]) < tol, k
+    # the same gradients and adjoints from one walk, each image's times its weight
+    w = rng.uniform(-2, 2, images)
+    dt = torch.float64 if precision == "fp64" else torch.float32
+    out = [torch.zeros(st.a.shape, dtype=dt, device="cuda") for _ in range(3)]
+    wd = torch.tensor(w, device="cuda")
+    torch.cuda.synchronize()
+    both = c.weighted_grad_device(wd.data_ptr(), *(v.data_ptr() for v in out), with_adjoint=True)
+    for k in comps:
+        f = w.astype(np.asarray(g[k]).dtype)[:, None, None, None]
+        assert relmax(out[k].cpu().numpy(), g[k] * f) < tol, k
+    np.testing.assert_allclose(both, adj, rtol=tol, atol=tol * np.abs(adj).max())
     if link:
         return
     b, j1, j2 = c.compute_jb()
@@ -101,3 +113,20 @@ def test_plans(images, spread, cubic):
         want = o.redistribute(s, getattr(st, k), images, cubic=cubic)
         want[-1] = getattr(st, k)[-1]
         assert relmax(getattr(got, k), want) < 1e-11 + 2e-16 * images * 10.0 ** spread, k
+
+
+def test_vmap_over_backward_passes():
+    """Weights without storage: the rows of the Jacobian by torch.func.vmap over autograd.grad."""
+    torch = pytest.importorskip("torch")
+    from mepgl_gb300.autograd import GLEnergy
+    rng = np.random.default_rng(3)
+    prob = problem(rng, 9, 7, True, False, True, 0.0)
+    st = random_state(rng, prob, images=3, amp=0.2)
+    x = [torch.tensor(getattr(st, k), dtype=torch.float64, device="cuda", requires_grad=True)
+         for k in ("a", "psi_1", "psi_2")]
+    e = GLEnergy(prob, 3)(*x)
+    eye = torch.eye(3, dtype=torch.float64, device="cuda")
+    rows = torch.func.vmap(lambda v: torch.autograd.grad(e, x, v, retain_graph=True))(eye)
+    for n in range(3):
+        for got, want in zip(rows, torch.autograd.grad(e, x, eye[n], retain_graph=True)):
+            torch.testing.assert_close(got[n], want, rtol=1e-15, atol=0)
