@@ -269,7 +269,8 @@ mepgl_status build_layout(mepgl_ctx *c)
     const size_t o_xf = take(LS_GRID), o_xd = take(LS_GRID), tables = at;
     size_t o_img[7];
     for (int k = 0; k < 4; ++k) o_img[k] = take(I);
-    const size_t o_poly = take(4 * I), o_tick = take((I + 1) / 2), o_stage = take((I + 1) / 2), o_queue = take(1),
+    const size_t o_poly = take(4 * I), o_tick = take((I + 1) / 2), o_queue = take(1),
+                 o_stage = take((STAGE_STRIDE * I + 1) / 2),   // right after the counter: cleared together
                  o_mail = at;   // from here on what fetch() brings to the host
     for (int k = 4; k < 7; ++k) o_img[k] = take(I);
     const size_t o_status = take(8), o_scr = take(3 * I + 64), o_ds = take(fmax + 1), o_jb = take(fmax + 1), zeroed = at,

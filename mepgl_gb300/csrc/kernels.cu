@@ -228,15 +228,16 @@ __device__ double line_search_scan(const double *c, const double *xt)
 
 // Smallest positive root of the quartic's derivative f = a0 + a1 x + a2 x^2 +
 // a3 x^3 with a0 < 0 < a3 (its first local minimum: f crosses zero upwards
-// there) by Newton's method from a point from which it converges
-// monotonically.  f has its turning points at c1 <= c2 where D = a2^2 - 3 a1
-// a3 > 0 and its inflection at cm.  Left of cm it is concave: if f rises from
-// 0 to its root there, Newton from 0 stays left of it.  Right of cm it is
-// convex: Newton from a bound above the root stays right of it.  The steps
-// divide by a float reciprocal (each still gains seven digits).  False where
-// a case is out of the ordinary (no such bound in float range, slow
-// convergence); the caller then takes the closed form, whose acos, cos and
-// cbrt cost a lone warp about 10 us.
+// there).  Newton's method in float, x and f in units (powers of two) that
+// make the constant about -1 and every other coefficient 1 at most, from a
+// point from which it converges monotonically: f has its turning points at c1
+// <= c2 where D = a2^2 - 3 a1 a3 > 0 and its inflection at cm.  Left of cm it
+// is concave: if f rises from 0 to its root there, Newton from 0 stays left of
+// it.  Right of cm it is convex: Newton from a bound above the root stays right
+// of it.  Then steps in double with that slope, each of which gains about five
+// digits.  False where a case is out of the ordinary (far out of float's range,
+// a turning point that float cannot tell from a root, steps that shrink by less
+// than 1000); the caller then takes the closed form.
 __device__ bool first_minimum(double a0, double a1, double a2, double a3, double &root)
 {
     if (!(a0 < 0.0)) return false;
@@ -245,35 +246,61 @@ __device__ bool first_minimum(double a0, double a1, double a2, double a3, double
         return a1 > 0.0;
     }
     if (!(a3 > 0.0)) return false;
-    const double b2 = 2.0 * a2, b3 = 3.0 * a3, D = a2 * a2 - a1 * b3;
-    const double cm = -a2 / b3, fm = a0 + cm * (a1 + cm * (a2 + cm * a3));
-    double x = 0.0;
-    bool right = fm < 0.0;   // monotone f: right of the inflection if it is still negative there
-    if (D > 0.0) {
-        const double sd = sqrt(D), c1 = cm - sd / b3;
-        const double f1 = a0 + c1 * (a1 + c1 * (a2 + c1 * a3));
-        right = !(c1 > 0.0 && f1 > 0.0);
-    } else if (!right && !(a1 > 0.0)) {
-        return false;
-    }
-    if (right) {
-        // x - cm <= max(sqrt(2 |P|), cbrt(2 |Q|)) of the depressed cubic z^3 + P z + Q
-        const float P = (float)(2.0 * fabs(D) / (b3 * a3)), Q = (float)(2.0 * fabs(fm) / a3);
-        const float z = 1.0001f * fmaxf(sqrtf(P), cbrtf(Q));
-        if (!(z > 1e-30f && z < 1e30f)) return false;
-        x = cm + (double)z;
-        if (!(x > 0.0)) return false;
-    }
-    for (int it = 0; it < 24; ++it) {
-        const double f = a0 + x * (a1 + x * (a2 + x * a3)), df = a1 + x * (b2 + x * b3);
-        const float d = (float)df;
-        if (!(d > 1e-30f && d < 1e30f)) return false;
-        const double dx = f * (double)(1.0f / d);
-        x -= dx;
-        if (fabs(dx) <= 1e-9 * fabs(x)) {
-            root = x;
-            return x > 0.0;
+    auto exponent = [](double v) { return ((__double2hiint(v) >> 20) & 0x7ff) - 1023; };
+    auto pow2 = [](int k) { return __hiloint2double((k + 1023) << 20, 0); };
+    const int e0 = exponent(a0), k1 = e0 - exponent(a1), k2 = (e0 - exponent(a2)) >> 1, k3 = (e0 - exponent(a3)) / 3 - 1;
+    const int ex = min(k1, min(k2, k3));
+    if (abs(e0) > 300 || abs(ex) > 200) return false;
+    const float A0 = (float)(a0 * pow2(-e0)), A1 = (float)(a1 * pow2(ex - e0)), A2 = (float)(a2 * pow2(2 * ex - e0)),
+                A3 = (float)(a3 * pow2(3 * ex - e0));
+    const float b2 = 2.0f * A2, b3 = 3.0f * A3;
+    float x = 0.0f;
+    if (k1 == ex && A1 > 0.0f && fabsf(A2) <= 0x1p-8f && A3 <= 0x1p-8f) {
+        x = -A0 / A1;   // nearly linear: 1 <= A1 < 2, so that f rises from 0 to 4 by more than |A0| < 2
+    } else {
+        const float p = A2 * A2, q = A1 * b3, D = p - q;
+        if (!(b3 > 1e-25f)) return false;
+        const float cm = -A2 / b3, fm = A0 + cm * (A1 + cm * (A2 + cm * A3));
+        const float noise = 1e-6f * (fabsf(A0) + fabsf(cm) * (fabsf(A1) + fabsf(cm) * (fabsf(A2) + fabsf(cm) * A3)));
+        if (fabsf(D) <= 1e-6f * (p + fabsf(q)) && !(fabsf(fm) > noise)) return false;
+        bool right = fm < 0.0f;   // monotone f: right of the inflection if it is still negative there
+        if (D > 0.0f) {
+            // c1 > 0 needs a2 < 0 (else it is the negative one of two roots, or both are negative)
+            const float c1 = A2 < 0.0f ? A1 / (sqrtf(D) - A2) : -1.0f;
+            const float f1 = A0 + c1 * (A1 + c1 * (A2 + c1 * A3));
+            if (c1 > 0.0f && !(fabsf(f1) > 1e-6f * (fabsf(A0) + c1 * (fabsf(A1) + c1 * (fabsf(A2) + c1 * A3))))) return false;
+            right = !(c1 > 0.0f && f1 > 0.0f);
+        } else if (!right && !(A1 > 0.0f)) {
+            return false;
         }
+        if (right) {
+            // x - cm <= max(sqrt(2 |P|), cbrt(2 |Q|)) of the depressed cubic z^3 + P z + Q
+            const float z = 1.0001f * fmaxf(sqrtf(2.0f * fabsf(D) / (b3 * A3)), cbrtf(2.0f * fabsf(fm) / A3));
+            if (!(z > 1e-30f && z < 1e30f)) return false;
+            x = cm + z;
+            if (!(x > 0.0f)) return false;
+        }
+    }
+    float r = 0.0f;   // 1 / slope
+    for (int it = 0; it < 24; ++it) {
+        const float f = A0 + x * (A1 + x * (A2 + x * A3)), d = A1 + x * (b2 + x * b3);
+        if (!(d > 1e-30f && d < 1e30f)) return false;
+        r = 1.0f / d;
+        const float dx = f * r;
+        x -= dx;
+        if (fabsf(dx) <= 1e-4f * fabsf(x)) break;
+    }
+    const double rs = pow2(ex - e0) * (double)r;
+    double y = (double)x * pow2(ex), last = fabs(y);
+    for (int it = 0; it < 8; ++it) {
+        const double dy = (a0 + y * (a1 + y * (a2 + y * a3))) * rs, ay = fabs(dy);
+        y -= dy;
+        if (ay <= 1e-13 * fabs(y)) {
+            root = y;
+            return y > 0.0;
+        }
+        if (!(ay <= 1e-3 * last)) return false;
+        last = ay;
     }
     return false;
 }
@@ -1215,8 +1242,7 @@ static cudaError_t nlcg_fused_launch(const Launch &L, const Scalars &sc, const S
             return e != cudaSuccess ? e : cudaErrorInvalidConfiguration;
         }
     }
-    const long long items = 2LL * L.n_stiles * steps;
-    const int grid = items < slots[ci] ? (int)items : slots[ci];
+    const int grid = L.n_stiles < slots[ci] ? L.n_stiles : slots[ci];
 #define FUSED_ARGS L.stile0, L.n_stiles, steps, plan, sc, queue, stage, max_polls
     switch (ci) {
     case 0: k_nlcg_s<T, 1, false><<<grid, NTS, 0, L.stream>>>(*L.batch, FUSED_ARGS); break;
@@ -1237,10 +1263,13 @@ cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlag
     plan.di0 = f0.din;
     plan.it0 = it0;
     plan.base = f0;
-    cudaError_t e = first_item ? cudaMemcpyAsync(queue, &first_item, sizeof(first_item), cudaMemcpyHostToDevice, L.stream)
-                               : cudaMemsetAsync(queue, 0, sizeof(unsigned long long), L.stream);
-    if (e == cudaSuccess && first_item) e = cudaStreamSynchronize(L.stream);   // first_item is a host local
-    if (e == cudaSuccess) e = cudaMemsetAsync(stage, 0, sizeof(unsigned) * (size_t)n_stage, L.stream);
+    // the counter and the stages lie in one piece of memory
+    char *const end = reinterpret_cast<char *>(stage + (size_t)n_stage * STAGE_STRIDE);
+    cudaError_t e = cudaMemsetAsync(queue, 0, end - reinterpret_cast<char *>(queue), L.stream);
+    if (e == cudaSuccess && first_item) {
+        e = cudaMemcpyAsync(queue, &first_item, sizeof(first_item), cudaMemcpyHostToDevice, L.stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream);   // first_item is a host local
+    }
     if (e != cudaSuccess) return e;
     return L.precision == 0 ? nlcg_fused_launch<float>(L, sc, plan, steps, queue, stage, max_polls)
            : L.paired       ? nlcg_fused_launch<ff>(L, sc, plan, steps, queue, stage, max_polls)

@@ -41,9 +41,12 @@ int fuse_waves(int precision);
 int strip_pass_slots(int precision, int paired, int ncomp);
 // `steps` NLCG steps (iterations it0, it0 + 1, ...; step 0 with the buffers
 // of f0) of the launch's tiles in one persistent launch; queue (one counter)
-// and stage (one per global image, n_stage) are reset on the stream first.
+// and stage (one per global image, n_stage, STAGE_STRIDE words apart: a line
+// each, because whole strips of warps poll them) lie in one allocation in this
+// order and are reset on the stream first.
 // first_item > 0 starts the queue there (the wait self-test); each per-image
 // wait polls at most max_polls times.
+constexpr int STAGE_STRIDE = 32;
 constexpr unsigned STAGE_WAIT_POLLS = 1u << 22;   // about 100 ns to 1 us per poll
 cudaError_t launch_nlcg_fused(const Launch &L, const Scalars &sc, const StepFlags &f0, int it0, int steps,
                               unsigned long long *queue, unsigned *stage, int n_stage,

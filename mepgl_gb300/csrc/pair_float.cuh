@@ -100,6 +100,13 @@ __device__ __forceinline__ ff shfl_down(ff v, int o)
     return ff(__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o));
 }
 
+__device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ ff shfl_xor(ff v, int o)
+{
+    return ff(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
+}
+
 // lane to the right (+1) / left (-1) of any lattice number type
 template <class T> __device__ __forceinline__ T shfl_right(T v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 template <class T> __device__ __forceinline__ T shfl_left(T v) { return __shfl_up_sync(0xffffffffu, v, 1); }

@@ -162,6 +162,17 @@ __device__ __forceinline__ void strip_load(vec2_t<T> (&c)[NA][1 + NC], const vec
             for (int k = 0; k < 1 + NC; ++k) c[a][k] = src[a][k][sc_];
 }
 
+// Zeros in place of the arrays that are not in `keep`.
+template <class T, int NC>
+__device__ __forceinline__ void drop_arrays(vec2_t<T> (&c)[3][1 + NC], unsigned keep)
+{
+#pragma unroll
+    for (int a = 1; a < 3; ++a)
+        if (!((keep >> a) & 1u))
+#pragma unroll
+            for (int k = 0; k < 1 + NC; ++k) c[a][k] = zero2<T>();
+}
+
 // Halo column of row j: lanes 0 and 31 copy arrays a < NR of hmask at their
 // halo column into slot[side][a] by cp.async (zero-filled outside the
 // lattice).  Every lane commits one group per call (empty for the others,
@@ -223,9 +234,76 @@ __device__ __forceinline__ uint16_t strip_code(const StringDesc &S, const StripL
     return S.mask[L.gi + S.nx * j];
 }
 
-// Warp form of finish_image: the tile's NV partials leave from lane 0; if
-// this tile is the last of its image, every lane receives the image sums
-// (its partials added in index order) and the function returns true.
+// Sums of N values over a warp with about N + 3 additions instead of 5 N: at
+// each of the first distances a lane gives half of its values away and adds
+// the other half, so that value k ends up in lane sum_lane<N>(k) (and in others).
+template <int N>
+__device__ constexpr int sum_lane(int k)
+{
+    int lane = 0;
+    for (int n = N, o = 16; n > 1; n = (n + 1) / 2, o >>= 1)
+        if (k >= (n + 1) / 2) {
+            lane |= o;
+            k -= (n + 1) / 2;
+        }
+    return lane;
+}
+
+template <int N, class T>
+__device__ __forceinline__ T warp_sums(T (&w)[N])
+{
+    const int lane = threadIdx.x & 31;
+    int n = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int h = (n + 1) / 2;
+        const bool up = n > 1 && (lane & o);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (i >= h) continue;
+            const T hi = n == 1 ? w[i] : i + h < n ? w[i + h < N ? i + h : i] : (T)0;
+            const T keep = up ? hi : w[i], give = up ? w[i] : hi;
+            w[i] = keep + shfl_xor(give, o);
+        }
+        n = h;
+    }
+    return w[0];
+}
+
+// Sums of n strips' partials (8 doubles each, NV used), added in index order
+// per lane, to every lane.  AHEAD strips' loads are in flight per lane.
+constexpr int AHEAD = 4;
+template <int NV>
+__device__ __forceinline__ void image_sums(const double *part, int n, double (&tot)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    double acc[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+    for (int t0 = 0; t0 < n; t0 += 32 * AHEAD) {
+        double q[AHEAD][NV];
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+            const int t = t0 + 32 * a + lane;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) q[a][k] = t < n ? __ldcg(part + (size_t)t * 8 + k) : 0.0;
+        }
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) acc[k] += q[a][k];
+    }
+    const double all = warp_sums<NV>(acc);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) tot[k] = __shfl_sync(FULL_MASK, all, sum_lane<NV>(k));
+}
+
+// The strip's NV partials leave the warp; if this strip is the last of its
+// image, every lane receives the image sums (its partials added in index
+// order) and the function returns true.  Everything that the lanes wrote
+// before is visible to whoever learns from the ticket (or from what the last
+// strip publishes) that the strip is done: the warp barrier orders the lanes'
+// writes before lane 0's fence, which is cumulative.
 template <int NV, class T>
 __device__ __forceinline__ bool finish_image_warp(const T (&v)[NV], const Scalars &sc, int tile, int first_tile,
                                                   int tiles_per_image, int img, double (&tot)[NV])
@@ -233,35 +311,22 @@ __device__ __forceinline__ bool finish_image_warp(const T (&v)[NV], const Scalar
     const int lane = threadIdx.x & 31;
     T w[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        w[k] = v[k];
+    for (int k = 0; k < NV; ++k) w[k] = v[k];
+    const double mine = (double)warp_sums<NV>(w);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) w[k] += shfl_down(w[k], o);
-    }
+    for (int k = 0; k < NV; ++k)
+        if (lane == sum_lane<NV>(k)) sc.part[(size_t)tile * 8 + k] = mine;
+    __syncwarp();
     int last = 0;
     if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sc.part[(size_t)tile * 8 + k] = (double)w[k];
         __threadfence();
         last = atomicAdd(&sc.ticket[img], 1u) == (unsigned)tiles_per_image - 1;
+        if (last) __threadfence();
     }
     last = __shfl_sync(FULL_MASK, last, 0);
     if (!last) return false;
-    __threadfence();
-    double acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-    for (int t = lane; t < tiles_per_image; t += 32) {
-        const double *p = sc.part + (size_t)(first_tile + t) * 8;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) acc[k] += __ldcg(p + k);
-    }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(FULL_MASK, acc[k], o);
-        tot[k] = __shfl_sync(FULL_MASK, acc[k], 0);
-    }
+    __syncwarp();
+    image_sums<NV>(sc.part + (size_t)first_tile * 8, tiles_per_image, tot);
     if (lane == 0) sc.ticket[img] = 0;
     return true;
 }
@@ -313,9 +378,8 @@ using GradRing = vec2_t<T>[3][2][2][1 + NC];
 // Gradient pass on one strip: x <- x + alpha_pend d over the strip (+ halo),
 // the gradient of every site, |g|^2 and g . (g - g_prev); the last strip of an
 // image computes beta.  Returns true (in every lane) when this strip finished
-// its image.  Before the strip's partials are counted every lane fences its
-// field stores, so that a consumer that has seen the image finished (same
-// launch) reads them.
+// its image; a consumer in the same launch that has seen the image finished
+// reads the field stores (finish_image_warp).
 template <class T, int NC, bool ONE>
 __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
@@ -336,14 +400,29 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         xout[c] = static_cast<V *>(S.x[f.xout][c]) + off;
         gcur[c] = static_cast<V *>(S.g[f.gcur][c]) + off;
     }
-    const T alpha = (T)__ldcg(sc.alpha_pend + img);
-    const unsigned fields = alpha != (T)0 ? 3u : 1u;   // d is not read when nothing is pending
-    // nor g_prev when it does not enter beta (restarted image, steepest descent)
-    const bool hist = f.use_cg && __ldcg((f.gprev ? sc.gn1 : sc.gn0) + img) <= 1.7976931348623157e308;
+    const double alpha_d = __ldcg(sc.alpha_pend + img), norm = f.use_cg ? __ldcg((f.gprev ? sc.gn1 : sc.gn0) + img) : INFINITY;
+    // the first three rows are loaded together, and before the scalars are looked
+    // at: one memory latency, not three or four.  What turns out not to be read
+    // (below) is dropped again.
+    V ra[3][1 + NC], rb[3][1 + NC], rc[3][1 + NC];
+    uint16_t ma, mb, rm;
+    auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, unsigned arrays) {
+        strip_load<T, NC, 3>(raw, src, S, L, j, arrays);
+        strip_halo<T, NC, 2, 3>(ring[(j + 3) % 3], src, S, L, j, arrays & 3u, true);
+        m = strip_code(S, L, j);
+    };
+    load(ra, ma, j0 - 1, 3u);
+    load(rb, mb, j0, f.use_cg ? 7u : 3u);
+    load(rc, rm, j0 + 1, f.use_cg ? 7u : 3u);
+    const T alpha = (T)alpha_d;
+    // d is not read when nothing is pending, nor g_prev when it does not enter
+    // beta (restarted image, steepest descent)
+    const unsigned fields = (alpha != (T)0 ? 3u : 1u) | (norm <= 1.7976931348623157e308 ? 4u : 0u);
+    drop_arrays<T, NC>(ra, fields);
+    drop_arrays<T, NC>(rb, fields);
+    drop_arrays<T, NC>(rc, fields);
     PackParams<T, NC> pp;
     pp.load(S);
-    V rc[3][1 + NC];
-    uint16_t rm;
     // raw row j -> window row (x + alpha d; left / right A by shuffles)
     auto take = [&](GradRow<T, NC> &R, int j, V (&hp)[NC], const V (&raw)[3][1 + NC], uint16_t m) {
         cp_async_wait_groups<0>();   // row j's halo is in the newest groups
@@ -368,11 +447,6 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         for (int c = 0; c < NC; ++c) hp[c] = hx[1 + c];
         R.m = m;
     };
-    auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, bool gold) {
-        strip_load<T, NC, 3>(raw, src, S, L, j, gold && hist ? fields | 4u : fields);
-        strip_halo<T, NC, 2, 3>(ring[(j + 3) % 3], src, S, L, j, fields, true);
-        m = strip_code(S, L, j);
-    };
     // FP64 and float-float rows hand their upper y-link and views on to the next
     // (21 of 233 FP64 instructions); FP32 forms them again from the row below,
     // because the carry costs 20 registers, i.e. warps (sweep of 16 strings:
@@ -381,12 +455,7 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     GradRow<T, NC> Rm, R0, Rp;
     V hp0[NC], hp1[NC];
     GradCarry<T, NC> up;   // from the row below
-    {   // the first three rows are loaded together: one memory latency, not three
-        V ra[3][1 + NC], rb[3][1 + NC];
-        uint16_t ma, mb;
-        load(ra, ma, j0 - 1, false);
-        load(rb, mb, j0, true);
-        load(rc, rm, j0 + 1, true);
+    {
         take(Rm, j0 - 1, hp0, ra, ma);
         take(R0, j0, hp0, rb, mb);
         if constexpr (CARRY) {
@@ -408,7 +477,7 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
         take(Rp, j + 1, hp1, rc, rm);
-        if (r + 1 < rows) load(rc, rm, j + 2, true);
+        if (r + 1 < rows) load(rc, rm, j + 2, fields);
         const int s = L.gi + S.nx * j;
         if (L.cok) {
             V o[1 + NC];
@@ -460,15 +529,13 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     }
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[2];
-    __threadfence();
-    __syncwarp();
     const bool fin = finish_image_warp<2>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
     if (fin && L.lane == 0) {
         (f.gcur ? sc.gn1 : sc.gn0)[img] = tot[0];
         sc.gdg[img] = tot[1];
         double beta = 0.0;
         if (f.use_cg) {
-            beta = tot[1] / __ldcg((f.gprev ? sc.gn1 : sc.gn0) + img);
+            beta = tot[1] / __ldcg((f.gprev ? sc.gn1 : sc.gn0) + img);   // again: a register pair held through the rows costs more
             beta = beta > 0.0 ? beta : 0.0;   // Polak-Ribiere clipped at 0; NaN -> 0
         }
         sc.beta[img] = beta;
@@ -498,8 +565,7 @@ using DirRing = vec2_t<T>[3][2][3][1 + NC];
 
 // Direction pass on one strip: d <- -g + beta d over the strip (+ halo), the
 // quartic coefficients of F(x + a d); the last strip of an image runs the line
-// search.  Returns true (in every lane) when this strip finished its image;
-// field stores are fenced as in grad_tile.
+// search.  Returns true (in every lane) when this strip finished its image.
 template <class T, int NC, bool ONE>
 __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                          DirRing<T, NC> &ring, double (&coef)[5])
@@ -519,12 +585,24 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
         src[2][c] = static_cast<const V *>(S.d[f.din][c]) + off;
         dout[c] = static_cast<V *>(S.d[f.dout][c]) + off;
     }
-    const T beta = (T)__ldcg(sc.beta + img);
+    const double beta_d = __ldcg(sc.beta + img);
+    V ra[3][1 + NC], rb[3][1 + NC], rc[3][1 + NC];   // as in grad_tile
+    uint16_t ma, mb, rm;
+    auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, unsigned arrays) {
+        strip_load<T, NC, 3>(raw, src, S, L, j, arrays);
+        strip_halo<T, NC, 3, 3>(ring[(j + 3) % 3], src, S, L, j, arrays, true);
+        m = strip_code(S, L, j);
+    };
+    load(ra, ma, j0 - 1, f.use_cg ? 7u : 3u);
+    load(rb, mb, j0, f.use_cg ? 7u : 3u);
+    load(rc, rm, j0 + 1, f.use_cg ? 7u : 3u);
+    const T beta = (T)beta_d;
     const unsigned fields = beta != (T)0 ? 7u : 3u;    // d is not read when it does not enter
+    drop_arrays<T, NC>(ra, fields);
+    drop_arrays<T, NC>(rb, fields);
+    drop_arrays<T, NC>(rc, fields);
     PackParams<T, NC> pp;
     pp.load(S);
-    V rc[3][1 + NC];
-    uint16_t rm;
     auto take = [&](DirRow<T, NC> &R, const V (&raw)[3][1 + NC], uint16_t m) {
 #pragma unroll
         for (int c = 0; c < 1 + NC; ++c) {
@@ -538,19 +616,9 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
         }
         R.m = m;
     };
-    auto load = [&](V (&raw)[3][1 + NC], uint16_t &m, int j, bool issue) {
-        strip_load<T, NC, 3>(raw, src, S, L, j, issue ? fields : 0u);
-        strip_halo<T, NC, 3, 3>(ring[(j + 3) % 3], src, S, L, j, fields, issue);
-        m = strip_code(S, L, j);
-    };
     DirRow<T, NC> R0, Rp;
     T xm_ax, dm_ax;   // row j - 1: only A_x of x and of d is read
-    {   // the first three rows are loaded together: one memory latency, not three
-        V ra[3][1 + NC], rb[3][1 + NC];
-        uint16_t ma, mb;
-        load(ra, ma, j0 - 1, true);
-        load(rb, mb, j0, true);
-        load(rc, rm, j0 + 1, true);
+    {
         take(R0, ra, ma);
         xm_ax = R0.x[0].x;
         dm_ax = R0.d[0].x;
@@ -566,7 +634,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
         take(Rp, rc, rm);
-        if (r + 1 < rows) load(rc, rm, j + 2, true);
+        if (r + 1 < rows) load(rc, rm, j + 2, fields);
         else strip_halo<T, NC, 3, 3>(ring[0], src, S, L, j + 2, 0u, false);
         cp_async_wait_groups<2>();   // groups of rows j + 1 and j + 2 may still be pending
         const int s = L.gi + S.nx * j;
@@ -644,8 +712,6 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     if constexpr (WIDE) sum.total(pp, v);
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[5];
-    __threadfence();
-    __syncwarp();
     const bool fin = finish_image_warp<5>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
     if (fin) {
         if (L.lane == 0) {
@@ -687,6 +753,15 @@ __global__ void __launch_bounds__(NTS, StripBlocks<T>::dir) k_dir_poly_s(const _
 // and an item is only taken by a running block, so the waits always end;
 // each is still bounded, and a wait that runs out sets status[0] and
 // ends its block.
+//
+// A small string's pass is a chain of latencies (67 x 61 sites, 9 images: 8 us,
+// of which the rows are 1.3): the wait's poll, three rows of loads, two rows of
+// arithmetic, the strip's sums and ticket, the image's sums over its strips,
+// the step, the publication.  So there is one fence in each of the last two
+// and none in the wait, the image's partials are loaded four strips at a time,
+// the stages lie a line apart and no more blocks run than a pass has strips
+// (more of them only poll).  Ten steps: 293 us before these, 200 with them;
+// 64 x 64 x 16 of two components in FP64 675 -> 632 with its reparametrization.
 
 // Step plan of a fused launch: the buffers and gradient slot of step k
 // follow from those of step 0 as the separate launches toggle them.
@@ -706,9 +781,9 @@ struct StepPlan {
     }
 };
 
-// Lane 0 waits until stage >= need (acquire, then a fence so that the whole
-// warp's later loads see what the finishing block wrote), polling at most
-// max_polls times; false if the wait ran out.
+// Lane 0 waits until stage >= need, polling at most max_polls times; false if
+// the wait ran out.  Its acquire and the warp barrier order the whole warp's
+// later loads after what the finishing block wrote.
 __device__ __forceinline__ bool wait_stage(const unsigned *stage, unsigned need, unsigned max_polls, int *status)
 {
     int ok = 1;
@@ -724,7 +799,6 @@ __device__ __forceinline__ bool wait_stage(const unsigned *stage, unsigned need,
             }
             __nanosleep(64);
         }
-        __threadfence();
     }
     ok = __shfl_sync(FULL_MASK, ok, 0);
     __syncwarp();
@@ -734,7 +808,6 @@ __device__ __forceinline__ bool wait_stage(const unsigned *stage, unsigned need,
 __device__ __forceinline__ void publish_stage(unsigned *stage, unsigned value)
 {
     if ((threadIdx.x & 31) == 0) {
-        __threadfence();
         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(stage), "r"(value) : "memory");
     }
     __syncwarp();
@@ -761,12 +834,12 @@ __global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __g
         const StripRef tr = strip_tile<ONE>(bt, tile0 + u);
         const int img = bt.s[ONE ? 0 : tr.s].img_base + tr.n;
         const unsigned need = 2u * (unsigned)k + (unsigned)pass;
-        if (need > 0 && !wait_stage(stage + img, need, max_polls, sc.status)) return;
+        if (need > 0 && !wait_stage(stage + (size_t)img * STAGE_STRIDE, need, max_polls, sc.status)) return;
         const StepFlags f = plan.step(k);
         if (pass == 0) {
-            if (grad_tile<T, NC, ONE>(bt, tr, sc, f, gring)) publish_stage(stage + img, need + 1);
+            if (grad_tile<T, NC, ONE>(bt, tr, sc, f, gring)) publish_stage(stage + (size_t)img * STAGE_STRIDE, need + 1);
         } else {
-            if (dir_tile<T, NC, ONE>(bt, tr, sc, f, dring, coef)) publish_stage(stage + img, need + 1);
+            if (dir_tile<T, NC, ONE>(bt, tr, sc, f, dring, coef)) publish_stage(stage + (size_t)img * STAGE_STRIDE, need + 1);
         }
     }
 }
