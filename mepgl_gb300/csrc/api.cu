@@ -5,7 +5,7 @@
 // count) and every device buffer they need, allocated at creation: fields
 // x (ping-pong), gradients g (two slots), directions d (ping-pong),
 // packed neighbour masks, per-site parameters when not uniform, per-image
-// scalars and per-tile partials.  The reference instead allocated and freed
+// scalars and per-strip partials.  The reference instead allocated and freed
 // scratch inside every call (mepgl/src/nlcg.cu:225-239,
 // mepgl/src/parallel_sum.cu:49-67, mepgl/src/interpolation.cu:410-480).
 #include <algorithm>
@@ -224,7 +224,7 @@ int layout_strips(mepgl_ctx *c)
     return base;
 }
 
-// (Re)build tile table, descriptors and per-image arrays for the current strings.
+// (Re)build strip layout, descriptors and per-image arrays for the current strings.
 mepgl_status build_layout(mepgl_ctx *c)
 {
     drop_graphs(c);
@@ -335,7 +335,7 @@ Launch make_launch(mepgl_ctx *c, int batch)
     return L;
 }
 
-// Launch of the tile kernels over one string.
+// Launch of the kernels over one string.
 Launch string_launch(mepgl_ctx *c, int si)
 {
     Launch L = make_launch(c, c->string_batch[si]);

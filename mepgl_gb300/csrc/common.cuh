@@ -22,7 +22,7 @@
 
 namespace mepgl {
 
-constexpr int TX = 32;        // tile width: one warp per tile row
+constexpr int TX = 32;        // strip width: a warp
 constexpr int NT = 256;       // threads per block for the lattice kernels
 constexpr int MAX_STRINGS = 16;   // strings per launch (descriptors travel as a kernel parameter)
 
@@ -220,7 +220,7 @@ struct Scalars {
     double *alpha_pend;   // step not yet applied to x (0 = nothing pending)
     double *fenergy;      // energy (polynomial constant term)
     double *poly;         // [img][4] = B, C, D, E
-    double *part;         // per-tile partials, [tile][8]
+    double *part;         // partial sums, [strip][8]
     unsigned *ticket;     // per-image arrival counters
     double *xtab_f, *xtab_d;   // line-search grid x_p, p = 0..2000, rounded to float / double
     int *status;          // device-side error flags

@@ -46,7 +46,7 @@ template <> struct MaskOf<ff> { using type = float; };
 
 template <class T>
 struct Wts {
-    static constexpr bool interior = false;
+    static constexpr bool interior = false, masses = true;
     T area, wfx, wbx, wfy, wby, lfx, lbx, lfy, lby, wsx, wsy;
     T vUR, vUL, vLL, vLR, ivs;
     __device__ __forceinline__ void load(unsigned mk)

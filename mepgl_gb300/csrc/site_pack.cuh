@@ -213,11 +213,18 @@ struct PackParams {
 // Weights of a site whose neighbours all lie inside both domains, as
 // constants (FP64 strips: a row of such sites drops every multiplication by a
 // weight, 26 of 212 instructions of the gradient and 24 of 290 of the quartic).
+// Without per-site arrays the quartic's link sums also leave out the mass, which
+// multiplies them once per strip (16 more; a step of 256 x 256 x 64: 3.90 ->
+// 3.79 ms).
 struct Ones {
-    static constexpr bool interior = true;
+    static constexpr bool interior = true, masses = false;   // masses: each site's own, so they stay in the links' sums
     static constexpr double area = 1, wfx = 1, wbx = 1, wfy = 1, wby = 1, wsx = 2, wsy = 2;
     static constexpr double lfx = 1, lbx = 1, lfy = 1, lby = 1;
     static constexpr double vUR = 1, vUL = 1, vLL = 1, vLR = 1, ivs = 0.25;
+};
+
+struct OnesPerSite : Ones {
+    static constexpr bool masses = true;
 };
 
 // FP64: a biquadratic coupling of zero is skipped (a uniform branch; its 26
@@ -502,16 +509,30 @@ __device__ __forceinline__ void site_gradient(const GradView<S, NC> &c, const Gr
 // scalars, and the magnetic sums with their factors outside.
 template <class S, int NC>
 struct PolySum {
-    pack_t<S, NC> ka, kb, kc, kd, ke;
+    // FP64 rows of interior sites: the links' sums without their mass, per direction
+    static constexpr int LINKS = std::is_same<S, double>::value ? 2 : 1;
+    pack_t<S, NC> ka, kb, kc, kd, ke, la[LINKS], lb[LINKS], lc[LINKS], ld[LINKS];
     S e, b, c, d, e4, em0, em1, em2;
     __device__ __forceinline__ void zero()
     {
         ka = kb = kc = kd = ke = Pk<S, NC>::bc(S(0.0f));
+#pragma unroll
+        for (int q = 0; q < LINKS; ++q) la[q] = lb[q] = lc[q] = ld[q] = ka;
         e = b = c = d = e4 = em0 = em1 = em2 = S(0.0f);
     }
-    __device__ __forceinline__ void total(const PackParams<S, NC> &pp, S (&o)[5]) const
+    __device__ __forceinline__ void total(const PackParams<S, NC> &pp, bool links, int compat, S (&o)[5])
     {
         using K = Pk<S, NC>;
+        if constexpr (LINKS == 2) if (links) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const auto f = q == 0 ? pp.hmxi : pp.hmyi;
+                ka = pfma(f, la[q], ka);
+                kb = pfma(f, lb[q], kb);
+                kc = pfma(f, lc[q], kc);
+                kd = pfma(q == 1 && compat ? pmul(f, K::bc(S(0.5f))) : f, ld[q], kd);
+            }
+        }
         o[0] = fma1(S(0.125f), em0, e + K::sum(ka));
         o[1] = fma1(pp.idx4, em1, b + K::sum(kb));
         o[2] = fma1(pp.idx8, em2, c + K::sum(kc));
@@ -529,7 +550,8 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
                                           const PackParams<S, NC> &pp, const Wt &w, int per_site, int compat,
                                           int thin_film, PolySum<S, NC> &sum)
 {
-    constexpr bool ones = Wt::interior;
+    constexpr bool ones = Wt::interior, bare = ones && !Wt::masses;
+    constexpr int LINKS = PolySum<S, NC>::LINKS;
     using K = Pk<S, NC>;
     using P = pack_t<S, NC>;
     const S half = S(0.5f);
@@ -558,7 +580,10 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
         const P s0 = pmul(pp.qd, K::bc(Ai + Aj)), s1 = pmul(pp.qd, K::bc(ai + aj));
         const P P0 = pfma(s0, Y, Dx), P1 = pfma(s0, Vd, pfma(s1, Y, Ex)), P2 = pmul(s1, Vd);
         const P Q0 = pfma(s0, X, Dy), Q1 = pfma(s0, U, pfma(s1, X, Ey)), Q2 = pmul(s1, U);
-        const P fDx = pmul(f, Dx), fDy = pmul(f, Dy), fEx = pmul(f, Ex), fEy = pmul(f, Ey);
+        const P fDx = bare ? Dx : pmul(f, Dx), fDy = bare ? Dy : pmul(f, Dy);
+        const P fEx = bare ? Ex : pmul(f, Ex), fEy = bare ? Ey : pmul(f, Ey);
+        P &la = bare ? sum.la[dir % LINKS] : ka, &lb = bare ? sum.lb[dir % LINKS] : kb;
+        P &lc = bare ? sum.lc[dir % LINKS] : kc, &ld = bare ? sum.ld[dir % LINKS] : kd;
         if (dir == 0) {
             w0 = pmul(W, W0);
             w1 = pmul(W, W1);
@@ -568,14 +593,14 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
             w1 = pfma(W, W1, w1);
             w2 = pfma(W, W2, w2);
         }
-        ka = pfma(fDx, P0, ka);
-        kb = pfma(fEx, P0, pfma(fDx, P1, kb));
-        kc = pfma(fEx, P1, pfma(fDx, P2, kc));
-        kd = pfma(fEx, P2, kd);
-        ka = pfma(fDy, Q0, ka);
-        kb = pfma(fEy, Q0, pfma(fDy, Q1, kb));
-        kc = pfma(fEy, Q1, pfma(fDy, Q2, kc));
-        kd = pfma(fEy, Q2, kd);
+        la = pfma(fDx, P0, la);
+        lb = pfma(fEx, P0, pfma(fDx, P1, lb));
+        lc = pfma(fEx, P1, pfma(fDx, P2, lc));
+        ld = pfma(fEx, P2, ld);
+        la = pfma(fDy, Q0, la);
+        lb = pfma(fEy, Q0, pfma(fDy, Q1, lb));
+        lc = pfma(fEy, Q1, pfma(fDy, Q2, lc));
+        ld = pfma(fEy, Q2, ld);
         if (compat) {
             if (dir == 0) {
                 // t1 carries charge -1 instead of q in its field term: t1 += e, e_k = (q + 1) dx a psi;
@@ -595,7 +620,7 @@ __device__ __forceinline__ void site_poly(const PackView<S, NC> &v, const PackVi
                 kd = pnfma(f, pfma(cj, pmul(qj, rhj), pmul(ci, pmul(qi, rh))), kd);
             } else {
                 kd_y = pfma(n2, pmul(W, W1), pmul(n1, pmul(W, W2)));
-                kd_y = pfma(fEx, P2, pfma(fEy, Q2, kd_y));
+                if (!bare) kd_y = pfma(fEx, P2, pfma(fEy, Q2, kd_y));
             }
         }
     }

@@ -630,6 +630,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     constexpr bool WIDE = !std::is_same<T, float>::value;
     PolySum<T, NC> sum;
     sum.zero();
+    bool links = false;   // some row was one of interior sites
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
@@ -684,12 +685,17 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
         }
         bool inner = false;
         if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
+        links |= inner && !S.per_site;
         if (L.cok) {
             if (S.per_site) pp.load_site(S, L.gi, j, s);
             if constexpr (!WIDE) sum.zero();
             if (inner) {
-                if constexpr (std::is_same<T, double>::value)
-                    site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, Ones(), S.per_site, f.poly_compat, S.thin_film, sum);
+                if constexpr (std::is_same<T, double>::value) {
+                    if (S.per_site)
+                        site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, OnesPerSite(), 1, f.poly_compat, S.thin_film, sum);
+                    else
+                        site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, Ones(), 0, f.poly_compat, S.thin_film, sum);
+                }
             } else {
                 Wts<T> w;
                 w.load(R0.m);
@@ -697,7 +703,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
             }
             if constexpr (!WIDE) {
                 T o[5];
-                sum.total(pp, o);
+                sum.total(pp, false, f.poly_compat, o);
 #pragma unroll
                 for (int k = 0; k < 5; ++k) v[k] += o[k];
             }
@@ -709,7 +715,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     // the halo copy of the row below the tile may still be in flight: complete it before the
     // ring can be reused (the fused kernel runs more tiles in the same block)
     cp_async_wait_groups<0>();
-    if constexpr (WIDE) sum.total(pp, v);
+    if constexpr (WIDE) sum.total(pp, links, f.poly_compat, v);
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[5];
     const bool fin = finish_image_warp<5>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
