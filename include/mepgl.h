@@ -77,8 +77,8 @@ enum { MEPGL_DISC_REFERENCE = 0, MEPGL_DISC_LINK = 1 };
 enum { MEPGL_FP64_NATIVE = 0, MEPGL_FP64_PAIRED = 1 };
 /* How the FP32 NLCG steps of a mepgl_nlcg_steps call are launched: two pass
  * kernels per step, or every step of the call in one persistent launch whose
- * tiles wait on per-image stage counters instead of kernel boundaries.  AUTO
- * fuses the batches of at most a few waves of tiles, where the boundaries
+ * strips wait on per-image stage counters instead of kernel boundaries.  AUTO
+ * fuses the batches of at most a few waves of strips, where the boundaries
  * idle much of the GPU.  Both give the same results bit for bit.  No
  * reference counterpart. */
 enum { MEPGL_FP32_STEPS_AUTO = 0, MEPGL_FP32_STEPS_PASSES = 1, MEPGL_FP32_STEPS_FUSED = 2 };
@@ -111,7 +111,7 @@ typedef struct mepgl_options {
     int32_t spline;            /* MEPGL_SPLINE_*                                */
     int32_t metric;            /* MEPGL_METRIC_*                                */
     int32_t use_graphs;        /* capture NLCG steps as CUDA graphs (default 1) */
-    int32_t tile_rows;         /* rows per stencil tile: 0 = auto, 4, 8 or 16   */
+    int32_t tile_rows;         /* not used: rows per strip follow the launch    */
     int32_t discretization;    /* MEPGL_DISC_*                                  */
     int32_t fp64_arith;        /* MEPGL_FP64_*                                  */
     int32_t fp32_steps;        /* MEPGL_FP32_STEPS_*                            */
@@ -318,8 +318,7 @@ mepgl_status mepgl_info(const mepgl_ctx *ctx, int *n_images, int *precision, int
 mepgl_status mepgl_profile_passes(mepgl_ctx *ctx, int steps, int use_cg, double *ms_grad, double *ms_dir_poly);
 
 /* Names of the kernels that run the two NLCG passes of this context in its
- * current precision and FP64 arithmetic (FP32 passes are warp-strip or
- * shared-memory-tile kernels, chosen when the library is built), and of the
+ * current precision and FP64 arithmetic, and of the
  * kernel that runs whole mepgl_nlcg_steps calls as one persistent launch
  * ("" when the passes are launched separately; mepgl_profile_passes always
  * times the separate pass kernels).  The strings are static.  No reference

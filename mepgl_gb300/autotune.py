@@ -1,11 +1,9 @@
-"""Autotuner for the tile shape and residency of the two NLCG passes.
+"""Autotuner for the strips of the two FP32 NLCG passes.
 
-The stencil tile is 32 sites wide with a one-site halo; its height (rows per
-tile, hence the halo-to-interior ratio) and the minimum resident blocks per
-SM requested from ptxas (hence the register budget) are compile-time
-template parameters, and the FP32 passes exist in two designs: warp strips
-(one warp per tile walking down its rows, neighbours by shuffles) and
-shared-memory tiles (eight warps per tile, with variants of the halo copy).  The tuner builds one library
+A strip is 32 sites wide and belongs to one warp; its most rows (hence the
+halo-to-interior ratio; small launches take fewer), the single-warp blocks per
+SM requested from ptxas (hence the register budget) and how many waves of
+strips still run fused are compile-time constants.  The tuner builds one library
 per candidate (in parallel, into a scratch directory), times the FP32 NLCG
 step of a workload with each (CUDA events on the context's stream, after
 warm-up), and writes the fastest candidate's definitions to
