@@ -95,11 +95,6 @@ __device__ __forceinline__ ff operator*(ff a, int i) { return a * ff(i); }
 // warp shuffle of any lattice number type (float, double, float-float)
 __device__ __forceinline__ float shfl_down(float v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ double shfl_down(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
-__device__ __forceinline__ ff shfl_down(ff v, int o)
-{
-    return ff(__shfl_down_sync(0xffffffffu, v.hi, o), __shfl_down_sync(0xffffffffu, v.lo, o));
-}
-
 __device__ __forceinline__ float shfl_xor(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ double shfl_xor(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ ff shfl_xor(ff v, int o)
