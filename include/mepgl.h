@@ -273,7 +273,8 @@ mepgl_status mepgl_arc_length(mepgl_ctx *ctx, int metric, double *s);
  * (cubic), else MEPGL_ERR_INVALID_ARG.  Two equal adjacent images (a
  * segment of zero length, 0/0 in the reference) resample to their state;
  * a string of zero arc length returns MEPGL_ERR_NAN, and a singular cubic
- * spline matrix too. */
+ * spline matrix (the first two images equal) too.  With F_new != F the string
+ * is then left as it was. */
 mepgl_status mepgl_redistribute(mepgl_ctx *ctx, int kind, int F_new);
 
 /* Batched strings.  No counterpart in the reference, which runs parameter

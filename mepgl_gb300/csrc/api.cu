@@ -510,16 +510,17 @@ mepgl_status nlcg_steps_body(mepgl_ctx *c, int iters, int use_cg, int maxwell)
 // Device-side error flags (STATUS_* in kernels.cuh): a stage wait of the
 // fused NLCG launch that ran out (the launch then stopped early), non-finite
 // per-image scalars after NLCG steps, a string of zero or non-finite arc
-// length.  Read on the stream after the work before it, then cleared; the
+// length, and (cubic: after a cubic reparametrization) a singular spline
+// matrix.  Read on the stream after the work before it, then cleared; the
 // first raised flag is reported.
-mepgl_status report_device_status(mepgl_ctx *c, const int *st);
+mepgl_status report_device_status(mepgl_ctx *c, const int *st, bool cubic);
 
-mepgl_status check_device_status(mepgl_ctx *c)
+mepgl_status check_device_status(mepgl_ctx *c, bool cubic = false)
 {
-    int st[4];
+    int st[STATUS_COUNT];
     CK(c, cudaMemcpyAsync(st, c->sc.status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    return report_device_status(c, st);
+    return report_device_status(c, st, cubic);
 }
 
 // Device doubles to the caller's arrays (NULL: skipped) and, with check, the
@@ -537,7 +538,7 @@ struct Fetch {
 mepgl_status fetch(mepgl_ctx *c, std::initializer_list<Fetch> items, bool check)
 {
     const double *status = reinterpret_cast<const double *>(c->sc.status), *lo = check ? status : nullptr,
-                 *hi = check ? status + 2 : nullptr;
+                 *hi = check ? status + (STATUS_COUNT + 1) / 2 : nullptr;
     for (const Fetch &f : items) {
         if (!f.dst) continue;
         if (!lo || f.src < lo) lo = f.src;
@@ -550,16 +551,17 @@ mepgl_status fetch(mepgl_ctx *c, std::initializer_list<Fetch> items, bool check)
     for (const Fetch &f : items)
         if (f.dst) memcpy(f.dst, mail + (f.src - lo), f.n * sizeof(double));
     if (!check) return MEPGL_OK;
-    int st[4];
+    int st[STATUS_COUNT];
     memcpy(st, mail + (status - lo), sizeof(st));
-    return report_device_status(c, st);
+    return report_device_status(c, st, false);
 }
 
 // The flags that a copy brought; raised ones are cleared on the device.
-mepgl_status report_device_status(mepgl_ctx *c, const int *st)
+mepgl_status report_device_status(mepgl_ctx *c, const int *st, bool cubic)
 {
-    if (!(st[STATUS_WAIT] | st[STATUS_NONFINITE] | st[STATUS_ARC])) return MEPGL_OK;
-    CK(c, cudaMemsetAsync(c->sc.status, 0, 4 * sizeof(int), c->stream));
+    const bool spline = cubic && st[STATUS_SPLINE];
+    if (!(st[STATUS_WAIT] | st[STATUS_NONFINITE] | st[STATUS_ARC]) && !spline) return MEPGL_OK;
+    CK(c, cudaMemsetAsync(c->sc.status, 0, STATUS_COUNT * sizeof(int), c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     if (st[STATUS_WAIT])
         return fail(c, MEPGL_ERR_CUDA, "fused NLCG launch: a per-image stage wait ran out; the steps are incomplete");
@@ -571,9 +573,11 @@ mepgl_status report_device_status(mepgl_ctx *c, const int *st)
                         " image(s), first: string " + std::to_string(si) + " image " +
                         std::to_string(g - c->hdesc[si].img_base));
     }
-    return fail(c, MEPGL_ERR_NAN,
-                "arc length of the string is zero or not finite (all images equal, or non-finite fields); "
-                "it was taken as uniform, so a linear resample kept the images");
+    if (st[STATUS_ARC])
+        return fail(c, MEPGL_ERR_NAN,
+                    "arc length of the string is zero or not finite (all images equal, or non-finite fields); "
+                    "it was taken as uniform, so a linear resample kept the images");
+    return fail(c, MEPGL_ERR_NAN, "spline matrix is singular (coincident images)");
 }
 
 // wait: until the copies are done
@@ -684,7 +688,7 @@ mepgl_status redistribute(mepgl_ctx *c, int kind, int F_new)
     }
     // resize: new buffers for F_new images, state moved in, history reset
     CK(c, cudaStreamSynchronize(c->stream));
-    st = check_device_status(c);    // before build_layout renews the flags
+    st = check_device_status(c, cubic);    // before build_layout renews the flags
     if (st != MEPGL_OK) {
         for (int f = 0; f < 1 + c->ncomp; ++f) cudaFree(target[f]);
         return st;
@@ -1265,16 +1269,7 @@ mepgl_status mepgl_redistribute(mepgl_ctx *c, int kind, int F_new)
         return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_redistribute: unknown kind");
     mepgl_status st = redistribute(c, kind, F_new);
     if (st != MEPGL_OK) return st;
-    int flags[5];
-    CK(c, cudaMemcpyAsync(flags, c->sc.status, sizeof(flags), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    st = report_device_status(c, flags);
-    if (st != MEPGL_OK) return st;
-    if (kind == MEPGL_REDIST_CUBIC && flags[STATUS_SPLINE]) {
-        CK(c, cudaMemset(c->sc.status + STATUS_SPLINE, 0, sizeof(int)));
-        return fail(c, MEPGL_ERR_NAN, "spline matrix is singular (coincident images)");
-    }
-    return MEPGL_OK;
+    return check_device_status(c, kind == MEPGL_REDIST_CUBIC);
 }
 
 mepgl_status mepgl_iteration(mepgl_ctx *c, char mode, int relaxation_steps, int use_cg)

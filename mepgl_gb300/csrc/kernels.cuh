@@ -95,7 +95,8 @@ cudaError_t launch_arc_cumulate(int F, double *s, int *bad, cudaStream_t st);
 // launch ran out; [1] count of non-finite per-image scalars after NLCG steps,
 // [2] the first such image + 1; [3] a string of zero or non-finite arc length;
 // [4] a singular spline matrix.
-constexpr int STATUS_WAIT = 0, STATUS_NONFINITE = 1, STATUS_NONFINITE_IMAGE = 2, STATUS_ARC = 3, STATUS_SPLINE = 4;
+constexpr int STATUS_WAIT = 0, STATUS_NONFINITE = 1, STATUS_NONFINITE_IMAGE = 2, STATUS_ARC = 3, STATUS_SPLINE = 4,
+              STATUS_COUNT = 5;
 // Checks energy and |g|^2 (slot 0 or 1) of n_images images (see STATUS_NONFINITE).
 cudaError_t launch_check_scalars(const Scalars &sc, int n_images, int slot, cudaStream_t st);
 // Initial-guess parameters of launch_generate (see mepgl_guess).
