@@ -85,10 +85,10 @@ struct Uniform {
     T a[2], b[2], hmx[2], hmy[2], aob[2], q[2];
     T eta, gamma, delta, h, idx, dx2, dx;
     // the same with the spacing folded in, as the stencils of site_pack.cuh
-    // use them: q dx, +- half of it, half of its square, (q + 1) dx, q / dx;
-    // -2 hm*, hm* / dx^2, and that times half of (q dx)^2; hm* q / dx; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
+    // use them: q dx, +- half of it, (q + 1) dx, q / dx; -2 hm*, hm* / dx^2, half
+    // of that; hm* q / dx; 2 a dx^2, 2 b dx^2; couplings times dx^2; h dx;
     // 1 / (4 dx), 1 / (8 dx^2)
-    T qd[2], hqd[2], nhqd[2], hqq[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hqmx[2], hqmy[2], jmx[2], jmy[2],
+    T qd[2], hqd[2], nhqd[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hhmx[2], hhmy[2], jmx[2], jmy[2],
         a2[2], b2[2];
     T etad, gammad, deltad, hd, idx4, idx8;
 };
@@ -100,15 +100,14 @@ inline void fold_spacing(Uniform<double> &U)
         U.qd[c] = U.q[c] * U.dx;
         U.hqd[c] = 0.5 * U.qd[c];
         U.nhqd[c] = -U.hqd[c];
-        U.hqq[c] = U.hqd[c] * U.qd[c];
         U.kq[c] = (U.q[c] + 1.0) * U.dx;
         U.qi[c] = U.q[c] * U.idx;
         U.n2hmx[c] = -2.0 * U.hmx[c];
         U.n2hmy[c] = -2.0 * U.hmy[c];
         U.hmxi[c] = U.hmx[c] * U.idx * U.idx;
         U.hmyi[c] = U.hmy[c] * U.idx * U.idx;
-        U.hqmx[c] = U.hqq[c] * U.hmxi[c];
-        U.hqmy[c] = U.hqq[c] * U.hmyi[c];
+        U.hhmx[c] = 0.5 * U.hmxi[c];
+        U.hhmy[c] = 0.5 * U.hmyi[c];
         U.jmx[c] = U.hmx[c] * U.qi[c];
         U.jmy[c] = U.hmy[c] * U.qi[c];
         U.a2[c] = 2.0 * U.a[c] * U.dx2;
@@ -136,15 +135,14 @@ inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
         r.qd[c] = T(U.qd[c]);
         r.hqd[c] = T(U.hqd[c]);
         r.nhqd[c] = T(U.nhqd[c]);
-        r.hqq[c] = T(U.hqq[c]);
         r.kq[c] = T(U.kq[c]);
         r.qi[c] = T(U.qi[c]);
         r.n2hmx[c] = T(U.n2hmx[c]);
         r.n2hmy[c] = T(U.n2hmy[c]);
         r.hmxi[c] = T(U.hmxi[c]);
         r.hmyi[c] = T(U.hmyi[c]);
-        r.hqmx[c] = T(U.hqmx[c]);
-        r.hqmy[c] = T(U.hqmy[c]);
+        r.hhmx[c] = T(U.hhmx[c]);
+        r.hhmy[c] = T(U.hhmy[c]);
         r.jmx[c] = T(U.jmx[c]);
         r.jmy[c] = T(U.jmy[c]);
         r.a2[c] = T(U.a2[c]);

@@ -84,7 +84,7 @@ struct EnergyOp {
         __device__ __forceinline__ void site(const EnergyOp &, const PackView<T, NC> &v, const StringDesc &S,
                                              PackParams<T, NC> &pp, const W &w, const WalkPos &q)
         {
-            e.v += site_energy<T, NC>(v, pp, w, S.per_site, S.thin_film);
+            e.v += site_energy<T, NC>(v, pp, w, S.thin_film);
         }
         __device__ __forceinline__ void link(const EnergyOp &, const PackView<T, NC> &v, const StringDesc &S,
                                              PackParams<T, NC> &, const Wts<T> &w, const WalkPos &q)
