@@ -31,7 +31,7 @@ namespace mepgl {
 template <class T>
 struct MaskTable {
     T sc[256][12];    // area, wfx, wbx, wfy, wby, lfx, lbx, lfy, lby, wfx + wbx, wfy + wby, 0
-    T cc[256][5];     // vUR, vUL, vLL, vLR, 1 / their sum
+    T cc[256][8];     // vUR, vUL, vLL, vLR, 1 / their sum, lower minus upper ones, right minus left ones, 0
 };
 // Defined here: kernels.cu is the only translation unit that includes this file.
 __constant__ MaskTable<float> c_mask_f;
@@ -48,7 +48,7 @@ template <class T>
 struct Wts {
     static constexpr bool interior = false, masses = true;
     T area, wfx, wbx, wfy, wby, lfx, lbx, lfy, lby, wsx, wsy;
-    T vUR, vUL, vLL, vLR, ivs;
+    T vUR, vUL, vLL, vLR, ivs, vdx, vdy;
     __device__ __forceinline__ void load(unsigned mk)
     {
         const auto &M = mask_table<typename MaskOf<T>::type>();
@@ -57,6 +57,7 @@ struct Wts {
         lfx = M.sc[s][5]; lbx = M.sc[s][6]; lfy = M.sc[s][7]; lby = M.sc[s][8];
         wsx = M.sc[s][9]; wsy = M.sc[s][10];
         vUR = M.cc[c][0]; vUL = M.cc[c][1]; vLL = M.cc[c][2]; vLR = M.cc[c][3]; ivs = M.cc[c][4];
+        vdx = M.cc[c][5]; vdy = M.cc[c][6];
     }
 };
 
@@ -85,6 +86,9 @@ inline void build_mask_table(MaskTable<T> &M)
         M.cc[k][3] = (T)(b(6) & b(7) & b(0));
         const T v = M.cc[k][0] + M.cc[k][1] + M.cc[k][2] + M.cc[k][3];
         M.cc[k][4] = v > (T)0 ? (T)1 / v : (T)0;
+        M.cc[k][5] = (M.cc[k][2] + M.cc[k][3]) - (M.cc[k][0] + M.cc[k][1]);
+        M.cc[k][6] = (M.cc[k][0] + M.cc[k][3]) - (M.cc[k][1] + M.cc[k][2]);
+        M.cc[k][7] = (T)0;
     }
 }
 

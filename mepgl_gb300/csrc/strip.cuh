@@ -363,11 +363,11 @@ __device__ __forceinline__ GradView<T, NC> grad_view(const GradRow<T, NC> &R)
 // The carry into row c from the row d below it.
 template <class T, int NC>
 __device__ __forceinline__ GradCarry<T, NC> grad_below(const GradRow<T, NC> &d, const GradRow<T, NC> &c,
-                                                       const PackParams<T, NC> &pp, const Wts<T> &w, T hd)
+                                                       const PackParams<T, NC> &pp, const Wts<T> &w)
 {
     GradCarry<T, NC> k;
     const GradView<T, NC> vd = grad_view(d);
-    grad_up<T, NC>(vd, grad_view(c), pp, w.wby, hd, vd.ar.y - vd.a.y, vd.a.y - vd.al.y, k);
+    grad_up<T, NC>(vd, grad_view(c), pp, w.wby, vd.ar.y - vd.a.y, vd.a.y - vd.al.y, k);
     return k;
 }
 
@@ -459,16 +459,10 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         take(Rm, j0 - 1, hp0, ra, ma);
         take(R0, j0, hp0, rb, mb);
         if constexpr (CARRY) {
-            // the link from row j0 - 1 with the weight and field sum that row j0 knows it by
+            // the link from row j0 - 1 with the weight that row j0 knows it by
             Wts<T> w;
             w.load(R0.m);
-            T hd = pp.hd + pp.hd;
-            if (S.per_site && L.cok) {
-                PackParams<T, NC> q = pp;
-                q.load_site(S, L.gi, j0, L.gi + S.nx * j0);
-                hd = field_sums(S, q, L.gi, j0, L.gi + S.nx * j0).d;
-            }
-            up = grad_below(Rm, R0, pp, w, hd);
+            up = grad_below(Rm, R0, pp, w);
         }
     }
     const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
@@ -503,13 +497,13 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
             if (inner) {
                 if constexpr (std::is_same<T, double>::value)
                     site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr),
-                                         pp, Ones(), h, f.maxwell, S.thin_film, up, g);
+                                         pp, Ones(), h, S.per_site, f.maxwell, S.thin_film, up, g);
             } else {
                 Wts<T> w;
                 w.load(R0.m);
-                if constexpr (!CARRY) up = grad_below(Rm, R0, pp, w, h.d);
+                if constexpr (!CARRY) up = grad_below(Rm, R0, pp, w);
                 site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr), pp,
-                                     w, h, f.maxwell, S.thin_film, up, g);
+                                     w, h, S.per_site, f.maxwell, S.thin_film, up, g);
             }
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) {

@@ -205,10 +205,10 @@ struct GradientOp {
             const GradView<T, NC> u{v.a[2][1], v.a[2][0], v.a[2][2], v.px[2][1], v.py[2][1]};
             if (q.r == 0) {
                 const GradView<T, NC> d{v.a[0][1], v.a[0][0], v.a[0][2], v.px[0][1], v.py[0][1]};
-                grad_up<T, NC>(d, c, pp, T(w.wby), h.d, d.ar.y - d.a.y, d.a.y - d.al.y, up);
+                grad_up<T, NC>(d, c, pp, T(w.wby), d.ar.y - d.a.y, d.a.y - d.al.y, up);
             }
             T g[2 + 2 * NC];
-            site_gradient<T, NC>(c, u, v.px[1][0], v.py[1][0], v.px[1][2], v.py[1][2], pp, w, h, op.maxwell, S.thin_film,
+            site_gradient<T, NC>(c, u, v.px[1][0], v.py[1][0], v.px[1][2], v.py[1][2], pp, w, h, S.per_site, op.maxwell, S.thin_film,
                                  up, g);
             store(op, S, g, q);
             if constexpr (ADJ) a.site(v, S, pp, w);

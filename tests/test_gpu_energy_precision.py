@@ -89,3 +89,33 @@ def test_energy_of_vortex_lattices(arith, comps, vortices, n, dx, h):
     for got, tol in ((e, u["fp32" if arith == "fp32" else "fp64"]), (q, u[arith])):
         err = max(float(abs((LD(v) - w) / s)) for v, (w, s) in zip(got, want))
         assert err <= tol, (err, tol)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("nx,ny", [(97, 40), (33, 18)])
+def test_a_uniform_field_leaves_no_rounding_in_the_gradient(precision, nx, ny):
+    """dF/dA of a string without psi and with A of 1e-3 in a field of 0.9: at sites
+    with all their views the field cancels exactly, and what is left is sums of
+    about ten differences of A, each a rounding of its own size."""
+    from mepgl_gb300 import native
+    dtype = np.float32 if precision == "fp32" else np.float64
+    prob = Problem.uniform(nx, ny, 0.4, h=0.9)
+    a = (1e-3 * np.random.default_rng(5).standard_normal((2, ny, nx, 2))).astype(dtype)
+    c = native.StringContext(prob, 2, precision)
+    c.set_state(StringState(a=a, psi_1=np.zeros_like(a), psi_2=None))
+    got = c.energy_grad()[1][0].astype(LD)[:, 2:-2, 2:-2]
+    c.close()
+    x = a.astype(LD)
+    ex, ey = x[:, :, 1:, 1] - x[:, :, :-1, 1], x[:, 1:, :, 0] - x[:, :-1, :, 0]
+    # the sum over the four collocated views of a plaquette of (mean) curl
+    want = np.zeros_like(x)
+    for b in (slice(0, -1), slice(1, None)):
+        for l in (slice(0, -1), slice(1, None)):
+            w = (ex[:, b] - ey[:, :, l]) / 4       # weight of each view; dF = w (d ex - d ey)
+            want[:, b, 1:, 1] += w
+            want[:, b, :-1, 1] -= w
+            want[:, 1:, l, 0] -= w
+            want[:, :-1, l, 0] += w
+    want = want[:, 2:-2, 2:-2]
+    u = 2.0 ** -24 if precision == "fp32" else 2.0 ** -53
+    assert float(np.max(np.abs(got - want))) <= 10 * u * float(np.max(np.abs(ex)) + np.max(np.abs(ey)))
