@@ -200,7 +200,7 @@ void drop_graphs(mepgl_ctx *c)
 int layout_strips(mepgl_ctx *c)
 {
     const int paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED;
-    const int slots = strip_pass_slots(c->precision, paired, c->ncomp), cap = strip_rows_cap(c->precision, paired);
+    const int slots = strip_pass_slots(c->precision, c->ncomp, c->sm_count), cap = strip_rows_cap(c->precision, paired);
     int base = 0;
     c->batch_stile0.clear();
     c->batch_nstiles.clear();
@@ -424,8 +424,7 @@ bool use_fused(const mepgl_ctx *c)
 {
     if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_PASSES) return false;
     if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED) return true;
-    const int paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED;
-    const long long cap = (long long)fuse_waves(c->precision) * strip_pass_slots(c->precision, paired, c->ncomp);
+    const long long cap = (long long)fuse_waves(c->precision) * strip_pass_slots(c->precision, c->ncomp, c->sm_count);
     for (int n : c->batch_nstiles)
         if (n > cap) return false;
     return true;

@@ -91,6 +91,7 @@ struct Uniform {
     T qd[2], hqd[2], nhqd[2], kq[2], qi[2], n2hmx[2], n2hmy[2], hmxi[2], hmyi[2], hhmx[2], hhmy[2], jmx[2], jmy[2],
         a2[2], b2[2];
     T etad, gammad, deltad, hd, idx4, idx8;
+    T hl;   // what rounding h to float left out, times dx (float only)
 };
 
 // The folded parameters from the plain ones (host, in double).
@@ -119,6 +120,7 @@ inline void fold_spacing(Uniform<double> &U)
     U.gammad = U.gamma * U.dx2;
     U.deltad = U.delta * U.dx2;
     U.hd = U.h * U.dx;
+    U.hl = 0.0;
 }
 
 // Rounded once from double: to float, or split into a float pair.
@@ -159,6 +161,7 @@ inline void round_uniform(Uniform<T> &r, const Uniform<double> &U)
     r.gammad = T(U.gammad);
     r.deltad = T(U.deltad);
     r.hd = T(U.hd);
+    r.hl = T(std::is_same<T, float>::value ? (U.h - (double)(float)U.h) * U.dx : 0.0);
     r.idx4 = T(U.idx4);
     r.idx8 = T(U.idx8);
 }

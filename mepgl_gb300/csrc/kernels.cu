@@ -30,12 +30,17 @@ namespace mepgl {
 // (registers per thread: 65536 / (32 x blocks)).  FP64 and float-float strips
 // hold twice the registers of FP32 ones; at 12 blocks they spill: a
 // float-float step of the 256 x 256 string took 2.1 ms instead of 1.5, FP64
-// gained nothing.
+// gained nothing.  The direction pass of several one-component FP32 strings
+// takes 119 registers if it may (16 blocks): ten steps of the 16 strings then take
+// 16.5 ms, with 18, 20, 22, 24, 28 blocks 16.2, 16.6, 16.3, 15.9, 16.8.
 #ifndef MEPGL_MINB_STRIP_GRAD
 #define MEPGL_MINB_STRIP_GRAD 16
 #endif
 #ifndef MEPGL_MINB_STRIP_DIR
 #define MEPGL_MINB_STRIP_DIR 16
+#endif
+#ifndef MEPGL_MINB_STRIP_DIR_SWEEP
+#define MEPGL_MINB_STRIP_DIR_SWEEP 24
 #endif
 #ifndef MEPGL_MINB_STRIP_FUSED
 #define MEPGL_MINB_STRIP_FUSED 12
@@ -43,11 +48,12 @@ namespace mepgl {
 #ifndef MEPGL_MINB_STRIP_F64
 #define MEPGL_MINB_STRIP_F64 8
 #endif
-template <class T> struct StripBlocks {
+template <class T, int NC, bool ONE> struct StripBlocks {
     static constexpr int grad = MEPGL_MINB_STRIP_F64, dir = MEPGL_MINB_STRIP_F64, fused = MEPGL_MINB_STRIP_F64;
 };
-template <> struct StripBlocks<float> {
-    static constexpr int grad = MEPGL_MINB_STRIP_GRAD, dir = MEPGL_MINB_STRIP_DIR, fused = MEPGL_MINB_STRIP_FUSED;
+template <int NC, bool ONE> struct StripBlocks<float, NC, ONE> {
+    static constexpr int grad = MEPGL_MINB_STRIP_GRAD, fused = MEPGL_MINB_STRIP_FUSED,
+                         dir = NC == 1 && !ONE ? MEPGL_MINB_STRIP_DIR_SWEEP : MEPGL_MINB_STRIP_DIR;
 };
 // Fused steps only for batches of at most this many waves of the pass kernels
 // (beyond that the boundaries cost little; FP32 pass kernels hold more warps)
@@ -1212,19 +1218,9 @@ static int resident(K kernel)
     return nb * sms;
 }
 
-template <class T>
-static int pass_slots(int ncomp)
-{
-    static int slots[2] = {0, 0};
-    int &n = slots[ncomp == 2];
-    if (n == 0) n = ncomp == 2 ? resident(k_dir_poly_s<T, 2, false>) : resident(k_dir_poly_s<T, 1, false>);
-    return n;
-}
-
-int strip_pass_slots(int precision, int paired, int ncomp)
-{
-    return precision == 0 ? pass_slots<float>(ncomp) : paired ? pass_slots<ff>(ncomp) : pass_slots<double>(ncomp);
-}
+// Constants and not what the compiler's register counts happen to give: the
+// rows of a strip, and with them the order of an image's sums, follow from it.
+int strip_pass_slots(int precision, int ncomp, int sms) { return sms * (precision == 1 ? 8 : ncomp == 2 ? 16 : 21); }
 
 template <class T>
 static cudaError_t nlcg_fused_launch(const Launch &L, const Scalars &sc, const StepPlan &plan, int steps,

@@ -36,9 +36,10 @@ int strip_rows(int precision, int paired, int ny, long tiles, int slots);
 // The same for the walks over one string, of `columns` image columns of strips.
 int walk_rows(int precision, int ny, long columns, int sms);
 // Steps are fused for batches of at most fuse_waves() x strip_pass_slots()
-// strips; strip_pass_slots(): resident warps of the pass kernels on the GPU.
+// strips; strip_pass_slots(): warps of the pass kernels that `sms` multiprocessors
+// hold, by type and components.
 int fuse_waves(int precision);
-int strip_pass_slots(int precision, int paired, int ncomp);
+int strip_pass_slots(int precision, int ncomp, int sms);
 // `steps` NLCG steps (iterations it0, it0 + 1, ...; step 0 with the buffers
 // of f0) of the launch's tiles in one persistent launch; queue (one counter)
 // and stage (one per global image, n_stage, STAGE_STRIDE words apart: a line

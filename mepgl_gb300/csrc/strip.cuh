@@ -538,7 +538,7 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::grad) k_grad_s(const __grid_constant__ batch_t<ONE> bt,
+__global__ void __launch_bounds__(NTS, (StripBlocks<T, NC, ONE>::grad)) k_grad_s(const __grid_constant__ batch_t<ONE> bt,
                                                                   int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) GradRing<T, NC> ring;
@@ -733,7 +733,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::dir) k_dir_poly_s(const __grid_constant__ batch_t<ONE> bt,
+__global__ void __launch_bounds__(NTS, (StripBlocks<T, NC, ONE>::dir)) k_dir_poly_s(const __grid_constant__ batch_t<ONE> bt,
                                                                       int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) DirRing<T, NC> ring;
@@ -814,7 +814,7 @@ __device__ __forceinline__ void publish_stage(unsigned *stage, unsigned value)
 }
 
 template <class T, int NC, bool ONE>
-__global__ void __launch_bounds__(NTS, StripBlocks<T>::fused) k_nlcg_s(const __grid_constant__ batch_t<ONE> bt, int tile0, int n_tiles, int steps,
+__global__ void __launch_bounds__(NTS, (StripBlocks<T, NC, ONE>::fused)) k_nlcg_s(const __grid_constant__ batch_t<ONE> bt, int tile0, int n_tiles, int steps,
                                             StepPlan plan, Scalars sc, unsigned long long *queue, unsigned *stage,
                                             unsigned max_polls)
 {

@@ -119,3 +119,24 @@ def test_a_uniform_field_leaves_no_rounding_in_the_gradient(precision, nx, ny):
     want = want[:, 2:-2, 2:-2]
     u = 2.0 ** -24 if precision == "fp32" else 2.0 ** -53
     assert float(np.max(np.abs(got - want))) <= 10 * u * float(np.max(np.abs(ex)) + np.max(np.abs(ey)))
+
+
+def test_fp32_energy_of_a_field_that_float_rounds():
+    """h = 0.9 loses 2.6e-8 of itself in float, and with it 5.3e-8 of its energy, which the couplings'
+    gain nearly cancels here (energy about a thirtieth of either).  A of 1e-3 decides how every site
+    rounds, so the sum keeps two units of roundoff of its parts' sum divided by the root of the sites."""
+    from mepgl_gb300 import native
+    n, p = 128, dict(PARS[2], a=(-1.0, -1.0), m_yy=(1.0, 1.0), eta=-0.375, gamma=0.0, delta=0.0)
+    prob = Problem.uniform(n, n, 0.5, multicomponent=True, h=0.9, q=(1.0, 1.0), **p)
+    rng = np.random.default_rng(3)
+    f = [(s + 1e-3 * rng.standard_normal((2, n, n, 2))).astype(np.float32) for s in (0.0, [1.0, 0.0], [1.0, 0.0])]
+    c = native.StringContext(prob, 2, "fp32", line_search=1, line_polynomial=1)
+    c.set_state(StringState(a=f[0], psi_1=f[1], psi_2=f[2]))
+    e = c.compute_free_energy()
+    c.nlcg_steps(1)
+    q = c.image_scalars()["fenergy"]
+    c.close()
+    for k in range(2):
+        want, parts = energy(f[0][k], [f[1][k], f[2][k]], 0.5, 0.9, p)
+        tol = 2 * 2.0 ** -24 * float(parts) / n * 8      # eight roundings of a site's sum
+        assert abs(float(LD(e[k]) - want)) <= tol and abs(float(LD(q[k]) - want)) <= tol
