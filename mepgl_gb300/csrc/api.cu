@@ -196,32 +196,48 @@ void drop_graphs(mepgl_ctx *c)
     c->graphs.clear();
 }
 
-// Strips of the NLCG passes: rows per strip by launch batch, global strip order.
+// Strips of the NLCG passes: rows per group of sums, strips, global orders.  The
+// groups come from the string and the GPU alone, so that its sums are added up
+// alike in a context of its own and in any batch.  Where a batch's strips are
+// many, a strip is several groups: the sums cost it little, two more halo rows per
+// group would cost a lot (ten FP32 steps of 64 strings of 96 x 100 x 24: 8.7 ms
+// with a strip per group, 6.3 with these).  Float-float strips, bound by issue, gain
+// nothing by more rows (16 strings of 64 x 64 x 16, two components: 5.1 against
+// 7.6 ms).  Returns the groups of all strings.
 int layout_strips(mepgl_ctx *c)
 {
     const int paired = c->opt.fp64_arith == MEPGL_FP64_PAIRED;
     const int slots = strip_pass_slots(c->precision, c->ncomp, c->sm_count), cap = strip_rows_cap(c->precision, paired);
-    int base = 0;
+    auto most = [&](const StringDesc &D) { return (long)D.F * D.tiles_x * ((D.ny + cap - 1) / cap); };   // strips of the most rows
+    int base = 0, part = 0;
     c->batch_stile0.clear();
     c->batch_nstiles.clear();
     size_t si = 0;
     for (Batch &B : c->batches) {
-        long most = 0;   // strips of the most rows
-        for (int k = 0; k < B.n; ++k) most += (long)B.s[k].F * B.s[k].tiles_x * ((B.s[k].ny + cap - 1) / cap);
+        long all = 0;
+        for (int k = 0; k < B.n; ++k) all += most(B.s[k]);
         c->batch_stile0.push_back(base);
         for (int k = 0; k < B.n; ++k, ++si) {
             StringDesc &D = B.s[k];
-            D.rows = strip_rows(c->precision, paired, D.ny, most, slots);
-            D.stiles_y = (D.ny + D.rows - 1) / D.rows;
+            D.grows = strip_rows(c->precision, paired, D.ny, most(D), slots);
+            const int ngroups = (D.ny + D.grows - 1) / D.grows;   // down an image
+            const int per = paired ? 1 : std::max(1, strip_rows(c->precision, paired, D.ny, all, slots) / D.grows);
+            D.stiles_y = (ngroups + per - 1) / per;
+            D.gper = (ngroups + D.stiles_y - 1) / D.stiles_y;
+            D.stiles_y = (ngroups + D.gper - 1) / D.gper;
+            D.rows = D.gper * D.grows;
             D.stile_base = base;
+            D.groups = ngroups * D.tiles_x;
+            D.part_base = part;
             D.wrows = walk_rows(c->precision, D.ny, (long)D.F * D.tiles_x, c->sm_count);
             D.wtiles_y = (D.ny + D.wrows - 1) / D.wrows;
             base += D.F * D.tiles_x * D.stiles_y;
+            part += D.F * D.groups;
             c->hdesc[si] = D;
         }
         c->batch_nstiles.push_back(base - c->batch_stile0.back());
     }
-    return base;
+    return part;
 }
 
 // (Re)build strip layout, descriptors and per-image arrays for the current strings.
@@ -248,13 +264,13 @@ mepgl_status build_layout(mepgl_ctx *c)
         img += D.F;
     }
     c->total_images = img;
-    const int n_stiles = layout_strips(c);
+    const int n_groups = layout_strips(c);
     Scalars &S = c->sc;
     const size_t I = (size_t)img;
     int fmax = 0;
     for (auto &s : c->strings) fmax = fmax > s.F ? fmax : s.F;
     // one allocation: the line-search grids, then what starts at zero, then the partial sums
-    size_t n_part = (size_t)n_stiles * 8;
+    size_t n_part = (size_t)n_groups * 8;
     for (size_t k = 0; k < c->strings.size(); ++k) {   // also of the walks, and of the arc lengths per image and site block
         const StringDesc &D = c->hdesc[k];
         const size_t w = (size_t)D.F * D.tiles_x * D.wtiles_y * 8, arc = 2 * (size_t)D.F * arc_blocks(D);

@@ -175,6 +175,8 @@ struct StringDesc {
     int tiles_x;              // strips across an image
     int img_base;             // first global image index of this string
     int rows;                 // rows per warp strip of the NLCG passes
+    int grows, gper;          // rows per group of their sums, groups per strip
+    int groups, part_base;    // groups of an image (all columns); first global group index
     int stiles_y, stile_base; // strips down an image; first global strip index
     int wrows, wtiles_y;      // the same of the walks over one string (walk.cuh)
     int thin_film;
@@ -221,7 +223,7 @@ struct Scalars {
     double *alpha_pend;   // step not yet applied to x (0 = nothing pending)
     double *fenergy;      // energy (polynomial constant term)
     double *poly;         // [img][4] = B, C, D, E
-    double *part;         // partial sums, [strip][8]
+    double *part;         // partial sums, [group of rows of a strip][8]
     unsigned *ticket;     // per-image arrival counters
     double *xtab_f, *xtab_d;   // line-search grid x_p, p = 0..2000, rounded to float / double
     int *status;          // device-side error flags

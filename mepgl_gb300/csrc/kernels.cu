@@ -30,9 +30,9 @@ namespace mepgl {
 // (registers per thread: 65536 / (32 x blocks)).  FP64 and float-float strips
 // hold twice the registers of FP32 ones; at 12 blocks they spill: a
 // float-float step of the 256 x 256 string took 2.1 ms instead of 1.5, FP64
-// gained nothing.  The direction pass of several one-component FP32 strings
-// takes 119 registers if it may (16 blocks): ten steps of the 16 strings then take
-// 16.5 ms, with 18, 20, 22, 24, 28 blocks 16.2, 16.6, 16.3, 15.9, 16.8.
+// gained nothing.  The passes of several one-component FP32 strings take 122
+// registers if they may (16 blocks): ten steps of the 16 strings then take 17.9 ms,
+// with 20, 22, 24 blocks 17.7, 16.8, 16.0.
 #ifndef MEPGL_MINB_STRIP_GRAD
 #define MEPGL_MINB_STRIP_GRAD 16
 #endif
@@ -41,6 +41,9 @@ namespace mepgl {
 #endif
 #ifndef MEPGL_MINB_STRIP_DIR_SWEEP
 #define MEPGL_MINB_STRIP_DIR_SWEEP 24
+#endif
+#ifndef MEPGL_MINB_STRIP_GRAD_SWEEP
+#define MEPGL_MINB_STRIP_GRAD_SWEEP 24
 #endif
 #ifndef MEPGL_MINB_STRIP_FUSED
 #define MEPGL_MINB_STRIP_FUSED 12
@@ -52,7 +55,8 @@ template <class T, int NC, bool ONE> struct StripBlocks {
     static constexpr int grad = MEPGL_MINB_STRIP_F64, dir = MEPGL_MINB_STRIP_F64, fused = MEPGL_MINB_STRIP_F64;
 };
 template <int NC, bool ONE> struct StripBlocks<float, NC, ONE> {
-    static constexpr int grad = MEPGL_MINB_STRIP_GRAD, fused = MEPGL_MINB_STRIP_FUSED,
+    static constexpr int grad = NC == 1 && !ONE ? MEPGL_MINB_STRIP_GRAD_SWEEP : MEPGL_MINB_STRIP_GRAD,
+                         fused = MEPGL_MINB_STRIP_FUSED,
                          dir = NC == 1 && !ONE ? MEPGL_MINB_STRIP_DIR_SWEEP : MEPGL_MINB_STRIP_DIR;
 };
 // Fused steps only for batches of at most this many waves of the pass kernels

@@ -29,7 +29,7 @@ struct StepFlags {
     int poly_compat, ls_exact;
 };
 
-// Rows per warp strip of an image column of ny rows, in a batch of `tiles`
+// Rows per warp strip of an image column of ny rows, of a string of `tiles`
 // strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
 int strip_rows_cap(int precision, int paired);
 int strip_rows(int precision, int paired, int ny, long tiles, int slots);

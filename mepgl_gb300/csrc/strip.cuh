@@ -13,8 +13,10 @@
 // 32) into a three-row ring in shared memory with cp.async and read it back
 // themselves, so no lane waits for another.  Rows j0 - 1 and j0 + S.rows are
 // read as halo rows.  While a row is computed, the loads of the next row are
-// in flight.  Every strip leaves one partial per quantity, and the last strip
-// of an image (atomic ticket) finishes it.
+// in flight.  Every strip leaves one partial per quantity and group of S.grows
+// rows, and the last strip of an image (atomic ticket) finishes it.  The groups
+// follow from the string alone and a strip is one of them, or in a batch, where
+// there are strips enough, several: a string's sums are the same in any batch.
 //
 // FP64: bound by the FP64 pipe, 64 clocks per warp instruction and SM
 // quarter, so 8 warps per SM (255 registers, no spills) keep it busy and the
@@ -221,10 +223,10 @@ __device__ __forceinline__ StripRef strip_tile(const batch_t<ONE> &bt, int g)
     return t;
 }
 
-// Slot of a strip's partial sums.
+// Slot of a strip's first partial sums (its next group's: tiles_x further).
 __device__ __forceinline__ int strip_slot(const StringDesc &S, const StripRef &tr)
 {
-    return S.stile_base + (tr.n * S.stiles_y + tr.ty) * S.tiles_x + tr.tx;
+    return S.part_base + tr.n * S.groups + tr.ty * S.gper * S.tiles_x + tr.tx;
 }
 
 // Packed neighbour codes of the lane's site in row j (0 outside the lattice).
@@ -298,15 +300,9 @@ __device__ __forceinline__ void image_sums(const double *part, int n, double (&t
     for (int k = 0; k < NV; ++k) tot[k] = __shfl_sync(FULL_MASK, all, sum_lane<NV>(k));
 }
 
-// The strip's NV partials leave the warp; if this strip is the last of its
-// image, every lane receives the image sums (its partials added in index
-// order) and the function returns true.  Everything that the lanes wrote
-// before is visible to whoever learns from the ticket (or from what the last
-// strip publishes) that the strip is done: the warp barrier orders the lanes'
-// writes before lane 0's fence, which is cumulative.
+// NV sums of a group of rows leave the warp.
 template <int NV, class T>
-__device__ __forceinline__ bool finish_image_warp(const T (&v)[NV], const Scalars &sc, int tile, int first_tile,
-                                                  int tiles_per_image, int img, double (&tot)[NV])
+__device__ __forceinline__ void store_sums(const T (&v)[NV], const Scalars &sc, int slot)
 {
     const int lane = threadIdx.x & 31;
     T w[NV];
@@ -315,20 +311,41 @@ __device__ __forceinline__ bool finish_image_warp(const T (&v)[NV], const Scalar
     const double mine = (double)warp_sums<NV>(w);
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-        if (lane == sum_lane<NV>(k)) sc.part[(size_t)tile * 8 + k] = mine;
+        if (lane == sum_lane<NV>(k)) sc.part[(size_t)slot * 8 + k] = mine;
+}
+
+// The strip is done.  If it is the last of its image's `strips`, every lane
+// receives the image sums (its `sums` partials from `first` on, added in index
+// order) and the function returns true.  Everything that the lanes wrote before,
+// the strip's partials among it, is visible to whoever learns from the ticket (or
+// from what the last strip publishes) that the strip is done: the warp barrier
+// orders the lanes' writes before lane 0's fence, which is cumulative.
+template <int NV>
+__device__ __forceinline__ bool finish_image(const Scalars &sc, int first, int sums, int strips, int img, double (&tot)[NV])
+{
+    const int lane = threadIdx.x & 31;
     __syncwarp();
     int last = 0;
     if (lane == 0) {
         __threadfence();
-        last = atomicAdd(&sc.ticket[img], 1u) == (unsigned)tiles_per_image - 1;
+        last = atomicAdd(&sc.ticket[img], 1u) == (unsigned)strips - 1;
         if (last) __threadfence();
     }
     last = __shfl_sync(FULL_MASK, last, 0);
     if (!last) return false;
     __syncwarp();
-    image_sums<NV>(sc.part + (size_t)first_tile * 8, tiles_per_image, tot);
+    image_sums<NV>(sc.part + (size_t)first * 8, sums, tot);
     if (lane == 0) sc.ticket[img] = 0;
     return true;
+}
+
+// The same for a strip of one group of rows, whose NV sums leave the warp first.
+template <int NV, class T>
+__device__ __forceinline__ bool finish_image_warp(const T (&v)[NV], const Scalars &sc, int slot, int first, int sums,
+                                                  int strips, int img, double (&tot)[NV])
+{
+    store_sums<NV>(v, sc, slot);
+    return finish_image<NV>(sc, first, sums, strips, img, tot);
 }
 
 // One row of x + alpha d as the gradient window holds it: fields of the
@@ -467,6 +484,7 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     }
     const int rows = S.ny - j0 < S.rows ? S.ny - j0 : S.rows;
     T v[2] = {(T)0, (T)0};
+    int slot = strip_slot(S, tr), left = S.grows;   // of the present group of rows; its rows to go
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
@@ -516,6 +534,13 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
                 v[1] = fma1(gv.x, gv.x - go.x, fma1(gv.y, gv.y - go.y, v[1]));
             }
         }
+        if constexpr (!ONE)
+            if (--left == 0 || r + 1 == rows) {
+                store_sums<2>(v, sc, slot);
+                v[0] = v[1] = (T)0;
+                slot += S.tiles_x;
+                left = S.grows;
+            }
         if constexpr (!CARRY) Rm = R0;
         R0 = Rp;
 #pragma unroll
@@ -523,7 +548,8 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     }
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[2];
-    const bool fin = finish_image_warp<2>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
+    if constexpr (ONE) store_sums<2>(v, sc, slot);
+    const bool fin = finish_image<2>(sc, S.part_base + tr.n * S.groups, S.groups, tpi, img, tot);
     if (fin && L.lane == 0) {
         (f.gcur ? sc.gn1 : sc.gn0)[img] = tot[0];
         sc.gdg[img] = tot[1];
@@ -625,6 +651,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     PolySum<T, NC> sum;
     sum.zero();
     bool links = false;   // some row was one of interior sites
+    int slot = strip_slot(S, tr), left = S.grows;   // of the present group of rows; its rows to go
 #pragma unroll 1
     for (int r = 0; r < rows; ++r) {
         const int j = j0 + r;
@@ -702,6 +729,18 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
                 for (int k = 0; k < 5; ++k) v[k] += o[k];
             }
         }
+        if constexpr (!ONE)
+            if (--left == 0 || r + 1 == rows) {
+                if constexpr (WIDE) {
+                    sum.total(pp, links, f.poly_compat, v);
+                    sum.zero();
+                    links = false;
+                }
+                store_sums<5>(v, sc, slot);
+                if constexpr (!WIDE) v[0] = v[1] = v[2] = v[3] = v[4] = (T)0;
+                slot += S.tiles_x;
+                left = S.grows;
+            }
         xm_ax = R0.x[0].x;
         dm_ax = R0.d[0].x;
         R0 = Rp;
@@ -709,10 +748,13 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     // the halo copy of the row below the tile may still be in flight: complete it before the
     // ring can be reused (the fused kernel runs more tiles in the same block)
     cp_async_wait_groups<0>();
-    if constexpr (WIDE) sum.total(pp, links, f.poly_compat, v);
+    if constexpr (ONE) {
+        if constexpr (WIDE) sum.total(pp, links, f.poly_compat, v);
+        store_sums<5>(v, sc, slot);
+    }
     const int tpi = S.tiles_x * S.stiles_y;
     double tot[5];
-    const bool fin = finish_image_warp<5>(v, sc, strip_slot(S, tr), S.stile_base + tr.n * tpi, tpi, img, tot);
+    const bool fin = finish_image<5>(sc, S.part_base + tr.n * S.groups, S.groups, tpi, img, tot);
     if (fin) {
         if (L.lane == 0) {
 #pragma unroll

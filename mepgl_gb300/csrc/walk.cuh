@@ -97,7 +97,7 @@ struct EnergyOp {
         {
             const double v[1] = {(double)e.total()};
             double tot[1];
-            if (finish_image_warp<1>(v, sc, u, n * tpi, tpi, img, tot) &&
+            if (finish_image_warp<1>(v, sc, u, n * tpi, tpi, tpi, img, tot) &&
                 (threadIdx.x & 31) == 0)
                 op.out[img] = S.disc ? tot[0] : tot[0] * S.ud.dx2;
         }
@@ -131,7 +131,7 @@ struct AdjointSums {
     {
         const double v[3] = {(double)h.total(), (double)eta.total(), (double)gamma.total()};
         double tot[3];
-        if (finish_image_warp<3>(v, sc, u, n * tpi, tpi, img, tot) &&
+        if (finish_image_warp<3>(v, sc, u, n * tpi, tpi, tpi, img, tot) &&
             (threadIdx.x & 31) == 0) {
             out[3 * img] = tot[0] * (S.disc ? 1.0 : -0.25 * S.ud.dx2);
             out[3 * img + 1] = tot[1] * S.ud.dx2;
@@ -304,7 +304,7 @@ struct FluxOp {
         {
             const double v[1] = {b};
             double tot[1];
-            if (finish_image_warp<1>(v, sc, u, n * tpi, tpi, img, tot) &&
+            if (finish_image_warp<1>(v, sc, u, n * tpi, tpi, tpi, img, tot) &&
                 (threadIdx.x & 31) == 0)
                 op.out[n] = tot[0] * S.ud.dx2;
         }
