@@ -1224,7 +1224,8 @@ static int resident(K kernel)
 
 // Constants and not what the compiler's register counts happen to give: the
 // rows of a strip, and with them the order of an image's sums, follow from it.
-int strip_pass_slots(int precision, int ncomp, int sms) { return sms * (precision == 1 ? 8 : ncomp == 2 ? 16 : 21); }
+// One component in FP32: 96 registers, five warps in each quarter of the SM.
+int strip_pass_slots(int precision, int ncomp, int sms) { return sms * (precision == 1 ? 8 : ncomp == 2 ? 16 : 20); }
 
 template <class T>
 static cudaError_t nlcg_fused_launch(const Launch &L, const Scalars &sc, const StepPlan &plan, int steps,
