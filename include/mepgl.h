@@ -200,7 +200,8 @@ mepgl_status mepgl_batch_generate_string(mepgl_ctx *ctx, int string, const mepgl
 mepgl_status mepgl_free_energy(mepgl_ctx *ctx, double *fenergy);
 
 /* Free energy and gradient dF/d(A, psi) of the current state.  Gradients
- * have the layout of the fields; NULL outputs are skipped.  Replaces the
+ * have the layout of the fields; NULL outputs are skipped.  Device outputs
+ * that are not aligned to an (x, y) pair take a copy more.  Replaces the
  * gradientPsi / gradientA launches (mepgl/src/nlcg.cu:1521-1537). */
 mepgl_status mepgl_energy_grad(mepgl_ctx *ctx, double *fenergy, void *g_a, void *g_psi_1, void *g_psi_2,
                                int memory);
@@ -210,7 +211,8 @@ mepgl_status mepgl_energy_grad(mepgl_ctx *ctx, double *fenergy, void *g_a, void 
  * and (adjoint non-NULL: host array of 3 F doubles) dF_n/d(H, eta, gamma)
  * without the weights at adjoint[3 n + k].  `weights` is a device array of F
  * doubles, rounded to the precision of the fields first.  g_psi_2 is ignored
- * with one component; the other arrays must not be NULL. */
+ * with one component; the other arrays must not be NULL, and take a copy more
+ * where they are not aligned to an (x, y) pair. */
 mepgl_status mepgl_weighted_grad(mepgl_ctx *ctx, const double *weights, double *adjoint, void *g_a, void *g_psi_1,
                                  void *g_psi_2);
 
@@ -345,7 +347,8 @@ mepgl_status mepgl_fused_wait_selftest(mepgl_ctx *ctx, int *timed_out);
  * Inputs (all device pointers): comp_code / sc_code are int32 neighbour
  * codes per site (the layout of the reference's buildNearestNeighbourMap),
  * the nine parameter arrays are per-site doubles, a / psi_1 / psi_2 are the
- * F images as double pairs; fenergy receives F doubles.  Scratch for the
+ * F images as double pairs, aligned to a pair (16 bytes; else
+ * MEPGL_ERR_INVALID_ARG); fenergy receives F doubles.  Scratch for the
  * reduction lives in fixed device arrays of the library (4 MiB + 16 KiB per
  * GPU that loads it, kept until the process exits): the string must satisfy
  * n_images <= 4096 and n_images * ceil(nx/32) * ceil(ny/8) <= 65536 (and the

@@ -10,6 +10,7 @@
 // mepgl/src/parallel_sum.cu:49-67, mepgl/src/interpolation.cu:410-480).
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
@@ -1131,36 +1132,52 @@ mepgl_status mepgl_batch_info(const mepgl_ctx *c, int string, int *nx, int *ny, 
 
 int mepgl_string_count(const mepgl_ctx *c) { return c ? (int)c->strings.size() : 0; }
 
+}  // extern "C"
+
+namespace {
+
+// The gradient kernels store whole (x, y) pairs: a caller's device array takes
+// them in place if it is aligned to a pair.
+bool pair_aligned(const mepgl_ctx *c, const void *p)
+{
+    return reinterpret_cast<uintptr_t>(p) % (2 * real_size(c->precision)) == 0;
+}
+
+// Gradient of string 0 into the caller's arrays (NULL: skipped), in place where
+// they are device arrays that allow it, else by way of the spare direction buffer.
+mepgl_status gradient_out(mepgl_ctx *c, void *const (&dst)[3], int memory, const double *weights, double *adjoint)
+{
+    StringHost &s = c->strings[0];
+    bool direct = memory == MEPGL_DEVICE;
+    for (int f = 0; f < 1 + c->ncomp; ++f) direct = direct && dst[f] && pair_aligned(c, dst[f]);
+    FieldPtrs out;
+    for (int f = 0; f < 3; ++f) out.p[f] = f > c->ncomp ? nullptr : direct ? dst[f] : s.d[c->di ^ 1][f];
+    Launch L = string_launch(c, 0);
+    L.paired = 0;   // the gradient a caller asks for is IEEE double in every FP64 mode
+    CK(c, launch_gradient_only(L, c->sc, c->xi, out, 0, weights, adjoint));
+    c->launches += 1;
+    const void *src[3] = {out.p[0], out.p[1], out.p[2]};
+    return direct ? MEPGL_OK : copy_fields(c, s, dst, src, memory, false, false);
+}
+
+}  // namespace
+
+extern "C" {
+
 mepgl_status mepgl_energy_grad(mepgl_ctx *c, double *fenergy, void *g_a, void *g_psi_1, void *g_psi_2, int memory)
 {
     if (!c) return MEPGL_ERR_INVALID_ARG;
     mepgl_status st = flush(c);
     if (st != MEPGL_OK) return st;
-    StringHost &s = c->strings[0];
     if (fenergy) {
         st = mepgl_free_energy(c, fenergy);
         if (st != MEPGL_OK) return st;
     }
     if (!g_a && !g_psi_1 && !g_psi_2) return MEPGL_OK;
-    const bool direct = memory == MEPGL_DEVICE && g_a && g_psi_1 && (c->ncomp == 1 || g_psi_2);
-    FieldPtrs out;
-    for (int f = 0; f < 3; ++f) out.p[f] = s.d[c->di ^ 1][f];   // spare direction buffer
-    if (direct) {
-        out.p[0] = g_a;
-        out.p[1] = g_psi_1;
-        out.p[2] = c->ncomp == 2 ? g_psi_2 : nullptr;
-    }
-    Launch L = string_launch(c, 0);
-    L.paired = 0;   // the gradient a caller asks for is IEEE double in every FP64 mode
-    CK(c, launch_gradient_only(L, c->sc, c->xi, out, 0));
-    c->launches += 1;
-    if (direct) {
-        CK(c, cudaStreamSynchronize(c->stream));
-        return MEPGL_OK;
-    }
-    void *dst[3] = {g_a, g_psi_1, g_psi_2};
-    const void *src[3] = {out.p[0], out.p[1], out.p[2]};
-    return copy_fields(c, s, dst, src, memory, false);
+    st = gradient_out(c, {g_a, g_psi_1, g_psi_2}, memory, nullptr, nullptr);
+    if (st != MEPGL_OK) return st;
+    CK(c, cudaStreamSynchronize(c->stream));
+    return MEPGL_OK;
 }
 
 mepgl_status mepgl_weighted_grad(mepgl_ctx *c, const double *weights, double *adjoint, void *g_a, void *g_psi_1,
@@ -1169,13 +1186,12 @@ mepgl_status mepgl_weighted_grad(mepgl_ctx *c, const double *weights, double *ad
     if (!c) return MEPGL_ERR_INVALID_ARG;
     if (!weights || !g_a || !g_psi_1 || (c->ncomp == 2 && !g_psi_2))
         return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_weighted_grad: null argument");
+    if (reinterpret_cast<uintptr_t>(weights) % sizeof(double))
+        return fail(c, MEPGL_ERR_INVALID_ARG, "mepgl_weighted_grad: weights are not aligned to a double");
     mepgl_status st = flush(c);
     if (st != MEPGL_OK) return st;
-    Launch L = string_launch(c, 0);
-    L.paired = 0;   // as mepgl_energy_grad
-    CK(c, launch_gradient_only(L, c->sc, c->xi, FieldPtrs{{g_a, g_psi_1, c->ncomp == 2 ? g_psi_2 : nullptr}}, 0, weights,
-                               adjoint ? c->dscratch : nullptr));
-    c->launches += 1;
+    st = gradient_out(c, {g_a, g_psi_1, g_psi_2}, MEPGL_DEVICE, weights, adjoint ? c->dscratch : nullptr);
+    if (st != MEPGL_OK) return st;
     if (adjoint) return fetch(c, {{adjoint, c->dscratch, 3 * (size_t)c->strings[0].F}}, false);
     CK(c, cudaStreamSynchronize(c->stream));
     return MEPGL_OK;

@@ -1664,6 +1664,9 @@ extern "C" mepgl_status mepgl_free_energy_noalloc(int nx, int ny, int n_images, 
         return noalloc_fail(MEPGL_ERR_INVALID_ARG,
                             "string too large for the fixed scratch: need n_images <= 4096 and "
                             "n_images * ceil(nx/32) * ceil(ny/8) <= 65536");
+    for (const void *p : {a, psi_1, multicomponent ? psi_2 : a})   // read as whole pairs
+        if (reinterpret_cast<uintptr_t>(p) % (2 * sizeof(double)))
+            return noalloc_fail(MEPGL_ERR_INVALID_ARG, "fields not aligned to a pair of doubles");
     // An error left pending by the caller's own earlier work is reported as
     // such and left in place, not taken for a failure of this call.
     cudaError_t pend = cudaPeekAtLastError();
