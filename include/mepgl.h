@@ -75,12 +75,12 @@ enum { MEPGL_DISC_REFERENCE = 0, MEPGL_DISC_LINK = 1 };
  * reductions, line search and every other kernel stay double.  No
  * reference counterpart. */
 enum { MEPGL_FP64_NATIVE = 0, MEPGL_FP64_PAIRED = 1 };
-/* How the FP32 NLCG steps of a mepgl_nlcg_steps call are launched: two pass
- * kernels per step, or every step of the call in one persistent launch whose
- * strips wait on per-image stage counters instead of kernel boundaries.  AUTO
- * fuses the batches of at most a few waves of strips, where the boundaries
- * idle much of the GPU.  Both give the same results bit for bit.  No
- * reference counterpart. */
+/* How the NLCG steps of a mepgl_nlcg_steps call are launched, in every
+ * precision (the names are older than that): two pass kernels per step, or the
+ * steps of the call in persistent launches whose strips wait on per-image stage
+ * counters instead of kernel boundaries.  AUTO fuses the batches of at most a few
+ * waves of strips (FP64: sixteen), where the boundaries idle much of the GPU.
+ * Both give the same results bit for bit.  No reference counterpart. */
 enum { MEPGL_FP32_STEPS_AUTO = 0, MEPGL_FP32_STEPS_PASSES = 1, MEPGL_FP32_STEPS_FUSED = 2 };
 
 /* The physical problem.  Replaces the generated headers config.cuh/real.cuh
@@ -322,7 +322,7 @@ mepgl_status mepgl_profile_passes(mepgl_ctx *ctx, int steps, int use_cg, double 
 
 /* Names of the kernels that run the two NLCG passes of this context in its
  * current precision and FP64 arithmetic, and of the
- * kernel that runs whole mepgl_nlcg_steps calls as one persistent launch
+ * kernel that runs mepgl_nlcg_steps calls as persistent launches
  * ("" when the passes are launched separately; mepgl_profile_passes always
  * times the separate pass kernels).  The strings are static.  No reference
  * counterpart; labels timings and profiler captures. */
@@ -333,8 +333,7 @@ mepgl_status mepgl_pass_kernels(const mepgl_ctx *ctx, const char **grad, const c
  * waits for an image stage that nothing sets, gives up after a short poll
  * limit and sets the device status flag.  *timed_out = 1 when the flag was
  * set (then cleared).  The launch writes no field or scalar, so the context
- * continues as before.  FP32 contexts of a build with fused steps; no
- * reference counterpart. */
+ * continues as before.  No reference counterpart. */
 mepgl_status mepgl_fused_wait_selftest(mepgl_ctx *ctx, int *timed_out);
 
 /* Allocation-free free energy.  No counterpart in the reference.  For callers

@@ -439,8 +439,7 @@ mepgl_status two_step_graph(mepgl_ctx *c, int use_cg, int maxwell, cudaGraphExec
 // single launch of seconds.
 bool use_fused(const mepgl_ctx *c)
 {
-    if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_PASSES) return false;
-    if (c->precision == 0 && c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED) return true;
+    if (c->opt.fp32_steps != MEPGL_FP32_STEPS_AUTO) return c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED;
     const long long cap = (long long)fuse_waves(c->precision) * strip_pass_slots(c->precision, c->ncomp, c->sm_count);
     for (int n : c->batch_nstiles)
         if (n > cap) return false;
@@ -1390,8 +1389,6 @@ mepgl_status mepgl_pass_kernels(const mepgl_ctx *c, const char **grad, const cha
 mepgl_status mepgl_fused_wait_selftest(mepgl_ctx *c, int *timed_out)
 {
     if (!c || !timed_out) return MEPGL_ERR_INVALID_ARG;
-    if (c->precision != MEPGL_FP32)
-        return fail(c, MEPGL_ERR_UNSUPPORTED, "mepgl_fused_wait_selftest: needs an FP32 context and fused steps");
     mepgl_status st = flush(c);
     if (st != MEPGL_OK) return st;
     const Launch L = make_launch(c, 0);
