@@ -434,9 +434,8 @@ mepgl_status two_step_graph(mepgl_ctx *c, int use_cg, int maxwell, cudaGraphExec
 // boundaries then idle much of the GPU).  FP32: on larger batches the pass
 // kernels, which hold more warps per SM, are faster.  FP64: both forms hold 8
 // warps per SM and are bound by arithmetic, so the fused launch keeps a small
-// lead (256 x 256 x 64, 7 waves, two steps: 8.96 ms against 9.24); it is
-// bounded so that one call of a large string does not hold the GPU in a
-// single launch of seconds.
+// lead (256 x 256 x 64, 7 waves, two steps: 8.96 ms against 9.24) up to the
+// waves measured.
 bool use_fused(const mepgl_ctx *c)
 {
     if (c->opt.fp32_steps != MEPGL_FP32_STEPS_AUTO) return c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED;
@@ -444,6 +443,18 @@ bool use_fused(const mepgl_ctx *c)
     for (int n : c->batch_nstiles)
         if (n > cap) return false;
     return true;
+}
+
+// Steps of one fused launch of a batch: a call of many is cut into launches of
+// about a fifth of a second at most (a wave of FP64 strips of two components, the
+// longest, takes 0.55 ms a step), so that others sharing the GPU get their turn
+// and a wait that runs out is reported.  The boundary costs some microseconds.
+int fused_steps_per_launch(const mepgl_ctx *c, int batch)
+{
+    constexpr int wave_steps = 400;
+    const int slots = strip_pass_slots(c->precision, c->ncomp, c->sm_count);
+    const int waves = (c->batch_nstiles[batch] + slots - 1) / slots;
+    return std::max(1, wave_steps / std::max(1, waves));
 }
 
 // Paired FP64 passes keep the fields x as float-float pairs:
@@ -493,14 +504,21 @@ mepgl_status nlcg_steps(mepgl_ctx *c, int iters, int use_cg, int maxwell)
 mepgl_status nlcg_steps_body(mepgl_ctx *c, int iters, int use_cg, int maxwell)
 {
     if (iters > 0 && use_fused(c)) {
-        // all steps of a batch in one persistent launch (per-image stages instead of kernel boundaries)
-        const StepFlags f0 = step_flags(c, 1, use_cg, maxwell);
-        for (size_t b = 0; b < c->batches.size(); ++b)
-            CK(c, launch_nlcg_fused(make_launch(c, (int)b), c->sc, f0, 1, iters, c->fqueue, c->fstage,
-                                    c->total_images));
+        // the steps of a batch in persistent launches (per-image stages instead of kernel boundaries)
+        for (size_t b = 0; b < c->batches.size(); ++b) {
+            StepFlags f = step_flags(c, 1, use_cg, maxwell);
+            const int most = fused_steps_per_launch(c, (int)b);
+            for (int it = 0, n; it < iters; it += n) {
+                n = std::min(most, iters - it);
+                CK(c, launch_nlcg_fused(make_launch(c, (int)b), c->sc, f, 1 + it, n, c->fqueue, c->fstage,
+                                        c->total_images));
+                f.xin ^= n & 1;
+                f.din ^= n & 1;
+                c->launches += 1;
+            }
+        }
         c->xi ^= iters & 1;
         c->di ^= iters & 1;
-        c->launches += (int64_t)c->batches.size();
         c->pending = true;
         return MEPGL_OK;
     }

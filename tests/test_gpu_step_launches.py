@@ -71,3 +71,26 @@ def test_waits_end(arith):
     np.testing.assert_array_equal(a.get_state().psi_1, b.get_state().psi_1)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("arith", ["fp32", "fp64", "paired"])
+@pytest.mark.parametrize("strings", [1, 2])
+def test_a_call_of_many_steps_is_several_launches(arith, strings):
+    """901 steps of strings of one wave: launches of 400 steps at most, the same bits as pass kernels."""
+    from mepgl_gb300 import native
+    rng = np.random.default_rng(23)
+    probs = [problem(rng, nx, ny, False, False, True, 0.0) for nx, ny in ((20, 17), (16, 12))[:strings]]
+    states = [random_state(rng, p, images=4, amp=0.2) for p in probs]
+    prec, kw = options(arith, native.FP32_STEPS_FUSED)
+    c = native.StringContext(probs[0], 4, prec, **kw)
+    c.set_state(states[0])
+    before = c.info()["kernel_launches"]
+    c.nlcg_steps(901)
+    assert 3 <= c.info()["kernel_launches"] - before < 20
+    c.close()
+    fused, passes = (run(arith, how, strings, probs, states, (901, 2))
+                     for how in (native.FP32_STEPS_FUSED, native.FP32_STEPS_PASSES))
+    for x, y in zip(fused, passes):
+        for key in x:
+            if x[key] is not None:
+                np.testing.assert_array_equal(x[key], y[key], err_msg=key)
