@@ -1452,15 +1452,25 @@ cudaError_t launch_winding(int precision, const void *psi, int nx, int ny, int F
     return cudaGetLastError();
 }
 
+// Dynamic shared memory of a reparametrization kernel, at most.  A kernel's limit
+// is one setting for the whole process, so every launch that needs more than the
+// default sets this, and none lowers what another thread's launch counts on.
+constexpr size_t REDIST_SMEM = 200 * 1024;
+
+template <class K>
+static cudaError_t allow_smem(K kernel, size_t need)
+{
+    if (need <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)REDIST_SMEM);
+}
+
 cudaError_t launch_redist_plan(double *s_f, double *s_jb, const double *s_use, int *status, int F, int F_new, int cubic,
                                int spline, const RedistPlan &p, cudaStream_t st)
 {
     const size_t sm = redist_plan_smem(F, F_new);
-    const int use_smem = sm <= 200 * 1024;   // about 2,300 images
-    if (use_smem && sm > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_redist_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-    }
+    const int use_smem = sm <= REDIST_SMEM;   // about 2,300 images
+    const cudaError_t e = allow_smem(k_redist_plan, use_smem ? sm : 0);
+    if (e != cudaSuccess) return e;
     k_redist_plan<<<1, 128, use_smem ? sm : 0, st>>>(s_f, s_jb, s_use, status, F, F_new, cubic, spline, p, use_smem);
     return cudaGetLastError();
 }
@@ -1497,7 +1507,7 @@ static void cubic_shape(int precision, int F, int F_new, int *tpb_out, size_t *s
     while (tpb > 32 && (size_t)tpb * F * cs > 32 * 1024) tpb >>= 1;
     const size_t sm = ub + (size_t)tpb * F * cs;
     *tpb_out = tpb;
-    *sm_out = sm <= 200 * 1024 ? sm : 0;
+    *sm_out = sm <= REDIST_SMEM ? sm : 0;
 }
 
 size_t redist_cubic_scratch_bytes(int precision, long pairs, int F, int F_new)
@@ -1522,23 +1532,18 @@ cudaError_t launch_redist_cubic(int precision, const void *f, void *fnew, void *
         const long blocks = (reals + tpb - 1) / tpb;
         const int grid = (int)(blocks < 152 * 32 ? blocks : 152 * 32);
         if (precision == 1) {
-            if (sm > 48 * 1024)
-                e = cudaFuncSetAttribute(k_redist_cubic_s<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            e = allow_smem(k_redist_cubic_s<double>, sm);
             if (e != cudaSuccess) return e;
             k_redist_cubic_s<double><<<grid, tpb, sm, st>>>((const double *)f, (double *)fnew, reals, F, F_new, p);
         } else {
-            if (sm > 48 * 1024)
-                e = cudaFuncSetAttribute(k_redist_cubic_s<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            e = allow_smem(k_redist_cubic_s<float>, sm);
             if (e != cudaSuccess) return e;
             k_redist_cubic_s<float><<<grid, tpb, sm, st>>>((const float *)f, (float *)fnew, reals, F, F_new, p);
         }
         return cudaGetLastError();
     }
-    if (ub > 200 * 1024 || !sigma) return cudaErrorInvalidValue;   // more than about 2,800 images
-    if (ub > 48 * 1024)
-        e = precision == 1
-                ? cudaFuncSetAttribute(k_redist_cubic<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ub)
-                : cudaFuncSetAttribute(k_redist_cubic<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ub);
+    if (ub > REDIST_SMEM || !sigma) return cudaErrorInvalidValue;   // more than about 2,800 images
+    e = precision == 1 ? allow_smem(k_redist_cubic<double>, ub) : allow_smem(k_redist_cubic<float>, ub);
     if (e != cudaSuccess) return e;
     if (precision == 1)
         k_redist_cubic<double><<<grid_for(reals), NT, ub, st>>>((const double *)f, (double *)fnew, (double *)sigma,
