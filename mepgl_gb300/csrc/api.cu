@@ -215,14 +215,17 @@ int layout_strips(mepgl_ctx *c)
     c->batch_nstiles.clear();
     size_t si = 0;
     for (Batch &B : c->batches) {
-        long all = 0;
-        for (int k = 0; k < B.n; ++k) all += most(B.s[k]);
+        long all = 0, columns = 0;
+        for (int k = 0; k < B.n; ++k) {
+            all += most(B.s[k]);
+            columns += (long)B.s[k].F * B.s[k].tiles_x;
+        }
         c->batch_stile0.push_back(base);
         for (int k = 0; k < B.n; ++k, ++si) {
             StringDesc &D = B.s[k];
-            D.grows = strip_rows(c->precision, paired, D.ny, most(D), slots);
+            D.grows = strip_rows(c->precision, paired, D.ny, (long)D.F * D.tiles_x, most(D), slots);
             const int ngroups = (D.ny + D.grows - 1) / D.grows;   // down an image
-            const int per = paired ? 1 : std::max(1, strip_rows(c->precision, paired, D.ny, all, slots) / D.grows);
+            const int per = paired ? 1 : std::max(1, strip_rows(c->precision, paired, D.ny, columns, all, slots) / D.grows);
             D.stiles_y = (ngroups + per - 1) / per;
             D.gper = (ngroups + D.stiles_y - 1) / D.stiles_y;
             D.stiles_y = (ngroups + D.gper - 1) / D.gper;
@@ -435,11 +438,28 @@ mepgl_status two_step_graph(mepgl_ctx *c, int use_cg, int maxwell, cudaGraphExec
 // kernels, which hold more warps per SM, are faster.  FP64: both forms hold 8
 // warps per SM and are bound by arithmetic, so the fused launch keeps a small
 // lead (256 x 256 x 64, 7 waves, two steps: 8.96 ms against 9.24) up to the
-// waves measured.
+// waves measured.  Float-float: warps of the two passes side by side on an SM,
+// each of some 40 KB of instructions, cost more than the boundaries (ten steps, fused
+// against separate: 256 x 256 x 64 13.6 / 12.2 ms, 200 x 160 x 24 3.4 / 2.8, 48 x 48 x
+// 300 7.1 / 2.9, 64 x 64 x 16 0.48 / 0.44), but for the smallest strings, whose strips
+// are single rows (67 x 61 x 9: 0.43 / 0.53, one component 0.30 / 0.40).  One
+// component has half the instructions: there, images of some fifty strips or more
+// are no worse fused in batches of two waves (256 x 256 x 32 3.5 / 3.9, 160 x 160 x 60
+// 2.7 / 3.0, 300 x 100 x 40 3.0 / 2.7), smaller ones are (64 x 40 x 600 4.0 / 3.0).
 bool use_fused(const mepgl_ctx *c)
 {
     if (c->opt.fp32_steps != MEPGL_FP32_STEPS_AUTO) return c->opt.fp32_steps == MEPGL_FP32_STEPS_FUSED;
-    const long long cap = (long long)fuse_waves(c->precision) * strip_pass_slots(c->precision, c->ncomp, c->sm_count);
+    const int slots = strip_pass_slots(c->precision, c->ncomp, c->sm_count);
+    if (c->precision == 1 && c->opt.fp64_arith == MEPGL_FP64_PAIRED) {
+        bool rows = true, large = c->ncomp == 1;
+        for (const StringDesc &D : c->hdesc) {
+            rows = rows && D.grows == 1;
+            large = large && D.tiles_x * D.stiles_y >= 48;
+        }
+        for (int n : c->batch_nstiles) large = large && n >= 2 * slots;
+        if (!rows && !large) return false;
+    }
+    const long long cap = (long long)fuse_waves(c->precision) * slots;
     for (int n : c->batch_nstiles)
         if (n > cap) return false;
     return true;

@@ -19,6 +19,7 @@
 //
 // Energies, gradients, adjoints and B, J of a string are formed by the same
 // kind of walk (walk.cuh).
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -84,7 +85,10 @@ int fuse_waves(int precision) { return precision == 1 ? MEPGL_FUSE_WAVES_F64 : M
 // 256 x 40 loses 3 % from 150 on), down to the fewest rows that still gain.
 // Float-float strips are bound by issue, and a second wave of them costs more
 // than long ones: four steps of 128 x 128 x 24 take 447 / 845 us at 80 % (one
-// wave of 12 rows), 613 / 1029 at 110 %, 522 / 903 at 150 %.
+// wave of 12 rows), 613 / 1029 at 110 %, 522 / 903 at 150 %.  So a string of
+// one to one and a half waves of the most rows takes up to half as many more and
+// is one wave (ten steps, two components: 200 x 160 x 24 4.2 -> 3.4 ms, 40 x 1000
+// x 10 3.1 -> 2.2).
 #ifndef MEPGL_STRIP_ROWS_F32
 #define MEPGL_STRIP_ROWS_F32 40
 #endif
@@ -118,10 +122,16 @@ static int equal_rows(int ny, int cap, int least, long tiles, long want)
     return (int)((ny + k - 1) / k);
 }
 
-int strip_rows(int precision, int paired, int ny, long tiles, int slots)
+int strip_rows(int precision, int paired, int ny, long columns, long tiles, int slots)
 {
+    const int cap = strip_rows_cap(precision, paired);
+    if (paired && tiles > slots && 2 * tiles <= 3L * slots) {
+        const long k = std::max(1L, slots / columns), rows = (ny + k - 1) / k;   // k strips a column: one wave
+        if (k * columns <= slots && 2 * rows <= 3 * cap) return (int)rows;
+        return equal_rows(ny, cap, 1, tiles, 3L * slots / 2);
+    }
     const int fill = precision == 0 ? MEPGL_STRIP_FILL_F32 : paired ? MEPGL_STRIP_FILL_FF : MEPGL_STRIP_FILL_F64;
-    return equal_rows(ny, strip_rows_cap(precision, paired), precision == 0 ? 2 : 1, tiles, (long)slots * fill / 100);
+    return equal_rows(ny, cap, precision == 0 ? 2 : 1, tiles, (long)slots * fill / 100);
 }
 
 #ifndef MEPGL_WALK_ROWS_F32
@@ -130,6 +140,7 @@ int strip_rows(int precision, int paired, int ny, long tiles, int slots)
 #ifndef MEPGL_WALK_ROWS_F64
 #define MEPGL_WALK_ROWS_F64 8
 #endif
+static_assert(MEPGL_WALK_ROWS_F32 <= 8, "a lane adds up its rows in float");
 int walk_rows(int precision, int ny, long columns, int sms)
 {
     const int cap = precision == 0 ? MEPGL_WALK_ROWS_F32 : MEPGL_WALK_ROWS_F64;

@@ -29,10 +29,10 @@ struct StepFlags {
     int poly_compat, ls_exact;
 };
 
-// Rows per warp strip of an image column of ny rows, of a string of `tiles`
-// strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
+// Rows per warp strip of an image column of ny rows, where `columns` such columns
+// are `tiles` strips of strip_rows_cap() rows on a GPU that holds `slots` warps.
 int strip_rows_cap(int precision, int paired);
-int strip_rows(int precision, int paired, int ny, long tiles, int slots);
+int strip_rows(int precision, int paired, int ny, long columns, long tiles, int slots);
 // The same for the walks over one string, of `columns` image columns of strips.
 int walk_rows(int precision, int ny, long columns, int sms);
 // Steps are fused for batches of at most fuse_waves() x strip_pass_slots()
