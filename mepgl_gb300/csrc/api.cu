@@ -94,6 +94,8 @@ void free_string_buffers(StringHost &s)
 void free_string_params(StringHost &s)
 {
     for (auto &p : s.dparams) { cudaFree(p); p = nullptr; }
+    cudaFree(s.dsites);
+    s.dsites = nullptr;
     cudaFree(s.dmask);
     s.dmask = nullptr;
 }
@@ -125,6 +127,10 @@ mepgl_status upload_string_params(mepgl_ctx *c, StringHost &s)
             cudaError_t e;
             s.dparams[k] = c->precision == 1 ? upload_as<double>(c, s.params[k], &e) : upload_as<float>(c, s.params[k], &e);
             CK(c, e);
+        }
+        if (c->precision == 1 && c->opt.fp64_arith == MEPGL_FP64_PAIRED) {
+            CK(c, cudaMalloc(&s.dsites, (size_t)(5 * c->ncomp + 1) * s.M() * sizeof(ff)));
+            CK(c, launch_pair_sites(s.dparams, c->ncomp, s.dsites, s.M()));
         }
     }
     return MEPGL_OK;
@@ -171,6 +177,16 @@ void fill_desc(mepgl_ctx *c, int si, int img_base)
     round_uniform(D.uff, U);      // the double values split into float pairs
     D.disc = c->opt.discretization;
     D.ph = s.dparams[8];
+    if (s.dsites) {
+        const size_t bytes = (size_t)s.M() * sizeof(ff);
+        const char *at = static_cast<const char *>(s.dsites);
+        for (int k = 0; k < c->ncomp; ++k)
+            for (const void **p : {&D.pairs.a[k], &D.pairs.b[k], &D.pairs.hmx[k], &D.pairs.hmy[k], &D.pairs.aob[k]}) {
+                *p = at;
+                at += bytes;
+            }
+        D.pairs.h = at;
+    }
     D.mask = s.dmask;
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < 3; ++f) {

@@ -21,6 +21,7 @@ struct StringHost {
     std::vector<int32_t> comp, sc;
     bool uniform;
     void *dparams[9] = {};             // per-site arrays (type T) when not uniform
+    void *dsites = nullptr;            // and those of the float-float passes (PairSites), in one piece
     uint16_t *dmask = nullptr;
     void *x[2][3] = {}, *g[2][3] = {}, *d[2][3] = {};
     double q[2], eta, gamma, delta, dx;

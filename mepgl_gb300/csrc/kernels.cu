@@ -177,16 +177,20 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid)
                      : "memory");
 }
 
-// (h + h_neighbour) dx of the four neighbours of site s = (i, j).
-template <class T, int NC>
+// (h + h_neighbour) dx of the four neighbours of site s = (i, j).  PAIRS: of a
+// float-float pass; PS: the string may have per-site parameters.
+template <class T, int NC, bool PAIRS = false, bool PS = true>
 __device__ __forceinline__ FieldSums<T> field_sums(const StringDesc &S, const PackParams<T, NC> &pp, int i, int j, int s)
 {
     const T hs = pp.hd + pp.hd;
     FieldSums<T> f{hs, hs, hs, hs};
-    if (S.per_site) {
-        const store_t<T> *h = static_cast<const store_t<T> *>(S.ph);
+    if (PS && S.per_site) {
+        auto at = [&](int n) {
+            if constexpr (PAIRS && std::is_same<T, ff>::value) return pair_site(S.pairs.h, n);
+            else return from_store<T>(static_cast<const store_t<T> *>(S.ph)[n]);
+        };
         const T dx = S.template u<T>().dx;
-        auto with = [&](int n) { return pp.hd + from_store<T>(h[n]) * dx; };
+        auto with = [&](int n) { return pp.hd + at(n) * dx; };
         f.u = with(j + 1 < S.ny ? s + S.nx : s);
         f.d = with(j > 0 ? s - S.nx : s);
         f.r = with(i + 1 < S.nx ? s + 1 : s);
@@ -445,6 +449,24 @@ __global__ void k_restart_cg(Scalars sc, int first, int last)
 {
     const int n = first + blockIdx.x * blockDim.x + threadIdx.x;
     if (n < last) sc.gn0[n] = sc.gn1[n] = INFINITY;
+}
+
+// PairSites' arrays of one component, or (a alone) of the field.
+__global__ void __launch_bounds__(NT) k_pair_sites(const double *a, const double *b, const double *mx, const double *my, float2 *out,
+                                                   long M)
+{
+    const long i = blockIdx.x * (long)NT + threadIdx.x;
+    if (i >= M) return;
+    auto put = [&](int k, double v) {
+        const ff w = to_ff(v);
+        out[k * M + i] = make_float2(w.hi, w.lo);
+    };
+    put(0, a[i]);
+    if (!b) return;
+    put(1, b[i]);
+    put(2, 0.5 / mx[i]);
+    put(3, 0.5 / my[i]);
+    put(4, a[i] / b[i]);
 }
 
 // Fields x between double pairs and float-float pairs, in place (an ff2
@@ -1181,7 +1203,9 @@ static cudaError_t walk(const Launch &L, const Scalars &sc, int xbuf, const Op &
 }
 
 // NLCG passes: one single-warp block per strip; launches of one string take
-// the kernels that read its descriptor at fixed offsets.
+// the kernels that read its descriptor at fixed offsets, and in float-float, where
+// the registers run out, those without per-site parameters have no code for them
+// (256 x 256 x 64, four steps: 5.65 ms with it, 5.32 without).
 #define DISPATCH_STRIP_T(L, KERNEL, T, ...)                                                         \
     do {                                                                                            \
         if (strip_one(L)) {                                                                         \
@@ -1196,7 +1220,11 @@ static cudaError_t walk(const Launch &L, const Scalars &sc, int xbuf, const Op &
 #define DISPATCH_STRIP(L, KERNEL, ...)                                                              \
     do {                                                                                            \
         if ((L).precision == 0) DISPATCH_STRIP_T(L, KERNEL, float, __VA_ARGS__);                    \
-        else if ((L).paired) DISPATCH_STRIP_T(L, KERNEL, ff, __VA_ARGS__);                          \
+        else if ((L).paired && strip_one(L) && !(L).batch->s[0].per_site) {                         \
+            const batch_t<true> one = only_string(L);                                               \
+            if ((L).ncomp == 2) KERNEL<ff, 2, true, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(one, __VA_ARGS__); \
+            else KERNEL<ff, 1, true, false><<<(L).n_stiles, NTS, 0, (L).stream>>>(one, __VA_ARGS__); \
+        } else if ((L).paired) DISPATCH_STRIP_T(L, KERNEL, ff, __VA_ARGS__);                        \
         else DISPATCH_STRIP_T(L, KERNEL, double, __VA_ARGS__);                                      \
     } while (0)
 
@@ -1563,6 +1591,18 @@ cudaError_t launch_redist_cubic(int precision, const void *f, void *fnew, void *
         k_redist_cubic<float><<<grid_for(reals), NT, ub, st>>>((const float *)f, (float *)fnew, (float *)sigma, reals,
                                                                F, F_new, p);
     return cudaGetLastError();
+}
+
+cudaError_t launch_pair_sites(void *const *p, int ncomp, void *out, long M)
+{
+    // behind the parameters' own copies, and done when the context's stream may read them
+    const unsigned grid = (unsigned)((M + NT - 1) / NT);
+    const double *const *q = reinterpret_cast<const double *const *>(p);
+    float2 *o = static_cast<float2 *>(out);
+    for (int k = 0; k < ncomp; ++k) k_pair_sites<<<grid, NT, 0, cudaStreamLegacy>>>(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3], o + 5 * k * M, M);
+    k_pair_sites<<<grid, NT, 0, cudaStreamLegacy>>>(q[8], nullptr, nullptr, nullptr, o + 5 * ncomp * M, M);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
 }
 
 cudaError_t launch_x_format(void *x, long pairs, int to_pairs, cudaStream_t st)

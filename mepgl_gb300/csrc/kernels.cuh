@@ -58,6 +58,9 @@ cudaError_t launch_grad(const Launch &L, const Scalars &sc, const StepFlags &f);
 // Pass 2: d <- -g + beta d (into d[dout]); quartic of F(x + a d); the last
 // tile of each image runs the line search and sets alpha, alpha_pend.
 cudaError_t launch_dir_poly(const Launch &L, const Scalars &sc, const StepFlags &f);
+// PairSites' arrays, one after the other (a, b, 1 / 2 m_xx, 1 / 2 m_yy, a / b per
+// component, h) in `out`, from the device arrays p (a_1 b_1 mxx_1 myy_1 a_2 .. h).
+cudaError_t launch_pair_sites(void *const *p, int ncomp, void *out, long M);
 // Paired FP64: the NLCG passes keep x as float-float pairs; the in-place
 // conversion of `pairs` complex values of x to (1) or from (0) them.
 cudaError_t launch_x_format(void *x, long pairs, int to_pairs, cudaStream_t st);

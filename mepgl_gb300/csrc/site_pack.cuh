@@ -137,6 +137,13 @@ struct PackView {
     P px[3][3], py[3][3];
 };
 
+// Value of a site in one of PairSites' arrays.
+__device__ __forceinline__ ff pair_site(const void *p, int s)
+{
+    const float2 v = static_cast<const float2 *>(p)[s];
+    return ff(v.x, v.y);
+}
+
 // Parameters as the stencils use them: read from the descriptor, and the
 // site's own where the string has per-site arrays.
 template <class S, int NC>
@@ -199,6 +206,35 @@ struct PackParams {
             x[c] = from_store<S>((St)0.5 / static_cast<const St *>(D.pmxx[c])[i > 0 ? s - 1 : s]);
             y[c] = from_store<S>((St)0.5 / static_cast<const St *>(D.pmyy[c])[j > 0 ? s - D.nx : s]);
         }
+        take_site(p, x, y);
+    }
+    // in the NLCG passes, whose float-float ones have them as pairs
+    __device__ __forceinline__ void load_pass_site(const StringDesc &D, int i, int j, int s)
+    {
+        if constexpr (!std::is_same<S, ff>::value) return load_site(D, i, j, s);
+        else load_pairs(D, i, j, s);
+    }
+    __device__ __forceinline__ void load_pairs(const StringDesc &D, int i, int j, int s)
+    {
+        SiteParams<S> p;
+        p.load_uniform(D);
+        S x[2], y[2];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            p.a[c] = pair_site(D.pairs.a[c], s);
+            p.b[c] = pair_site(D.pairs.b[c], s);
+            p.hmx[c] = pair_site(D.pairs.hmx[c], s);
+            p.hmy[c] = pair_site(D.pairs.hmy[c], s);
+            p.aob[c] = pair_site(D.pairs.aob[c], s);
+            x[c] = pair_site(D.pairs.hmx[c], i > 0 ? s - 1 : s);
+            y[c] = pair_site(D.pairs.hmy[c], j > 0 ? s - D.nx : s);
+        }
+        p.h = pair_site(D.pairs.h, s);
+        take_site(p, x, y);
+    }
+    // x, y: 1 / (2 m) at the left and the lower neighbour
+    __device__ __forceinline__ void take_site(const SiteParams<S> &p, const S (&x)[2], const S (&y)[2])
+    {
         const S d2 = p.dx2, two = S(2.0f), n2 = S(-2.0f);
         const P i2 = K::bc(idx * idx);
         hmx = K::mk(p.hmx[0], p.hmx[NC - 1]);

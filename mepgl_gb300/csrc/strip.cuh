@@ -397,7 +397,7 @@ using GradRing = vec2_t<T>[3][2][2][1 + NC];
 // image computes beta.  Returns true (in every lane) when this strip finished
 // its image; a consumer in the same launch that has seen the image finished
 // reads the field stores (finish_image_warp).
-template <class T, int NC, bool ONE>
+template <class T, int NC, bool ONE, bool PS = true>
 __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
 {
@@ -508,20 +508,20 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         bool inner = false;
         if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
-            if (S.per_site) pp.load_site(S, L.gi, j, s);
+            if (PS && S.per_site) pp.load_pass_site(S, L.gi, j, s);
             const GradView<T, NC> vc = grad_view(R0), vu = grad_view(Rp);
-            const FieldSums<T> h = field_sums(S, pp, L.gi, j, s);
+            const FieldSums<T> h = field_sums<T, NC, true, PS>(S, pp, L.gi, j, s);
             T g[2 + 2 * NC];
             if (inner) {
                 if constexpr (std::is_same<T, double>::value)
                     site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr),
-                                         pp, Ones(), h, S.per_site, f.maxwell, S.thin_film, up, g);
+                                         pp, Ones(), h, PS && S.per_site, f.maxwell, S.thin_film, up, g);
             } else {
                 Wts<T> w;
                 w.load(R0.m);
                 if constexpr (!CARRY) up = grad_below(Rm, R0, pp, w);
                 site_gradient<T, NC>(vc, vu, psi_x<T, NC>(pl), psi_y<T, NC>(pl), psi_x<T, NC>(pr), psi_y<T, NC>(pr), pp,
-                                     w, h, S.per_site, f.maxwell, S.thin_film, up, g);
+                                     w, h, PS && S.per_site, f.maxwell, S.thin_film, up, g);
             }
 #pragma unroll
             for (int c = 0; c < 1 + NC; ++c) {
@@ -563,12 +563,12 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
     return fin;
 }
 
-template <class T, int NC, bool ONE>
+template <class T, int NC, bool ONE, bool PS = true>
 __global__ void __launch_bounds__(NTS, (StripBlocks<T, NC, ONE>::grad)) k_grad_s(const __grid_constant__ batch_t<ONE> bt,
                                                                   int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) GradRing<T, NC> ring;
-    grad_tile<T, NC, ONE>(bt, strip_tile<ONE>(bt, tile0 + (int)blockIdx.x), sc, f, ring);
+    grad_tile<T, NC, ONE, PS>(bt, strip_tile<ONE>(bt, tile0 + (int)blockIdx.x), sc, f, ring);
 }
 
 // One row of the polynomial window: fields and new direction of the lane's
@@ -586,7 +586,7 @@ using DirRing = vec2_t<T>[3][2][3][1 + NC];
 // Direction pass on one strip: d <- -g + beta d over the strip (+ halo), the
 // quartic coefficients of F(x + a d); the last strip of an image runs the line
 // search.  Returns true (in every lane) when this strip finished its image.
-template <class T, int NC, bool ONE>
+template <class T, int NC, bool ONE, bool PS = true>
 __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                          DirRing<T, NC> &ring, double (&coef)[5])
 {
@@ -706,13 +706,13 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
         }
         bool inner = false;
         if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
-        links |= inner && !S.per_site;
+        links |= inner && !(PS && S.per_site);
         if (L.cok) {
-            if (S.per_site) pp.load_site(S, L.gi, j, s);
+            if (PS && S.per_site) pp.load_pass_site(S, L.gi, j, s);
             if constexpr (!WIDE) sum.zero();
             if (inner) {
                 if constexpr (std::is_same<T, double>::value) {
-                    if (S.per_site)
+                    if (PS && S.per_site)
                         site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, OnesPerSite(), 1, f.poly_compat, S.thin_film, sum);
                     else
                         site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, Ones(), 0, f.poly_compat, S.thin_film, sum);
@@ -720,7 +720,7 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
             } else {
                 Wts<T> w;
                 w.load(R0.m);
-                site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, w, S.per_site, f.poly_compat, S.thin_film, sum);
+                site_poly<T, NC>(pack_view(vx), pack_view(vd), pp, w, PS && S.per_site, f.poly_compat, S.thin_film, sum);
             }
             if constexpr (!WIDE) {
                 T o[5];
@@ -774,13 +774,13 @@ __device__ __forceinline__ bool dir_tile(const batch_t<ONE> &bt, const StripRef 
     return fin;
 }
 
-template <class T, int NC, bool ONE>
+template <class T, int NC, bool ONE, bool PS = true>
 __global__ void __launch_bounds__(NTS, (StripBlocks<T, NC, ONE>::dir)) k_dir_poly_s(const __grid_constant__ batch_t<ONE> bt,
                                                                       int tile0, Scalars sc, StepFlags f)
 {
     __shared__ __align__(16) DirRing<T, NC> ring;
     __shared__ double coef[5];
-    dir_tile<T, NC, ONE>(bt, strip_tile<ONE>(bt, tile0 + (int)blockIdx.x), sc, f, ring, coef);
+    dir_tile<T, NC, ONE, PS>(bt, strip_tile<ONE>(bt, tile0 + (int)blockIdx.x), sc, f, ring, coef);
 }
 
 // ------------------------------------------------------------ fused steps
