@@ -61,7 +61,11 @@ enum { MEPGL_HOST = 0, MEPGL_DEVICE = 1,          /* where a caller buffer lives
 enum { MEPGL_LS_COMPAT = 0, MEPGL_LS_EXACT = 1 }; /* step: geometric scan | its exact
                                                      first local minimum     */
 enum { MEPGL_POLY_COMPAT = 0, MEPGL_POLY_EXACT = 1 };       /* line polynomial        */
-enum { MEPGL_SPLINE_COMPAT = 0, MEPGL_SPLINE_FMM = 1 };     /* cubic evaluation       */
+/* Cubic evaluation, the reference's or the textbook's.  Both find an image's
+ * segment on the arc length s[k] itself, which ends at 1: the reference walks
+ * running sums of its differences, whose last bits may end below 1, and then
+ * reads past its array (mepgl/src/interpolation.cu:380-386). */
+enum { MEPGL_SPLINE_COMPAT = 0, MEPGL_SPLINE_FMM = 1 };
 enum { MEPGL_METRIC_FIELDS = 0, MEPGL_METRIC_JB = 1 };      /* arc-length metric      */
 enum { MEPGL_REDIST_LINEAR = 0, MEPGL_REDIST_CUBIC = 1 };
 /* Kinetic and magnetic terms: the reference's linearised covariant differences

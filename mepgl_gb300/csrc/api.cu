@@ -452,9 +452,9 @@ mepgl_status two_step_graph(mepgl_ctx *c, int use_cg, int maxwell, cudaGraphExec
 // Fused steps pay where a batch is a few waves of the pass kernels (the kernel
 // boundaries then idle much of the GPU).  FP32: on larger batches the pass
 // kernels, which hold more warps per SM, are faster.  FP64: both forms hold 8
-// warps per SM and are bound by arithmetic, so the fused launch keeps a small
-// lead (256 x 256 x 64, 7 waves, two steps: 8.96 ms against 9.24) up to the
-// waves measured.  Float-float: warps of the two passes side by side on an SM,
+// warps per SM and are bound by arithmetic, so the fused launch keeps a lead up to
+// the waves measured (ten steps, two components, fused against separate: 200 x 160 x
+// 24 7.4 / 9.3 ms, 400 x 300 x 8 8.3 / 10.6, 48 x 48 x 300 8.5 / 8.8).  Float-float: warps of the two passes side by side on an SM,
 // each of some 40 KB of instructions, cost more than the boundaries (ten steps, fused
 // against separate: 256 x 256 x 64 13.6 / 12.2 ms, 200 x 160 x 24 3.4 / 2.8, 48 x 48 x
 // 300 7.1 / 2.9, 64 x 64 x 16 0.48 / 0.44), but for the smallest strings, whose strips

@@ -9,7 +9,7 @@
 // partials in a fixed order.
 //
 // Precision.  Fields are float or double (T).  Sums are formed in T inside
-// a block (fixed pairwise shuffle trees), then in double across tiles and
+// a warp (fixed shuffle trees), then in double across groups of rows and
 // images.  GB300's FP64 pipe is a small fraction of its FP32
 // rate, so FP32 kernels avoid any per-site double arithmetic or conversion.
 #pragma once
@@ -62,8 +62,9 @@ template <> __device__ __forceinline__ void store2<ff>(double2 *p, ff2 v)
 // type itself for float and double; float-float pairs in the paired FP64 mode
 // (ff2 fills the same 16 bytes as double2), so the paired passes move them
 // without conversions.  The arrays are internal to the NLCG passes and the
-// pending-step update, and are zeroed (a valid value in every format)
-// whenever the history is reset.
+// pending-step update.  A restart does not clear them: after one, no pass uses what
+// they hold (beta is 0 and |g|^2 infinite; what a pass has loaded ahead is dropped)
+// before it has written them, in its own format.
 template <class T> __device__ __forceinline__ vec2_t<T> loadw(const vec2_t<store_t<T>> *p) { return load2<T>(p); }
 template <> __device__ __forceinline__ ff2 loadw<ff>(const double2 *p)
 {

@@ -753,11 +753,11 @@ __device__ void arc_cumulate(int F, double *const (&s)[2], int *bad, double *r)
     }
 }
 
-__global__ void k_arc_cumulate(int F, double *s_f, double *s_jb, int *bad, int use_smem)
+__global__ void k_arc_cumulate(int F, double *s, int *bad, int use_smem)
 {
     extern __shared__ double cum_sm[];
-    double *const s[2] = {s_f ? s_f : s_jb, s_f ? s_jb : nullptr};
-    arc_cumulate(F, s, bad, use_smem ? cum_sm : nullptr);
+    double *const one[2] = {s, nullptr};
+    arc_cumulate(F, one, bad, use_smem ? cum_sm : nullptr);
 }
 
 // Finiteness of the per-image scalars after a call's NLCG steps: the energy
@@ -789,7 +789,8 @@ __global__ void k_check_scalars(const double *fenergy, const double *gn, int n_i
 // from the continuants p_q = d_q p_{q-1} - dl_q du_{q-1} p_{q-2} (a multiply-add
 // per image; d'_q = p_q / p_{q-1} are then independent divisions), polished by
 // two sweeps of d'_q = d_q - dl_q du_{q-1} / d'_{q-1}, each of which shrinks an
-// error by dl_q du_{q-1} / d'_{q-1}^2 <= 1/4.  If a pivot would have been exchanged, or one is not
+// error by dl_q du_{q-1} / d'_{q-1}^2: at most 1/4, except 1 at q = 1, where the
+// first sweep leaves d'_0 = d_0 exact and the second d'_1.  Hence two.  If a pivot would have been exchanged, or one is not
 // a normal number, the elimination runs as written.  With both
 // cumulations before it, 32 images, cubic: 45 us -> 26; 64 images, linear: 34 us
 // -> 14.  The arrays live in shared memory when they fit, else in the plan's
@@ -1462,7 +1463,7 @@ cudaError_t launch_arc_distances(const Launch &L, const Scalars &sc, int xbuf, i
 cudaError_t launch_arc_cumulate(int F, double *s, int *bad, cudaStream_t st)
 {
     const int smem = F <= ARC_CUM_MAX;
-    k_arc_cumulate<<<1, NT, smem ? F * sizeof(double) : 0, st>>>(F, s, nullptr, bad, smem);
+    k_arc_cumulate<<<1, NT, smem ? F * sizeof(double) : 0, st>>>(F, s, bad, smem);
     return cudaGetLastError();
 }
 

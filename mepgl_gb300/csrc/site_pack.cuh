@@ -27,19 +27,17 @@
 // with the u squared.  The energy by itself (site_energy) squares the u, which
 // costs about as much there; in the quartic it would be a tenth of a float-float
 // step (256 x 256 x 64, four steps: 5.8 against 6.6 ms; FP64, two: 7.7 against
-// 8.1).  Spacings
-// are folded into the parameters: the gradient's kinetic and magnetic terms
-// carry no 1/dx (dx^2 / dx^2 = 1).
+// 8.1).  Spacings are folded into the parameters: the gradient's kinetic and
+// magnetic terms carry no 1/dx (dx^2 / dx^2 = 1).
 //
 // Why: GB300 issues two FP64 operations per SM and clock, so the double
 // passes take 16 clocks per warp instruction and are bound by their count
 // alone (95 % of that rate measured); the float-float and FP32 passes are
 // bound by issue.  The forms the reference writes out cost 345 FP64
 // instructions per two-component site in the gradient and 486 in the
-// quartic.  With these forms, on the two-component 256 x 256 string of 64
-// images: an FP64 step 6.43 -> 4.60 ms, FP32 reparametrization and ten steps
-// 2.66 -> 2.42 ms; 1024 x 1024, FP32 passes: 3.46 -> 3.17 ms a step; the FP64
-// gradient and energy of 512 x 512 x 16, with its copies, 4.83 -> 4.00 ms.
+// quartic.  These forms alone, on the two-component 256 x 256 string of 64
+// images, took an FP64 step from 6.43 to 4.60 ms (3.83 with the strips), FP32
+// reparametrization and ten steps from 2.66 to 2.42 (2.27).
 #pragma once
 
 #include "site_ops.cuh"
@@ -259,14 +257,12 @@ struct PackParams {
 
 // Weights of a site whose neighbours all lie inside both domains, as
 // constants (FP64 strips: a row of such sites drops every multiplication by a
-// weight, 26 of 212 instructions of the gradient and 24 of 290 of the quartic).
+// weight, some 26 of the instructions of the gradient and 24 of the quartic).
 // Without per-site arrays the quartic's link sums also leave out the mass, which
-// multiplies them once per strip (16 more; a step of 256 x 256 x 64: 3.90 ->
-// 3.79 ms).
+// multiplies them once per strip (16 more; steps of 256 x 256 x 64 3 % quicker).
 struct Ones {
     static constexpr bool interior = true, masses = false;   // masses: each site's own, so they stay in the links' sums
     static constexpr double area = 1, wfx = 1, wbx = 1, wfy = 1, wby = 1, wsx = 2, wsy = 2;
-    static constexpr double lfx = 1, lbx = 1, lfy = 1, lby = 1;
     static constexpr double vUR = 1, vUL = 1, vLL = 1, vLR = 1, ivs = 0.25;
 };
 

@@ -19,14 +19,12 @@
 // there are strips enough, several: a string's sums are the same in any batch.
 //
 // FP64: bound by the FP64 pipe, 64 clocks per warp instruction and SM
-// quarter, so 8 warps per SM (255 registers, no spills) keep it busy and the
-// strips' equal sharing of the quarters counts.  256 x 256 x 64, two
-// components, per step: 4.48 ms, 4.66 as shared-memory tiles of 256 threads
-// and two launches; 64 x 64 x 16, ten steps with reparametrization: 744 us
-// against 1070.  Float-float: 1.53 ms per step against 1.68.  With what the
-// wider types save on top (the carry from row to row, rows of interior sites
-// without weights, one running sum per coefficient): FP64 3.92 ms, float-float
-// 1.43 ms per step.
+// quarter, so 8 warps per SM (255 registers; the fused launch of two components
+// spills some 80 of its values around a pass) keep it busy and the strips' equal
+// sharing of the quarters counts.  256 x 256 x 64, two components, per step: FP64
+// 3.83 ms, float-float 1.33, against 6.5 and 1.7 as shared-memory tiles of 256
+// threads; 64 x 64 x 16, one component, ten steps with reparametrization in FP64:
+// 0.63 ms against 1.17.
 #pragma once
 
 constexpr int NTS = 32;   // threads per block of the strip kernels
@@ -396,7 +394,7 @@ using GradRing = vec2_t<T>[3][2][2][1 + NC];
 // the gradient of every site, |g|^2 and g . (g - g_prev); the last strip of an
 // image computes beta.  Returns true (in every lane) when this strip finished
 // its image; a consumer in the same launch that has seen the image finished
-// reads the field stores (finish_image_warp).
+// reads the field stores (finish_image).
 template <class T, int NC, bool ONE, bool PS = true>
 __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef tr, const Scalars &sc, const StepFlags &f,
                                           GradRing<T, NC> &ring)
@@ -465,7 +463,7 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         R.m = m;
     };
     // FP64 and float-float rows hand their upper y-link and views on to the next
-    // (21 of 233 FP64 instructions); FP32 forms them again from the row below,
+    // (21 FP64 instructions fewer a site); FP32 forms them again from the row below,
     // because the carry costs 20 registers, i.e. warps (sweep of 16 strings:
     // 15.8 ms against 16.5 with the carry)
     constexpr bool CARRY = !std::is_same<T, float>::value;

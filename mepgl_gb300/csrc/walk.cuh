@@ -31,9 +31,9 @@ __device__ __forceinline__ uint16_t walk_code(const StringDesc &S, const StripLa
     return (uint16_t)((S.code_comp[s] & 0xff) | ((S.code_sc[s] & 0xff) << 8));
 }
 
-// Where a lane is: image (of the string, of the context), site and row of the strip.
+// Where a lane is: image of the string, site and row of the strip.
 struct WalkPos {
-    int n, img, gi, j, s, r;
+    int n, gi, j, s, r;
 };
 
 // Neighbourhood of a site as the gauge-link terms read it.
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(NTS, sizeof(T) == 4 ? 16 : 8) k_walk(const __g
         bool inner = false;
         if constexpr (std::is_same<T, double>::value) inner = !S.disc && __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
-            const WalkPos q{n, S.img_base + n, L.gi, j, L.gi + S.nx * j, r};
+            const WalkPos q{n, L.gi, j, L.gi + S.nx * j, r};
             if (S.per_site) pp.load_site(S, q.gi, q.j, q.s);
             if (inner) {
                 if constexpr (std::is_same<T, double>::value) st.site(op, v, S, pp, Ones(), q);
