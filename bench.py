@@ -327,7 +327,7 @@ def run_ours(args):
     # site-image counted by ncu (profiles/fp64_passes_flops_config2.md) over the
     # event-timed passes; no FP64 peak is measured on this machine, so the
     # denominator is GB300's nominal FP64 rate
-    fp64_flop = {"k_grad_s": 293.7, "k_dir_poly_s": 430.3}
+    fp64_flop = {"k_grad_s": 295.0, "k_dir_poly_s": 437.4}
     nominal_fp64_tflops = 1.25
     fp64["flop_roofline"] = {
         k: {"flop_per_site_image": f, "tflops": f * units_per_step / (ms_ / 1e3) / 1e12,
