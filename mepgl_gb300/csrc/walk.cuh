@@ -11,9 +11,9 @@
 // rows of interior sites skip the weights.
 
 // Sum over a strip of a lane's terms: in float for FP32, over eight rows at most
-// (walk_rows), then in double.  No conversion before the strip's end: three sums of
-// 512 x 768 x 12 sites in FP32 take 85 us with one conversion each, 122 with two and
-// an FP64 addition.
+// (walk_rows), then in double.  No conversion before the strip's end: the three sums
+// of the adjoints of 768 x 512 x 12 sites in FP32 took 85 us with one conversion each,
+// 122 with two and an FP64 addition (three rows in flight).
 template <class T>
 struct RowSum {
     T v;
@@ -288,9 +288,12 @@ struct FluxOp {
 // One strip per single-warp block; strips of the string in (image, row, column)
 // order.  Rows in flight beyond the window: a walk reads a third of what an
 // NLCG pass does per row, so where it is bound by memory (FP32, and the flux)
-// one row per warp keeps too few bytes in flight.
+// one row per warp keeps few bytes in flight; a third costs registers (FP32, two
+// components, 768 x 512 x 12, whole calls at 1, 2, 3 rows: energies 78, 79, 91 us,
+// adjoints 74, 74, 85, gradients 87, 89, 93; 200 x 160 x 24 with holes, gradients:
+// 49, 47, 51).
 #ifndef MEPGL_WALK_AHEAD
-#define MEPGL_WALK_AHEAD 3
+#define MEPGL_WALK_AHEAD 2
 #endif
 template <class T, int NC, class Op>
 __global__ void __launch_bounds__(NTS, sizeof(T) == 4 ? 16 : 8) k_walk(const __grid_constant__ StringDesc S, Scalars sc,
