@@ -177,24 +177,45 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid)
                      : "memory");
 }
 
-// (h + h_neighbour) dx of the four neighbours of site s = (i, j).  PAIRS: of a
-// float-float pass; PS: the string may have per-site parameters.
+// Per-site strings: the fields at the four neighbours of site s = (i, j).  FP32
+// loads them ahead of the site's parameters (PackParams::load_site); the wider types
+// where they are used (held over the divisions they cost FP64 gradients 5 %).
+template <class T>
+struct FieldSites {
+    T u, d, r, l;
+    static constexpr bool ahead = std::is_same<T, float>::value;
+    template <class At>
+    __device__ __forceinline__ void take(const StringDesc &S, int i, int j, int s, const At &at)
+    {
+        u = at(j + 1 < S.ny ? s + S.nx : s);
+        d = at(j > 0 ? s - S.nx : s);
+        r = at(i + 1 < S.nx ? s + 1 : s);
+        l = at(i > 0 ? s - 1 : s);
+    }
+    __device__ __forceinline__ void load(const StringDesc &S, int i, int j, int s)
+    {
+        if constexpr (ahead) take(S, i, j, s, [&](int n) { return static_cast<const T *>(S.ph)[n]; });
+    }
+};
+
+// (h + h_neighbour) dx of the four neighbours of site s = (i, j), near loaded.
+// PAIRS: of a float-float pass; PS: the string may have per-site parameters.
 template <class T, int NC, bool PAIRS = false, bool PS = true>
-__device__ __forceinline__ FieldSums<T> field_sums(const StringDesc &S, const PackParams<T, NC> &pp, int i, int j, int s)
+__device__ __forceinline__ FieldSums<T> field_sums(const StringDesc &S, const PackParams<T, NC> &pp, FieldSites<T> near, int i,
+                                                   int j, int s)
 {
     const T hs = pp.hd + pp.hd;
     FieldSums<T> f{hs, hs, hs, hs};
     if (PS && S.per_site) {
-        auto at = [&](int n) {
+        if constexpr (!FieldSites<T>::ahead) near.take(S, i, j, s, [&](int n) {
             if constexpr (PAIRS && std::is_same<T, ff>::value) return pair_site(S.pairs.h, n);
             else return from_store<T>(static_cast<const store_t<T> *>(S.ph)[n]);
-        };
+        });
         const T dx = S.template u<T>().dx;
-        auto with = [&](int n) { return pp.hd + at(n) * dx; };
-        f.u = with(j + 1 < S.ny ? s + S.nx : s);
-        f.d = with(j > 0 ? s - S.nx : s);
-        f.r = with(i + 1 < S.nx ? s + 1 : s);
-        f.l = with(i > 0 ? s - 1 : s);
+        f.u = pp.hd + near.u * dx;
+        f.d = pp.hd + near.d * dx;
+        f.r = pp.hd + near.r * dx;
+        f.l = pp.hd + near.l * dx;
     }
     return f;
 }

@@ -506,9 +506,13 @@ __device__ __forceinline__ bool grad_tile(const batch_t<ONE> &bt, const StripRef
         bool inner = false;
         if constexpr (std::is_same<T, double>::value) inner = __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
-            if (PS && S.per_site) pp.load_pass_site(S, L.gi, j, s);
+            FieldSites<T> near;
+            if (PS && S.per_site) {
+                near.load(S, L.gi, j, s);
+                pp.load_pass_site(S, L.gi, j, s);
+            }
             const GradView<T, NC> vc = grad_view(R0), vu = grad_view(Rp);
-            const FieldSums<T> h = field_sums<T, NC, true, PS>(S, pp, L.gi, j, s);
+            const FieldSums<T> h = field_sums<T, NC, true, PS>(S, pp, near, L.gi, j, s);
             T g[2 + 2 * NC];
             if (inner) {
                 if constexpr (std::is_same<T, double>::value)

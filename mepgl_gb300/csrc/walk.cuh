@@ -62,7 +62,7 @@ __device__ __forceinline__ SiteParams<T> site_params(const StringDesc &S, int s,
 // ------------------------------------------------------------- operations
 // Free energy per image (computeFreeEnergy).
 struct EnergyOp {
-    static constexpr bool psi = true;
+    static constexpr bool psi = true, field = false;
     double *out;
     template <class T, int NC>
     struct State {
@@ -121,7 +121,7 @@ struct AdjointSums {
 };
 
 struct AdjointOp {
-    static constexpr bool psi = true;
+    static constexpr bool psi = true, field = false;
     double *out;
     template <class T, int NC>
     struct State {
@@ -153,7 +153,7 @@ struct AdjointOp {
 // in FP32 from 0.78 to 0.65 ms.
 template <bool ADJ>
 struct GradientOp {
-    static constexpr bool psi = true;
+    static constexpr bool psi = true, field = true;
     void *p[3];
     int maxwell;
     const double *weights;
@@ -162,6 +162,8 @@ struct GradientOp {
     struct State {
         GradCarry<T, NC> up;
         AdjointSums<T, NC> a;
+        FieldSites<T> near;   // of a per-site string, loaded with the site's parameters
+        __device__ __forceinline__ void ahead(const StringDesc &S, const WalkPos &q) { near.load(S, q.gi, q.j, q.s); }
         __device__ __forceinline__ void store(const GradientOp &op, const StringDesc &S, const T *g, const WalkPos &q) const
         {
             const size_t k = (size_t)q.n * S.nx * S.ny + q.s;
@@ -179,7 +181,7 @@ struct GradientOp {
         __device__ __forceinline__ void site(const GradientOp &op, const PackView<T, NC> &v, const StringDesc &S,
                                              PackParams<T, NC> &pp, const W &w, const WalkPos &q)
         {
-            const FieldSums<T> h = field_sums(S, pp, q.gi, q.j, q.s);
+            const FieldSums<T> h = field_sums(S, pp, near, q.gi, q.j, q.s);
             const GradView<T, NC> c{v.a[1][1], v.a[1][0], v.a[1][2], v.px[1][1], v.py[1][1]};
             const GradView<T, NC> u{v.a[2][1], v.a[2][0], v.a[2][2], v.px[2][1], v.py[2][1]};
             if (q.r == 0) {
@@ -222,7 +224,7 @@ struct GradientOp {
 
 // B (reals) and J (pairs) of every site (computeJB).
 struct JbOp {
-    static constexpr bool psi = true;
+    static constexpr bool psi = true, field = false;
     void *b, *j1, *j2;
     template <class T, int NC>
     struct State {
@@ -256,7 +258,7 @@ struct JbOp {
 // Magnetic flux of every image, Phi = dx^2 sum of B (post.py:131-133): reads A
 // only.  Sums in double.
 struct FluxOp {
-    static constexpr bool psi = false;
+    static constexpr bool psi = false, field = false;
     double *out;      // by image of the string
     template <class T, int NC>
     struct State {
@@ -399,7 +401,10 @@ __global__ void __launch_bounds__(NTS, sizeof(T) == 4 ? 16 : 8) k_walk(const __g
         if constexpr (std::is_same<T, double>::value) inner = !S.disc && __all_sync(FULL_MASK, !L.cok || R0.m == 0xffffu);
         if (L.cok) {
             const WalkPos q{n, L.gi, j, L.gi + S.nx * j, r};
-            if (S.per_site) pp.load_site(S, q.gi, q.j, q.s);
+            if (S.per_site) {
+                if constexpr (Op::field) st.ahead(S, q);
+                pp.load_site(S, q.gi, q.j, q.s);
+            }
             if (inner) {
                 if constexpr (std::is_same<T, double>::value) st.site(op, v, S, pp, Ones(), q);
             } else {
