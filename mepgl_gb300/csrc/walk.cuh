@@ -297,9 +297,17 @@ struct FluxOp {
 #ifndef MEPGL_WALK_AHEAD
 #define MEPGL_WALK_AHEAD 2
 #endif
+// Blocks per SM: FP32 is bound by the latency of its loads.  One component fits 20
+// warps' registers (gradients at 16 / 20 / 24 blocks: 180 x 150 x 24 with per-site
+// parameters 31 / 25 / 29 us, uniform 24 / 22 / 25; 512 x 512 x 32 165 / 148 / 182
+// and 113 / 109 / 145), two lose beyond 16 (512 x 512 x 32 at 16 / 20: 145 / 175).
+template <class T, int NC>
+struct WalkBlocks {
+    static constexpr int v = sizeof(T) == 4 ? (NC == 1 ? 20 : 16) : 8;
+};
 template <class T, int NC, class Op>
-__global__ void __launch_bounds__(NTS, sizeof(T) == 4 ? 16 : 8) k_walk(const __grid_constant__ StringDesc S, Scalars sc,
-                                                                       int xbuf, Op op)
+__global__ void __launch_bounds__(NTS, WalkBlocks<T, NC>::v) k_walk(const __grid_constant__ StringDesc S, Scalars sc,
+                                                                    int xbuf, Op op)
 {
     using St = store_t<T>;
     using V = vec2_t<T>;
